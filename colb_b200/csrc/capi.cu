@@ -11,6 +11,7 @@ static std::string g_err;
 std::string& abd_global_error() { return g_err; }
 
 int eng_energy_masked(Engine* E, int slot, const int* skip);
+int eng_energy_candidates(Engine* E, int slot, const int* skip);
 Geo eng_geo(Engine* E);
 
 template <class T>
@@ -511,7 +512,16 @@ int abd_energy(AbdHandle* h, double* e) {
     if (!e) return E->fail(ABD_ERR_INVALID_ARG, "abd_energy: null");
     int* skip = E->sci + SI_NACT * E->ns;
     CUDA_TRY(cudaMemsetAsync(skip, 0, sizeof(int) * E->ns, E->stream));
-    int rc = eng_energy_masked(E, SD_E0, skip);
+    // Every active pair is a candidate (dhat <= cand_dist), so where the
+    // body-pair broad phase applies the energy is summed over its list: the
+    // grid query walks buckets that mostly hold the same body's primitives
+    // (4096-sphere pile: edge query 5.8 ms and point query 1.0 ms against
+    // about 0.3 ms for the detection and the list; energy + gradient +
+    // increment of its Newton system 8.70 -> 1.76 ms).  Bodies without contiguous ranges, and
+    // a list that does not fit, keep the grid query.
+    int rc = eng_use_bp(E) ? detect_full(E) : ABD_ERR_CONTACT_OVERFLOW;
+    if (rc == ABD_OK) rc = eng_energy_candidates(E, SD_E0, skip);
+    else if (rc == ABD_ERR_CONTACT_OVERFLOW) { E->err.clear(); rc = eng_energy_masked(E, SD_E0, skip); }
     if (rc) return rc;
     CUDA_TRY(cudaMemcpyAsync(e, E->scd + SD_E0 * E->ns, sizeof(double) * E->ns, cudaMemcpyDeviceToHost, E->stream));
     CUDA_TRY(cudaStreamSynchronize(E->stream));

@@ -352,7 +352,7 @@ __global__ void k_list_energy(int n, const int* __restrict__ n_dev, const int4* 
             }
         }
         warp_reduce_add(Eo, s, e, valid);
-        warp_reduce_add(En, s, en, valid);
+        if (En) warp_reduce_add(En, s, en, valid);
     }
 }
 
@@ -384,6 +384,26 @@ int eng_energy_list(Engine* E, const LsUnits& U, int slot, const int* skip, bool
         E->launches++;
     }
     return eng_pg_energy(E, U.bunit, Eo, En, skip);
+}
+
+// energy per scene into scd[slot] over the candidate list of a detection that
+// has just run at the current positions (hcnt holds its counts)
+int eng_energy_candidates(Engine* E, int slot, const int* skip) {
+    cudaStream_t s = E->stream;
+    const AbdParams& P = E->P;
+    double* Eo = E->scd + slot * E->ns;
+    CUDA_TRY(cudaMemsetAsync(Eo, 0, sizeof(double) * E->ns, s));
+    int rc = eng_body_energy(E, E->bscene, Eo, nullptr, skip);
+    if (rc) return rc;
+    const int n = E->hcnt->n_ee + E->hcnt->n_pt;
+    if (n > 0) {
+        int ph = phase_begin(E, PH_ELIST);
+        k_list_energy<<<grid_for(n, 128), 128, 0, s>>>(n, nullptr, E->contacts, eng_geo(E), E->bscene, skip, P.ee_f32, P.dhat,
+                                                      P.barrier, P.kappa * P.dt * P.dt, Eo, nullptr);
+        phase_end(E, ph, n * (16.0 + 16.0 + 4 * 24.0));
+        E->launches++;
+    }
+    return eng_pg_energy(E, E->bscene, Eo, nullptr, skip);
 }
 
 // ------------------------------------------------------------------ detection from the list

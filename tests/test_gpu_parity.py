@@ -255,3 +255,27 @@ def test_net_trajectory_matches_oracle():
         assert np.abs(xe - xo).max() <= 1e-6 * np.abs(xo).max()
     assert se.n_active > 0
     assert e.count_intersections() == 0
+
+
+@pytest.mark.parametrize("which", ["chain", "net", "cubes", "pile"])
+def test_energy_over_candidates_equals_grid_query(which, chain_scene, chain_pairs):
+    """abd_energy sums over the body-pair candidate list (broadphase 2) or
+    queries the hashed grid (broadphase 1): the same active set, so equal up to
+    the order of an FP64 sum."""
+    p = dict(chain=P.reference_params, net=P.config_params, cubes=P.config_params, pile=P.config_params)[which]
+    if which == "chain":
+        sc = dict(chain_scene, state=chain_pairs["states"][2])
+    elif which == "net":
+        sc = S.config2_chain_net(n=4, seed=1, pitch=1.5 - 5e-4)
+    elif which == "cubes":
+        sc = S.config1_cubes(seed=3)
+        st = sc["state"].copy()
+        st[:, [1, 25]] -= S.transform(sc)[:, 1].min() - 5e-4
+        sc = dict(sc, state=st)
+    else:
+        sc = S.config5_pile(n=27, seed=2)
+        st = sc["state"].copy()
+        st[:, [1, 25]] -= S.transform(sc)[:, 1].min() - 5e-4
+        sc = dict(sc, state=st)
+    e = [Engine(p(broadphase=b), sc).energy()[0] for b in (1, 2)]
+    assert e[0] != 0.0 and e[1] == pytest.approx(e[0], rel=1e-11)

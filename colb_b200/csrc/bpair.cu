@@ -1,33 +1,47 @@
-// bpair.cu — two-level broad phase: bodies first, then primitives of each
-// overlapping body pair staged in shared memory.
+// bpair.cu — three-level broad phase: bodies, then clusters of primitives of
+// each overlapping body pair, then the primitives of each overlapping
+// cluster pair.
 //
 // Affine bodies are rigid-ish meshes whose primitives are mostly surrounded
 // by primitives of the same body, which never pair with them when
 // self-contact is off.  A uniform grid over primitives therefore spends its
 // time rejecting same-body neighbours.  Here:
-//   1. one warp per body reduces the body's swept, padded box;
+//   1. one block per body forms the step's displacement and the swept,
+//      padded box of every vertex and of the body;
 //   2. one warp per body A tests A against every later body B of its scene
 //      (and A against itself when self-contact is on) and appends the
 //      overlapping pairs;
-//   3. one CTA per body pair stages the primitives of A and of B whose boxes
-//      touch the two bodies' box overlap into shared memory (block
-//      compaction), tests all staged pairs, and appends hits;
-//   4. hits are sorted by a 64-bit (kind, a, b) key, so the list comes out
+//   3. one block per body that has a pair forms the boxes of its clusters of
+//      32 consecutive vertices, edges and triangles (neighbours in a mesh's
+//      numbering are mostly neighbours in space), and one warp per body pair
+//      and kind appends the overlapping cluster pairs;
+//   4. one warp per cluster pair tests its (at most 32 x 32) primitive boxes
+//      and runs the exact test on the overlapping ones, 32 at a time from a
+//      queue, and appends hits;
+//   5. hits are sorted by a 64-bit (kind, a, b) key, so the list comes out
 //      in the same canonical order as the grid-based detection.
-// Step 3 runs the reference's pair predicate (contact.py:158-168) in
+// Step 4 runs the reference's pair predicate (contact.py:158-168) in
 // `detect` mode, or the Lipschitz reachability test along a step (see
 // swept.cu) in `swept` mode.  Bodies must own contiguous vertex, edge and
 // triangle ranges (as geometry.py:31-73 lays them out).
+//
+// What bounds it is the latency of dependent loads and the warp count, not
+// bytes (7 MB of positions for a 16 x 16 net of 288-vertex links).  Staging
+// all primitives of both bodies of a pair in one block, as an earlier form
+// of step 4 did, forms every primitive box once per body pair (14 times more
+// boxes than step 3 on that net) and leaves most of the block idle in the
+// narrow tests; the figures are at bp_build.
 #include "contact.cuh"
 #include <cub/cub.cuh>
+#include <climits>
+#include <cstring>
 
 Geo eng_geo(Engine* E);
 int eng_grow_swept(Engine* E, int need);
 int eng_grow_contacts(Engine* E, int need);
 int eng_pg_candidates(Engine* E, double filt);
 
-#define BP_CHUNK 1024
-#define BP_THREADS 256
+#define BP_CL 32            // primitives of a cluster: one per lane
 
 DV float4 fmin4(float4 a, float4 b) { return make_float4(fminf(a.x, b.x), fminf(a.y, b.y), fminf(a.z, b.z), 0.f); }
 DV float4 fmax4(float4 a, float4 b) { return make_float4(fmaxf(a.x, b.x), fmaxf(a.y, b.y), fmaxf(a.z, b.z), 0.f); }
@@ -36,27 +50,24 @@ DV bool overlap(float4 al, float4 ah, float4 bl, float4 bh) {
 }
 
 // swept (x .. x+p) padded box of one vertex, outward rounded
-DV void vbox(const double* x, const double* p, int v, float pad, float4& lo, float4& hi) {
-    double a0 = x[3*v], a1 = x[3*v+1], a2 = x[3*v+2];
-    double b0 = a0, b1 = a1, b2 = a2;
-    if (p) { b0 += p[3*v]; b1 += p[3*v+1]; b2 += p[3*v+2]; }
+DV void vbox(const double* x, const double* p, float pad, float4& lo, float4& hi) {
+    double a0 = x[0], a1 = x[1], a2 = x[2];
+    double b0 = a0 + p[0], b1 = a1 + p[1], b2 = a2 + p[2];
     lo = make_float4(__fsub_rd(__double2float_rd(fmin(a0, b0)), pad), __fsub_rd(__double2float_rd(fmin(a1, b1)), pad),
                      __fsub_rd(__double2float_rd(fmin(a2, b2)), pad), 0.f);
     hi = make_float4(__fadd_ru(__double2float_ru(fmax(a0, b0)), pad), __fadd_ru(__double2float_ru(fmax(a1, b1)), pad),
                      __fadd_ru(__double2float_ru(fmax(a2, b2)), pad), 0.f);
 }
 
-// 1. body boxes: one warp per body over its vertices; with vlo/vhi given,
-// every vertex's box is kept too (the primitive boxes of the pair tests are
-// the min/max over their vertices' boxes, exact in float)
+// body boxes alone, one warp per body (contact groups of a step that was
+// listed by the grid)
 __global__ void k_body_boxes(int nb, const int* __restrict__ vbeg, const double* __restrict__ x, const double* __restrict__ p,
-                             float pad, float4* blo, float4* bhi, float4* vlo = nullptr, float4* vhi = nullptr) {
+                             float pad, float4* blo, float4* bhi) {
     int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     for (int b = warp; b < nb; b += (gridDim.x * blockDim.x) >> 5) {
         float4 lo = make_float4(3e38f, 3e38f, 3e38f, 0.f), hi = make_float4(-3e38f, -3e38f, -3e38f, 0.f);
         for (int v = vbeg[b] + lane; v < vbeg[b+1]; v += 32) {
-            float4 l, h; vbox(x, p, v, pad, l, h);
-            if (vlo) { vlo[v] = l; vhi[v] = h; }
+            float4 l, h; vbox(x + 3L * v, p + 3L * v, pad, l, h);
             lo = fmin4(lo, l); hi = fmax4(hi, h);
         }
         for (int o = 16; o > 0; o >>= 1) {
@@ -71,7 +82,7 @@ __global__ void k_body_boxes(int nb, const int* __restrict__ vbeg, const double*
 // 2. body pairs (a <= b, same scene); a == b only with self-contact
 __global__ void k_body_pairs(int nb, const int* __restrict__ bscene, const int* __restrict__ sc_body_begin,
                              const float4* __restrict__ blo, const float4* __restrict__ bhi, int self_contact,
-                             int2* out, int cap, int* count) {
+                             int2* out, int cap, int* count, int* paired) {
     int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     for (int a = warp; a < nb; a += (gridDim.x * blockDim.x) >> 5) {
         int s = bscene[a];
@@ -81,35 +92,16 @@ __global__ void k_body_pairs(int nb, const int* __restrict__ bscene, const int* 
             if (!overlap(al, ah, blo[b], bhi[b])) continue;
             int at = atomicAdd(count, 1);
             if ((unsigned)at < (unsigned)cap) out[at] = make_int2(a, b);
+            paired[a] = 1; paired[b] = 1;
         }
     }
-}
-
-// block-wide compaction of an index range into shared memory
-template <class BoxFn>
-DV int stage(int begin, int end, float4 rlo, float4 rhi, BoxFn box, int* idx, float4* lo, float4* hi, int* scount) {
-    if (threadIdx.x == 0) *scount = 0;
-    __syncthreads();
-    for (int i = begin + threadIdx.x; i < end; i += blockDim.x) {
-        float4 l, h; box(i, l, h);
-        if (overlap(l, h, rlo, rhi)) {
-            int at = atomicAdd(scount, 1);
-            if (at < BP_CHUNK) { idx[at] = i; lo[at] = l; hi[at] = h; }
-        }
-    }
-    __syncthreads();
-    int n = min(*scount, BP_CHUNK);
-    __syncthreads();     // everyone has read the count before it can be reset
-    return n;
 }
 
 struct BpArgs {
-    Geo G; const double* p; const float* pmag;
+    Geo G; const float* pmag;
     const float4* vlo; const float4* vhi;          // per-vertex swept boxes of this build
-    const int* ebeg; const int* tbeg; const int* vbeg;
-    const float4* blo; const float4* bhi;
-    float pad; double lim; double filt; int mode;   // mode 0 swept (Lipschitz, lim), 1 detect (predicate, filt)
-    int f32; int self_contact; int do_ee; int do_pt;
+    double lim; double filt; int mode;              // mode 0 swept (Lipschitz, lim), 1 detect (predicate, filt)
+    int f32;
     unsigned long long* out; int cap; int* count;
 };
 
@@ -142,80 +134,291 @@ DV void bp_emit(const BpArgs& A, int kind, int a, int b) {
     if ((unsigned)at < (unsigned)A.cap) A.out[at] = ((unsigned long long)kind << 62) | ((unsigned long long)a << 31) | (unsigned long long)b;
 }
 
-// 3. one CTA per body pair
-__global__ void __launch_bounds__(BP_THREADS) k_bp_prims(const int2* __restrict__ bpairs, const int* __restrict__ npairs,
-                                                        int bp_cap, BpArgs A) {
-    extern __shared__ float4 smem[];
-    float4* alo = smem;                  float4* ahi = alo + BP_CHUNK;
-    float4* blo = ahi + BP_CHUNK;        float4* bhi = blo + BP_CHUNK;
-    int* aidx = reinterpret_cast<int*>(bhi + BP_CHUNK);
-    int* bidx = aidx + BP_CHUNK;
-    __shared__ int sa, sb;
+// ---- step 1: displacements and boxes
+// Clusters of body b start at beg[b] / 32 + b: with at most ceil(n / 32) of
+// them per body the ranges of successive bodies never overlap, so no table
+// is needed.
+DV int cl_first(const int* beg, int b) { return (beg[b] >> 5) + b; }
+DV int cl_count(const int* beg, int b) { return (beg[b + 1] - beg[b] + BP_CL - 1) >> 5; }
+// float <-> int with the same order, for the integer warp reductions
+DV int f_ord(float f) { int i = __float_as_int(f); return i ^ ((i >> 31) & 0x7fffffff); }
+DV float f_unord(int i) { return __int_as_float(i ^ ((i >> 31) & 0x7fffffff)); }
+// union of the lanes' boxes in every lane (a lane without one passes an
+// empty box); NaN bounds are ignored, as fminf / fmaxf do
+DV void warp_union(float4& lo, float4& hi) {
+    const unsigned full = 0xffffffffu;
+    lo.x = f_unord(__reduce_min_sync(full, f_ord(fminf(lo.x, 3e38f)))); lo.y = f_unord(__reduce_min_sync(full, f_ord(fminf(lo.y, 3e38f))));
+    lo.z = f_unord(__reduce_min_sync(full, f_ord(fminf(lo.z, 3e38f)))); hi.x = f_unord(__reduce_max_sync(full, f_ord(fmaxf(hi.x, -3e38f))));
+    hi.y = f_unord(__reduce_max_sync(full, f_ord(fmaxf(hi.y, -3e38f)))); hi.z = f_unord(__reduce_max_sync(full, f_ord(fmaxf(hi.z, -3e38f))));
+}
+DV void empty_box(float4& lo, float4& hi) { lo = make_float4(3e38f, 3e38f, 3e38f, 0.f); hi = make_float4(-3e38f, -3e38f, -3e38f, 0.f); }
+
+struct BpBoxes {
+    float4 *vlo, *vhi, *blo, *bhi, *cl[3], *ch[3];   // clusters of vertices, edges, triangles
+    int* still;                                      // the body did not move in the swept build that wrote its boxes
+    int* paired;                                     // the body is in a body pair of this build
+    int* clok;                                       // its cluster boxes belong to its present vertex boxes
+};
+struct BpDisp {                                                      // dq null: static positions
+    const double* dq; double sign; const double* xbar; const double* mass; const int* bscene; const int* done;
+    double* pv; float* pmag;
+};
+constexpr int BOX_THREADS = 128;
+__global__ void __launch_bounds__(BOX_THREADS) k_bp_boxes(int nb, const int* __restrict__ vbeg, const double* __restrict__ x,
+        BpDisp D, float pad, int keep, BpBoxes B) {
+    __shared__ float4 slo[BOX_THREADS / 32], shi[BOX_THREADS / 32];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int b = blockIdx.x; b < nb; b += gridDim.x) {
+        double d[12];
+        bool dyn = false;
+        if (threadIdx.x == 0) B.paired[b] = 0;
+        if (D.dq) {
+            dyn = D.mass[b] > 0.0 && !D.done[D.bscene[b]];
+            // pinned, or its scene has converged: the boxes of the last
+            // build, in which it did not move either, are still its boxes
+            if (!dyn && keep && B.still[b]) continue;
+            if (dyn) {
+#pragma unroll
+                for (int k = 0; k < 12; k++) d[k] = D.dq[12L * b + k];
+            }
+        }
+        float4 rlo, rhi;
+        empty_box(rlo, rhi);
+        for (int v = vbeg[b] + threadIdx.x, v1 = vbeg[b + 1]; v < v1; v += BOX_THREADS) {
+            double q[3] = {0.0, 0.0, 0.0};
+            if (D.dq) {
+                if (dyn) {
+                    const double x0 = D.xbar[3*v], x1 = D.xbar[3*v+1], x2 = D.xbar[3*v+2];
+#pragma unroll
+                    for (int k = 0; k < 3; k++) q[k] = D.sign * (d[k] + x0 * d[3+k] + x1 * d[6+k] + x2 * d[9+k]);
+                }
+                D.pv[3*v] = q[0]; D.pv[3*v+1] = q[1]; D.pv[3*v+2] = q[2];
+                D.pmag[v] = __double2float_ru(sqrt(q[0] * q[0] + q[1] * q[1] + q[2] * q[2]));
+            }
+            float4 l, h;
+            vbox(x + 3L * v, q, pad, l, h);
+            B.vlo[v] = l; B.vhi[v] = h;
+            rlo = fmin4(rlo, l); rhi = fmax4(rhi, h);
+        }
+        warp_union(rlo, rhi);
+        if (lane == 0) { slo[warp] = rlo; shi[warp] = rhi; }
+        __syncthreads();           // everyone has read the body's flag
+        if (threadIdx.x == 0) {
+            for (int w = 1; w < BOX_THREADS / 32; w++) { rlo = fmin4(rlo, slo[w]); rhi = fmax4(rhi, shi[w]); }
+            B.blo[b] = rlo; B.bhi[b] = rhi;
+            B.still[b] = !dyn;
+            B.clok[b] = 0;
+        }
+        __syncthreads();           // slo / shi are read before the next body writes them
+    }
+}
+
+// ---- step 3: cluster boxes of the bodies that have a pair
+__global__ void __launch_bounds__(BOX_THREADS) k_bp_clboxes(int nb, const int* __restrict__ vbeg, const int* __restrict__ ebeg,
+        const int* __restrict__ tbeg, const int2* __restrict__ edges, const int* __restrict__ tris, int do_ee, int do_pt,
+        BpBoxes B) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const float4* __restrict__ vlo = B.vlo;
+    const float4* __restrict__ vhi = B.vhi;
+    for (int b = blockIdx.x; b < nb; b += gridDim.x) {
+        const bool todo = B.paired[b] && !B.clok[b];
+        __syncthreads();           // read by all before thread 0 sets the flag
+        if (!todo) continue;
+        const int v0 = vbeg[b], v1 = vbeg[b + 1], vc = cl_first(vbeg, b);
+        const int e0 = ebeg[b], e1 = ebeg[b + 1], ec = cl_first(ebeg, b);
+        const int t0 = tbeg[b], t1 = tbeg[b + 1], tc = cl_first(tbeg, b);
+        const int nv = do_pt ? cl_count(vbeg, b) : 0, ne = do_ee ? cl_count(ebeg, b) : 0, nt = do_pt ? cl_count(tbeg, b) : 0;
+        for (int j = warp; j < nv + ne + nt; j += BOX_THREADS / 32) {
+            float4 l, h;
+            empty_box(l, h);
+            if (j < ne) {
+                const int e = e0 + j * BP_CL + lane;
+                if (e < e1) {
+                    const int2 ed = edges[e];
+                    l = fmin4(vlo[ed.x], vlo[ed.y]); h = fmax4(vhi[ed.x], vhi[ed.y]);
+                }
+                warp_union(l, h);
+                if (lane == 0) { B.cl[1][ec + j] = l; B.ch[1][ec + j] = h; }
+            } else if (j < ne + nt) {
+                const int t = t0 + (j - ne) * BP_CL + lane;
+                if (t < t1) {
+                    const int a0 = tris[3*t], a1 = tris[3*t+1], a2 = tris[3*t+2];
+                    l = fmin4(vlo[a0], fmin4(vlo[a1], vlo[a2])); h = fmax4(vhi[a0], fmax4(vhi[a1], vhi[a2]));
+                }
+                warp_union(l, h);
+                if (lane == 0) { B.cl[2][tc + j - ne] = l; B.ch[2][tc + j - ne] = h; }
+            } else {
+                const int v = v0 + (j - ne - nt) * BP_CL + lane;
+                if (v < v1) { l = vlo[v]; h = vhi[v]; }
+                warp_union(l, h);
+                if (lane == 0) { B.cl[0][vc + j - ne - nt] = l; B.ch[0][vc + j - ne - nt] = h; }
+            }
+        }
+        if (threadIdx.x == 0) B.clok[b] = 1;
+    }
+}
+
+// ---- step 3: overlapping cluster pairs of each body pair, as primitive
+// ranges {first of a, first of b, counts | kind | same body}.  The counter
+// is 64-bit and exact: the host grows the list once and runs the kernel
+// again.  `q0`, `q1`: the slice of body pairs to expand.
+DV int4 cl_item(int a0, int na, int b0, int nb, int kind, int same) {
+    return make_int4(a0, b0, min(na, BP_CL) | (min(nb, BP_CL) << 8) | (kind << 16) | (same << 17), 0);
+}
+__global__ void k_bp_clusters(const int2* __restrict__ bpairs, const int* __restrict__ npairs, int bp_cap, int q0, int q1,
+                              const int* __restrict__ vbeg, const int* __restrict__ ebeg, const int* __restrict__ tbeg,
+                              BpBoxes B, int do_ee, int do_pt, int4* out, long long cap, unsigned long long* count) {
+    const int lane = threadIdx.x & 31;
+    const int n = min(min(*npairs, bp_cap), q1);     // an overflowing pair list is rebuilt larger by the host
+    // pass 0: edges of a x edges of b; 1: vertices of a x triangles of b; 2: the reverse.
+    // One warp per pair and pass: three times the warps, a third of the dependent loads each.
+    const int first = do_ee ? 0 : 1, np = (do_pt ? 3 : 1) - first;
+    if (np <= 0) return;
+    for (long long w = (long long)q0 * np + ((blockIdx.x * blockDim.x + threadIdx.x) >> 5); w < (long long)n * np;
+         w += (gridDim.x * blockDim.x) >> 5) {
+        const int2 bp = bpairs[w / np];
+        const int same = bp.x == bp.y;
+        const float4 rlo = fmax4(B.blo[bp.x], B.blo[bp.y]), rhi = fmin4(B.bhi[bp.x], B.bhi[bp.y]);
+        {
+            const int pass = first + (int)(w % np);
+            if (same && pass == 2) continue;
+            const int kind = pass == 0 ? ABD_CONTACT_EE : ABD_CONTACT_PT;
+            const int ba = pass == 2 ? bp.y : bp.x, bb = pass == 2 ? bp.x : bp.y;
+            const int* abeg = pass == 0 ? ebeg : vbeg;
+            const int* bbeg = pass == 0 ? ebeg : tbeg;
+            const float4* AL = pass == 0 ? B.cl[1] : B.cl[0];
+            const float4* AH = pass == 0 ? B.ch[1] : B.ch[0];
+            const float4* BL = pass == 0 ? B.cl[1] : B.cl[2];
+            const float4* BH = pass == 0 ? B.ch[1] : B.ch[2];
+            const int na = cl_count(abeg, ba), nb = cl_count(bbeg, bb);
+            const int ca = cl_first(abeg, ba), cb = cl_first(bbeg, bb);
+            for (int a0 = 0; a0 < na; a0 += 32) {
+                float4 al, ah;
+                empty_box(al, ah);
+                if (a0 + lane < na) { al = AL[ca + a0 + lane]; ah = AH[ca + a0 + lane]; }
+                const unsigned am = __ballot_sync(0xffffffffu, a0 + lane < na && overlap(al, ah, rlo, rhi));
+                if (!am) continue;
+                for (int b0 = 0; b0 < nb; b0 += 32) {
+                    float4 bl, bh;
+                    empty_box(bl, bh);
+                    bool bin = b0 + lane < nb;
+                    if (bin) { bl = BL[cb + b0 + lane]; bh = BH[cb + b0 + lane]; }
+                    bin = bin && overlap(bl, bh, rlo, rhi);
+                    if (!__any_sync(0xffffffffu, bin)) continue;
+                    for (unsigned m = am; m; m &= m - 1) {
+                        const int i = __ffs(m) - 1;
+                        const float4 l = make_float4(__shfl_sync(0xffffffffu, al.x, i), __shfl_sync(0xffffffffu, al.y, i), __shfl_sync(0xffffffffu, al.z, i), 0.f);
+                        const float4 h = make_float4(__shfl_sync(0xffffffffu, ah.x, i), __shfl_sync(0xffffffffu, ah.y, i), __shfl_sync(0xffffffffu, ah.z, i), 0.f);
+                        const bool hit = bin && overlap(l, h, bl, bh) && !(same && pass == 0 && b0 + lane < a0 + i);
+                        const unsigned hm = __ballot_sync(0xffffffffu, hit);
+                        if (!hm) continue;
+                        unsigned long long at = 0;
+                        if (lane == 0) at = atomicAdd(count, (unsigned long long)__popc(hm));
+                        at = __shfl_sync(0xffffffffu, at, 0) + __popc(hm & ((1u << lane) - 1));
+                        if (hit && at < (unsigned long long)cap) {
+                            const int pa = abeg[ba] + (a0 + i) * BP_CL, pb = bbeg[bb] + (b0 + lane) * BP_CL;
+                            out[at] = cl_item(pa, abeg[ba + 1] - pa, pb, bbeg[bb + 1] - pb, kind, same);
+                        }
+                    }
+                }
+            }
+        }
+    }
+}
+
+// ---- step 4: one warp per cluster pair
+constexpr int PRIM_THREADS = 128;
+__global__ void __launch_bounds__(PRIM_THREADS) k_bp_prims(const int4* __restrict__ items,
+                                                           const unsigned long long* __restrict__ nitems, long long cap, BpArgs A) {
+    __shared__ int2 queue[PRIM_THREADS / 32][64];
+    const int lane = threadIdx.x & 31;
+    int2* Q = queue[threadIdx.x >> 5];
     const Geo& G = A.G;
-    const float pad = A.pad;
-    int n = min(*npairs, bp_cap);      // an overflowing pair list is rebuilt larger by the host
-    for (int q = blockIdx.x; q < n; q += gridDim.x) {
-        int2 bp = bpairs[q];
-        int ba = bp.x, bb = bp.y;
-        float4 rlo = fmax4(A.blo[ba], A.blo[bb]), rhi = fmin4(A.bhi[ba], A.bhi[bb]);
-        const float4* __restrict__ vlo = A.vlo;
-        const float4* __restrict__ vhi = A.vhi;
-        auto ebox = [&](int e, float4& l, float4& h) {
-            int2 ed = G.edges[e];
-            l = fmin4(__ldg(vlo + ed.x), __ldg(vlo + ed.y)); h = fmax4(__ldg(vhi + ed.x), __ldg(vhi + ed.y));
-        };
-        auto tbox = [&](int t, float4& l, float4& h) {
-            const int v0 = G.tris[3*t], v1 = G.tris[3*t+1], v2 = G.tris[3*t+2];
-            l = fmin4(__ldg(vlo + v0), fmin4(__ldg(vlo + v1), __ldg(vlo + v2)));
-            h = fmax4(__ldg(vhi + v0), fmax4(__ldg(vhi + v1), __ldg(vhi + v2)));
-        };
-        auto pbox = [&](int v, float4& l, float4& h) { l = __ldg(vlo + v); h = __ldg(vhi + v); };
-        // ---- edge-edge
-        if (A.do_ee) {
-            for (int a0 = A.ebeg[ba]; a0 < A.ebeg[ba+1]; a0 += BP_CHUNK) {
-                int na = stage(a0, min(a0 + BP_CHUNK, A.ebeg[ba+1]), rlo, rhi, ebox, aidx, alo, ahi, &sa);
-                if (na == 0) continue;
-                for (int b0 = A.ebeg[bb]; b0 < A.ebeg[bb+1]; b0 += BP_CHUNK) {
-                    int nbb = stage(b0, min(b0 + BP_CHUNK, A.ebeg[bb+1]), rlo, rhi, ebox, bidx, blo, bhi, &sb);
-                    // a staged box per warp row (in registers), the other side across the lanes
-                    for (int ia = threadIdx.x >> 5; ia < na; ia += blockDim.x >> 5) {
-                        const float4 al = alo[ia], ah = ahi[ia];
-                        const int i = aidx[ia];
-                        for (int ib = threadIdx.x & 31; ib < nbb; ib += 32) {
-                            const int j = bidx[ib];
-                            if (ba == bb && i >= j) continue;
-                            if (!overlap(al, ah, blo[ib], bhi[ib])) continue;
-                            int lo_ = min(i, j), hi_ = max(i, j);
-                            if (bp_ee_ok(A, lo_, hi_)) bp_emit(A, ABD_CONTACT_EE, lo_, hi_);
-                        }
-                    }
-                    __syncthreads();
-                }
+    int qn = 0;                                   // queued box overlaps of this warp
+    auto test = [&](int at) {
+        const int2 e = Q[at];
+        const int a = e.x & 0x7fffffff, b = e.y;
+        if (e.x >= 0) { if (bp_ee_ok(A, min(a, b), max(a, b))) bp_emit(A, ABD_CONTACT_EE, min(a, b), max(a, b)); }
+        else if (bp_pt_ok(A, a, b)) bp_emit(A, ABD_CONTACT_PT, a, b);
+    };
+    const long long n = min((long long)*nitems, cap);
+    for (long long w = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5; w < n; w += ((long long)gridDim.x * blockDim.x) >> 5) {
+        const int4 it = items[w];
+        const int na = it.z & 0xff, nb = (it.z >> 8) & 0xff, pt = (it.z >> 16) & 1, same = (it.z >> 17) & 1;
+        float4 al, ah, bl, bh;
+        empty_box(al, ah);
+        empty_box(bl, bh);
+        if (lane < na) {
+            if (pt) { al = A.vlo[it.x + lane]; ah = A.vhi[it.x + lane]; }
+            else {
+                const int2 ed = G.edges[it.x + lane];
+                al = fmin4(__ldg(A.vlo + ed.x), __ldg(A.vlo + ed.y)); ah = fmax4(__ldg(A.vhi + ed.x), __ldg(A.vhi + ed.y));
             }
         }
-        // ---- point-triangle, both directions
-        if (A.do_pt) {
-            for (int dir = 0; dir < (ba == bb ? 1 : 2); dir++) {
-                int pb = dir == 0 ? ba : bb, tb = dir == 0 ? bb : ba;
-                for (int p0 = A.vbeg[pb]; p0 < A.vbeg[pb+1]; p0 += BP_CHUNK) {
-                    int na = stage(p0, min(p0 + BP_CHUNK, A.vbeg[pb+1]), rlo, rhi, pbox, aidx, alo, ahi, &sa);
-                    if (na == 0) continue;
-                    for (int t0 = A.tbeg[tb]; t0 < A.tbeg[tb+1]; t0 += BP_CHUNK) {
-                        int nt = stage(t0, min(t0 + BP_CHUNK, A.tbeg[tb+1]), rlo, rhi, tbox, bidx, blo, bhi, &sb);
-                        for (int ia = threadIdx.x >> 5; ia < na; ia += blockDim.x >> 5) {
-                            const float4 al = alo[ia], ah = ahi[ia];
-                            const int pv = aidx[ia];
-                            for (int ib = threadIdx.x & 31; ib < nt; ib += 32) {
-                                if (!overlap(al, ah, blo[ib], bhi[ib])) continue;
-                                const int tr = bidx[ib];
-                                if (bp_pt_ok(A, pv, tr)) bp_emit(A, ABD_CONTACT_PT, pv, tr);
-                            }
-                        }
-                        __syncthreads();
-                    }
-                }
+        if (lane < nb) {
+            if (pt) {
+                const int* t = G.tris + 3L * (it.y + lane);
+                const int v0 = t[0], v1 = t[1], v2 = t[2];
+                bl = fmin4(__ldg(A.vlo + v0), fmin4(__ldg(A.vlo + v1), __ldg(A.vlo + v2)));
+                bh = fmax4(__ldg(A.vhi + v0), fmax4(__ldg(A.vhi + v1), __ldg(A.vhi + v2)));
+            } else {
+                const int2 ed = G.edges[it.y + lane];
+                bl = fmin4(__ldg(A.vlo + ed.x), __ldg(A.vlo + ed.y)); bh = fmax4(__ldg(A.vhi + ed.x), __ldg(A.vhi + ed.y));
             }
         }
+        float4 ul = bl, uh = bh;
+        warp_union(ul, uh);
+        for (unsigned m = __ballot_sync(0xffffffffu, lane < na && overlap(al, ah, ul, uh)); m; m &= m - 1) {
+            const int i = __ffs(m) - 1;
+            const float4 l = make_float4(__shfl_sync(0xffffffffu, al.x, i), __shfl_sync(0xffffffffu, al.y, i), __shfl_sync(0xffffffffu, al.z, i), 0.f);
+            const float4 h = make_float4(__shfl_sync(0xffffffffu, ah.x, i), __shfl_sync(0xffffffffu, ah.y, i), __shfl_sync(0xffffffffu, ah.z, i), 0.f);
+            const bool hit = lane < nb && overlap(l, h, bl, bh) && !(same && !pt && it.x + i >= it.y + lane);
+            const unsigned hm = __ballot_sync(0xffffffffu, hit);
+            if (!hm) continue;
+            if (hit) Q[qn + __popc(hm & ((1u << lane) - 1))] = make_int2((it.x + i) | (pt ? 0x80000000 : 0), it.y + lane);
+            qn += __popc(hm);
+            __syncwarp();
+            if (qn >= 32) {
+                test(lane);
+                __syncwarp();
+                qn -= 32;
+                int2 rest;
+                if (lane < qn) rest = Q[32 + lane];
+                __syncwarp();
+                if (lane < qn) Q[lane] = rest;
+                __syncwarp();
+            }
+        }
+    }
+    __syncwarp();
+    if (lane < qn) test(lane);
+}
+
+// ---- step 5 for lists of at most RANK_MAX hits: a key's place is the number
+// of smaller keys (keys are distinct), counted by BR_SPLIT threads per key
+// over the whole list and written decoded, one launch instead of a radix
+// sort's histogram, scan and eight passes plus the decoding.
+constexpr int RANK_MAX = 16384, BR_THREADS = 256, BR_SPLIT = 8, BR_KEYS = BR_THREADS / BR_SPLIT;
+__global__ void __launch_bounds__(BR_THREADS) k_bp_rank(int n, const unsigned long long* __restrict__ keys, int4* out, int* n_ee) {
+    __shared__ unsigned long long tile[BR_THREADS * 4];
+    const int k = blockIdx.x * BR_KEYS + threadIdx.x / BR_SPLIT, part = threadIdx.x % BR_SPLIT;
+    const unsigned long long key = k < n ? keys[k] : 0;
+    int rank = 0;
+    for (int t0 = 0; t0 < n; t0 += BR_THREADS * 4) {
+        const int m = min(BR_THREADS * 4, n - t0);
+        __syncthreads();
+        for (int i = threadIdx.x; i < m; i += BR_THREADS) tile[i] = keys[t0 + i];
+        __syncthreads();
+#pragma unroll 4
+        for (int i = part; i < m; i += BR_SPLIT) rank += tile[i] < key;
+    }
+#pragma unroll
+    for (int o = BR_SPLIT / 2; o > 0; o >>= 1) rank += __shfl_xor_sync(0xffffffffu, rank, o);
+    if (part == 0 && k < n) {
+        const int kind = (int)(key >> 62);
+        out[rank] = make_int4(kind, (int)((key >> 31) & 0x7fffffffull), (int)(key & 0x7fffffffull), 0);
+        // the last edge-edge pair gives their count
+        if (kind == ABD_CONTACT_EE) atomicMax(n_ee, rank + 1);
     }
 }
 
@@ -232,47 +435,58 @@ __global__ void k_bp_decode(int n, const unsigned long long* __restrict__ keys, 
 }
 
 struct BpScratch {
-    float4* blo = nullptr; float4* bhi = nullptr;
-    float4* vlo = nullptr; float4* vhi = nullptr;   // per-vertex boxes of the latest build
+    BpBoxes B = {};
     int2* bpairs = nullptr; int bp_cap = 0;
+    int4* items = nullptr; long long item_cap = 0;   // cluster pairs
     unsigned long long* keys = nullptr; unsigned long long* keys_s = nullptr; int key_cap = 0;
-    int* cnt = nullptr;                     // [0] body pairs, [1] hits, [2] n_ee
+    int* cnt = nullptr;                     // [0] body pairs, [1] hits, [2] n_ee, [4..5] cluster pairs (64-bit)
+    bool swept = false;                     // the boxes are those of a swept build (k_bp_boxes keeps bodies that stay put)
     void* tmp = nullptr; size_t tmp_bytes = 0;
 };
+constexpr long long BP_ITEM_LIMIT = 1LL << 27;     // cluster pairs held at once (2 GiB)
 static BpScratch* bps(Engine* E) { return reinterpret_cast<BpScratch*>(E->bp_state); }
 
 void eng_bp_free(Engine* E) {
     BpScratch* S = bps(E);
     if (!S) return;
-    void* ps[] = {S->blo, S->bhi, S->vlo, S->vhi, S->bpairs, S->keys, S->keys_s, S->cnt, S->tmp};
+    void* ps[] = {S->B.vlo, S->B.vhi, S->B.blo, S->B.bhi, S->B.cl[0], S->B.cl[1], S->B.cl[2], S->B.ch[0], S->B.ch[1], S->B.ch[2],
+                  S->B.still, S->bpairs, S->items, S->keys, S->keys_s, S->cnt, S->tmp};
     for (void* p : ps) if (p) cudaFree(p);
     delete S;
     E->bp_state = nullptr;
 }
 
-static int bp_reserve(Engine* E, int bp_need, int key_need) {
+static int bp_reserve(Engine* E, int bp_need, long long item_need, int key_need) {
     BpScratch* S = bps(E);
     if (!S) {
         S = new BpScratch(); E->bp_state = S;
-        if (cudaMalloc(&S->blo, sizeof(float4) * E->nb) != cudaSuccess || cudaMalloc(&S->bhi, sizeof(float4) * E->nb) != cudaSuccess ||
-            cudaMalloc(&S->vlo, sizeof(float4) * std::max(E->nv, 1)) != cudaSuccess ||
-            cudaMalloc(&S->vhi, sizeof(float4) * std::max(E->nv, 1)) != cudaSuccess ||
-            cudaMalloc(&S->cnt, sizeof(int) * 4) != cudaSuccess)
+        auto box = [](float4** p, size_t n) { return cudaMalloc(p, sizeof(float4) * std::max<size_t>(n, 1)) == cudaSuccess; };
+        const size_t nc[3] = {(size_t)E->nv / 32 + E->nb + 1, (size_t)E->ne / 32 + E->nb + 1, (size_t)E->nt / 32 + E->nb + 1};
+        bool ok = box(&S->B.blo, E->nb) && box(&S->B.bhi, E->nb) && box(&S->B.vlo, E->nv) && box(&S->B.vhi, E->nv);
+        for (int k = 0; k < 3; k++) ok = ok && box(&S->B.cl[k], nc[k]) && box(&S->B.ch[k], nc[k]);
+        if (!ok || cudaMalloc(&S->cnt, sizeof(int) * 8) != cudaSuccess || cudaMalloc(&S->B.still, sizeof(int) * 3 * E->nb) != cudaSuccess)
             return E->fail(ABD_ERR_CUDA, "cudaMalloc body boxes");
-        cudaFuncSetAttribute(k_bp_prims, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)(4 * BP_CHUNK * sizeof(float4) + 2 * BP_CHUNK * sizeof(int)));
+        S->B.paired = S->B.still + E->nb; S->B.clok = S->B.paired + E->nb;
     }
     // buffers in use by queued work are freed only after the stream drains
-    if (bp_need > S->bp_cap || key_need > S->key_cap) eng_stream_sync(E);
+    if (bp_need > S->bp_cap || item_need > S->item_cap || key_need > S->key_cap) eng_stream_sync(E);
     if (bp_need > S->bp_cap) {
         if (S->bpairs) cudaFree(S->bpairs);
+        S->bpairs = nullptr;
         S->bp_cap = bp_need + bp_need / 2 + 1024;
         if (cudaMalloc(&S->bpairs, sizeof(int2) * S->bp_cap) != cudaSuccess) return E->fail(ABD_ERR_CUDA, "cudaMalloc body pairs");
+    }
+    if (item_need > S->item_cap) {
+        if (S->items) cudaFree(S->items);
+        S->items = nullptr;
+        S->item_cap = std::min(item_need + item_need / 2 + 4096, BP_ITEM_LIMIT);
+        if (cudaMalloc(&S->items, sizeof(int4) * (size_t)S->item_cap) != cudaSuccess) return E->fail(ABD_ERR_CUDA, "cudaMalloc cluster pairs");
     }
     if (key_need > S->key_cap) {
         if (S->keys) cudaFree(S->keys);
         if (S->keys_s) cudaFree(S->keys_s);
         if (S->tmp) cudaFree(S->tmp);
+        S->keys = S->keys_s = nullptr; S->tmp = nullptr;
         S->key_cap = key_need + key_need / 2 + 4096;
         if (cudaMalloc(&S->keys, sizeof(unsigned long long) * S->key_cap) != cudaSuccess ||
             cudaMalloc(&S->keys_s, sizeof(unsigned long long) * S->key_cap) != cudaSuccess)
@@ -285,42 +499,86 @@ static int bp_reserve(Engine* E, int bp_need, int key_need) {
 }
 
 // Build a sorted (kind, a, b) list of EE and PT candidates into `out`
-// (capacity *cap, grown through `grow`).  p may be null (static positions).
+// (capacity *cap, grown through `grow`).  disp.dq null: static positions.
 // mode 0: swept list with limit lim; mode 1: detection with distance filt.
 // The list length comes back to the host; its EE count stays on the device
 // (copied to nee_dev when given; BpScratch::cnt[2] until the next build).
-static int bp_build(Engine* E, const double* p, double lim, double filt, int mode, int4*& out, int& cap, int& n_out,
+// Steps of the resting 16 x 16 net, one handle: 13.51 -> 11.85 ms per step, of
+// eight nets in one handle 24.5 -> 18.1 ms, against one block per body pair
+// with both bodies' primitives staged in shared memory (90 and 464 us per
+// build there; boxes, pairs, clusters and primitive tests 45 and 190 us here)
+// and a radix sort over 64 bits for every list (35 us for short ones, k_bp_rank
+// 12 us; the sort stays for longer lists, where counting is quadratic).
+static int bp_build(Engine* E, const BpDisp& disp, double lim, double filt, int mode, int4*& out, int& cap, int& n_out,
                     int* nee_dev, int (*grow)(Engine*, int)) {
     cudaStream_t s = E->stream;
     const AbdParams& P = E->P;
     int rc;
-    if ((rc = bp_reserve(E, 4 * E->nb + 1024, std::max(cap, 4096)))) return rc;
+    if ((rc = bp_reserve(E, 4 * E->nb + 1024, 64LL * E->nb + 4096, std::max(cap, 4096)))) return rc;
     BpScratch* S = bps(E);
-    float pad = (float)(0.5 * lim);
+    const float pad = (float)(0.5 * lim);
+    const int do_ee = P.contact_ee && E->ne > 0, do_pt = P.contact_pt && E->nt > 0;
+    // the positions are those the last swept build's step led to, so a body
+    // that stays put in both has the same boxes
+    const int keep = mode == 0 && S->swept && E->sw_valid;
+    S->swept = false;
+    const int body_grid = std::min(E->nb, NUM_SMS * 16);
+    k_bp_boxes<<<body_grid, BOX_THREADS, 0, s>>>(E->nb, E->bd_vbeg, E->x, disp, pad, keep, S->B);
+    E->launches++;
     for (int attempt = 0; attempt < 8; attempt++) {
-        CUDA_TRY(cudaMemsetAsync(S->cnt, 0, sizeof(int) * 4, s));
-        k_body_boxes<<<grid_for(32L * E->nb), 256, 0, s>>>(E->nb, E->bd_vbeg, E->x, p, pad, S->blo, S->bhi, S->vlo, S->vhi);
-        k_body_pairs<<<grid_for(32L * E->nb), 256, 0, s>>>(E->nb, E->bscene, E->sc_body_begin, S->blo, S->bhi,
-                                                            P.self_contact, S->bpairs, S->bp_cap, S->cnt);
+        CUDA_TRY(cudaMemsetAsync(S->cnt, 0, sizeof(int) * 8, s));
+        k_body_pairs<<<grid_for(32L * E->nb), 256, 0, s>>>(E->nb, E->bscene, E->sc_body_begin, S->B.blo, S->B.bhi,
+                                                            P.self_contact, S->bpairs, S->bp_cap, S->cnt, S->B.paired);
+        k_bp_clboxes<<<body_grid, BOX_THREADS, 0, s>>>(E->nb, E->bd_vbeg, E->bd_ebeg, E->bd_tbeg, E->edges, E->tris, do_ee,
+                                                       do_pt, S->B);
         BpArgs A;
-        A.G = eng_geo(E); A.p = p; A.pmag = E->pmag; A.ebeg = E->bd_ebeg; A.tbeg = E->bd_tbeg; A.vbeg = E->bd_vbeg;
-        A.vlo = S->vlo; A.vhi = S->vhi;
-        A.blo = S->blo; A.bhi = S->bhi; A.pad = pad; A.lim = lim; A.filt = filt; A.mode = mode; A.f32 = P.ee_f32;
-        A.self_contact = P.self_contact; A.do_ee = P.contact_ee && E->ne > 0; A.do_pt = P.contact_pt && E->nt > 0;
+        A.G = eng_geo(E); A.pmag = E->pmag; A.vlo = S->B.vlo; A.vhi = S->B.vhi;
+        A.lim = lim; A.filt = filt; A.mode = mode; A.f32 = P.ee_f32;
         A.out = S->keys; A.cap = S->key_cap; A.count = S->cnt + 1;
-        size_t smem = 4 * BP_CHUNK * sizeof(float4) + 2 * BP_CHUNK * sizeof(int);
-        k_bp_prims<<<NUM_SMS * 2, BP_THREADS, smem, s>>>(S->bpairs, S->cnt, S->bp_cap, A);
-        E->launches += 3;
-        int h[2];
-        CUDA_TRY(cudaMemcpyAsync(h, S->cnt, sizeof(int) * 2, cudaMemcpyDeviceToHost, s));
+        unsigned long long* nitems = reinterpret_cast<unsigned long long*>(S->cnt + 4);
+        auto expand = [&](int q0, int q1) {
+            k_bp_clusters<<<NUM_SMS * 4, 256, 0, s>>>(S->bpairs, S->cnt, S->bp_cap, q0, q1, E->bd_vbeg, E->bd_ebeg, E->bd_tbeg,
+                                                       S->B, do_ee, do_pt, S->items, S->item_cap, nitems);
+            k_bp_prims<<<NUM_SMS * 8, PRIM_THREADS, 0, s>>>(S->items, nitems, S->item_cap, A);
+            E->launches += 2;
+        };
+        expand(0, INT_MAX);
+        E->launches += 2;
+        CUDA_TRY(cudaMemcpyAsync(E->hcnt->bp, S->cnt, sizeof(int) * 8, cudaMemcpyDeviceToHost, s));
         CUDA_TRY(eng_stream_sync(E));
-        if (h[0] > S->bp_cap || h[1] > S->key_cap) {
-            if ((rc = bp_reserve(E, h[0], h[1]))) return rc;
+        const int npairs = E->hcnt->bp[0];
+        long long items;
+        memcpy(&items, E->hcnt->bp + 4, sizeof items);
+        if (npairs > S->bp_cap || (items > S->item_cap && S->item_cap < BP_ITEM_LIMIT) || E->hcnt->bp[1] > S->key_cap) {
+            if ((rc = bp_reserve(E, npairs, std::min(items, BP_ITEM_LIMIT), E->hcnt->bp[1]))) return rc;
             continue;
         }
-        int n = h[1];
+        if (items > S->item_cap) {
+            // more cluster pairs than the list may hold: slices of body pairs
+            // small enough to fit whatever they overlap
+            auto most = [&](int n) { return (long long)n / 32 + 1; };
+            const long long per = most(E->ne) * most(E->ne) + 2 * most(E->nv) * most(E->nt);
+            const int step = (int)std::max<long long>(1, S->item_cap / std::max<long long>(per, 1));
+            CUDA_TRY(cudaMemsetAsync(S->cnt + 1, 0, sizeof(int), s));
+            for (int q0 = 0; q0 < npairs; q0 += step) {
+                CUDA_TRY(cudaMemsetAsync(nitems, 0, sizeof(long long), s));
+                expand(q0, std::min(npairs, q0 + step));
+                CUDA_TRY(cudaMemcpyAsync(E->hcnt->bp, S->cnt, sizeof(int) * 8, cudaMemcpyDeviceToHost, s));
+                CUDA_TRY(eng_stream_sync(E));
+                memcpy(&items, E->hcnt->bp + 4, sizeof items);
+                if (items > S->item_cap) return E->fail(ABD_ERR_CONTACT_OVERFLOW, "body-pair broad phase: one body pair's cluster pairs do not fit");
+            }
+            if (E->hcnt->bp[1] > S->key_cap) {
+                if ((rc = bp_reserve(E, npairs, 0, E->hcnt->bp[1]))) return rc;
+                continue;
+            }
+        }
+        const int n = E->hcnt->bp[1];
         if (n > cap) { if ((rc = grow(E, n))) return rc; }
-        if (n > 0) {
+        if (n > 0 && n <= RANK_MAX) {
+            k_bp_rank<<<(n + BR_KEYS - 1) / BR_KEYS, BR_THREADS, 0, s>>>(n, S->keys, out, S->cnt + 2);
+            E->launches++;
+        } else if (n > 0) {
             size_t bytes = S->tmp_bytes;
             CUDA_TRY(cub::DeviceRadixSort::SortKeys(S->tmp, bytes, S->keys, S->keys_s, n, 0, 64, s));
             k_bp_decode<<<grid_for(n), 256, 0, s>>>(n, S->keys_s, out, S->cnt + 2);
@@ -328,6 +586,7 @@ static int bp_build(Engine* E, const double* p, double lim, double filt, int mod
         }
         if (nee_dev) CUDA_TRY(cudaMemcpyAsync(nee_dev, S->cnt + 2, sizeof(int), cudaMemcpyDeviceToDevice, s));
         n_out = n;
+        S->swept = mode == 0;
         return ABD_OK;
     }
     return E->fail(ABD_ERR_CONTACT_OVERFLOW, "body-pair broad phase did not fit after growing");
@@ -336,10 +595,12 @@ static int bp_build(Engine* E, const double* p, double lim, double filt, int mod
 static int grow_sw(Engine* E, int need) { return eng_grow_swept(E, need); }
 static int grow_ct(Engine* E, int need) { return eng_grow_contacts(E, need); }
 
-// swept list along p = E->pv (computed by the caller), limit lim
-int eng_swept_bp(Engine* E, double lim) {
+// swept list along the displacement sign * J dq (left in E->pv), limit lim;
+// bodies of scenes flagged done do not move
+int eng_swept_bp(Engine* E, const double* dq, double sign, const int* done, double lim) {
     int n = 0;
-    int rc = bp_build(E, E->pv, lim, lim, 0, E->sw, E->sw_cap, n, E->sw_nee, grow_sw);
+    const BpDisp disp = {dq, sign, E->xbar, E->mass, E->bscene, done, E->pv, E->pmag};
+    int rc = bp_build(E, disp, lim, lim, 0, E->sw, E->sw_cap, n, E->sw_nee, grow_sw);
     if (rc) return rc;
     E->n_sw = n; E->n_sw_ee = -1; E->sw_valid = true;   // EE count on the device only (E->sw_nee)
     return ABD_OK;
@@ -356,7 +617,7 @@ int eng_detect_bp(Engine* E, double filt) {
     CUDA_TRY(cudaMemsetAsync(E->dcnt, 0, DETECT_COUNTER_BYTES, E->stream));
     double lim = filt * (1.0 + 1e-6) + 1e-7;
     int n = 0;
-    if ((rc = bp_build(E, nullptr, lim, filt, 1, E->contacts, E->cap, n, nullptr, grow_ct))) return rc;
+    if ((rc = bp_build(E, BpDisp{}, lim, filt, 1, E->contacts, E->cap, n, nullptr, grow_ct))) return rc;
     k_bp_counts<<<1, 32, 0, E->stream>>>(E->dcnt, bps(E)->cnt + 2, n);
     E->launches++;
     return eng_pg_candidates(E, filt);

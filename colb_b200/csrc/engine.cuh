@@ -94,6 +94,7 @@ struct Counters {
     int nkeys, grp_fail, ls_trials, ls_nsw;   // ls_*: trial count and list length of a graph line search
     int n_sw, n_sw_ee, sw_overflow, pos_changed;   // pos_changed: abd_set_state moved a body
     int du_guard;                                  // mixed-precision increments replaced (du_guard)
+    alignas(8) int bp[8];                          // host only: counts of a body-pair build (bpair.cu)
 };
 #define DETECT_COUNTER_BYTES (5 * sizeof(int))   // n_ee .. overflow
 
@@ -321,7 +322,7 @@ void eng_lsgraph_free(Engine* E);
 int eng_groups(Engine* E, const int* done);   // contact groups of the listed step (after eng_swept)
 void eng_groups_free(Engine* E);
 int eng_detect_list(Engine* E);
-int eng_swept_bp(Engine* E, double lim);
+int eng_swept_bp(Engine* E, const double* dq, double sign, const int* done, double lim);
 int eng_detect_bp(Engine* E, double filt);
 void eng_bp_free(Engine* E);
 bool eng_use_bp(const Engine* E);

@@ -196,14 +196,11 @@ int eng_swept(Engine* E, const double* dq, double sign, const int* done) {
         // length at that fraction (k_ls_init), so the list still covers every
         // position it visits
         for (double scale = 1.0;; scale *= 0.25) {
-            k_vertex_disp2<<<grid_for(E->nv), 256, 0, s>>>(E->nv, E->vbody, E->xbar, dq, sign * scale, E->mass, E->bscene,
-                                                            done, E->pv, E->pmag);
-            E->launches++;
             if ((E->P.test_inject & ABD_INJECT_SWEPT_FULL) && !E->sw_inject_done && scale == 1.0) {
                 E->sw_inject_done = true;        // test hook: the full step's list "does not fit"
                 continue;
             }
-            rc = eng_swept_bp(E, lim);
+            rc = eng_swept_bp(E, dq, sign * scale, done, lim);
             if (rc == ABD_ERR_CONTACT_OVERFLOW && scale > 1e-6) { E->err.clear(); continue; }
             if (rc == ABD_OK) E->sw_scale = scale;
             return rc;

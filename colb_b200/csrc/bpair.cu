@@ -435,6 +435,7 @@ __global__ void k_bp_decode(int n, const unsigned long long* __restrict__ keys, 
 }
 
 struct BpScratch {
+    void* slab = nullptr;                   // boxes, flags and counters
     BpBoxes B = {};
     int2* bpairs = nullptr; int bp_cap = 0;
     int4* items = nullptr; long long item_cap = 0;   // cluster pairs
@@ -446,11 +447,16 @@ struct BpScratch {
 constexpr long long BP_ITEM_LIMIT = 1LL << 27;     // cluster pairs held at once (2 GiB)
 static BpScratch* bps(Engine* E) { return reinterpret_cast<BpScratch*>(E->bp_state); }
 
+void eng_step_boxes(Engine* E, const float4** lo, const float4** hi) {
+    BpScratch* S = bps(E);
+    *lo = S && S->swept ? S->B.blo : nullptr;
+    *hi = S && S->swept ? S->B.bhi : nullptr;
+}
+
 void eng_bp_free(Engine* E) {
     BpScratch* S = bps(E);
     if (!S) return;
-    void* ps[] = {S->B.vlo, S->B.vhi, S->B.blo, S->B.bhi, S->B.cl[0], S->B.cl[1], S->B.cl[2], S->B.ch[0], S->B.ch[1], S->B.ch[2],
-                  S->B.still, S->bpairs, S->items, S->keys, S->keys_s, S->cnt, S->tmp};
+    void* ps[] = {S->slab, S->bpairs, S->items, S->keys, S->tmp};
     for (void* p : ps) if (p) cudaFree(p);
     delete S;
     E->bp_state = nullptr;
@@ -460,13 +466,21 @@ static int bp_reserve(Engine* E, int bp_need, long long item_need, int key_need)
     BpScratch* S = bps(E);
     if (!S) {
         S = new BpScratch(); E->bp_state = S;
-        auto box = [](float4** p, size_t n) { return cudaMalloc(p, sizeof(float4) * std::max<size_t>(n, 1)) == cudaSuccess; };
-        const size_t nc[3] = {(size_t)E->nv / 32 + E->nb + 1, (size_t)E->ne / 32 + E->nb + 1, (size_t)E->nt / 32 + E->nb + 1};
-        bool ok = box(&S->B.blo, E->nb) && box(&S->B.bhi, E->nb) && box(&S->B.vlo, E->nv) && box(&S->B.vhi, E->nv);
-        for (int k = 0; k < 3; k++) ok = ok && box(&S->B.cl[k], nc[k]) && box(&S->B.ch[k], nc[k]);
-        if (!ok || cudaMalloc(&S->cnt, sizeof(int) * 8) != cudaSuccess || cudaMalloc(&S->B.still, sizeof(int) * 3 * E->nb) != cudaSuccess)
+        // one allocation for all boxes, flags and counters of the handle
+        const size_t nb = E->nb, nv = E->nv;
+        const size_t nc[3] = {nv / 32 + nb + 1, (size_t)E->ne / 32 + nb + 1, (size_t)E->nt / 32 + nb + 1};
+        const size_t boxes = 2 * (nb + nv + nc[0] + nc[1] + nc[2]);
+        if (cudaMalloc(&S->slab, sizeof(float4) * boxes + sizeof(int) * (8 + 3 * nb)) != cudaSuccess) {
+            S->slab = nullptr;
             return E->fail(ABD_ERR_CUDA, "cudaMalloc body boxes");
-        S->B.paired = S->B.still + E->nb; S->B.clok = S->B.paired + E->nb;
+        }
+        float4* at = reinterpret_cast<float4*>(S->slab);
+        auto take = [&](float4*& lo, float4*& hi, size_t n) { lo = at; hi = at + n; at += 2 * n; };
+        take(S->B.blo, S->B.bhi, nb);
+        take(S->B.vlo, S->B.vhi, nv);
+        for (int k = 0; k < 3; k++) take(S->B.cl[k], S->B.ch[k], nc[k]);
+        S->cnt = reinterpret_cast<int*>(at);
+        S->B.still = S->cnt + 8; S->B.paired = S->B.still + nb; S->B.clok = S->B.paired + nb;
     }
     // buffers in use by queued work are freed only after the stream drains
     if (bp_need > S->bp_cap || item_need > S->item_cap || key_need > S->key_cap) eng_stream_sync(E);
@@ -484,13 +498,12 @@ static int bp_reserve(Engine* E, int bp_need, long long item_need, int key_need)
     }
     if (key_need > S->key_cap) {
         if (S->keys) cudaFree(S->keys);
-        if (S->keys_s) cudaFree(S->keys_s);
         if (S->tmp) cudaFree(S->tmp);
         S->keys = S->keys_s = nullptr; S->tmp = nullptr;
         S->key_cap = key_need + key_need / 2 + 4096;
-        if (cudaMalloc(&S->keys, sizeof(unsigned long long) * S->key_cap) != cudaSuccess ||
-            cudaMalloc(&S->keys_s, sizeof(unsigned long long) * S->key_cap) != cudaSuccess)
+        if (cudaMalloc(&S->keys, 2 * sizeof(unsigned long long) * S->key_cap) != cudaSuccess)
             return E->fail(ABD_ERR_CUDA, "cudaMalloc pair keys");
+        S->keys_s = S->keys + S->key_cap;
         S->tmp_bytes = 0;
         cub::DeviceRadixSort::SortKeys(nullptr, S->tmp_bytes, S->keys, S->keys_s, S->key_cap);
         if (cudaMalloc(&S->tmp, S->tmp_bytes) != cudaSuccess) return E->fail(ABD_ERR_CUDA, "cudaMalloc sort scratch");

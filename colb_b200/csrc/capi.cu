@@ -162,7 +162,7 @@ void eng_free(Engine* E) {
                   E->sc_plane_begin, E->sc_body_begin, E->edge_scene, E->tri_scene, E->st, E->backup, E->du, E->g, E->x,
                   E->xf, E->pv, E->ws, E->contacts, E->cst, E->ctype, E->cxb, E->cbody, E->cblk, E->keys, E->keys_s,
                   E->ukeys, E->row_ptr, E->bcol, E->vals, E->dinv, E->scd, E->sci, E->cub_tmp, E->dcnt, E->prof_d,
-                  E->sw, E->sw_flag, E->sw_off, E->pmag, E->zero_int, E->zero_ns, E->sw_nee};
+                  E->sw, E->sw_flag, E->sw_off, E->pmag, E->vchunk, E->zero_int, E->zero_ns, E->sw_nee};
     for (void* p : ps) if (p) cudaFree(p);
     for (int i = 0; i < 10; i++) if (E->kv[i]) cudaFree(E->kv[i]);
     if (E->hcnt) cudaFreeHost(E->hcnt);
@@ -298,6 +298,23 @@ int abd_create(const AbdParams* params, const AbdSceneDesc* scenes, int32_t n_sc
         g_err = E->err; eng_free(E); delete E; return rc;
     }
     E->edges = reinterpret_cast<int2*>(edges_i);
+    // runs of vertices of one body, in vertex order; a body without vertices
+    // gets an empty run, so that its state is written too
+    {
+        std::vector<int4> ch;
+        std::vector<char> seen(nb, 0);
+        for (int v = 0; v < nv;) {
+            const int b = vbody[v];
+            int e = v + 1;
+            while (e < nv && e - v < VCHUNK && vbody[e] == b) e++;
+            ch.push_back(make_int4(b, v, e - v, !seen[b]));
+            seen[b] = 1;
+            v = e;
+        }
+        for (int b = 0; b < nb; b++) if (!seen[b]) ch.push_back(make_int4(b, 0, 0, 1));
+        E->nvchunk = (int)ch.size();
+        if ((rc = up(E->vchunk, ch))) { g_err = E->err; eng_free(E); delete E; return rc; }
+    }
     // per-body primitive ranges for the body-pair broad phase
     {
         std::vector<int> vb(nb + 1, 0), eb(nb + 1, 0), tb(nb + 1, 0);
@@ -383,7 +400,7 @@ int abd_set_state(AbdHandle* h, const double* st, int32_t n) {
     CUDA_TRY(cudaMemcpyAsync(E->st, E->st_in, bytes, cudaMemcpyDeviceToDevice, E->stream));
     CUDA_TRY(cudaMemcpyAsync(&E->hcnt->pos_changed, &E->dcnt->pos_changed, sizeof(int), cudaMemcpyDeviceToHost, E->stream));
     CUDA_TRY(cudaStreamSynchronize(E->stream));
-    if (E->hcnt->pos_changed) E->sw_valid = false;
+    if (E->hcnt->pos_changed) { E->sw_valid = false; E->x_fresh = false; }
     return ABD_OK;
 }
 
@@ -686,7 +703,7 @@ extern "C" int abd_get_autotune(AbdHandle* h, int32_t* shapes, int32_t cap, int3
     v[0] = cc < 0 ? -1 : TUNE_CONTACT_THREADS[cc];
     v[1] = cc < 0 ? -1 : TUNE_CONTACT_PER_BLOCK[cc];
     v[2] = E->tune[TK_LIST_ENERGY].chosen < 0 ? -1 : TUNE_THREADS[E->tune[TK_LIST_ENERGY].chosen];
-    v[3] = E->tune[TK_BODY_ENERGY].chosen < 0 ? -1 : TUNE_THREADS[E->tune[TK_BODY_ENERGY].chosen];
+    v[3] = v[2];          // one kernel evaluates both
     for (int i = 0; i < 4 && i < cap; i++) shapes[i] = v[i];
     *n = 4;
     return ABD_OK;

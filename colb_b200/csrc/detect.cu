@@ -12,7 +12,7 @@
 // rebuilds a hashed uniform grid (one radix sort), counts pairs per query
 // item, scans, and writes each item's pairs in index order, so the list is
 // sorted and exact-size; overflow is reported instead of wrapping.
-#include "contact.cuh"
+#include "energy.cuh"
 #include <cub/cub.cuh>
 
 // ------------------------------------------------------------------ transform
@@ -35,13 +35,18 @@ __global__ void k_transform(int nv, const double* __restrict__ xbar, const int* 
     }
 }
 
-int eng_body_energy(Engine* E, const int* bunit, double* Eo, double* En, const int* skip);
-int eng_pg_energy(Engine* E, const int* bunit, double* Eo, double* En, const int* skip);
+int eng_body_energy(Engine* E, double* Eo, const int* skip);
+int eng_pg_energy(Engine* E, double* Eo, const int* skip);
 int eng_pg_candidates(Engine* E, double filt);
 
+// Vertex positions of the nxt state.  The line search leaves them behind with
+// every state it writes, so they are formed here only after the state came
+// from outside.
 int eng_transform(Engine* E) {
+    if (E->x_fresh) return ABD_OK;
     k_transform<<<grid_for(E->nv), 256, 0, E->stream>>>(E->nv, E->xbar, E->vbody, E->st, E->x, E->xf);
     E->launches++;
+    E->x_fresh = true;
     return ABD_OK;
 }
 
@@ -104,65 +109,6 @@ __global__ void k_point_boxes(int nv, const double* __restrict__ x, const int* _
         float l[3], h[3];
 #pragma unroll
         for (int k = 0; k < 3; k++) { l[k] = __fsub_rd(f_rd(x[3*v+k]), pad); h[k] = __fadd_ru(f_ru(x[3*v+k]), pad); }
-        lo[v] = make_float4(l[0], l[1], l[2], 0.f); hi[v] = make_float4(h[0], h[1], h[2], 0.f); scene[v] = vscene[v];
-        ext = fmaxf(ext, fmaxf(h[0] - l[0], fmaxf(h[1] - l[1], h[2] - l[2])));
-    }
-    for (int o = 16; o > 0; o >>= 1) ext = fmaxf(ext, __shfl_xor_sync(0xffffffffu, ext, o));
-    if ((threadIdx.x & 31) == 0 && ext > 0.f) atomic_max_pos(cell, ext);
-}
-
-// swept boxes of a displacement p (vertex array, 3 doubles each)
-__global__ void k_swept_edge_boxes(int ne, const int2* __restrict__ edges, const double* __restrict__ x,
-                                   const double* __restrict__ p, const int* __restrict__ escene,
-                                   float4* lo, float4* hi, int* scene, float* cell) {
-    float ext = 0.f;
-    GS_LOOP(e, ne) {
-        int2 ed = edges[e];
-        float l[3], h[3];
-#pragma unroll
-        for (int k = 0; k < 3; k++) {
-            double a = x[3*ed.x+k], b = x[3*ed.y+k], a1 = a + p[3*ed.x+k], b1 = b + p[3*ed.y+k];
-            l[k] = __fsub_rd(f_rd(fmin(fmin(a, b), fmin(a1, b1))), 1e-6f);
-            h[k] = __fadd_ru(f_ru(fmax(fmax(a, b), fmax(a1, b1))), 1e-6f);
-        }
-        lo[e] = make_float4(l[0], l[1], l[2], 0.f); hi[e] = make_float4(h[0], h[1], h[2], 0.f); scene[e] = escene[e];
-        ext = fmaxf(ext, fmaxf(h[0] - l[0], fmaxf(h[1] - l[1], h[2] - l[2])));
-    }
-    for (int o = 16; o > 0; o >>= 1) ext = fmaxf(ext, __shfl_xor_sync(0xffffffffu, ext, o));
-    if ((threadIdx.x & 31) == 0 && ext > 0.f) atomic_max_pos(cell, ext);
-}
-__global__ void k_swept_tri_boxes(int nt, const int* __restrict__ tris, const double* __restrict__ x,
-                                  const double* __restrict__ p, const int* __restrict__ tscene,
-                                  float4* lo, float4* hi, int* scene, float* cell) {
-    float ext = 0.f;
-    GS_LOOP(t, nt) {
-        float l[3], h[3];
-#pragma unroll
-        for (int k = 0; k < 3; k++) {
-            double mn = 1e300, mx = -1e300;
-            for (int q = 0; q < 3; q++) {
-                int v = tris[3*t+q];
-                double a = x[3*v+k], b = a + p[3*v+k];
-                mn = fmin(mn, fmin(a, b)); mx = fmax(mx, fmax(a, b));
-            }
-            l[k] = __fsub_rd(f_rd(mn), 1e-6f); h[k] = __fadd_ru(f_ru(mx), 1e-6f);
-        }
-        lo[t] = make_float4(l[0], l[1], l[2], 0.f); hi[t] = make_float4(h[0], h[1], h[2], 0.f); scene[t] = tscene[t];
-        ext = fmaxf(ext, fmaxf(h[0] - l[0], fmaxf(h[1] - l[1], h[2] - l[2])));
-    }
-    for (int o = 16; o > 0; o >>= 1) ext = fmaxf(ext, __shfl_xor_sync(0xffffffffu, ext, o));
-    if ((threadIdx.x & 31) == 0 && ext > 0.f) atomic_max_pos(cell, ext);
-}
-__global__ void k_swept_point_boxes(int nv, const double* __restrict__ x, const double* __restrict__ p,
-                                    const int* __restrict__ vscene, float4* lo, float4* hi, int* scene, float* cell) {
-    float ext = 0.f;
-    GS_LOOP(v, nv) {
-        float l[3], h[3];
-#pragma unroll
-        for (int k = 0; k < 3; k++) {
-            double a = x[3*v+k], b = a + p[3*v+k];
-            l[k] = __fsub_rd(f_rd(fmin(a, b)), 1e-6f); h[k] = __fadd_ru(f_ru(fmax(a, b)), 1e-6f);
-        }
         lo[v] = make_float4(l[0], l[1], l[2], 0.f); hi[v] = make_float4(h[0], h[1], h[2], 0.f); scene[v] = vscene[v];
         ext = fmaxf(ext, fmaxf(h[0] - l[0], fmaxf(h[1] - l[1], h[2] - l[2])));
     }
@@ -398,36 +344,16 @@ int eng_pg_candidates(Engine* E, double filt) {
 
 // ------------------------------------------------------------------ energies
 __global__ void k_body_energy(int nb, const double* __restrict__ st, const double* __restrict__ mass,
-                              const double* __restrict__ J, const int* __restrict__ bscene, double dt,
-                              double g0, double g1, double g2, double k_ortho, const int* done, double* E,
-                              double* En) {
+                              const double* __restrict__ J, const int* __restrict__ bscene, BodyTerms T, const int* done,
+                              double* E) {
     for (long base = (long)blockIdx.x * blockDim.x; base < nb; base += (long)gridDim.x * blockDim.x) {
         long b = base + threadIdx.x;
         bool valid = b < nb;
         int s = valid ? bscene[b] : 0;
         double e = 0, en = 0;
-        if (valid && !done[s]) {
-            const double* now = st + ST_STRIDE * b + ST_NOW; const double* nx = st + ST_STRIDE * b + ST_NXT;
-            double eo = ortho_energy(nx + ST_Q, k_ortho);
-            double gv[3] = {g0, g1, g2};
-            double n0 = 0, n1 = 0, s0 = 0, s1 = 0;
-#pragma unroll
-            for (int k = 0; k < 3; k++) {
-                double ct = now[ST_C+k] + dt * now[ST_V+k] + dt * dt * gv[k];
-                double d = nx[ST_C+k] - ct; n0 += d * d;
-                s0 += fabs(d) * (fabs(nx[ST_C+k]) + fabs(ct));
-            }
-#pragma unroll
-            for (int r = 0; r < 9; r++) {
-                double qt = now[ST_Q+r] + dt * now[ST_QD+r];
-                double d = nx[ST_Q+r] - qt; n1 += d * d;
-                s1 += fabs(d) * (fabs(nx[ST_Q+r]) + fabs(qt));
-            }
-            e = eo * dt * dt + 0.5 * (n0 * mass[b] + n1 * J[b]);
-            if (En) en = (e + s0 * fabs(mass[b]) + s1 * fabs(J[b]) + dt * dt * ortho_noise(nx + ST_Q, k_ortho)) * DBL_EPSILON;
-        } else valid = false;
+        if (valid && !done[s]) body_energy(st + ST_STRIDE * b, mass[b], J[b], T, e, en);
+        else valid = false;
         warp_reduce_add(E, s, e, valid);
-        if (En) warp_reduce_add(En, s, en, valid);
     }
 }
 
@@ -481,29 +407,16 @@ __global__ void k_pt_energy(int nv, GridView GV, Geo G, const float4* __restrict
         warp_reduce_add(E, s, e, valid);
     }
 }
-// planes come from the vertex's scene; the energy goes to the unit of its body
-__global__ void k_pg_energy(int nv, Geo G, const int* __restrict__ vscene, const int* __restrict__ bunit, double dhat,
-                            int barrier, double sc, const int* done, double* E, double* En) {
+__global__ void k_pg_energy(int nv, Geo G, const int* __restrict__ vscene, PairTerms T, const int* done, double* E) {
     for (long base = (long)blockIdx.x * blockDim.x; base < nv; base += (long)gridDim.x * blockDim.x) {
         long v = base + threadIdx.x;
         bool valid = v < nv;
         int s = valid ? vscene[v] : 0;
-        int u = valid ? bunit[G.vbody[v]] : 0;
         double e = 0, en = 0;
-        if (valid && !done[u]) {
-            double xh = dhat * dhat;
-            double L = fmax(fabs(G.x[3*v]), fmax(fabs(G.x[3*v+1]), fabs(G.x[3*v+2])));
-            for (int pl = G.sc_plane_begin[s]; pl < G.sc_plane_begin[s+1]; pl++) {
-                const double* n = G.planes + 4*pl;
-                double d = n[0] * G.x[3*v] + n[1] * G.x[3*v+1] + n[2] * G.x[3*v+2] - n[3];
-                if (!(d < dhat)) continue;
-                double b0, b1, b2; barrier3(barrier, d * d, xh, b0, b1, b2);
-                e += b0 * sc;
-                en += contact_noise(sc, b0, b1, d * d, fmax(L, fabs(n[3])), 1.0) * DBL_EPSILON;
-            }
+        if (valid && !done[s]) {
+            for (int pl = G.sc_plane_begin[s]; pl < G.sc_plane_begin[s+1]; pl++) plane_energy(G.x + 3*v, G.planes + 4*pl, T, e, en);
         } else valid = false;
-        warp_reduce_add(E, u, e, valid);
-        if (En) warp_reduce_add(En, u, en, valid);
+        warp_reduce_add(E, s, e, valid);
     }
 }
 
@@ -516,7 +429,7 @@ static int energy_impl(Engine* E, int slot, const int* skip) {
     CUDA_TRY(cudaMemsetAsync(Eo, 0, sizeof(double) * E->ns, s));
     if ((rc = eng_transform(E))) return rc;
     const AbdParams& P = E->P;
-    if ((rc = eng_body_energy(E, E->bscene, Eo, nullptr, skip))) return rc;
+    if ((rc = eng_body_energy(E, Eo, skip))) return rc;
     double sc = P.kappa * P.dt * P.dt;
     Geo G = geo(E);
     if (P.contact_ee && E->ne > 1) {
@@ -539,144 +452,22 @@ static int energy_impl(Engine* E, int slot, const int* skip) {
         phase_end(E, ph, E->nv * (32.0 + 4.0 + 24.0) + E->nt * (12.0 + 32.0 + 4.0 + 4.0) + g.H * 8.0);
         E->launches++;
     }
-    return eng_pg_energy(E, E->bscene, Eo, nullptr, skip);
+    return eng_pg_energy(E, Eo, skip);
 }
-// En (may be null) accumulates the scale of the FP64 evaluation error
-int eng_body_energy(Engine* E, const int* bunit, double* Eo, double* En, const int* skip) {
-    const AbdParams& P = E->P;
-    int tb = TUNE_THREADS[tune_begin(E, TK_BODY_ENERGY, 4, 2)];
-    k_body_energy<<<grid_for(E->nb, tb), tb, 0, E->stream>>>(E->nb, E->st, E->mass, E->J, bunit, P.dt, P.gravity[0],
-                                                            P.gravity[1], P.gravity[2], P.k_ortho, skip, Eo, En);
-    tune_end(E, TK_BODY_ENERGY);
+int eng_body_energy(Engine* E, double* Eo, const int* skip) {
+    k_body_energy<<<grid_for(E->nb), 256, 0, E->stream>>>(E->nb, E->st, E->mass, E->J, E->bscene, body_terms(E->P), skip, Eo);
     E->launches++;
     return ABD_OK;
 }
-int eng_pg_energy(Engine* E, const int* bunit, double* Eo, double* En, const int* skip) {
-    const AbdParams& P = E->P;
+int eng_pg_energy(Engine* E, double* Eo, const int* skip) {
     if (E->npl > 0) {
-        k_pg_energy<<<grid_for(E->nv), 256, 0, E->stream>>>(E->nv, geo(E), E->vscene, bunit, P.dhat, P.barrier,
-                                                            P.kappa * P.dt * P.dt, skip, Eo, En);
+        k_pg_energy<<<grid_for(E->nv), 256, 0, E->stream>>>(E->nv, geo(E), E->vscene, pair_terms(E->P), skip, Eo);
         E->launches++;
     }
     return ABD_OK;
 }
 int eng_energy(Engine* E, int slot) { return energy_impl(E, slot, E->sci + SI_DONE * E->ns); }
 int eng_energy_masked(Engine* E, int slot, const int* skip) { return energy_impl(E, slot, skip); }
-
-// ------------------------------------------------------------------ CCD
-__global__ void k_vertex_disp(int nv, const int* __restrict__ vbody, const double* __restrict__ xbar,
-                              const double* __restrict__ dq, double sign, const double* __restrict__ mass,
-                              double* p) {
-    GS_LOOP(v, nv) {
-        int b = vbody[v];
-        const double* d = dq + 12 * b;
-        double x0 = xbar[3*v], x1 = xbar[3*v+1], x2 = xbar[3*v+2];
-        bool dyn = mass[b] > 0.0;
-#pragma unroll
-        for (int k = 0; k < 3; k++)
-            p[3*v+k] = dyn ? sign * (d[k] + x0 * d[3+k] + x1 * d[6+k] + x2 * d[9+k]) : 0.0;
-    }
-}
-
-__global__ void k_ccd_ee(int ne, GridView GV, Geo G, const double* __restrict__ p, const float4* __restrict__ qlo,
-                         const float4* __restrict__ qhi, const int* __restrict__ qscene, int self_contact,
-                         double s_ccd, int ccd_it, const int* done, double* toi, int* capped) {
-    GS_LOOP(i, ne) {
-        int s = qscene[i];
-        if (done[s]) continue;
-        int ii = (int)i;
-        double best = 1.0;
-        grid_visit(GV, qlo[i], qhi[i], s, [&](int j) {
-            if (j <= ii) return;
-            int2 a = G.edges[ii], b = G.edges[j];
-            if (a.x == b.x || a.x == b.y || a.y == b.x || a.y == b.y) return;
-            if (!self_contact && G.vbody[a.x] == G.vbody[b.x]) return;
-            int v[4] = {a.x, a.y, b.x, b.y};
-            double xx[12], pp[12];
-            for (int k = 0; k < 4; k++) for (int c = 0; c < 3; c++) { xx[3*k+c] = G.x[3*v[k]+c]; pp[3*k+c] = p[3*v[k]+c]; }
-            double t;
-            if (accd(0, xx, pp, s_ccd, best, &t, capped, ccd_it) && t < best) best = t;
-        });
-        if (best < 1.0) atomic_min_pos(toi + s, best);
-    }
-}
-__global__ void k_ccd_pt(int nv, GridView GV, Geo G, const double* __restrict__ p, const float4* __restrict__ qlo,
-                         const float4* __restrict__ qhi, const int* __restrict__ qscene, int self_contact,
-                         double s_ccd, int ccd_it, const int* done, double* toi, int* capped) {
-    GS_LOOP(pi, nv) {
-        int s = qscene[pi];
-        if (done[s]) continue;
-        int pp0 = (int)pi;
-        double best = 1.0;
-        grid_visit(GV, qlo[pi], qhi[pi], s, [&](int t) {
-            int a = G.tris[3*t], b = G.tris[3*t+1], c = G.tris[3*t+2];
-            if (pp0 == a || pp0 == b || pp0 == c) return;
-            if (!self_contact && G.vbody[pp0] == G.vbody[a]) return;
-            int v[4] = {pp0, a, b, c};
-            double xx[12], pp[12];
-            for (int k = 0; k < 4; k++) for (int q = 0; q < 3; q++) { xx[3*k+q] = G.x[3*v[k]+q]; pp[3*k+q] = p[3*v[k]+q]; }
-            double tt;
-            if (accd(1, xx, pp, s_ccd, best, &tt, capped, ccd_it) && tt < best) best = tt;
-        });
-        if (best < 1.0) atomic_min_pos(toi + s, best);
-    }
-}
-__global__ void k_ccd_pg(int nv, Geo G, const double* __restrict__ p, const int* __restrict__ vscene, double s_ccd,
-                         const int* done, double* toi) {
-    GS_LOOP(v, nv) {
-        int s = vscene[v];
-        if (done[s]) continue;
-        double best = 1.0;
-        for (int pl = G.sc_plane_begin[s]; pl < G.sc_plane_begin[s+1]; pl++) {
-            const double* n = G.planes + 4*pl;
-            double d = n[0] * G.x[3*v] + n[1] * G.x[3*v+1] + n[2] * G.x[3*v+2] - n[3];
-            double vn = n[0] * p[3*v] + n[1] * p[3*v+1] + n[2] * p[3*v+2];
-            if (vn < 0) { double t = (1 - s_ccd) * d / (-vn); if (t < 0) t = 0; if (t < best) best = t; }
-        }
-        if (best < 1.0) atomic_min_pos(toi + s, best);
-    }
-}
-__global__ void k_fill(double* a, int n, double v) { GS_LOOP(i, n) a[i] = v; }
-
-// per-scene largest step fraction along x -> x + sign * J dq
-int eng_ccd(Engine* E, const double* dq, double sign) {
-    cudaStream_t s = E->stream;
-    int rc;
-    double* toi = E->scd + SD_TOI * E->ns;
-    k_fill<<<grid_for(E->ns), 256, 0, s>>>(toi, E->ns, 1.0);
-    if ((rc = eng_transform(E))) return rc;
-    k_vertex_disp<<<grid_for(E->nv), 256, 0, s>>>(E->nv, E->vbody, E->xbar, dq, sign, E->mass, E->pv);
-    E->launches += 2;
-    const AbdParams& P = E->P;
-    const int* done = E->sci + SI_DONE * E->ns;
-    Geo G = geo(E);
-    if (P.contact_ee && E->ne > 1) {
-        Grid& g = E->gee;
-        CUDA_TRY(cudaMemsetAsync(g.cell, 0, sizeof(float), s));
-        k_swept_edge_boxes<<<grid_for(g.n), 256, 0, s>>>(g.n, E->edges, E->x, E->pv, E->edge_scene, g.lo, g.hi, g.scene, g.cell);
-        E->launches++;
-        if ((rc = eng_grid_build(E, g))) return rc;
-        k_ccd_ee<<<grid_for(E->ne, 64), 64, 0, s>>>(E->ne, eng_view(g), G, E->pv, g.lo, g.hi, g.scene, P.self_contact, P.ccd_scale,
-                                                    ccd_iters(P), done, toi, &E->dcnt->ccd_capped);
-        E->launches++;
-    }
-    if (P.contact_pt && E->nt > 0) {
-        Grid& g = E->gpt;
-        CUDA_TRY(cudaMemsetAsync(g.cell, 0, sizeof(float), s));
-        k_swept_tri_boxes<<<grid_for(g.n), 256, 0, s>>>(g.n, E->tris, E->x, E->pv, E->tri_scene, g.lo, g.hi, g.scene, g.cell);
-        k_swept_point_boxes<<<grid_for(g.nq), 256, 0, s>>>(g.nq, E->x, E->pv, E->vscene, g.qlo, g.qhi, g.qscene, g.cell);
-        E->launches += 2;
-        if ((rc = eng_grid_build(E, g))) return rc;
-        k_ccd_pt<<<grid_for(E->nv, 64), 64, 0, s>>>(E->nv, eng_view(g), G, E->pv, g.qlo, g.qhi, g.qscene, P.self_contact, P.ccd_scale,
-                                                    ccd_iters(P), done, toi, &E->dcnt->ccd_capped);
-        E->launches++;
-    }
-    if (E->npl > 0) {
-        k_ccd_pg<<<grid_for(E->nv), 256, 0, s>>>(E->nv, G, E->pv, E->vscene, P.ccd_scale, done, toi);
-        E->launches++;
-    }
-    return ABD_OK;
-}
 
 // ------------------------------------------------------------------ intersections
 DV double orient3(d3 a, d3 b, d3 c, d3 d) { return dot(cross(b - a, c - a), d - a); }

@@ -94,6 +94,7 @@ struct Counters {
     int nkeys, grp_fail, ls_trials, ls_nsw;   // ls_*: trial count and list length of a graph line search
     int n_sw, n_sw_ee, sw_overflow, pos_changed;   // pos_changed: abd_set_state moved a body
     int du_guard;                                  // mixed-precision increments replaced (du_guard)
+    int ticket;                                    // blocks that have finished the current search kernel
     alignas(8) int bp[8];                          // host only: counts of a body-pair build (bpair.cu)
 };
 #define DETECT_COUNTER_BYTES (5 * sizeof(int))   // n_ee .. overflow
@@ -115,7 +116,7 @@ struct Engine {
         float sum[8] = {0}; int cnt[8] = {0};
         cudaEvent_t a = nullptr, b = nullptr;
     };
-    Tuner tune[3];
+    Tuner tune[2];
 
     // host-side scene offsets
     std::vector<int> h_body_begin, h_vert_begin, h_edge_begin, h_tri_begin, h_plane_begin;
@@ -153,6 +154,8 @@ struct Engine {
     // memory in the assembly's own sync for the direct solver's analysis
     unsigned long long* h_ukeys = nullptr; int h_ukeys_cap = 0; int* h_done = nullptr; bool keys_host = false;
     int* sw_flag = nullptr; int* sw_off = nullptr;
+    int4* vchunk = nullptr; int nvchunk = 0;       // runs of <= VCHUNK vertices of one body {body, first, count, first run}
+    bool x_fresh = false;          // x and xf are the vertices of st's nxt state
     float* pmag = nullptr;         // |displacement| per vertex of the listed step
     int* zero_int = nullptr;       // a device 0
     int* zero_ns = nullptr;        // ns device zeros (no scene skipped)
@@ -281,12 +284,12 @@ DV int find_block(const int* row_ptr, const int* bcol, int r, int c) {
 // launch-shape autotuner (capi.cu): tune_begin returns the candidate index to
 // launch (the chosen one once timed, the default when autotune is off) and
 // brackets it with events until every candidate was timed TUNE_REPS times
-enum { TK_CONTACT = 0, TK_LIST_ENERGY, TK_BODY_ENERGY, TK_COUNT };
+enum { TK_CONTACT = 0, TK_LIST_ENERGY, TK_COUNT };
 // contact assembly: one warp per contact with 2, 4 (default) or 8 per block,
 // or one block of 64 or 128 threads per contact
 constexpr int TUNE_CONTACT_THREADS[5] = {64, 128, 256, 64, 128};
 constexpr int TUNE_CONTACT_PER_BLOCK[5] = {2, 4, 8, 1, 1};
-constexpr int TUNE_THREADS[4] = {64, 128, 256, 512};         // defaults 128 (list energy), 256 (body energy)
+constexpr int TUNE_THREADS[3] = {64, 128, 256};              // energies of the search, default 128
 constexpr int TUNE_REPS = 3;
 int tune_begin(Engine* E, int kernel, int ncand, int dflt);
 void tune_end(Engine* E, int kernel);
@@ -304,7 +307,6 @@ void eng_mlp_free(Engine* E);
 int eng_features(Engine* E, float* feat_dev);     // per-body features at the nxt state
 int eng_learned_ws(Engine* E);                     // network increment into ws
 long long eng_dense_bytes(Engine* E);
-int eng_ccd(Engine* E, const double* dq, double sign); // per-scene toi into scd[SD_TOI]
 int eng_step(Engine* E, int n_steps, AbdStepStats* stats);
 int eng_intersections(Engine* E, int* count);
 int eng_sync_counters(Engine* E);
@@ -314,10 +316,14 @@ void eng_keys_ahead_synced(Engine* E);                // after that sync: keys o
 int eng_grid_build(Engine* E, Grid& G);
 GridView eng_view(const Grid& G);
 int eng_swept(Engine* E, const double* dq, double sign, const int* done);
-int eng_ccd_list(Engine* E, const LsUnits& U, const int* skip);
-// dev_count: the listed-pair kernel reads the list length from
-// dcnt->ls_nsw and runs a fixed grid (for a graph that outlives one list)
-int eng_energy_list(Engine* E, const LsUnits& U, int slot, const int* skip, bool dev_count = false);
+// line search (search.cu)
+constexpr int LS_MAX_TRIALS = 64;
+constexpr int VCHUNK = 64;                             // vertices of a chunk: two per lane
+int eng_ls_begin(Engine* E, const LsUnits& U, const int* udone);
+int eng_ls_apply(Engine* E, const LsUnits& U);
+int eng_ls_energy(Engine* E, const LsUnits& U, int decide, cudaGraphConditionalHandle loop = 0);
+// body boxes of the listed step, null when the grid listed it (bpair.cu)
+void eng_step_boxes(Engine* E, const float4** lo, const float4** hi);
 void eng_lsgraph_free(Engine* E);
 int eng_groups(Engine* E, const int* done);   // contact groups of the listed step (after eng_swept)
 void eng_groups_free(Engine* E);

@@ -5,33 +5,6 @@
 // device; the host only reads "how many scenes are still iterating".
 #include "engine.cuh"
 
-int eng_energy_masked(Engine* E, int slot, const int* skip);
-
-// nxt.c / nxt.q are 12 consecutive doubles in DoF order [c, q0, q1, q2]
-__global__ void k_backup(int nb, const double* __restrict__ st, double* backup) {
-    GS_LOOP(i, 12L * nb) backup[i] = st[ST_STRIDE * (i / 12) + ST_NXT + (i % 12)];
-}
-// abd.py:768-785: nxt = backup - alpha du, for scenes not yet accepted
-__global__ void k_apply(int nb, const double* __restrict__ backup, const double* __restrict__ du,
-                        const double* __restrict__ alpha, const int* __restrict__ skip, const int* __restrict__ bscene,
-                        double* st) {
-    GS_LOOP(i, 12L * nb) {
-        long b = i / 12;
-        int s = bscene[b];
-        if (skip[s]) continue;
-        st[ST_STRIDE * b + ST_NXT + (i % 12)] = __fma_rn(-alpha[s], du[i], backup[i]);
-    }
-}
-// cap: the fraction of the increment the swept list covers (its CCD bound is a
-// fraction of that shorter step)
-__global__ void k_ls_init(int ns, const int* done, int* acc, double* alpha, const double* toi, int ccd, int* stall,
-                          double cap) {
-    GS_LOOP(s, ns) {
-        acc[s] = done[s];
-        alpha[s] = (ccd ? fmin(1.0, toi[s]) : 1.0) * cap;
-        if (!done[s]) stall[s] = 0;
-    }
-}
 // contact groups -> scenes: the smallest step length and CCD bound of the
 // scene's groups (for the profile and the step statistics); the scene
 // stalls when every group that searched gave up below ABD_LS_STALL_ALPHA
@@ -60,45 +33,6 @@ __global__ void k_grp_scene_stall(int ns, const int* done, const int* gact, cons
         stall[s] = gact[s] > 0 && gstall[s] == gact[s];
     }
 }
-// gauss_newton.py:107-113; an energy change within the FP64 evaluation
-// error of the two energies (N0 + N1) is no increase
-// one block: returns (to thread 0) the number of units still searching
-DV int ls_decide_block(int ns, int* acc, double* alpha, const double* E0, const double* E1, const double* N0,
-                       const double* N1, double min_alpha, int* stall) {
-    __shared__ int pending;
-    if (threadIdx.x == 0) pending = 0;
-    __syncthreads();
-    for (int s = threadIdx.x; s < ns; s += blockDim.x) {
-        if (acc[s]) continue;
-        if (E1[s] < E0[s] || E1[s] - E0[s] <= N0[s] + N1[s]) acc[s] = 1;
-        else if (alpha[s] * 0.5 < min_alpha) { acc[s] = 1; if (alpha[s] < ABD_LS_STALL_ALPHA) stall[s] = 1; }
-        else { alpha[s] *= 0.5; atomicAdd(&pending, 1); }
-    }
-    __syncthreads();
-    return pending;
-}
-__global__ void k_ls_decide(int ns, int* acc, double* alpha, const double* E0, const double* E1, const double* N0,
-                            const double* N1, double min_alpha, int* stall, Counters* cnt) {
-    int pending = ls_decide_block(ns, acc, alpha, E0, E1, N0, N1, min_alpha, stall);
-    if (threadIdx.x == 0) cnt->ls_pending = pending;
-}
-// the same decision inside the line-search graph: counts the trial and
-// keeps the graph's while-node running while units are pending, for at most
-// LS_MAX_TRIALS trials (the host loop's cap)
-constexpr int LS_MAX_TRIALS = 64;
-__global__ void k_ls_decide_graph(int ns, int* acc, double* alpha, const double* E0, const double* E1, const double* N0,
-                                  const double* N1, double min_alpha, int* stall, Counters* cnt,
-                                  cudaGraphConditionalHandle loop) {
-    int pending = ls_decide_block(ns, acc, alpha, E0, E1, N0, N1, min_alpha, stall);
-    if (threadIdx.x == 0) {
-        cnt->ls_pending = pending;
-        int t = cnt->ls_trials + 1;
-        cnt->ls_trials = t;
-        cudaGraphSetConditional(loop, (pending > 0 && t < LS_MAX_TRIALS) ? 1u : 0u);
-    }
-}
-__global__ void k_ls_graph_prep(Counters* cnt, int n_sw) { cnt->ls_trials = 0; cnt->ls_nsw = n_sw; }
-
 // Line-search graphs (ls_graph): one per unit kind (scenes, contact
 // groups), each a while-node whose body is one trial: apply the step
 // length, the energies of the listed step, the decision.  Every pointer in
@@ -107,7 +41,7 @@ __global__ void k_ls_graph_prep(Counters* cnt, int n_sw) { cnt->ls_trials = 0; c
 struct LsGraph {
     cudaGraph_t g = nullptr; cudaGraphExec_t x = nullptr;
     const void* sw = nullptr;       // swept list the body was captured with
-    int shapes[2] = {-2, -2};       // autotuner choice (list, body energy) it was captured with
+    int shape = -2;                 // autotuner choice it was captured with
     int body_launches = 0;          // kernels per trial
 };
 struct LsGraphState { LsGraph gr[2]; bool failed = false; };
@@ -118,7 +52,7 @@ void eng_lsgraph_free(Engine* E) {
     delete S;
     E->ls_graph_state = nullptr;
 }
-static int ls_graph_build(Engine* E, LsGraph& G, const LsUnits& U, const int* uacc, double* ualpha, int* ustall) {
+static int ls_graph_build(Engine* E, LsGraph& G, const LsUnits& U) {
     cudaStream_t s = E->stream;
     if (G.x) { cudaGraphExecDestroy(G.x); G.x = nullptr; }
     if (G.g) { cudaGraphDestroy(G.g); G.g = nullptr; }
@@ -135,23 +69,20 @@ static int ls_graph_build(Engine* E, LsGraph& G, const LsUnits& U, const int* ua
     cudaGraph_t body = cp.conditional.phGraph_out[0];
     const int l0 = E->launches;
     CUDA_TRY(cudaStreamBeginCaptureToGraph(s, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-    const AbdParams& P = E->P;
     E->capturing = true;
-    k_apply<<<grid_for(12L * E->nb), 256, 0, s>>>(E->nb, E->backup, E->du, ualpha, uacc, U.bunit, E->st);
-    int rc = eng_energy_list(E, U, SD_E1, uacc, true);
-    k_ls_decide_graph<<<1, 256, 0, s>>>(U.n, const_cast<int*>(uacc), ualpha, U.d + SD_E0 * U.n, U.d + SD_E1 * U.n,
-                                        U.d + SD_E0N * U.n, U.d + SD_E1N * U.n, P.ls_min_alpha, ustall, E->dcnt, h);
+    int rc = eng_ls_apply(E, U);
+    if (!rc) rc = eng_ls_energy(E, U, 2, h);
     E->capturing = false;
     cudaGraph_t captured = nullptr;
     cudaError_t ce = cudaStreamEndCapture(s, &captured);
-    G.body_launches = E->launches - l0 + 2;
+    G.body_launches = E->launches - l0;
     E->launches = l0;
     if (rc) return rc;
     CUDA_TRY(ce);
     CUDA_TRY(cudaGetLastError());
     CUDA_TRY(cudaGraphInstantiate(&G.x, G.g, 0));
     G.sw = E->sw;
-    G.shapes[0] = E->tune[TK_LIST_ENERGY].chosen; G.shapes[1] = E->tune[TK_BODY_ENERGY].chosen;
+    G.shape = E->tune[TK_LIST_ENERGY].chosen;
     return ABD_OK;
 }
 // the line search of one Newton iteration as one graph launch, not waited
@@ -159,8 +90,7 @@ static int ls_graph_build(Engine* E, LsGraph& G, const LsUnits& U, const int* ua
 // host sync that follows; *body_launches gets the kernels per trial.
 // Returns ABD_OK with *ran = 0 when the graph cannot be used (the caller then
 // runs the host loop).
-static int ls_graph_run(Engine* E, bool groups, const LsUnits& U, const int* uacc, double* ualpha, int* ustall,
-                        int* body_launches, int* ran) {
+static int ls_graph_run(Engine* E, bool groups, const LsUnits& U, int* body_launches, int* ran) {
     *ran = 0;
     if (!E->ls_graph_state) E->ls_graph_state = new LsGraphState();
     auto* S = reinterpret_cast<LsGraphState*>(E->ls_graph_state);
@@ -168,9 +98,8 @@ static int ls_graph_run(Engine* E, bool groups, const LsUnits& U, const int* uac
     LsGraph& G = S->gr[groups ? 1 : 0];
     // captured again when the swept list moved or the autotuner settled
     // on a launch shape after the capture
-    if (!G.x || G.sw != E->sw || G.shapes[0] != E->tune[TK_LIST_ENERGY].chosen ||
-        G.shapes[1] != E->tune[TK_BODY_ENERGY].chosen) {
-        if (ls_graph_build(E, G, U, uacc, ualpha, ustall)) {
+    if (!G.x || G.sw != E->sw || G.shape != E->tune[TK_LIST_ENERGY].chosen) {
+        if (ls_graph_build(E, G, U)) {
             // graphs unavailable: keep the host loop for this handle
             S->failed = true;
             cudaGetLastError();
@@ -178,7 +107,6 @@ static int ls_graph_run(Engine* E, bool groups, const LsUnits& U, const int* uac
             return ABD_OK;
         }
     }
-    k_ls_graph_prep<<<1, 1, 0, E->stream>>>(E->dcnt, E->n_sw);
     CUDA_TRY(cudaGraphLaunch(G.x, E->stream));
     E->launches += 1;
     *body_launches = G.body_launches;
@@ -295,17 +223,14 @@ int eng_step(Engine* E, int n_steps, AbdStepStats* stats) {
             // now + a ws, a = min(1, toi) halved until the energy is below
             // that of now (at most 7 halvings, else a = 0)
             if ((rc = eng_swept(E, E->ws, 1.0, done))) return rc;
-            if (P.ccd && (rc = eng_ccd_list(E, scene_units(E), done))) return rc;
             k_ws_to_du<<<grid_for(12L * E->nb), 256, 0, s>>>(E->nb, E->ws, E->mass, E->du);
-            k_backup<<<grid_for(12L * E->nb), 256, 0, s>>>(E->nb, E->st, E->backup);
-            k_ls_init<<<grid_for(ns), 256, 0, s>>>(ns, done, acc, alpha, E->scd + SD_TOI * ns, P.ccd, stall, E->sw_scale);
-            E->launches += 3;
-            if ((rc = eng_energy_list(E, scene_units(E), SD_E0, done))) return rc;
+            E->launches++;
+            const LsUnits U = scene_units(E);
+            if ((rc = eng_ls_begin(E, U, done))) return rc;
             for (int trial = 0;; trial++) {
-                k_apply<<<grid_for(12L * E->nb), 256, 0, s>>>(E->nb, E->backup, E->du, alpha, acc, E->bscene, E->st);
-                E->launches++;
+                if ((rc = eng_ls_apply(E, U))) return rc;
                 if (trial == 8) break;
-                if ((rc = eng_energy_list(E, scene_units(E), SD_E1, acc))) return rc;
+                if ((rc = eng_ls_energy(E, U, 0))) return rc;
                 k_ws_decide<<<1, 256, 0, s>>>(ns, acc, alpha, E->scd + SD_E0 * ns, E->scd + SD_E1 * ns, trial == 7, E->dcnt);
                 E->launches++;
                 if ((rc = eng_sync_counters(E))) return rc;
@@ -358,33 +283,25 @@ int eng_step(Engine* E, int n_steps, AbdStepStats* stats) {
             if (groups && !(E->grp && E->gscd && E->gsci)) return E->fail(ABD_ERR_CUDA, "contact groups not allocated");
             LsUnits U = groups ? group_units(E) : scene_units(E);
             const int* udone = U.i + SI_DONE * U.n;
-            int* uacc = U.i + SI_ACC * U.n;
             int* ustall = U.i + SI_STALL * U.n;
             double* ualpha = U.d + SD_ALPHA * U.n;
             if (!groups) udone = done;
-            if (P.ccd) {
-                int ph = phase_begin(E, PH_CCD); rc = eng_ccd_list(E, U, udone); phase_end(E, ph, 0);
-                if (rc) return rc;
-            }
-            // gauss_newton.py:98-115 line search
-            { int ph = phase_begin(E, PH_ENERGY); rc = eng_energy_list(E, U, SD_E0, udone); phase_end(E, ph, 0); if (rc) return rc; }
-            k_backup<<<grid_for(12L * E->nb), 256, 0, s>>>(E->nb, E->st, E->backup);
-            E->launches++;
-            k_ls_init<<<grid_for(U.n), 256, 0, s>>>(U.n, udone, uacc, ualpha, U.d + SD_TOI * U.n, P.ccd, ustall,
-                                                     E->sw_scale);
-            E->launches++;
+            // gauss_newton.py:98-115 line search, its CCD bound and start energy first
+            { int ph = phase_begin(E, PH_CCD); rc = eng_ls_begin(E, U, udone); phase_end(E, ph, 0); if (rc) return rc; }
             int ph_tr = phase_begin(E, PH_TRIALS);
             int graph_ran = 0, graph_body = 0;
             if (P.ls_graph) {
-                if ((rc = ls_graph_run(E, groups, U, uacc, ualpha, ustall, &graph_body, &graph_ran))) return rc;
+                if ((rc = ls_graph_run(E, groups, U, &graph_body, &graph_ran))) return rc;
                 if (graph_ran) st.ls_graph_launches++;
             }
             for (int trial = 0; trial < LS_MAX_TRIALS && !graph_ran; trial++) {
-                k_apply<<<grid_for(12L * E->nb), 256, 0, s>>>(E->nb, E->backup, E->du, ualpha, uacc, U.bunit, E->st);
-                { int ph = phase_begin(E, PH_ENERGY); rc = eng_energy_list(E, U, SD_E1, uacc); phase_end(E, ph, 0); if (rc) return rc; }
-                k_ls_decide<<<1, 256, 0, s>>>(U.n, uacc, ualpha, U.d + SD_E0 * U.n, U.d + SD_E1 * U.n, U.d + SD_E0N * U.n,
-                                              U.d + SD_E1N * U.n, P.ls_min_alpha, ustall, E->dcnt);
-                E->launches += 2;
+                if ((rc = eng_ls_apply(E, U))) return rc;
+                int ph = phase_begin(E, PH_ENERGY), pl = phase_begin(E, PH_ELIST);
+                rc = eng_ls_energy(E, U, 1);
+                // per listed pair: the entry, its 2-4 vertex ids and positions
+                phase_end(E, pl, E->n_sw * (16.0 + 16.0 + 4 * 24.0));
+                phase_end(E, ph, 0);
+                if (rc) return rc;
                 st.ls_trials++;
                 if ((rc = eng_sync_counters(E))) return rc;
                 if (E->hcnt->grp_fail) return E->fail(ABD_ERR_CUDA, "contact groups: union-find did not settle");

@@ -16,7 +16,7 @@
 // then evaluated over this list only.  The list is sorted by (kind, a, b),
 // so filtering it yields the same sorted candidate list as a fresh
 // detection.
-#include "contact.cuh"
+#include "energy.cuh"
 #include <cub/cub.cuh>
 
 Geo eng_geo(Engine* E);
@@ -263,65 +263,9 @@ int eng_swept(Engine* E, const double* dq, double sign, const int* done) {
     return ABD_OK;
 }
 
-// ------------------------------------------------------------------ CCD over the list
-__global__ void k_ccd_list(int n, const int4* __restrict__ list, Geo G, const double* __restrict__ p,
-                           const int* __restrict__ bscene, const int* __restrict__ skip, double s_ccd, int ccd_it,
-                           double* toi, int* capped) {
-    GS_LOOP(c, n) {
-        int4 C = list[c];
-        int v[4];
-        int kind;
-        if (C.x == ABD_CONTACT_EE) { int2 a = G.edges[C.y], b = G.edges[C.z]; v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y; kind = 0; }
-        else { v[0] = C.y; v[1] = G.tris[3*C.z]; v[2] = G.tris[3*C.z+1]; v[3] = G.tris[3*C.z+2]; kind = 1; }
-        int s = bscene[G.vbody[v[0]]];
-        if (skip[s]) continue;
-        double xx[12], pp[12];
-        for (int k = 0; k < 4; k++) for (int q = 0; q < 3; q++) { xx[3*k+q] = G.x[3*v[k]+q]; pp[3*k+q] = p[3*v[k]+q]; }
-        double t;
-        if (accd(kind, xx, pp, s_ccd, 1.0, &t, capped, ccd_it)) atomic_min_pos(toi + s, t);
-    }
-}
-// planes come from the vertex's scene; the bound goes to the unit of its body
-__global__ void k_ccd_pg2(int nv, Geo G, const double* __restrict__ p, const int* __restrict__ vscene,
-                          const int* __restrict__ bunit, double s_ccd, const int* skip, double* toi) {
-    GS_LOOP(v, nv) {
-        int s = vscene[v];
-        int u = bunit[G.vbody[v]];
-        if (skip[u]) continue;
-        double best = 1.0;
-        for (int pl = G.sc_plane_begin[s]; pl < G.sc_plane_begin[s+1]; pl++) {
-            const double* n = G.planes + 4*pl;
-            double d = n[0] * G.x[3*v] + n[1] * G.x[3*v+1] + n[2] * G.x[3*v+2] - n[3];
-            double vn = n[0] * p[3*v] + n[1] * p[3*v+1] + n[2] * p[3*v+2];
-            if (vn < 0) { double t = (1 - s_ccd) * d / (-vn); if (t < 0) t = 0; if (t < best) best = t; }
-        }
-        if (best < 1.0) atomic_min_pos(toi + u, best);
-    }
-}
-__global__ void k_fill1(double* a, int n, double v) { GS_LOOP(i, n) a[i] = v; }
-
-// per-unit (scene or contact group) largest conservative fraction of the
-// listed displacement (E->pv) into U's SD_TOI slots
-int eng_ccd_list(Engine* E, const LsUnits& U, const int* skip) {
-    cudaStream_t s = E->stream;
-    double* toi = U.d + SD_TOI * U.n;
-    k_fill1<<<grid_for(U.n), 256, 0, s>>>(toi, U.n, 1.0);
-    int rc = eng_transform(E);
-    if (rc) return rc;
-    Geo G = eng_geo(E);
-    if (E->n_sw > 0)
-        k_ccd_list<<<grid_for(E->n_sw, 64), 64, 0, s>>>(E->n_sw, E->sw, G, E->pv, U.bunit, skip, E->P.ccd_scale,
-                                                        ccd_iters(E->P), toi, &E->dcnt->ccd_capped);
-    if (E->npl > 0) k_ccd_pg2<<<grid_for(E->nv), 256, 0, s>>>(E->nv, G, E->pv, E->vscene, U.bunit, E->P.ccd_scale, skip, toi);
-    E->launches += 1 + (E->n_sw > 0) + (E->npl > 0);
-    return ABD_OK;
-}
-
-// ------------------------------------------------------------------ energy over the list
-__global__ void k_list_energy(int n, const int* __restrict__ n_dev, const int4* __restrict__ list, Geo G,
-                              const int* __restrict__ bscene, const int* __restrict__ skip, int f32, double dhat,
-                              int barrier, double sc, double* Eo, double* En) {
-    if (n_dev) n = *n_dev;
+// ------------------------------------------------------------------ energy over a candidate list
+__global__ void k_list_energy(int n, const int4* __restrict__ list, Geo G, const int* __restrict__ bscene,
+                              const int* __restrict__ skip, PairTerms T, double* Eo) {
     for (long base = (long)blockIdx.x * blockDim.x; base < n; base += (long)gridDim.x * blockDim.x) {
         long c = base + threadIdx.x;
         bool valid = c < n;
@@ -332,56 +276,14 @@ __global__ void k_list_energy(int n, const int* __restrict__ n_dev, const int4* 
             int v0 = C.x == ABD_CONTACT_EE ? G.edges[C.y].x : C.y;
             s = bscene[G.vbody[v0]];
             if (skip[s]) valid = false;
-            else {
-                int4 stv; int type; double xb;
-                if (classify(G, C.x, C.y, C.z, f32, dhat, stv, type, xb)) {
-                    double b0, b1, b2; barrier3(barrier, xb, dhat * dhat, b0, b1, b2);
-                    e = b0 * sc;
-                    int vs[4] = {stv.x, stv.y, stv.z, stv.w};
-                    double L = 0;
-#pragma unroll
-                    for (int k = 0; k < 4; k++)
-                        if (vs[k] >= 0)
-                            L = fmax(L, fmax(fabs(G.x[3*vs[k]]), fmax(fabs(G.x[3*vs[k]+1]), fabs(G.x[3*vs[k]+2]))));
-                    // FP32 distances carry 2^29 times the FP64 rounding
-                    en = contact_noise(sc, b0, b1, xb, L, (f32 && C.x == ABD_CONTACT_EE) ? 536870912.0 : 1.0) * DBL_EPSILON;
-                }
-            }
+            else pair_energy(G, C, T, e, en);
         }
         warp_reduce_add(Eo, s, e, valid);
-        if (En) warp_reduce_add(En, s, en, valid);
     }
 }
 
-int eng_body_energy(Engine* E, const int* bunit, double* Eo, double* En, const int* skip);
-int eng_pg_energy(Engine* E, const int* bunit, double* Eo, double* En, const int* skip);
-
-// energy per unit (scene or contact group) into U's slot and the scale of
-// its FP64 evaluation error into the noise slot (SD_E0 -> SD_E0N,
-// SD_E1 -> SD_E1N)
-int eng_energy_list(Engine* E, const LsUnits& U, int slot, const int* skip, bool dev_count) {
-    cudaStream_t s = E->stream;
-    const AbdParams& P = E->P;
-    double* Eo = U.d + slot * U.n;
-    double* En = U.d + (slot == SD_E0 ? SD_E0N : SD_E1N) * U.n;
-    CUDA_TRY(cudaMemsetAsync(Eo, 0, sizeof(double) * U.n, s));
-    CUDA_TRY(cudaMemsetAsync(En, 0, sizeof(double) * U.n, s));
-    int rc = eng_transform(E);
-    if (rc) return rc;
-    if ((rc = eng_body_energy(E, U.bunit, Eo, En, skip))) return rc;
-    if (E->n_sw > 0 || dev_count) {
-        int ph = phase_begin(E, PH_ELIST);
-        int tb = TUNE_THREADS[tune_begin(E, TK_LIST_ENERGY, 4, 1)];
-        const int grid = dev_count ? NUM_SMS * 4 : grid_for(E->n_sw, tb);
-        k_list_energy<<<grid, tb, 0, s>>>(E->n_sw, dev_count ? &E->dcnt->ls_nsw : nullptr, E->sw, eng_geo(E), U.bunit,
-                                          skip, P.ee_f32, P.dhat, P.barrier, P.kappa * P.dt * P.dt, Eo, En);
-        tune_end(E, TK_LIST_ENERGY);
-        // per listed pair: the entry, its 2-4 vertex ids and positions
-        phase_end(E, ph, E->n_sw * (16.0 + 16.0 + 4 * 24.0));
-        E->launches++;
-    }
-    return eng_pg_energy(E, U.bunit, Eo, En, skip);
-}
+int eng_body_energy(Engine* E, double* Eo, const int* skip);
+int eng_pg_energy(Engine* E, double* Eo, const int* skip);
 
 // energy per scene into scd[slot] over the candidate list of a detection that
 // has just run at the current positions (hcnt holds its counts)
@@ -390,17 +292,16 @@ int eng_energy_candidates(Engine* E, int slot, const int* skip) {
     const AbdParams& P = E->P;
     double* Eo = E->scd + slot * E->ns;
     CUDA_TRY(cudaMemsetAsync(Eo, 0, sizeof(double) * E->ns, s));
-    int rc = eng_body_energy(E, E->bscene, Eo, nullptr, skip);
+    int rc = eng_body_energy(E, Eo, skip);
     if (rc) return rc;
     const int n = E->hcnt->n_ee + E->hcnt->n_pt;
     if (n > 0) {
         int ph = phase_begin(E, PH_ELIST);
-        k_list_energy<<<grid_for(n, 128), 128, 0, s>>>(n, nullptr, E->contacts, eng_geo(E), E->bscene, skip, P.ee_f32, P.dhat,
-                                                      P.barrier, P.kappa * P.dt * P.dt, Eo, nullptr);
+        k_list_energy<<<grid_for(n, 128), 128, 0, s>>>(n, E->contacts, eng_geo(E), E->bscene, skip, pair_terms(P), Eo);
         phase_end(E, ph, n * (16.0 + 16.0 + 4 * 24.0));
         E->launches++;
     }
-    return eng_pg_energy(E, E->bscene, Eo, nullptr, skip);
+    return eng_pg_energy(E, Eo, skip);
 }
 
 // ------------------------------------------------------------------ detection from the list

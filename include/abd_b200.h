@@ -308,8 +308,8 @@ int abd_trainer_params(AbdTrainer* t, float* params);
 /* Launch shapes chosen by the autotuner (no reference counterpart): [0]
  * threads per block and [1] contacts per block of the contact assembly (one
  * warp per contact, or one block of 64 / 128 threads per contact), [2]
- * threads per block of the listed-pair energy, [3] of the body energy; -1
- * while still timing candidates.  *n gets the number of entries (4). */
+ * threads per block of the listed-pair energy, [3] of the body energy (one
+ * kernel evaluates both: the same value); -1 while still timing candidates.  *n gets the number of entries (4). */
 int abd_get_autotune(AbdHandle* h, int32_t* shapes, int32_t cap, int32_t* n);
 
 /* Number of edge-triangle intersections between different bodies at the
@@ -320,7 +320,7 @@ int abd_count_intersections(AbdHandle* h, int32_t* count);
  * step() in wp.ScopedTimer, abd.py:676).  When on, every phase launch is
  * bracketed by CUDA events on the handle's stream and summed per phase:
  *   0 detect (pair list)        1 assemble (all of it)    2 solve
- *   3 line-search energy        4 CCD                     5 other
+ *   3 energies of the trials    4 CCD and start energy    5 other
  *   6 contact-energy kernels    7 SpMV kernels            8 assembly: keys, sort, blocks
  *   9 assembly: bodies          10 assembly: contacts     11 assembly: block inverse
  *   12 dense factor + solve     13 swept candidate list   14 contact-energy list kernel

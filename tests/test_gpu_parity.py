@@ -279,3 +279,21 @@ def test_energy_over_candidates_equals_grid_query(which, chain_scene, chain_pair
         sc = dict(sc, state=st)
     e = [Engine(p(broadphase=b), sc).energy()[0] for b in (1, 2)]
     assert e[0] != 0.0 and e[1] == pytest.approx(e[0], rel=1e-11)
+
+
+@pytest.mark.parametrize("nu,nv,cand", [(3, 3, 0.3), (4, 8, 0.2), (11, 3, 0.2), (16, 8, 0.3), (24, 12, 0.4)])
+def test_body_pair_candidates_equal_grid_at_cluster_edges(nu, nv, cand):
+    """Bodies of 9 to 288 vertices (27 to 864 edges, 18 to 576 triangles: below,
+    at and above the 32-primitive clusters, with remainders) and lists from a
+    few hundred pairs to far above 16,384, where the ordering changes from
+    counting to the radix sort: the same sorted list as the hashed grid."""
+    V, F = S.torus_mesh(1.0, 0.25, nu, nv)
+    rng = np.random.default_rng(nu)
+    bodies = [S._body(V, F, 1000.0, rng.uniform(-0.6, 0.6, 3), S._rand_rotation(rng)) for _ in range(5)]
+    sc = S.assemble_bodies(bodies, planes=[[0.0, 1.0, 0.0, -1.5]])
+    got = []
+    for b in (1, 2):
+        quads, kinds = Engine(P.config_params(cand_dist=cand, broadphase=b), sc).pairs()
+        got.append((quads, kinds))
+    assert len(got[0][0]) > 0
+    assert np.array_equal(got[0][0], got[1][0]) and np.array_equal(got[0][1], got[1][1])

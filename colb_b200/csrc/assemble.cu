@@ -15,7 +15,7 @@
 // contact adds its four body blocks into that structure with FP64/FP32
 // atomics.
 #include "contact.cuh"
-#include "warp_eig.cuh"
+#include "contact_hess.cuh"
 #include <cub/cub.cuh>
 
 Geo eng_geo(Engine* E);
@@ -86,10 +86,10 @@ __global__ void __launch_bounds__(32 * BA_WARPS) k_body_assemble(int nb, const d
                                 const double* __restrict__ mass, const double* __restrict__ J, double dt, double g0,
                                 double g1, double g2, double k_ortho, int project, double pinned_diag,
                                 const int* __restrict__ row_ptr, const int* __restrict__ bcol, T* vals, double* grad) {
-    __shared__ WarpEigSmem sm[BA_WARPS];
+    __shared__ double sA[BA_WARPS][108];       // 9 x 9, leading dimension 12
     __shared__ double sq[BA_WARPS][9];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    WarpEigSmem& E = sm[w];
+    double* A = sA[w];
     for (int b = blockIdx.x * BA_WARPS + w; b < nb; b += gridDim.x * BA_WARPS) {
         int bi = find_block(row_ptr, bcol, b, b);
         if (bi < 0) continue;                              // every row holds its diagonal key
@@ -118,11 +118,11 @@ __global__ void __launch_bounds__(32 * BA_WARPS) k_body_assemble(int nb, const d
             g[lane] = dt * dt * (gi * 4.0 * k_ortho) + (q[r] - qt) * Jb;
         }
         if (project) {
-            ortho_hess_psd_warp(q, k_ortho * dt * dt, E.A, lane);    // analytic eigensystem
+            ortho_hess_psd_warp(q, k_ortho * dt * dt, A, lane);    // analytic eigensystem
         } else {
             for (int e = lane; e < 81; e += 32) {
                 int rr = e / 9, cc = e % 9;
-                E.A[rr*12 + cc] = ortho_hess(q, k_ortho, rr / 3, cc / 3, rr % 3, cc % 3) * dt * dt;
+                A[rr*12 + cc] = ortho_hess(q, k_ortho, rr / 3, cc / 3, rr % 3, cc % 3) * dt * dt;
             }
         }
         __syncwarp();
@@ -130,7 +130,7 @@ __global__ void __launch_bounds__(32 * BA_WARPS) k_body_assemble(int nb, const d
             int row = e % 12, col = e / 12;
             double v;
             if (row < 3 || col < 3) v = (row == col) ? m : 0.0;
-            else v = E.A[(row-3)*12 + (col-3)] + (row == col ? Jb : 0.0);
+            else v = A[(row-3)*12 + (col-3)] + (row == col ? Jb : 0.0);
             V[e] = (T)v;
         }
         __syncwarp();
@@ -138,363 +138,123 @@ __global__ void __launch_bounds__(32 * BA_WARPS) k_body_assemble(int nb, const d
 }
 
 // ---------------------------------------------------- contacts (abd.py:198-571)
-// One warp per active contact.  The stencil's squared-distance gradient and
-// Hessian are built lane-parallel in shared memory (auxiliary vectors by
-// lane 0, matrix entries by all lanes), chained through the barrier,
-// projected to PSD by the warp Jacobi (warp_eig.cuh), and scattered into the
-// body blocks: lanes own block entries, each summing the stencil vertices
-// that map to it through J = [1, xbar^T] (x) I3.
+// A warp takes `per` contacts.  First groups of 32 / per lanes form one
+// contact each: its stencil's five directions and its 5 x 5 matrix
+// (contact_hess.cuh, every lane of a group the same numbers, so there is
+// nothing to exchange).  Then the whole warp adds one contact after the other
+// to the body blocks: the directions map to body DoFs through
+// J = [1, xbar^T] (x) I3 as U_p, and block (a, b) is U_a M U_b^T.
+// The time is the latency of the eigenproblem's dependent rotations, so `per`
+// grows only once there are more contacts than warps that run at a time.
+// 147 contacts of the resting 16 x 16 net: 87 -> 28 us per launch against one
+// warp (or block) per contact with a 12 x 12 Jacobi over its lanes; 1,176
+// contacts of eight nets 114 -> 40 us.
+constexpr int CA_PER = 8;
 struct ContactSmem {
-    WarpEigSmem E;
-    double x[12], g[12], gy[9], aux[48], J[4][4];
-    double B0, B1, B2;
-    int v[4], vb[4], np, type, bodies[2], nbd;
+    double m[CA_PER][15], frame[CA_PER][9], w[CA_PER][12], gd[CA_PER], J[4][4];
+    int v[CA_PER][4], type[CA_PER];
+    double U[2][5][12], Z[2][5][12];
 };
 
-// C[point][aux] maps for the (w, u, v) and (w, e) parameterisations
-__constant__ signed char c_map_ee[4][3] = {{1, -1, 0}, {0, 1, 0}, {-1, 0, -1}, {0, 0, 1}};
-__constant__ signed char c_map_pt[4][3] = {{1, 0, 0}, {-1, -1, -1}, {0, 1, 0}, {0, 0, 1}};
-__constant__ signed char c_map_pe[3][2] = {{1, 0}, {-1, -1}, {0, 1}};
-
-DV void skew9(const double* a, double* S) {
-    S[0] = 0; S[1] = -a[2]; S[2] = a[1]; S[3] = a[2]; S[4] = 0; S[5] = -a[0]; S[6] = -a[1]; S[7] = a[0]; S[8] = 0;
-}
-DV void cross3(const double* a, const double* b, double* o) {
-    o[0] = a[1]*b[2] - a[2]*b[1]; o[1] = a[2]*b[0] - a[0]*b[2]; o[2] = a[0]*b[1] - a[1]*b[0];
-}
-
-// squared distance gradient (C.g) and Hessian (C.E.A, ld 12) of the stencil
-DV void warp_distance_derivs(ContactSmem& C, const Geo& G) {
-    const int lane = threadIdx.x & 31;
-    const int m = 3 * C.np;
-    double* A = C.E.A; double* Hy = C.E.T;
-    if (C.type == T_PG) {
-        if (lane == 0) {
-            const double* nn = G.planes + 4 * C.v[1];
-            double d = nn[0] * C.x[0] + nn[1] * C.x[1] + nn[2] * C.x[2] - nn[3];
-            for (int k = 0; k < 3; k++) { C.g[k] = 2 * d * nn[k]; C.aux[k] = nn[k]; }
-        }
-        __syncwarp();
-        if (lane < 9) A[(lane / 3) * 12 + lane % 3] = 2 * C.aux[lane / 3] * C.aux[lane % 3];
-    } else if (C.type == T_PP) {
-        if (lane < 6) { int k = lane % 3; double d = C.x[k] - C.x[3 + k]; C.g[lane] = lane < 3 ? 2 * d : -2 * d; }
-        for (int e = lane; e < 36; e += 32) {
-            int i = e / 6, j = e % 6;
-            A[i*12+j] = (i % 3 == j % 3) ? ((i < 3) == (j < 3) ? 2.0 : -2.0) : 0.0;
-        }
-    } else if (C.type == T_PE) {
-        // w = p - e0, e = e1 - e0, f = w.w - (w.e)^2/(e.e)
-        if (lane == 0) {
-            double w[3], e[3];
-            for (int k = 0; k < 3; k++) { w[k] = C.x[k] - C.x[3+k]; e[k] = C.x[6+k] - C.x[3+k]; }
-            double c = w[0]*e[0] + w[1]*e[1] + w[2]*e[2], s2 = e[0]*e[0] + e[1]*e[1] + e[2]*e[2], is = 1.0 / s2;
-            for (int k = 0; k < 3; k++) {
-                C.aux[k] = w[k]; C.aux[3+k] = e[k];
-                C.gy[k] = 2*w[k] - 2*c*is*e[k];
-                C.gy[3+k] = -2*c*is*w[k] + 2*c*c*is*is*e[k];
-            }
-            C.aux[6] = c; C.aux[7] = is;
-        }
-        __syncwarp();
-        const double* W = C.aux; const double* Ev = C.aux + 3;
-        double c = C.aux[6], is = C.aux[7];
-        for (int e = lane; e < 36; e += 32) {
-            int i = e / 6, j = e % 6, bi = i / 3, bj = j / 3, r = i % 3, q = j % 3;
-            double I = (r == q) ? 1.0 : 0.0, h;
-            if (bi == 0 && bj == 0) h = 2*I - 2*is*Ev[r]*Ev[q];
-            else if (bi == 0 && bj == 1) h = -2*is*Ev[r]*W[q] - 2*c*is*I + 4*c*is*is*Ev[r]*Ev[q];
-            else if (bi == 1 && bj == 0) h = -2*is*Ev[q]*W[r] - 2*c*is*I + 4*c*is*is*Ev[q]*Ev[r];
-            else h = -2*is*W[r]*W[q] + 4*c*is*is*(W[r]*Ev[q] + Ev[r]*W[q]) - 8*c*c*is*is*is*Ev[r]*Ev[q] + 2*c*c*is*is*I;
-            Hy[i*6+j] = h;
-        }
-        __syncwarp();
-        if (lane < 9) {
-            int pnt = lane / 3, k = lane % 3;
-            C.g[lane] = c_map_pe[pnt][0] * C.gy[k] + c_map_pe[pnt][1] * C.gy[3+k];
-        }
-        for (int e = lane; e < 81; e += 32) {
-            int i = e / 9, j = e % 9, pi = i / 3, pj = j / 3, r = i % 3, q = j % 3;
-            double acc = 0;
-            for (int a = 0; a < 2; a++) if (c_map_pe[pi][a])
-                for (int b = 0; b < 2; b++) if (c_map_pe[pj][b])
-                    acc += c_map_pe[pi][a] * c_map_pe[pj][b] * Hy[(3*a+r)*6 + 3*b+q];
-            A[i*12+j] = acc;
-        }
-    } else {
-        // f = (w.n)^2/(n.n), n = u x v; EE: w = a0-b0, u = a1-a0, v = b1-b0;
-        // PT: w = p-t0, u = t1-t0, v = t2-t0
-        if (lane == 0) {
-            double w[3], u[3], v[3];
-            for (int k = 0; k < 3; k++) {
-                if (C.type == T_EE) { w[k] = C.x[k] - C.x[6+k]; u[k] = C.x[3+k] - C.x[k]; v[k] = C.x[9+k] - C.x[6+k]; }
-                else { w[k] = C.x[k] - C.x[3+k]; u[k] = C.x[6+k] - C.x[3+k]; v[k] = C.x[9+k] - C.x[3+k]; }
-            }
-            double n[3]; cross3(u, v, n);
-            double a = w[0]*n[0] + w[1]*n[1] + w[2]*n[2], b = n[0]*n[0] + n[1]*n[1] + n[2]*n[2], ib = 1.0 / b;
-            double vw[3], wu[3], vn[3], nu[3];
-            cross3(v, w, vw); cross3(w, u, wu); cross3(v, n, vn); cross3(n, u, nu);
-            double* ga = C.aux; double* gb = C.aux + 9;
-            for (int k = 0; k < 3; k++) {
-                ga[k] = n[k]; ga[3+k] = vw[k]; ga[6+k] = wu[k];
-                gb[k] = 0; gb[3+k] = 2*vn[k]; gb[6+k] = 2*nu[k];
-            }
-            skew9(u, C.aux + 18); skew9(v, C.aux + 27); skew9(w, C.aux + 36);
-            double Sn[9]; skew9(n, Sn);
-            // Sn is needed only in the (u,v) blocks: keep it in gy's slot after gy is consumed
-            for (int i = 0; i < 9; i++) C.gy[i] = 2*a*ib*ga[i] - a*a*ib*ib*gb[i];
-            C.aux[45] = a; C.aux[46] = ib;
-            for (int i = 0; i < 9; i++) C.E.V[i] = Sn[i];          // V is free until the projection
-        }
-        __syncwarp();
-        const double* ga = C.aux; const double* gb = C.aux + 9;
-        const double* Su = C.aux + 18; const double* Sv = C.aux + 27; const double* Sw = C.aux + 36;
-        const double* Sn = C.E.V;
-        double a = C.aux[45], ib = C.aux[46];
-        double c1 = 2*ib, c2 = 2*a*ib, c3 = 2*a*ib*ib, c4 = 2*a*a*ib*ib*ib, c5 = a*a*ib*ib;
-        for (int e = lane; e < 81; e += 32) {
-            int i = e / 9, j = e % 9, bi = i / 3, bj = j / 3, r = i % 3, c = j % 3;
-            double ha = 0, hb = 0;
-            if (bi == 0 && bj == 1) ha = -Sv[3*r+c];
-            else if (bi == 1 && bj == 0) ha = -Sv[3*c+r];
-            else if (bi == 0 && bj == 2) ha = Su[3*r+c];
-            else if (bi == 2 && bj == 0) ha = Su[3*c+r];
-            else if (bi == 1 && bj == 2) ha = -Sw[3*r+c];
-            else if (bi == 2 && bj == 1) ha = -Sw[3*c+r];
-            if (bi == 1 && bj == 1) { double t = 0; for (int q = 0; q < 3; q++) t += Sv[3*q+r] * Sv[3*q+c]; hb = 2*t; }
-            else if (bi == 1 && bj == 2) { double t = 0; for (int q = 0; q < 3; q++) t += Sv[3*r+q] * Su[3*q+c]; hb = 2*t - 2*Sn[3*r+c]; }
-            else if (bi == 2 && bj == 1) { double t = 0; for (int q = 0; q < 3; q++) t += Su[3*r+q] * Sv[3*q+c]; hb = 2*t + 2*Sn[3*r+c]; }
-            else if (bi == 2 && bj == 2) { double t = 0; for (int q = 0; q < 3; q++) t += Su[3*q+r] * Su[3*q+c]; hb = 2*t; }
-            Hy[i*9+j] = c1*ga[i]*ga[j] + c2*ha - c3*(ga[i]*gb[j] + gb[i]*ga[j]) + c4*gb[i]*gb[j] - c5*hb;
-        }
-        __syncwarp();
-        const signed char (*Cm)[3] = C.type == T_EE ? c_map_ee : c_map_pt;
-        if (lane < 12) {
-            int pnt = lane / 3, k = lane % 3;
-            double acc = 0;
-            for (int q = 0; q < 3; q++) acc += Cm[pnt][q] * C.gy[3*q+k];
-            C.g[lane] = acc;
-        }
-        for (int e = lane; e < 144; e += 32) {
-            int i = e / 12, j = e % 12, pi = i / 3, pj = j / 3, r = i % 3, q = j % 3;
-            double acc = 0;
-            for (int aa = 0; aa < 3; aa++) if (Cm[pi][aa])
-                for (int bb = 0; bb < 3; bb++) if (Cm[pj][bb])
-                    acc += Cm[pi][aa] * Cm[pj][bb] * Hy[(3*aa+r)*9 + 3*bb+q];
-            A[i*12+j] = acc;
-        }
-    }
-    (void)m;
-    __syncwarp();
-}
-
 template <class T, int CAW>
-__global__ void __launch_bounds__(32 * CAW, 1) k_contact_assemble(const Counters* cnt, const int4* __restrict__ cst,
+__global__ void __launch_bounds__(32 * CAW) k_contact_assemble(const Counters* cnt, const int4* __restrict__ cst,
                                    const int* __restrict__ ctype, const double* __restrict__ cxb, Geo G, int barrier,
-                                   double dhat, double sc, int hess_mode, const int* __restrict__ row_ptr,
+                                   double dhat, double sc, int hess_mode, int per, const int* __restrict__ row_ptr,
                                    const int* __restrict__ bcol, T* vals, double* grad) {
     __shared__ ContactSmem sm[CAW];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     ContactSmem& C = sm[w];
     const int n = cnt->n_total;
-    for (int c = blockIdx.x * CAW + w; c < n; c += gridDim.x * CAW) {
-        int type = ctype[c];
-        if (type < 0) continue;                       // warp-uniform
-        if (lane == 0) {
-            int4 s4 = cst[c];
-            int sv[4] = {s4.x, s4.y, s4.z, s4.w};
-            C.type = type;
-            C.np = stencil_np(type);
-            for (int i = 0; i < 4; i++) C.v[i] = sv[i];
-            int nx = type == T_PG ? 1 : C.np;
-            for (int i = 0; i < nx; i++) {
-                int v = sv[i];
-                for (int k = 0; k < 3; k++) C.x[3*i+k] = G.x[3*v+k];
-                C.vb[i] = G.vbody[v];
-                C.J[i][0] = 1.0; C.J[i][1] = G.xbar[3*v]; C.J[i][2] = G.xbar[3*v+1]; C.J[i][3] = G.xbar[3*v+2];
+    for (int base = (blockIdx.x * CAW + w) * per; base < n; base += gridDim.x * CAW * per) {
+        const int span = 32 / per, mine = lane / span, c = base + mine;
+        int type = -1;
+        if (mine < per && c < n) type = ctype[c];
+        if (type >= 0) {
+            const int4 s4 = cst[c];
+            const int sv[4] = {s4.x, s4.y, s4.z, s4.w};
+            const int np = stencil_np(type);
+            d3 x[4];
+#pragma unroll
+            for (int i = 0; i < 4; i++) x[i] = i < np ? ld3(G.x + 3L * sv[i]) : mk3(0, 0, 0);
+            Stencil5 S;
+            stencil_hessian(type, x, type == T_PG ? G.planes + 4L * sv[1] : nullptr, S);
+            double B0, B1, B2;
+            barrier3(barrier, cxb[c], dhat * dhat, B0, B1, B2);
+            contact_matrix5(type, hess_mode == ABD_HESS_PROJECTED, B1, B2, S);
+            if (lane % span == 0) {
+#pragma unroll
+                for (int i = 0; i < 15; i++) C.m[mine][i] = S.a[i] * sc;
+#pragma unroll
+                for (int i = 0; i < 3; i++) { C.frame[mine][i] = S.n[i]; C.frame[mine][3 + i] = S.e1[i]; C.frame[mine][6 + i] = S.e2[i]; }
+#pragma unroll
+                for (int i = 0; i < 4; i++) { C.w[mine][i] = S.c[i]; C.w[mine][4 + i] = S.b2[i]; C.w[mine][8 + i] = S.b3[i]; C.v[mine][i] = sv[i]; }
+                C.gd[mine] = 2.0 * S.d * S.cn * B1 * sc;
             }
-            barrier3(barrier, cxb[c], dhat * dhat, C.B0, C.B1, C.B2);
-            C.bodies[0] = C.vb[0]; C.nbd = 1;
-            for (int i = 1; i < C.np; i++) if (C.vb[i] != C.bodies[0]) { C.bodies[1] = C.vb[i]; C.nbd = 2; break; }
         }
+        if (mine < per && lane % span == 0) C.type[mine] = type;
         __syncwarp();
-        warp_distance_derivs(C, G);
-        const int np = C.np, m = 3 * np;
-        const double B1 = C.B1, B2 = C.B2;
-        double* A = C.E.A;
-        if (hess_mode == ABD_HESS_REFERENCE) {
-            if (C.type == T_EE) team_psd_project_fast<32>(C.E, 12);      // abd.py:247
-            for (int e = lane; e < m * m; e += 32) {
-                int i = e / m, j = e % m;
-                double h = (C.type == T_PP) ? 0.0 : B1 * A[i*12+j];       // abd.py:381-382
-                A[i*12+j] = (h + B2 * C.g[i] * C.g[j]) * sc;
+        for (int q = 0; q < per; q++) {
+            const int tq = C.type[q];
+            if (tq < 0) continue;                         // warp-uniform
+            const int np = stencil_np(tq);
+            // bodies of the (at most two) sides
+            int vb[4];
+#pragma unroll
+            for (int i = 0; i < 4; i++) vb[i] = i < np ? G.vbody[C.v[q][i]] : -1;
+            int ba = vb[0], bb = -1;
+#pragma unroll
+            for (int i = 3; i > 0; i--) if (i < np && vb[i] != ba) bb = vb[i];
+            const bool da = G.mass[ba] > 0.0, db = bb >= 0 && G.mass[bb] > 0.0;
+            if (lane < 16) {
+                const int i = lane >> 2, k = lane & 3;
+                C.J[i][k] = i < np ? (k == 0 ? 1.0 : G.xbar[3L * C.v[q][i] + k - 1]) : 0.0;
             }
             __syncwarp();
-        } else if (C.type == T_PG || C.type == T_PP) {
-            // analytic projection.  With d the separation (g = 2d on the first
-            // point), B1 H + B2 g g^T is [M] (point-plane, d along the normal)
-            // or [M -M; -M M] (point-point) with M = 2 B1 I + 4 B2 d d^T for
-            // point-point and M = (2 B1 + 4 B2 d^2) n n^T for point-plane; the
-            // projection clamps M's eigenvalues 2 B1 (across d) and
-            // 2 B1 + 4 B2 |d|^2 (along d) at zero.
-            const double dx = 0.5 * C.g[0], dy = 0.5 * C.g[1], dz = 0.5 * C.g[2];
-            const double dd = dx * dx + dy * dy + dz * dz;
-            const double lam_t = C.type == T_PP ? fmax(2.0 * B1, 0.0) : 0.0;
-            const double lam_n = fmax(2.0 * B1 + 4.0 * B2 * dd, 0.0);
-            const double dv[3] = {dx, dy, dz};
-            for (int e = lane; e < m * m; e += 32) {
-                int i = e / m, j = e % m, a = i % 3, b = j % 3;
-                double nn = dd > 0.0 ? dv[a] * dv[b] / dd : 0.0;
-                double Mab = lam_t * ((a == b ? 1.0 : 0.0) - nn) + lam_n * nn;
-                A[i*12+j] = ((i / 3) == (j / 3) ? Mab : -Mab) * sc;
+            // U_p of both bodies, and Z = M U
+            if (lane < 24) {
+                const int side = lane / 12, row = lane % 12, al = row / 3, r = row % 3, body = side ? bb : ba;
+                double sc_ = 0, s2 = 0, s3 = 0;
+#pragma unroll
+                for (int i = 0; i < 4; i++) if (i < np && vb[i] == body) {
+                    sc_ += C.J[i][al] * C.w[q][i]; s2 += C.J[i][al] * C.w[q][4 + i]; s3 += C.J[i][al] * C.w[q][8 + i];
+                }
+                const double u[5] = {sc_ * C.frame[q][r], s2 * C.frame[q][r], s3 * C.frame[q][r], sc_ * C.frame[q][3 + r], sc_ * C.frame[q][6 + r]};
+#pragma unroll
+                for (int p = 0; p < 5; p++) {
+                    double z = 0;
+#pragma unroll
+                    for (int k = 0; k < 5; k++) z += C.m[q][s5(p, k)] * u[k];
+                    C.U[side][p][row] = u[p]; C.Z[side][p][row] = z;
+                }
+                // gradient: 2 d |c| B1 along the first direction
+                if (side ? db : da) atomicAdd(grad + 12L * body + row, C.gd[q] * u[0]);
+            }
+            // the four blocks' places, one lane each
+            int at = -1;
+            if (lane < 4) {
+                const int pa = lane >> 1, pb = lane & 1;
+                if ((pa ? db : da) && (pb ? db : da)) at = find_block(row_ptr, bcol, pa ? bb : ba, pb ? bb : ba);
             }
             __syncwarp();
-        } else {
-            for (int e = lane; e < m * m; e += 32) {
-                int i = e / m, j = e % m;
-                A[i*12+j] = B1 * A[i*12+j] + B2 * C.g[i] * C.g[j];
-            }
-            __syncwarp();
-            team_psd_project_fast<32>(C.E, m);
-            for (int e = lane; e < m * m; e += 32) { int i = e / m, j = e % m; A[i*12+j] *= sc; }
-            __syncwarp();
-        }
-        // gradient: G[b][3 al + k] += J_i[al] g_i[k] * B1 * sc for dynamic bodies
-        for (int e = lane; e < np * 12; e += 32) {
-            int i = e / 12, al = (e % 12) / 3, k = e % 3;
-            int b = C.vb[i];
-            if (G.mass[b] > 0.0) atomicAdd(grad + 12L * b + 3 * al + k, C.J[i][al] * C.g[3*i+k] * B1 * sc);
-        }
-        // Hessian blocks of the (at most two) bodies
-        for (int pa = 0; pa < C.nbd; pa++)
-            for (int pb = 0; pb < C.nbd; pb++) {
-                int Ba = C.bodies[pa], Bb = C.bodies[pb];
-                if (!(G.mass[Ba] > 0.0) || !(G.mass[Bb] > 0.0)) continue;
-                int bi = find_block(row_ptr, bcol, Ba, Bb);
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const int bi = __shfl_sync(0xffffffffu, at, k);
                 if (bi < 0) continue;
+                const double (*U)[12] = C.U[k >> 1];
+                const double (*Z)[12] = C.Z[k & 1];
                 T* V = vals + (long)bi * 144;
                 for (int e = lane; e < 144; e += 32) {
-                    int row = e % 12, col = e / 12;          // column-major block entry (row, col)
-                    int al = row / 3, r = row % 3, be = col / 3, q = col % 3;
+                    const int row = e % 12, col = e / 12;          // column-major block entry (row, col)
                     double sum = 0;
-                    for (int i = 0; i < np; i++) {
-                        if (C.vb[i] != Ba) continue;
-                        for (int j = 0; j < np; j++) {
-                            if (C.vb[j] != Bb) continue;
-                            sum += C.J[i][al] * C.J[j][be] * A[(3*i+r)*12 + 3*j+q];
-                        }
-                    }
+#pragma unroll
+                    for (int p = 0; p < 5; p++) sum += U[p][row] * Z[p][col];
                     if (sum != 0.0) atomicAdd(V + e, (T)sum);
                 }
             }
-        __syncwarp();
+            __syncwarp();
+        }
     }
 }
-
-// One block of NT threads per active contact: the same work as
-// k_contact_assemble, with the PSD projection spread over the whole block.
-template <class T, int NT>
-__global__ void __launch_bounds__(NT, 1) k_contact_assemble_team(const Counters* cnt, const int4* __restrict__ cst,
-                                   const int* __restrict__ ctype, const double* __restrict__ cxb, Geo G, int barrier,
-                                   double dhat, double sc, int hess_mode, const int* __restrict__ row_ptr,
-                                   const int* __restrict__ bcol, T* vals, double* grad) {
-    __shared__ ContactSmem C;
-    const int tid = threadIdx.x, warp = threadIdx.x >> 5;
-    const int n = cnt->n_total;
-    for (int c = blockIdx.x; c < n; c += gridDim.x) {
-        int type = ctype[c];
-        if (type < 0) continue;                       // block-uniform
-        if (tid == 0) {
-            int4 s4 = cst[c];
-            int sv[4] = {s4.x, s4.y, s4.z, s4.w};
-            C.type = type;
-            C.np = stencil_np(type);
-            for (int i = 0; i < 4; i++) C.v[i] = sv[i];
-            int nx = type == T_PG ? 1 : C.np;
-            for (int i = 0; i < nx; i++) {
-                int v = sv[i];
-                for (int k = 0; k < 3; k++) C.x[3*i+k] = G.x[3*v+k];
-                C.vb[i] = G.vbody[v];
-                C.J[i][0] = 1.0; C.J[i][1] = G.xbar[3*v]; C.J[i][2] = G.xbar[3*v+1]; C.J[i][3] = G.xbar[3*v+2];
-            }
-            barrier3(barrier, cxb[c], dhat * dhat, C.B0, C.B1, C.B2);
-            C.bodies[0] = C.vb[0]; C.nbd = 1;
-            for (int i = 1; i < C.np; i++) if (C.vb[i] != C.bodies[0]) { C.bodies[1] = C.vb[i]; C.nbd = 2; break; }
-        }
-        __syncthreads();
-        if (warp == 0) warp_distance_derivs(C, G);
-        __syncthreads();
-        const int np = C.np, m = 3 * np;
-        const double B1 = C.B1, B2 = C.B2;
-        double* A = C.E.A;
-        if (hess_mode == ABD_HESS_REFERENCE) {
-            if (C.type == T_EE) team_psd_project_fast<NT>(C.E, 12);          // abd.py:247
-            for (int e = tid; e < m * m; e += NT) {
-                int i = e / m, j = e % m;
-                double h = (C.type == T_PP) ? 0.0 : B1 * A[i*12+j];       // abd.py:381-382
-                A[i*12+j] = (h + B2 * C.g[i] * C.g[j]) * sc;
-            }
-            __syncthreads();
-        } else if (C.type == T_PG || C.type == T_PP) {
-            // analytic projection.  With d the separation (g = 2d on the first
-            // point), B1 H + B2 g g^T is [M] (point-plane, d along the normal)
-            // or [M -M; -M M] (point-point) with M = 2 B1 I + 4 B2 d d^T for
-            // point-point and M = (2 B1 + 4 B2 d^2) n n^T for point-plane; the
-            // projection clamps M's eigenvalues 2 B1 (across d) and
-            // 2 B1 + 4 B2 |d|^2 (along d) at zero.
-            const double dx = 0.5 * C.g[0], dy = 0.5 * C.g[1], dz = 0.5 * C.g[2];
-            const double dd = dx * dx + dy * dy + dz * dz;
-            const double lam_t = C.type == T_PP ? fmax(2.0 * B1, 0.0) : 0.0;
-            const double lam_n = fmax(2.0 * B1 + 4.0 * B2 * dd, 0.0);
-            const double dv[3] = {dx, dy, dz};
-            for (int e = tid; e < m * m; e += NT) {
-                int i = e / m, j = e % m, a = i % 3, b = j % 3;
-                double nn = dd > 0.0 ? dv[a] * dv[b] / dd : 0.0;
-                double Mab = lam_t * ((a == b ? 1.0 : 0.0) - nn) + lam_n * nn;
-                A[i*12+j] = ((i / 3) == (j / 3) ? Mab : -Mab) * sc;
-            }
-            __syncthreads();
-        } else {
-            for (int e = tid; e < m * m; e += NT) {
-                int i = e / m, j = e % m;
-                A[i*12+j] = B1 * A[i*12+j] + B2 * C.g[i] * C.g[j];
-            }
-            __syncthreads();
-            team_psd_project_fast<NT>(C.E, m);
-            for (int e = tid; e < m * m; e += NT) { int i = e / m, j = e % m; A[i*12+j] *= sc; }
-            __syncthreads();
-        }
-        // gradient: G[b][3 al + k] += J_i[al] g_i[k] * B1 * sc for dynamic bodies
-        for (int e = tid; e < np * 12; e += NT) {
-            int i = e / 12, al = (e % 12) / 3, k = e % 3;
-            int b = C.vb[i];
-            if (G.mass[b] > 0.0) atomicAdd(grad + 12L * b + 3 * al + k, C.J[i][al] * C.g[3*i+k] * B1 * sc);
-        }
-        // Hessian blocks of the (at most two) bodies
-        for (int pa = 0; pa < C.nbd; pa++)
-            for (int pb = 0; pb < C.nbd; pb++) {
-                int Ba = C.bodies[pa], Bb = C.bodies[pb];
-                if (!(G.mass[Ba] > 0.0) || !(G.mass[Bb] > 0.0)) continue;
-                int bi = find_block(row_ptr, bcol, Ba, Bb);
-                if (bi < 0) continue;
-                T* V = vals + (long)bi * 144;
-                for (int e = tid; e < 144; e += NT) {
-                    int row = e % 12, col = e / 12;          // column-major block entry (row, col)
-                    int al = row / 3, r = row % 3, be = col / 3, q = col % 3;
-                    double sum = 0;
-                    for (int i = 0; i < np; i++) {
-                        if (C.vb[i] != Ba) continue;
-                        for (int j = 0; j < np; j++) {
-                            if (C.vb[j] != Bb) continue;
-                            sum += C.J[i][al] * C.J[j][be] * A[(3*i+r)*12 + 3*j+q];
-                        }
-                    }
-                    if (sum != 0.0) atomicAdd(V + e, (T)sum);
-                }
-            }
-        __syncthreads();
-    }
-}
-
 
 // ---------------------------------------------------- block-Jacobi inverse
 // One warp per body: Gauss-Jordan with partial pivoting on [D | I] in shared
@@ -587,21 +347,20 @@ int eng_sync_counters(Engine* E) {
 
 int eng_grow_blocks(Engine* E, int need);
 
-// the contact assembly with the autotuned launch shape: one warp per
-// contact (2, 4 or 8 contacts per block) or one block of 64 / 128 threads per
-// contact
+// the contact assembly with the autotuned launch shape: 2, 4 or 8 warps per
+// block, one contact per warp until every scheduler of the GPU has a warp
 template <class T>
 static void launch_contact_assemble(Engine* E, int n, Geo G, double sc, T* V) {
     const AbdParams& P = E->P;
     cudaStream_t s = E->stream;
-    int c = tune_begin(E, TK_CONTACT, 5, 1);
-    const int threads = TUNE_CONTACT_THREADS[c], per_block = TUNE_CONTACT_PER_BLOCK[c];
-    dim3 block(threads), grid(grid_for((long)n, per_block));
-#define CA_ARGS E->dcnt, E->cst, E->ctype, E->cxb, G, P.barrier, P.dhat, sc, P.hess_mode, E->row_ptr, E->bcol, V, E->g
+    int c = tune_begin(E, TK_CONTACT, 3, 1);
+    const int threads = TUNE_CONTACT_THREADS[c], warps = TUNE_CONTACT_PER_BLOCK[c];
+    int per = 1;
+    while (per < CA_PER && (long)per * NUM_SMS * 4 < n) per *= 2;
+    dim3 block(threads), grid(grid_for((long)n, warps * per));
+#define CA_ARGS E->dcnt, E->cst, E->ctype, E->cxb, G, P.barrier, P.dhat, sc, P.hess_mode, per, E->row_ptr, E->bcol, V, E->g
     if (c == 0) k_contact_assemble<T, 2><<<grid, block, 0, s>>>(CA_ARGS);
     else if (c == 2) k_contact_assemble<T, 8><<<grid, block, 0, s>>>(CA_ARGS);
-    else if (c == 3) k_contact_assemble_team<T, 64><<<grid, block, 0, s>>>(CA_ARGS);
-    else if (c == 4) k_contact_assemble_team<T, 128><<<grid, block, 0, s>>>(CA_ARGS);
     else k_contact_assemble<T, 4><<<grid, block, 0, s>>>(CA_ARGS);
 #undef CA_ARGS
     tune_end(E, TK_CONTACT);

@@ -1,5 +1,7 @@
 // warp_eig.cuh — one warp projects a small symmetric matrix (n <= 12) held
-// in shared memory onto the PSD cone: V max(L, 0) V^T.
+// in shared memory onto the PSD cone: V max(L, 0) V^T.  The contact assembly
+// takes the 5 x 5 form of contact_hess.cuh; this general one is what the CPU
+// test checks projections against.
 //
 // Parallel cyclic Jacobi with round-robin ("tournament") pair ordering:
 // each round rotates n/2 disjoint index pairs at once, so for a product R of

@@ -307,7 +307,7 @@ int abd_trainer_params(AbdTrainer* t, float* params);
 
 /* Launch shapes chosen by the autotuner (no reference counterpart): [0]
  * threads per block and [1] contacts per block of the contact assembly (one
- * warp per contact, or one block of 64 / 128 threads per contact), [2]
+ * contact per warp; more per warp when there are more contacts than warps), [2]
  * threads per block of the listed-pair energy, [3] of the body energy (one
  * kernel evaluates both: the same value); -1 while still timing candidates.  *n gets the number of entries (4). */
 int abd_get_autotune(AbdHandle* h, int32_t* shapes, int32_t cap, int32_t* n);

@@ -6,17 +6,18 @@
 // edges are the off-diagonal 12x12 blocks (two dynamic bodies joined by an
 // active contact).  A component is factored on its own:
 //   - one body: the 12x12 block inverse written by the assembly;
-//   - FP64, Hessian projected to PSD and, in reverse Cuthill-McKee order, a
-//     body bandwidth of at most BAND_MAX: one CTA per component runs a banded
-//     block Cholesky with a sliding window in shared memory, all such
-//     components in one launch;
+//   - Hessian projected to PSD and, in reverse Cuthill-McKee order, a body
+//     bandwidth of at most BAND_WIDE: a banded L D L^T with the active window in
+//     registers, all such components of bandwidth up to BAND_MAX in one launch
+//     and the wider ones in another;
 //   - otherwise up to SMALL_MAX_BODIES bodies: one CTA per component factors
 //     it in shared memory (blocked Cholesky by 12-wide body columns; LU with
 //     partial pivoting when a pivot is not positive), all in one launch;
 //   - larger components: the 12x12 blocks are scattered into a dense
 //     column-major matrix and factored with cuSOLVER (Cholesky, or LU when
 //     Cholesky reports a non-positive pivot).
-// Mixed precision factors in FP32.
+// Mixed precision factors its FP32 blocks in FP64 on the band path, in FP32 on
+// the others.
 #include "engine.cuh"
 #include <cstring>
 #include <cusolverDn.h>
@@ -291,49 +292,55 @@ DV void band_cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" :
 DV void band_cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
 
 // A component whose bodies, in reverse Cuthill-McKee order, couple only
-// bodies at most BAND_MAX apart is a block band matrix: its Cholesky factor
-// L has the same band.  One CTA factors it with a sliding window of
-// (BAND_MAX + 1)^2 12x12 blocks in shared memory, all band components in
-// one launch, with no host synchronisation.  The inverse diagonal factors
-// Linv_k = L_kk^-1 are kept explicitly, so every panel entry is an
-// independent dot product.  Block column k:
-//   1. panel L_ik = A_ik Linv_k^T: warp 0 computes block row k + 1 and
-//      signals it at a named barrier without waiting; warps 1..6 compute
-//      the rows below, warp 7 the forward elimination y_k = Linv_k g_k;
-//   2. warp 0 goes straight on: A_{k+1,k+1} - L_{k+1,k} L_{k+1,k}^T into
-//      registers, then its Cholesky factor and inverse (Linv_{k+1}) in one
-//      sweep of 12 pivots; warps 1..7, once the whole panel is there (named
-//      barrier), apply column k to the rest of the window
-//      (A_ij -= L_ik L_jk^T), eliminate the right-hand sides below, write
-//      the factor column to global scratch and bring the next block row
-//      into the window.
-// One block barrier closes the column.  Warp 0's chain (one panel block
-// row, the diagonal update, 12 pivots) is the critical path.  The backward
-// solve, x_k = Linv_k^T (y_k - sum_d L_{k+d,k}^T x_{k+d}), is one short
-// dependent chain per column and runs on warp 0 alone under warp-level
-// synchronisation, each factor column prefetched two columns ahead.
-// FP64 mode only: FP32 roundings of a stiff PSD-projected Hessian can leave
-// the matrix indefinite (the rounded 12-body blocks of a chain mail in contact
-// have negative eigenvalues), which a Cholesky factorization without pivoting
-// cannot take, so mixed-precision components use the shared-memory and
-// cuSOLVER paths, which fall back to LU.  A non-positive pivot, which a
-// PSD-projected FP64 Hessian does not produce, is replaced by its magnitude.
-constexpr int BAND_MAX = 8;
-constexpr int BAND_W = BAND_MAX + 1;
-constexpr int BAND_THREADS = 256;
-// shared-memory stride of one 12x12 block: 146 doubles put the 81 block
-// bases of the window on different banks (144 would start every block on
-// bank 0, and tiles of different blocks read by one warp would conflict)
-constexpr int BAND_BLK = 146;
-constexpr int BAND_CREC = BAND_W * 144 + 12;   // backward record: factor column blocks, then y_k
+// bodies at most wb apart is a block band matrix: its factor A = L D L^T (L unit
+// lower) has the same band.  A CTA factors it with the active window, the
+// W = wb + 1 bodies that the current one couples, in registers.  Window thread
+// (tr, tc) of a 12 x 12 grid owns entry (tr, tc) of every block (i, j), j <= i < W,
+// of the window, whose slot i holds body k + i; after each body the window moves
+// one block up and left (register moves), so every register index is a
+// constant and the loop over bodies is short enough for the instruction
+// caches.  Row threads own one or two window rows each: they eliminate.  Six
+// pivots (half a body) take two barriers:
+//   - the window threads have published the six pivot rows in shared memory;
+//   - a row thread factors the 6 x 6 pivot block (every thread the same) and
+//     eliminates its row's six entries, which gives the row's part of the
+//     factor, the two vectors of the rank-6 update and its right-hand side's;
+//   - the window threads publish the next pivot rows with that update applied,
+//     and then apply it to their registers while the row threads go on.
+// The chain (per pivot a reciprocal of 74 cycles and two operations of 8, per
+// six pivots two barriers and one publishing) bounds the kernel; everything
+// else is kept off it.  The right-hand side is one more column of the pivot
+// rows.  After a body's pivots the row threads form
+//   M_{k,d} = L_kk^-T L_{k+d,k}^T  and  a_k = L_kk^-T D^-1 y_k
+// row by row (independent solves) and store them instead of the factor, so the
+// backward recurrence x_k = a_k - sum_d M_{k,d} x_{k+d}, on one warp, is a short
+// product per body, its records fetched four bodies at a time by the others.
+// 46 bodies of bandwidth 5 take 97 us (a blocked Cholesky with the window in
+// shared memory and one barrier per 12 x 12 factorization and product: 180),
+// 20 of 3 43 us, 45 of 8 162, 61 of 9 201 (cuSOLVER's dense LDL^T, which
+// took such a component before: 420), 92 of 11 363.
+// PSD-projected FP64 matrices have positive pivots (one that is not sets bit 1
+// of *status and is replaced by its magnitude).  SIGNED: mixed precision, whose
+// FP32-rounded blocks can be indefinite (the 12-body blocks of a chain mail
+// in contact have eigenvalues down to -2.9e3 of 1e9), factors them in FP64 with
+// pivots of either sign.
+constexpr int BAND_MAX = 8;            // body bandwidths up to here: narrow kernel
+constexpr int BAND_W = BAND_MAX + 1;   // its blocks per body
+constexpr int BAND_WIDE = 11;          // up to here: wide kernel (78 window entries per thread)
+constexpr int BAND_WTHREADS = 160;     // window threads: 12 x 12 in whole warps
+constexpr int BAND_RTHREADS = 96;      // row threads: one row each up to 8 bodies, two rows in wider windows
+constexpr int BAND_THREADS = BAND_WTHREADS + BAND_RTHREADS;
 constexpr int BAND_ORD_MAX = 1024;     // bodies of a band component (order kept in shared memory)
-// dynamic shared memory of k_band_solve in doubles: window, staged block
-// rows, inverse diagonal factors, right-hand sides, y_k, solution blocks,
-// staged right-hand sides, backward records, then the body order (ints)
-// and the block-pair tables (bytes)
-constexpr int band_smem_doubles() {
-    return BAND_W * BAND_W * BAND_BLK + 2 * BAND_W * 144 + 2 * 144 + BAND_W * 12 + 12 + BAND_W * 12 + 2 * 12 +
-           3 * BAND_CREC + BAND_ORD_MAX / 2 + (BAND_MAX * (BAND_MAX + 1) + 7) / 8;
+constexpr int BAND_P = 6;              // pivots per step
+constexpr int BAND_CHUNK = 4;          // bodies whose backward records are fetched at once
+constexpr int band_ld(int w) { return 12 * w + 2; }            // a pivot row: columns, then its right-hand side
+constexpr int band_ldr(int w) { return 12 * (w - 1) + 2; }     // a backward record's row: 12 wb entries of M, then a_k's
+// dynamic shared memory in doubles for windows of at most bw bodies: two
+// staged block rows, two chunks of backward records, the latest solution
+// blocks, two sets of pivot rows and of the update's two vectors, the
+// right-hand sides in passing, two L_kk, and the body order (ints)
+constexpr int band_smem_doubles(int bw = BAND_W) {
+    return (2 + 2 * BAND_CHUNK) * (bw * 144 + 12) + 16 * 12 + 6 * BAND_P * band_ld(bw) + 12 * bw + 288 + BAND_ORD_MAX / 2;
 }
 // a component of n bodies and body bandwidth wb is split between the two
 // CTAs of its cluster at position m = (n - wb) / 2 when both halves keep at
@@ -342,22 +349,23 @@ inline int band_split_point(int n, int wb) { return n >= 2 * wb + 12 ? (n - wb) 
 
 
 // Band blocks of every band component, contiguous and in FP64: A(i, i - d)
-// of position i (component order), d = 0..BAND_MAX, row-major, at
-// (loff + i BAND_W + d); blocks outside the band or absent are zero.  One
+// of position i (component order), d = 0..bw - 1, row-major, at
+// (loff + i bw + d); blocks outside the band or absent are zero.  One
 // warp per block.
 template <class TV>
-__global__ void k_band_gather(int npos, const int* __restrict__ pcomp, const int* __restrict__ cptr,
+__global__ void k_band_gather(int bw, int npos, const int* __restrict__ pcomp, const int* __restrict__ cptr,
                               const int* __restrict__ order, const int* __restrict__ cbw, const long long* __restrict__ loff,
                               const int* __restrict__ row_ptr, const int* __restrict__ bcol, const TV* __restrict__ vals,
                               double* Ab) {
     const int lane = threadIdx.x & 31;
-    for (long item = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; item < (long)npos * BAND_W;
+    for (long item = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; item < (long)npos * bw;
          item += ((long)gridDim.x * blockDim.x) >> 5) {
-        int p = (int)(item / BAND_W), d = (int)(item % BAND_W);
+        int p = (int)(item / bw), d = (int)(item % bw);
         int c = pcomp[p], i = p - cptr[c], j = i - d;
+        if (d > cbw[c]) continue;                       // never read
         int bi = -1;
-        if (j >= 0 && d <= cbw[c]) bi = find_block(row_ptr, bcol, order[p], order[cptr[c] + j]);
-        double* dst = Ab + (loff[c] + (long)i * BAND_W + d) * 144;
+        if (j >= 0) bi = find_block(row_ptr, bcol, order[p], order[cptr[c] + j]);
+        double* dst = Ab + (loff[c] + (long)i * bw + d) * 144;
         for (int e = lane; e < 144; e += 32) {
             int r = e / 12, cc = e % 12;
             dst[e] = bi >= 0 ? (double)vals[(long)bi * 144 + cc * 12 + r] : 0.0;     // row-major from column-major
@@ -365,79 +373,419 @@ __global__ void k_band_gather(int npos, const int* __restrict__ pcomp, const int
     }
 }
 
-// Warp-wide Cholesky factorization and inversion of a 12x12 SPD block in
-// one sweep of its 12 pivots.  On entry lane i < 12 holds row i of the
-// (symmetric) block in a[]; on exit it holds row i of W = L^-1, zeros right
-// of the diagonal, where L L^T is the block.  Step j: lane j owns the pivot
-// d_j = a[j]; every lane i > j forms t = a_ij / d_j and subtracts t times
-// lane j's row.  Right of column j that row is the remaining block row, so
-// this is the Schur update a_ic -= a_ij a_jc / d_j; left of column j it is
-// row j of the unscaled inverse w, so this is the forward substitution
-// w_i -= (L_ij / L_jj) w_j of L w = I; slot j itself becomes w_ij = -t.
-// Finally W_i = w_i / sqrt(d_i).  Lane j's row is final one step before it
-// is needed, so each pivot costs one reciprocal square root and one
-// broadcast on the dependent chain.  A non-positive pivot sets bit 1 of
-// *status and is replaced by its magnitude.
-DV void band_chol_inverse_rows(double (&a)[12], int* status) {
-    const int lane = threadIdx.x & 31;
-    double rown = 0.0;
-#pragma unroll
-    for (int j = 0; j < 12; j++) {
-        double s = 0.0;
-        if (lane == j) {
-            double d = a[j];
-            if (!(d > 0.0)) { atomicOr(status, 2); d = fabs(d) + 1e-30; }
-            rown = rsqrt(d);        // the double-precision rsqrt: ~76 cycles of latency on sm_100
-            s = rown * rown;
+// Warp-wide Cholesky factorization and inversion of 12 x 12 diagonal blocks
+// would be a chain of 12 square roots and divisions per body; here the pivots
+// are scalars, six divisions per step, which every row thread does for itself.
+
+// What a CTA of k_band_solve works on: one sub-component in its own order.
+struct BandJob {
+    int N, wb, ncol1;                  // bodies, body bandwidth, bodies eliminated before the merge
+    const double* A;                   // block A(i, i - d) at (i BW + d)
+    double* L;                         // backward record of body k at (k BW) blocks
+    double* Y;                         // right-hand sides of a handed-over separator at 12 k
+    const int* ord;                    // bodies in order (shared memory)
+    const double* g;
+};
+struct __align__(16) band_d2 { double x, y; };     // one 16-byte shared-memory access
+struct BandSmem { double *stage, *cst, *xs, *rows, *pass, *lkk; int* ord; };
+template <int BW>
+DV BandSmem band_smem(unsigned char* raw) {
+    BandSmem S;
+    S.stage = (double*)raw;                                   // [2][BW * 144 + 12] (16-byte aligned for cp.async)
+    S.cst = S.stage + 2 * (BW * 144 + 12);                    // [2][BAND_CHUNK][BW * 144 + 12]
+    S.xs = S.cst + 2 * BAND_CHUNK * (BW * 144 + 12);          // [16][12]
+    S.rows = S.xs + 16 * 12;                                  // [2] pivot rows, [2][2] update vectors, of BAND_P rows each
+    S.pass = S.rows + 6 * BAND_P * band_ld(BW);               // [12 BW]
+    S.lkk = S.pass + 12 * BW;                                 // [2][12][12]
+    S.ord = (int*)(S.lkk + 288);                              // [BAND_ORD_MAX]
+    return S;
+}
+
+// Shared memory of the elimination, and the pieces both roles use.  W: bodies of the window.
+template <int W, int BW>
+struct BandShared {
+    static constexpr int LD = band_ld(W), M = 12 * W;         // right-hand side at column M
+    const BandJob& J;
+    const BandSmem& S;
+    DV BandShared(const BandJob& j, const BandSmem& s) : J(j), S(s) {}
+    DV double* pivots(int buf) const { return S.rows + buf * BAND_P * LD; }                  // P[BAND_P][LD]
+    DV double* vec_c(int buf) const { return S.rows + (2 + 2 * buf) * BAND_P * LD; }         // c[row][BAND_P]: eliminated entries
+    DV double* vec_t(int buf) const { return vec_c(buf) + BAND_P * LD; }                     // t[row][BAND_P]: the factor's
+    DV const double* staged(int m) const { return S.stage + (m & 1) * (BW * 144 + 12); }
+};
+
+// Window threads (see above): the entries in registers.
+template <int W, int BW>
+struct BandWindow : BandShared<W, BW> {
+    using B = BandShared<W, BW>;
+    using B::LD; using B::J; using B::S; using B::pivots; using B::vec_c; using B::vec_t; using B::staged;
+    static constexpr int off(int i, int j) { return i * (i + 1) / 2 + j; }
+    double a[off(W, 0)];
+    const int tid, tr, tc;
+    DV BandWindow(const BandJob& j, const BandSmem& s)
+        : BandShared<W, BW>(j, s), tid(threadIdx.x), tr(threadIdx.x / 12), tc(threadIdx.x % 12) {}
+    DV bool owner() const { return tid < 144; }
+
+    // block row m and its right-hand side into staging buffer m & 1
+    DV void fetch_row(int m) const {
+        double* dst = S.stage + (m & 1) * (BW * 144 + 12);
+        const double* src = J.A + (long)m * BW * 144;
+        for (int e = tid; e < W * 72 + 6; e += BAND_WTHREADS) {
+            if (e < W * 72) band_cp16(dst + 2 * e, src + 2 * e);
+            else { const int c = e - W * 72; band_cp16(dst + BW * 144 + 2 * c, J.g + 12L * J.ord[m] + 2 * c); }
         }
-        if (j < 11) {
-            s = __shfl_sync(0xffffffffu, s, j);
-            const bool upd = lane > j && lane < 12;
-            const double t = a[j] * s;
+        band_cp_commit();
+    }
+    // the first W bodies
+    DV void load() {
 #pragma unroll
-            for (int c = 0; c < 12; c++) {
-                if (c == j) continue;
-                const double v = __shfl_sync(0xffffffffu, a[c], j);
-                if (upd) a[c] = fma(-t, v, a[c]);
+        for (int i = 0; i < W; i++)
+#pragma unroll
+            for (int j = 0; j <= i; j++) a[off(i, j)] = owner() ? J.A[((long)i * BW + i - j) * 144 + tid] : 0.0;
+        if (W < J.N) fetch_row(W);
+    }
+    // window entry of block (i, j) with the update of vectors c, t applied
+    template <int I, int JJ>
+    DV double updated(const double* t, const double (&cv)[BAND_P]) const {
+        const band_d2* tv = reinterpret_cast<const band_d2*>(t + (tr + 12 * I) * BAND_P);
+        double v = a[off(I, JJ)], w = 0.0;
+#pragma unroll
+        for (int m = 0; m < BAND_P / 2; m++) {
+            const band_d2 u = tv[m];
+            v -= u.x * cv[2 * m];
+            w -= u.y * cv[2 * m + 1];
+        }
+        return v + w;
+    }
+    // rows 6 .. 11 of slot 0 with the update applied; a pivot row's columns
+    // are block (0, 0)'s row and, transposed, the blocks (i, 0) below it
+    template <int I>
+    DV void publish_half(double* P, const double* t, const double (&cv)[BAND_P]) const {
+        if constexpr (I < W) {
+            const double v = updated<I, 0>(t, cv);
+            if (I == 0) { if (tr >= BAND_P) P[(tr - BAND_P) * LD + tc] = v; }
+            else if (tc >= BAND_P) P[(tc - BAND_P) * LD + 12 * I + tr] = v;
+            publish_half<I + 1>(P, t, cv);
+        }
+    }
+    // rows 0 .. 5 of slot 1, which becomes slot 0, with the update applied
+    template <int I>
+    DV void publish_next(double* P, const double* t, const double (&cv)[BAND_P]) const {
+        if constexpr (I < W) {
+            const double v = updated<I, 1>(t, cv);
+            if (I == 1) { if (tr < BAND_P) P[tr * LD + tc] = v; }
+            else if (tc < BAND_P) P[tc * LD + 12 * (I - 1) + tr] = v;
+            publish_next<I + 1>(P, t, cv);
+        }
+    }
+    // the update of vectors `cb`
+    DV void flush(int cb) {
+        const band_d2* c = reinterpret_cast<const band_d2*>(vec_c(cb) + tc * BAND_P);
+        const band_d2* t = reinterpret_cast<const band_d2*>(vec_t(cb) + tr * BAND_P);
+#pragma unroll
+        for (int m = 0; m < BAND_P / 2; m++) {
+            band_d2 cv[W];
+#pragma unroll
+            for (int j = 0; j < W; j++) cv[j] = c[j * 6 * BAND_P + m];
+#pragma unroll
+            for (int i = 0; i < W; i++) {
+                const band_d2 tv = t[i * 6 * BAND_P + m];
+#pragma unroll
+                for (int j = 0; j <= i; j++) { a[off(i, j)] -= tv.x * cv[j].x; a[off(i, j)] -= tv.y * cv[j].y; }
             }
-            if (upd) a[j] = -t;
-        }
-        if (lane == j) {
-            a[j] = 1.0;
-#pragma unroll
-            for (int c = j + 1; c < 12; c++) a[c] = 0.0;
         }
     }
+    // eliminates bodies [k0, k1); before it slot i holds body k0 + i, after it body k1 + i
+    DV void columns(int k0, int k1) {
+        if (owner()) {
+            double* P = pivots(0);
+            if (tr < BAND_P) P[tr * LD + tc] = a[off(0, 0)];
 #pragma unroll
-    for (int c = 0; c < 12; c++) a[c] *= rown;
+            for (int i = 1; i < W; i++) if (tc < BAND_P) P[tc * LD + 12 * i + tr] = a[off(i, 0)];
+        }
+        band_bar_arrive(1, BAND_THREADS);                    // the first pivot rows are there
+#pragma unroll 1
+        for (int h = 2 * k0; h < 2 * k1; h++) {              // half bodies
+            const int k = h >> 1, m = k + W, buf = h & 1;    // k0 may be odd: 2 k0 is even
+            if (buf) band_cp_wait_all();                     // the entering body's row
+            __syncthreads();                                 // the update's vectors (and that row) are there
+            double* P = pivots(buf ^ 1);
+            const double* t = vec_t(buf);
+            const double* c = vec_c(buf) + (tc + (buf ? 12 : 0)) * BAND_P;
+            const double* st = staged(m);
+            const bool in = m < J.N;
+            if (owner()) {
+                double cv[BAND_P];
+#pragma unroll
+                for (int n = 0; n < BAND_P; n++) cv[n] = c[n];
+                if (!buf) publish_half<0>(P, t, cv);
+                else {
+                    publish_next<1>(P, t, cv);
+                    if (tc < BAND_P) P[tc * LD + 12 * (W - 1) + tr] = in ? st[(W - 1) * 144 + tid] : 0.0;
+                }
+            }
+            if (h + 1 < 2 * k1) band_bar_arrive(1, BAND_THREADS);
+            if (owner()) flush(buf);
+            if (buf) {
+                // one block up and left; body m enters below
+#pragma unroll
+                for (int i = 0; i + 1 < W; i++)
+#pragma unroll
+                    for (int j = 0; j <= i; j++) a[off(i, j)] = a[off(i + 1, j + 1)];
+#pragma unroll
+                for (int j = 0; j < W; j++) a[off(W - 1, j)] = in && owner() ? st[(W - 1 - j) * 144 + tid] : 0.0;
+                if (m + 1 < J.N) fetch_row(m + 1);
+            }
+        }
+        __syncthreads();
+    }
+    // the separator (bodies ncol1..N-1, slots 0..wb-1) into this sub-component's
+    // unused record slots: block (p, q), p >= q, at (p BW + p - q), right-hand sides at Y + 12 p
+    DV void hand_over() const {
+        if (!owner()) return;
+#pragma unroll
+        for (int i = 0; i + 1 < W; i++)
+#pragma unroll
+            for (int j = 0; j <= i; j++) J.L[((long)(J.ncol1 + i) * BW + i - j) * 144 + tid] = a[off(i, j)];
+    }
+    // S = W0 + W1 - A_SS: adds the other CTA's separator (its blocks L1, right-hand
+    // sides Y1; forward position i is its position nt1 - i, so its block (nt1 - j,
+    // nt1 - i) is the transpose of block (i, j) here)
+    DV void merge(const double* L1, const double*, int nt1) {
+        if (!owner()) return;
+        const int p0 = J.ncol1;
+#pragma unroll
+        for (int i = 0; i + 1 < W; i++)
+#pragma unroll
+            for (int j = 0; j <= i; j++)
+                a[off(i, j)] += __ldcg(L1 + ((long)(nt1 - p0 - j) * BW + i - j) * 144 + tc * 12 + tr) -
+                                J.A[((long)(p0 + i) * BW + i - j) * 144 + tid];
+    }
+};
+
+// Row threads (see above): the elimination.
+template <int W, int BW, bool SIGNED>
+struct BandRows : BandShared<W, BW> {
+    using B = BandShared<W, BW>;
+    using B::LD; using B::M; using B::J; using B::S; using B::pivots; using B::vec_c; using B::vec_t; using B::staged;
+    static constexpr int NR = 12 * W > BAND_RTHREADS ? 2 : 1; // rows of a thread: row, row + BAND_RTHREADS
+    double rhs[NR];                      // right-hand sides of its rows
+    int* status;
+    const int row;
+    DV BandRows(const BandJob& j, const BandSmem& s, int* st)
+        : BandShared<W, BW>(j, s), status(st), row((int)threadIdx.x - BAND_WTHREADS) {}
+    DV bool has_row(int n) const { return row + n * BAND_RTHREADS < 12 * W; }
+    DV void load() {
+#pragma unroll
+        for (int n = 0; n < NR; n++) {
+            const int r = row + n * BAND_RTHREADS;
+            rhs[n] = has_row(n) ? J.g[12L * J.ord[r / 12] + r % 12] : 0.0;
+        }
+    }
+    DV double pivot_inverse(double d) const {
+        if (!SIGNED && !(d > 0.0)) { if (row == 0) atomicOr(status, 2); d = fabs(d) + 1e-30; }
+        return 1.0 / d;
+    }
+    // rows of M_{k,d}, d >= 1, and a_k: entry n of row 12 (d - 1) + i at n LDR + row,
+    // a_k's at n LDR + 12 wb (neighbouring threads write neighbouring places)
+    DV void backward_record(int k, const double (&rec)[NR][12]) const {
+        const double* lkk = S.lkk + (k & 1) * 144;
+#pragma unroll
+        for (int r = 0; r < NR; r++) {
+            const int e = row + r * BAND_RTHREADS;
+            if (!has_row(r) || (e > 0 && e < 12) || k + e / 12 >= J.N) continue;
+            double v[12];
+#pragma unroll
+            for (int n = 0; n < 12; n++) v[n] = rec[r][n];
+#pragma unroll
+            for (int j = 11; j > 0; j--)
+#pragma unroll
+                for (int n = 0; n < j; n++) v[n] -= lkk[j * 12 + n] * v[j];
+            double* o = J.L + (long)k * BW * 144 + (e == 0 ? 12 * (W - 1) : e - 12);
+#pragma unroll
+            for (int n = 0; n < 12; n++) o[n * band_ldr(W)] = v[n];
+        }
+    }
+    DV void columns(int k0, int k1) {
+        double rec[NR][12];              // the body's factor rows (thread 0, row 0: D^-1 y_k)
+        if (row < BAND_P) pivots(0)[row * LD + M] = rhs[0];
+#pragma unroll 1
+        for (int h = 2 * k0; h < 2 * k1; h++) {
+            const int k = h >> 1, buf = h & 1, q = buf * BAND_P;
+            band_bar_sync(1, BAND_THREADS);
+            const double* P = pivots(buf);
+            double inv[BAND_P], l[BAND_P][BAND_P], y[BAND_P], c[NR][BAND_P];
+            {
+                double d[BAND_P][BAND_P];
+#pragma unroll
+                for (int n = 0; n < BAND_P; n++) {
+#pragma unroll
+                    for (int m = n; m < BAND_P; m++) d[m][n] = P[n * LD + q + m];
+                    y[n] = P[n * LD + M];
+#pragma unroll
+                    for (int r = 0; r < NR; r++) c[r][n] = has_row(r) ? P[n * LD + row + r * BAND_RTHREADS] : 0.0;
+                }
+#pragma unroll
+                for (int n = 0; n < BAND_P; n++) {
+                    inv[n] = pivot_inverse(d[n][n]);
+#pragma unroll
+                    for (int m = n + 1; m < BAND_P; m++) l[m][n] = d[m][n] * inv[n];
+#pragma unroll
+                    for (int m = n + 1; m < BAND_P; m++) {
+#pragma unroll
+                        for (int o = n + 1; o <= m; o++) d[m][o] -= l[m][n] * d[o][n];
+                        y[m] -= l[m][n] * y[n];
+#pragma unroll
+                        for (int r = 0; r < NR; r++) c[r][m] -= l[m][n] * c[r][n];
+                    }
+                }
+            }
+            double t[NR][BAND_P];
+#pragma unroll
+            for (int r = 0; r < NR; r++) {
+                if (!has_row(r)) continue;
+                const int e = row + r * BAND_RTHREADS;
+                double r0 = rhs[r], r1 = 0.0;
+#pragma unroll
+                for (int n = 0; n < BAND_P; n++) {
+                    t[r][n] = c[r][n] * inv[n];
+                    vec_c(buf)[e * BAND_P + n] = c[r][n]; vec_t(buf)[e * BAND_P + n] = t[r][n];
+                    if (n & 1) r1 -= t[r][n] * y[n]; else r0 -= t[r][n] * y[n];
+                }
+                rhs[r] = r0 + r1;
+                // the next pivots' right-hand sides: rows 6 .. 11, or the next body's first six
+                const int next = buf ? 12 : BAND_P;
+                if (e >= next && e < next + BAND_P) pivots(buf ^ 1)[(e - next) * LD + M] = rhs[r];
+                if (buf) S.pass[e] = rhs[r];
+            }
+            // L_kk for the solves
+            if (row < 12) {
+#pragma unroll
+                for (int n = 0; n < BAND_P; n++) S.lkk[(k & 1) * 144 + row * 12 + q + n] = t[0][n];
+            }
+            __syncthreads();                                     // the update's vectors are there
+            if (!buf) {
+                // the window threads are publishing: the previous body's record
+                if (k > k0) backward_record(k - 1, rec);
+#pragma unroll
+                for (int n = 0; n < BAND_P; n++)
+#pragma unroll
+                    for (int r = 0; r < NR; r++) rec[r][n] = r == 0 && row == 0 ? y[n] * inv[n] : t[r][n];
+                continue;
+            }
+            // right-hand sides move up with the window
+#pragma unroll
+            for (int r = 0; r < NR; r++) {
+#pragma unroll
+                for (int n = 0; n < BAND_P; n++) rec[r][BAND_P + n] = r == 0 && row == 0 ? y[n] * inv[n] : t[r][n];
+                if (!has_row(r)) continue;
+                const int e = row + r * BAND_RTHREADS;
+                rhs[r] = e < 12 * (W - 1) ? S.pass[e + 12] : (k + W < J.N ? staged(k + W)[BW * 144 + e - 12 * (W - 1)] : 0.0);
+            }
+        }
+        if (k1 > k0) backward_record(k1 - 1, rec);
+        __syncthreads();
+    }
+    DV void hand_over() const {
+#pragma unroll
+        for (int r = 0; r < NR; r++) {
+            const int e = row + r * BAND_RTHREADS;
+            if (e < 12 * (W - 1)) J.Y[12L * J.ncol1 + e] = rhs[r];
+        }
+    }
+    DV void merge(const double*, const double* Y1, int nt1) {
+        const int p0 = J.ncol1;
+#pragma unroll
+        for (int r = 0; r < NR; r++) {
+            const int e = row + r * BAND_RTHREADS, p = p0 + e / 12;
+            if (e < 12 * (W - 1)) rhs[r] += __ldcg(Y1 + 12L * (nt1 - p) + e % 12) - J.g[12L * J.ord[p] + e % 12];
+        }
+    }
+};
+
+// both roles' elimination of a sub-component; the roles meet at the same barriers
+template <class Role>
+DV void band_eliminate(Role& role, const BandJob& J, bool split, int crank, const double* L1, const double* Y1, int nt1) {
+    role.load();
+    // one loop, so that the elimination's code is there once
+    int k0 = 0, k1 = J.ncol1;
+#pragma unroll 1
+    for (;;) {
+        role.columns(k0, k1);
+        if (!split || crank == 1 || k1 == J.N) break;
+        band_cluster_arrive(); band_cluster_wait();       // CTA 1's half of S is in global memory
+        role.merge(L1, Y1, nt1);
+        k0 = k1; k1 = J.N;
+    }
+    if (split && crank == 1) role.hand_over();
 }
 
-// Panel rows in place: R (one row of a block below the diagonal) becomes
-// R Linv^T, i.e. entry c = sum_{s <= c} R[s] Linv[c][s].  Two lanes (adjacent
-// or 12 apart) share a row and write six entries each; every lane of the
-// warp must call it, `act` says whether this lane has a row.
-DV void band_panel_row(double* R, const double* Li, int half, bool act) {
-    double v[12];
-    if (act) {
-#pragma unroll
-        for (int s = 0; s < 12; s++) v[s] = R[s];
-    }
-    __syncwarp();
-    if (act) {
-#pragma unroll
-        for (int c6 = 0; c6 < 6; c6++) {
-            const int c = half * 6 + c6;
-            double acc = 0.0;
-#pragma unroll
-            for (int s = 0; s < 12; s++) if (s <= c) acc += v[s] * Li[c * 12 + s];
-            R[c] = acc;
+// x_k = a_k - sum_d M_{k,d} x_{k+d} for k = kfirst down to klast, by warp 0, the
+// solution blocks above kfirst already in xs (a ring of 16).  The records of
+// BAND_CHUNK bodies are fetched at once by the other warps, one chunk ahead.
+// Every thread calls it.
+template <int W, int BW>
+DV void band_backward(const BandJob& J, const BandSmem& S, int kfirst, int klast, double* du) {
+    constexpr int LDR = band_ldr(W), REC = 12 * LDR;
+    const int lane = threadIdx.x & 31;
+    const bool solver = threadIdx.x < 32;
+    if (kfirst < klast) return;
+    // chunk q: bodies kfirst - q BAND_CHUNK and the BAND_CHUNK - 1 below it
+    auto fetch = [&](int q) {
+        for (int b = 0; b < BAND_CHUNK; b++) {
+            const int k = kfirst - q * BAND_CHUNK - b;
+            if (k < klast) break;
+            double* dst = S.cst + ((q & 1) * BAND_CHUNK + b) * REC;
+            const double* src = J.L + (long)k * BW * 144;
+            for (int e = threadIdx.x - 32; e < REC / 2; e += BAND_THREADS - 32) band_cp16(dst + 2 * e, src + 2 * e);
         }
+        band_cp_commit();
+    };
+    if (!solver) fetch(0);
+    const int jj = lane % 12, hh = lane / 12;            // lanes jj and jj + 12 take half of each block's rows
+    const int nq = (kfirst - klast) / BAND_CHUNK + 1;
+#pragma unroll 1
+    for (int q = 0; q < nq; q++) {
+        if (!solver) {
+            fetch(q + 1);                                // into the buffer chunk q - 1 used
+            band_cp_wait_but_one();                      // chunk q
+        }
+        __syncthreads();                                 // chunk q is there
+        if (solver) {
+#pragma unroll 1
+            for (int b = 0; b < BAND_CHUNK; b++) {
+                const int k = kfirst - q * BAND_CHUNK - b;
+                if (k < klast) break;
+                const int nk = min(W - 1, J.N - 1 - k);
+                double x = 0.0;
+                if (lane < 24) {
+                    const double* rec = S.cst + ((q & 1) * BAND_CHUNK + b) * REC + jj * LDR;
+                    double acc[3] = {hh == 0 ? rec[12 * (W - 1)] : 0.0, 0.0, 0.0};
+                    const band_d2* M = reinterpret_cast<const band_d2*>(rec + 6 * hh);
+#pragma unroll
+                    for (int d = 1; d < W; d++) {
+                        if (d > nk) break;
+                        const band_d2* xi = reinterpret_cast<const band_d2*>(S.xs + ((k + d) & 15) * 12 + 6 * hh);
+#pragma unroll
+                        for (int r = 0; r < 3; r++) {
+                            const band_d2 u = M[(d - 1) * 6 + r], w = xi[r];
+                            acc[r] = fma(-u.x, w.x, acc[r]);
+                            acc[r] = fma(-u.y, w.y, acc[r]);
+                        }
+                    }
+                    x = acc[0] + acc[1] + acc[2];
+                }
+                x += __shfl_sync(0xffffffffu, x, (lane + 12) & 31);
+                if (lane < 12) { S.xs[(k & 15) * 12 + lane] = x; du[12L * J.ord[k] + lane] = x; }
+                __syncwarp();
+            }
+        }
+        __syncthreads();                                 // chunk q's buffer is free
     }
-    __syncwarp();
 }
 
-// One job per cluster of two CTAs.  A job is a band component (sub-component
-// ct) factored by CTA 0 alone, or a large one split in two: ct holds its
+// One sub-component of a job on this CTA.  A job is a band component (ct)
+// factored by CTA 0 alone, or a large one split in two: ct holds its
 // bodies [0, m + wb) in order, cb the bodies [m, N) in reverse order, and
 // S = [m, m + wb) separates [0, m) from [m + wb, N) (the band couples bodies
 // at most wb apart).  CTA 0 eliminates [0, m) while CTA 1 eliminates
@@ -445,34 +793,64 @@ DV void band_panel_row(double* R, const double* Li, int half, bool act) {
 // Schur update applied.  After a cluster barrier CTA 0 adds CTA 1's update
 // (S = W0 + W1 - A_SS, right-hand sides likewise), factors and solves S,
 // and signals the solution at a second cluster barrier; then both CTAs run
-// their backward halves.  The dependent chain shrinks from N block columns
-// each way to about (N - wb) / 2 + wb.  jobs holds (ct, cb, m) per job,
-// cb = -1 for an unsplit component (m is then its size).
-// one CTA per SM (its shared memory allows no second), so the register cap is set for one
+// their backward halves.  The dependent chain shrinks from N bodies each
+// way to about (N - wb) / 2 + wb.
+// Not inlined, and its arguments by value: each width gets its own register
+// allocation, and what the loops read stays in registers (46 bodies of
+// bandwidth 5: 97 us, with all widths in one function 127).
+template <int W, int BW, bool SIGNED>
+__device__ __attribute__((noinline)) void band_job(BandJob J, bool split, int crank, const double* L1, const double* Y1,
+                                                   int nt1, double* du, int* status) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const BandSmem S = band_smem<BW>(smem_raw);
+    if ((int)threadIdx.x < BAND_WTHREADS) {
+        BandWindow<W, BW> role(J, S);
+        band_eliminate(role, J, split, crank, L1, Y1, nt1);
+    } else {
+        BandRows<W, BW, SIGNED> role(J, S, status);
+        band_eliminate(role, J, split, crank, L1, Y1, nt1);
+    }
+    int first = J.N - 1;
+    if (split && crank == 1) {
+        __threadfence();
+        band_cluster_arrive(); band_cluster_wait();       // S handed over
+        band_cluster_arrive(); band_cluster_wait();       // S solved by CTA 0
+        for (int e = threadIdx.x; e < J.wb * 12; e += BAND_THREADS) {
+            const int p = J.ncol1 + e / 12;
+            S.xs[(p & 15) * 12 + e % 12] = __ldcg(du + 12L * J.ord[p] + e % 12);
+        }
+        first = J.ncol1 - 1;
+        __syncthreads();
+    }
+    int last = split && crank == 0 ? J.ncol1 : 0;
+#pragma unroll 1
+    for (;;) {
+        band_backward<W, BW>(J, S, first, last, du);
+        if (last == 0) break;
+        __threadfence();
+        band_cluster_arrive();                            // S solved
+        first = last - 1; last = 0;
+    }
+    if (split && crank == 0) band_cluster_wait();
+    if (!split) {
+        band_cluster_arrive(); band_cluster_wait();
+        band_cluster_arrive(); band_cluster_wait();
+    }
+}
+
+// One job per cluster of two CTAs (band_job).  jobs holds (ct, cb, m) per
+// job, cb = -1 for an unsplit component (m is then its size).  One CTA per SM
+// (its registers allow no second).
+template <int BW = BAND_W, bool SIGNED = false>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(BAND_THREADS, 1)
 k_band_solve(int njobs, const int* __restrict__ jobs, const int* __restrict__ cptr,
         const int* __restrict__ order, const int* __restrict__ cbw, const long long* __restrict__ loff,
         const double* __restrict__ Ab, long long ltot, const double* __restrict__ g, double* Lg, double* du,
         int* status) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    double* win = (double*)smem_raw;                          // [BAND_W][BAND_W] row-major 12x12 blocks, BAND_BLK apart
-    double* stage = win + BAND_W * BAND_W * BAND_BLK;         // [2][BAND_W][144]: next block row
-    double* linv = stage + 2 * BAND_W * 144;                  // [2][144] inverse diagonal factors
-    double* rhs = linv + 2 * 144;                             // [BAND_W][12]
-    double* ybuf = rhs + BAND_W * 12;                         // [12] y_k of the current column
-    double* xs = ybuf + 12;                                   // [BAND_W][12] latest solution blocks (backward)
-    double* gst = xs + BAND_W * 12;                           // [2][12] right-hand side of each staged block row
-    double* cst = gst + 2 * 12;                               // [3][BAND_CREC] backward factor columns and y_k
-    int* ord = (int*)(cst + 3 * BAND_CREC);                   // [BAND_ORD_MAX] bodies of the sub-component
-    unsigned char* tri_a = (unsigned char*)(ord + BAND_ORD_MAX);   // block pair p -> (a, b), b <= a
-    unsigned char* tri_b = tri_a + BAND_MAX * (BAND_MAX + 1) / 2;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int t1 = tid - 32, n1 = blockDim.x - 32;            // thread index among warps 1..7
+    int* ord = band_smem<BW>(smem_raw).ord;
+    const int tid = threadIdx.x;
     const int crank = blockIdx.x & 1;                         // rank in the cluster
-    if (tid < BAND_MAX * (BAND_MAX + 1) / 2) {
-        int a = 0; while ((a + 1) * (a + 2) / 2 <= tid) a++;
-        tri_a[tid] = (unsigned char)a; tri_b[tid] = (unsigned char)(tid - a * (a + 1) / 2);
-    }
     for (int jb = blockIdx.x >> 1; jb < njobs; jb += gridDim.x >> 1) {
         const int ct = jobs[3 * jb], cb = jobs[3 * jb + 1], msplit = jobs[3 * jb + 2];
         const bool split = cb >= 0;
@@ -483,303 +861,25 @@ k_band_solve(int njobs, const int* __restrict__ jobs, const int* __restrict__ cp
             continue;
         }
         const int cc = crank == 0 ? ct : cb;
-        const int N = cptr[cc + 1] - cptr[cc], wb = cbw[cc];
-        // columns this CTA eliminates before the merge
-        const int ncol1 = !split ? N : (crank == 0 ? msplit : N - wb);
-        for (int e = tid; e < N; e += blockDim.x) ord[e] = order[cptr[cc] + e];
-        double* L = Lg + loff[cc] * 144;                      // Linv_k at (k BAND_W), L(k + d, k) at (k BAND_W + d)
-        double* Y = Lg + ltot * 144 + (loff[cc] / BAND_W) * 12;   // y_k at k * 12
-        const double* A = Ab + loff[cc] * 144;                // block A(i, i - d) at (i BAND_W + d)
+        BandJob J;
+        J.N = cptr[cc + 1] - cptr[cc]; J.wb = cbw[cc];
+        J.ncol1 = !split ? J.N : (crank == 0 ? msplit : J.N - J.wb);
+        J.A = Ab + loff[cc] * 144;
+        J.L = Lg + loff[cc] * 144;
+        J.Y = Lg + ltot * 144 + (loff[cc] / BW) * 12;
+        J.ord = ord; J.g = g;
+        for (int e = tid; e < J.N; e += BAND_THREADS) ord[e] = order[cptr[cc] + e];
         __syncthreads();
-        auto slot = [&](int i, int j) { return win + ((i % BAND_W) * BAND_W + (j % BAND_W)) * BAND_BLK; };
-        // window rows 0..min(wb, N - 1), their right-hand sides, and block
-        // row wb + 1 fetched ahead into its staging buffer
-        const int r0 = min(wb, N - 1);
-        for (int e = tid; e < (r0 + 1) * BAND_W * 144; e += blockDim.x) {
-            int i = e / (BAND_W * 144), d = (e / 144) % BAND_W, q = e % 144;
-            if (d <= i) slot(i, i - d)[q] = A[(long)e];
-        }
-        for (int e = tid; e < (r0 + 1) * 12; e += blockDim.x) rhs[(e / 12) * 12 + e % 12] = g[12L * ord[e / 12] + e % 12];
-        // block row m and its right-hand side into staging buffer m & 1 by
-        // warps 1..7; the stored row holds A(m, m - d) at block d, staged at
-        // block wb - d (column m - wb + (wb - d)); the same threads wait for
-        // it before the named barrier of the next column
-        auto fetch_row = [&](int m) {
-            double* dst = stage + (m & 1) * BAND_W * 144;
-            const double* src = A + (long)m * BAND_W * 144;
-            for (int e = t1; e < (wb + 1) * 72 + 6; e += n1) {
-                if (e < (wb + 1) * 72) {
-                    const int d = e / 72, c = e % 72;
-                    band_cp16(dst + (wb - d) * 144 + 2 * c, src + d * 144 + 2 * c);
-                } else {
-                    const int c = e - (wb + 1) * 72;
-                    band_cp16(gst + (m & 1) * 12 + 2 * c, g + 12L * ord[m] + 2 * c);
-                }
-            }
-            band_cp_commit();
-        };
-        // warp 0: factor and invert the diagonal block in slot(k, k) into linv[k & 1]
-        auto factor_diag = [&](int k) {
-            const double* D = slot(k, k);
-            double a[12];
-#pragma unroll
-            for (int c = 0; c < 12; c++) a[c] = lane < 12 ? D[lane * 12 + c] : 0.0;
-            band_chol_inverse_rows(a, status);
-            if (lane < 12) {
-#pragma unroll
-                for (int c = 0; c < 12; c++) linv[(k & 1) * 144 + lane * 12 + c] = a[c];
-            }
-        };
-        // block columns k0..k1-1; Linv_k0 is in linv[k0 & 1].  When k1 < N
-        // the last column leaves the next diagonal block unfactored, its
-        // update applied by warps 1..7 like every other block pair.
-        auto columns = [&](int k0, int k1) {
-            for (int k = k0; k < k1; k++) {
-                const int nk = min(wb, N - 1 - k);               // blocks below the diagonal in this column
-                const bool factor_next = k + 1 < k1;
-                const double* Li = linv + (k & 1) * 144;
-                if (warp == 0) {
-                    // panel block row k + 1 (lanes r and r + 12 share row r), signalled to warps 1..7
-                    const int r = lane % 12, half = lane / 12;
-                    double* P = slot(k + 1, k);
-                    if (nk > 0) band_panel_row(P + r * 12, Li, half, lane < 24);
-                    band_bar_arrive(1, blockDim.x);
-                    if (nk > 0 && factor_next) {
-                        // row r of A_{k+1,k+1} - L_{k+1,k} L_{k+1,k}^T: lane r forms entries 0..5,
-                        // lane r + 12 entries 6..11 and passes them to lane r
-                        const double* Dk = slot(k + 1, k + 1);
-                        double h[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-                        if (lane < 24) {
-                            double lr[12];
-#pragma unroll
-                            for (int s = 0; s < 12; s++) lr[s] = P[r * 12 + s];
-#pragma unroll
-                            for (int c6 = 0; c6 < 6; c6++) {
-                                const int c = half * 6 + c6;
-                                double acc0 = Dk[r * 12 + c], acc1 = 0.0;
-#pragma unroll
-                                for (int s = 0; s < 12; s += 2) {
-                                    acc0 = fma(-lr[s], P[c * 12 + s], acc0);
-                                    acc1 = fma(-lr[s + 1], P[c * 12 + s + 1], acc1);
-                                }
-                                h[c6] = acc0 + acc1;
-                            }
-                        }
-                        double a[12];
-#pragma unroll
-                        for (int c6 = 0; c6 < 6; c6++) {
-                            const double o = __shfl_sync(0xffffffffu, h[c6], (lane + 12) & 31);
-                            a[c6] = lane < 12 ? h[c6] : 0.0;
-                            a[6 + c6] = lane < 12 ? o : 0.0;
-                        }
-                        band_chol_inverse_rows(a, status);
-                        if (lane < 12) {
-                            double* Ln = linv + ((k + 1) & 1) * 144;
-#pragma unroll
-                            for (int c = 0; c < 12; c++) Ln[lane * 12 + c] = a[c];
-                        }
-                    }
-                } else {
-                    if (warp < 7) {
-                        // panel rows of blocks k + 2 .. k + nk, two adjacent lanes per row
-                        const int q = 12 + (t1 >> 1);
-                        const bool act = q < 12 * nk;
-                        band_panel_row(act ? slot(k + 1 + q / 12, k) + (q % 12) * 12 : win, Li, t1 & 1, act);
-                    } else if (lane < 12) {
-                        const double* rk = rhs + (k % BAND_W) * 12;
-                        double y = 0.0;
-#pragma unroll
-                        for (int s = 0; s < 12; s++) if (s <= lane) y += Li[lane * 12 + s] * rk[s];
-                        ybuf[lane] = y;
-                        Y[(long)k * 12 + lane] = y;
-                    }
-                    band_cp_wait_all();              // this thread's copies of the staged block row
-                    band_bar_sync(1, blockDim.x);    // panel (warp 0's row included), y_k and the staged row are there
-                    // A_ij -= L_ik L_jk^T over the window in 3 x 4 tiles (12 per
-                    // block pair); pair 0, (k+1, k+1), is warp 0's unless it stays unfactored
-                    const int npair = nk * (nk + 1) / 2;
-                    for (int e = t1 + (factor_next ? 12 : 0); e < npair * 12; e += n1) {
-                        int p = e / 12, tile = e % 12;
-                        int i = k + 1 + tri_a[p], j = k + 1 + tri_b[p];
-                        int r0t = (tile / 3) * 3, c0t = (tile % 3) * 4;
-                        const double* Lia = slot(i, k) + r0t * 12;
-                        const double* Ljb = slot(j, k) + c0t * 12;
-                        // rows 0, 4 and 8 of a block share a bank (12 doubles per
-                        // row): the lanes of the three column groups walk the 12
-                        // columns rotated by 0, 1 and 2, so the rows they read at
-                        // once lie on different banks
-                        const int rot = c0t >> 2;
-                        double acc[3][4] = {};
-#pragma unroll
-                        for (int s0 = 0; s0 < 12; s0++) {
-                            const int s = s0 + rot < 12 ? s0 + rot : s0 + rot - 12;
-                            double li[3], lj[4];
-#pragma unroll
-                            for (int a2 = 0; a2 < 3; a2++) li[a2] = Lia[a2 * 12 + s];
-#pragma unroll
-                            for (int b2 = 0; b2 < 4; b2++) lj[b2] = Ljb[b2 * 12 + s];
-#pragma unroll
-                            for (int a2 = 0; a2 < 3; a2++)
-#pragma unroll
-                                for (int b2 = 0; b2 < 4; b2++) acc[a2][b2] += li[a2] * lj[b2];
-                        }
-                        double* Aij = slot(i, j);
-#pragma unroll
-                        for (int a2 = 0; a2 < 3; a2++)
-#pragma unroll
-                            for (int b2 = 0; b2 < 4; b2++) Aij[(r0t + a2) * 12 + c0t + b2] -= acc[a2][b2];
-                    }
-                    // rhs_i -= L_ik y_k
-                    for (int t = t1; t < 12 * nk; t += n1) {
-                        int i = k + 1 + t / 12, r = t % 12;
-                        const double* R = slot(i, k) + r * 12;
-                        double acc = 0.0;
-#pragma unroll
-                        for (int c = 0; c < 12; c++) acc += R[c] * ybuf[c];
-                        rhs[(i % BAND_W) * 12 + r] -= acc;
-                    }
-                    // factor column k to global: Linv_k, then L(k + d, k)
-                    for (int e = t1; e < (nk + 1) * 144; e += n1) {
-                        int d = e / 144, q = e % 144;
-                        L[((long)k * BAND_W + d) * 144 + q] = d == 0 ? Li[q] : slot(k + d, k)[q];
-                    }
-                    // block row k + 1 + wb enters the window (staged during the
-                    // previous column; its ring row is that of row k, free now),
-                    // and row k + 2 + wb is fetched
-                    const int m1 = k + 1 + wb, m2 = k + 2 + wb;
-                    if (m1 < N) {
-                        const double* src = stage + (m1 & 1) * BAND_W * 144;
-                        for (int e = t1; e < (wb + 1) * 144; e += n1) {
-                            int q = e / 144, x = e % 144;             // block q: column k + 1 + q
-                            slot(m1, k + 1 + q)[x] = src[e];
-                        }
-                        if (t1 < 12) rhs[(m1 % BAND_W) * 12 + t1] = gst[(m1 & 1) * 12 + t1];
-                    }
-                    if (m2 < N) fetch_row(m2);
-                }
-                __syncthreads();
-            }
-        };
-        // warp 0: x_k = Linv_k^T (y_k - sum_d L_{k+d,k}^T x_{k+d}) for
-        // k = kfirst down to 0, the solution blocks above kfirst already in
-        // xs.  The record of column k (its factor blocks, then y_k) sits in
-        // ring buffer k % 3 of cst, fetched two columns ahead.  After column
-        // kcall the callback runs (once).
-        auto backward = [&](int kfirst, int kcall, auto&& callback) {
-            auto fetch_col = [&](int kk) {
-                const int nkk = min(wb, N - 1 - kk);
-                double* dst = cst + (kk % 3) * BAND_CREC;
-                const double* src = L + (long)kk * BAND_W * 144;
-                for (int e = lane; e < (nkk + 1) * 72 + 6; e += 32) {
-                    if (e < (nkk + 1) * 72) band_cp16(dst + 2 * e, src + 2 * e);
-                    else band_cp16(dst + BAND_W * 144 + 2 * (e - (nkk + 1) * 72), Y + (long)kk * 12 + 2 * (e - (nkk + 1) * 72));
-                }
-                band_cp_commit();
-            };
-            fetch_col(kfirst);
-            if (kfirst >= 1) { fetch_col(kfirst - 1); band_cp_wait_but_one(); } else band_cp_wait_all();
-            __syncwarp();
-            const int r = lane % 12, half = lane / 12;
-            for (int k = kfirst; k >= 0; k--) {
-                const int nk = min(wb, N - 1 - k);
-                const double* col = cst + (k % 3) * BAND_CREC;
-                if (k >= 2) fetch_col(k - 2);        // into the buffer column k + 1 used
-                // t_r = y_k[r] - sum_d (L_{k+d,k}^T x_{k+d})[r]: lanes r and r + 12 take alternate blocks d
-                double t = 0.0;
-                if (lane < 24) {
-                    double acc0 = half == 0 ? col[BAND_W * 144 + r] : 0.0, acc1 = 0.0;
-                    for (int d = 1 + half; d <= nk; d += 2) {
-                        const double* B = col + d * 144;
-                        const double* xi = xs + ((k + d) % BAND_W) * 12;
-#pragma unroll
-                        for (int c = 0; c < 12; c += 2) {
-                            acc0 = fma(-B[c * 12 + r], xi[c], acc0);
-                            acc1 = fma(-B[(c + 1) * 12 + r], xi[c + 1], acc1);
-                        }
-                    }
-                    t = acc0 + acc1;
-                }
-                t += __shfl_sync(0xffffffffu, t, (lane + 12) & 31);
-                // x_k[lane] = sum_{c >= lane} Linv[c][lane] t_c
-                double x = 0.0;
-#pragma unroll
-                for (int c = 0; c < 12; c++) {
-                    const double tc = __shfl_sync(0xffffffffu, t, c);
-                    if (lane < 12 && c >= lane) x += col[c * 12 + lane] * tc;
-                }
-                if (lane < 12) { du[12L * ord[k] + lane] = x; xs[(k % BAND_W) * 12 + lane] = x; }
-                if (k == kcall) callback();
-                // column k - 1 (fetched during column k + 1) must have landed; the
-                // fetch issued in this column may still be in flight
-                if (k >= 2) band_cp_wait_but_one(); else band_cp_wait_all();
-                __syncwarp();
-            }
-        };
-        auto nothing = [] {};
-
-        if (warp > 0 && wb + 1 < N) fetch_row(wb + 1);
-        __syncthreads();
-        if (warp == 0) factor_diag(0);
-        __syncthreads();
-        // with a body bandwidth wb >= 1 (a connected component of two or more
-        // bodies), every column but the last has nk >= 1 blocks below the diagonal
-        columns(0, ncol1);
-        if (!split) {
-            if (warp == 0) backward(N - 1, -1, nothing);
-            band_cluster_arrive(); band_cluster_wait();
-            band_cluster_arrive(); band_cluster_wait();
-        } else if (crank == 1) {
-            // hand S (positions ncol1..N-1, the separator in reverse order)
-            // to CTA 0 in this sub-component's unused factor slots: block
-            // (p, q) at (p BAND_W + p - q), its right-hand side at Y + 12 p
-            for (int e = tid; e < wb * BAND_W * 144; e += blockDim.x) {
-                const int p = ncol1 + e / (BAND_W * 144), d = (e / 144) % BAND_W, x = e % 144;
-                if (p - d >= ncol1) L[((long)p * BAND_W + d) * 144 + x] = slot(p, p - d)[x];
-            }
-            for (int e = tid; e < wb * 12; e += blockDim.x) Y[(long)(ncol1 + e / 12) * 12 + e % 12] = rhs[((ncol1 + e / 12) % BAND_W) * 12 + e % 12];
-            __threadfence();
-            band_cluster_arrive(); band_cluster_wait();       // S handed over
-            band_cluster_arrive(); band_cluster_wait();       // S solved by CTA 0
-            if (warp == 0) {
-                // x of the separator from du, then the backward half
-                for (int e = lane; e < wb * 12; e += 32) {
-                    const int p = ncol1 + e / 12;
-                    xs[(p % BAND_W) * 12 + e % 12] = __ldcg(du + 12L * ord[p] + e % 12);
-                }
-                __syncwarp();
-                backward(ncol1 - 1, -1, nothing);
-            }
+        const double* L1 = split ? Lg + loff[cb] * 144 : nullptr;
+        const double* Y1 = split ? Lg + ltot * 144 + (loff[cb] / BW) * 12 : nullptr;
+        const int nt1 = split ? msplit + (cptr[cb + 1] - cptr[cb]) - 1 : 0;
+#define BAND_CASE(w) case w: band_job<w, BW, SIGNED>(J, split, crank, L1, Y1, nt1, du, status); break
+        if constexpr (BW == BAND_W) {
+            switch (J.wb + 1) { BAND_CASE(2); BAND_CASE(3); BAND_CASE(4); BAND_CASE(5); BAND_CASE(6); BAND_CASE(7); BAND_CASE(8); BAND_CASE(9); }
         } else {
-            band_cluster_arrive(); band_cluster_wait();       // CTA 1's half of S is in global memory
-            // S = W0 + W1 - A_SS: window row i (forward position) takes block
-            // (i, j) of CTA 1 as its transposed reverse block (pj, pi),
-            // pi = Nt - 1 - i with Nt = m + N1 the component size
-            const int ncb = cptr[cb + 1] - cptr[cb];
-            const double* L1 = Lg + loff[cb] * 144;
-            const double* Y1 = Lg + ltot * 144 + (loff[cb] / BAND_W) * 12;
-            const int nt1 = msplit + ncb - 1;                 // forward position i <-> reverse position nt1 - i
-            for (int e = tid; e < wb * wb * 144; e += blockDim.x) {
-                const int i = msplit + e / (wb * 144), j = msplit + (e / 144) % wb, x = e % 144;
-                if (j > i) continue;
-                const int rr = x / 12, c = x % 12, pi = nt1 - i, pj = nt1 - j;
-                const double w1 = __ldcg(L1 + ((long)pj * BAND_W + (pj - pi)) * 144 + c * 12 + rr);
-                slot(i, j)[x] += w1 - A[((long)i * BAND_W + (i - j)) * 144 + x];
-            }
-            for (int e = tid; e < wb * 12; e += blockDim.x) {
-                const int i = msplit + e / 12, rr = e % 12;
-                rhs[(i % BAND_W) * 12 + rr] += __ldcg(Y1 + (long)(nt1 - i) * 12 + rr) - g[12L * ord[i] + rr];
-            }
-            __syncthreads();
-            if (warp == 0) factor_diag(msplit);
-            __syncthreads();
-            columns(msplit, N);
-            if (warp == 0) {
-                backward(N - 1, msplit, [&] { __threadfence(); band_cluster_arrive(); });
-            } else {
-                band_cluster_arrive();
-            }
-            band_cluster_wait();
+            switch (J.wb + 1) { BAND_CASE(10); BAND_CASE(11); BAND_CASE(12); }
         }
+#undef BAND_CASE
         __syncthreads();
     }
 }
@@ -800,7 +900,7 @@ struct DenseState {
     std::vector<int> done, parent, size, root, bmap, fill;
     std::vector<int> adj_ptr, adj, pos, deg, members, mptr, bfs;
     bool smem_set[2] = {false, false};
-    bool band_smem_set = false;
+    bool band_smem_set[2][2] = {};
 };
 static DenseState* ds_of(Engine* E) { return reinterpret_cast<DenseState*>(E->dense_state); }
 
@@ -836,7 +936,7 @@ static int dense_init(Engine* E) {
     cusolverDnSetStream(D->h, E->stream);
     // component maps, small-component lists, band sub-components (a split
     // component's separator appears in both halves) and band jobs
-    size_t ni = 10 * (size_t)E->nb + 16;
+    size_t ni = 12 * (size_t)E->nb + 32;
     if (cudaMalloc(&D->imap_d, sizeof(int) * ni) != cudaSuccess) return E->fail(ABD_ERR_CUDA, "cudaMalloc maps");
     if (cudaMallocHost(&D->imap_h, sizeof(int) * ni) != cudaSuccess) return E->fail(ABD_ERR_CUDA, "cudaMallocHost maps");
     if (cudaMalloc(&D->loff_d, sizeof(long long) * (E->nb + 1)) != cudaSuccess) return E->fail(ABD_ERR_CUDA, "cudaMalloc band offsets");
@@ -1005,41 +1105,48 @@ static int dense_solve_t(Engine* E, int* iters, int* fallback) {
     // ones (cuSOLVER)
     D->root.assign(nb, -1);
     D->bmap.assign(nb, -1);
-    std::vector<int> small_root, large_n, band_cptr(1, 0), band_bw, band_order, ord, band_jobs;
+    std::vector<int> small_root, large_n, ord;
     std::vector<long long> large_off, large_rhs;
-    long long aoff = 0, roff = 0, lblocks = 0;
-    int nmax_large = 0, nmax_small = 0, small_bodies = 0, nband = 0, ncomp_band = 0;
+    long long aoff = 0, roff = 0;
+    int nmax_large = 0, nmax_small = 0, small_bodies = 0, ncomp_band = 0, nsub = 0;
+    // band components of the narrow and the wide kernel
+    struct BandSet {
+        int stride;                              // blocks per body
+        std::vector<int> cptr{0}, bw, order, jobs;
+        std::vector<long long> loff;
+        long long blocks = 0;
+    } sets[2] = {{BAND_W}, {BAND_WIDE + 1}};
     // a band sub-component: bodies in factor order, body bandwidth
-    auto band_sub = [&](const int* bodies, int len, int bw) {
-        D->loff_h[nband] = lblocks;
-        lblocks += (long long)len * BAND_W;
-        band_order.insert(band_order.end(), bodies, bodies + len);
-        band_cptr.push_back((int)band_order.size());
-        band_bw.push_back(bw);
-        return nband++;
+    auto band_sub = [&](BandSet& B, const int* bodies, int len, int bw) {
+        B.loff.push_back(B.blocks);
+        B.blocks += (long long)len * B.stride;
+        B.order.insert(B.order.end(), bodies, bodies + len);
+        B.cptr.push_back((int)B.order.size());
+        B.bw.push_back(bw);
+        nsub++;
+        return (int)B.bw.size() - 1;
     };
     for (int b = 0; b < nb; b++) {
         int r = find(b), sz = D->size[r];
         if (sz < 2 || D->done[E->h_bscene[b]]) continue;
-        // FP32 roundings of a stiff projected Hessian can make it indefinite
-        // (the band Cholesky has no pivoting), so the band path runs in FP64
-        // mode only; there it takes every component of body bandwidth <= 8,
-        // large ones split between the two CTAs of a cluster, and cuSOLVER
-        // only the components of wider bandwidth
-        if (D->root[r] == -1 && projected && !E->mixed) {
+        // the band path takes every component of body bandwidth <= BAND_WIDE
+        // of a projected Hessian, large ones split between the two CTAs of a
+        // cluster, and cuSOLVER only wider ones
+        if (D->root[r] == -1 && projected) {
             int bw = rcm(r, ord);
-            if (bw >= 1 && bw <= BAND_MAX && sz <= BAND_ORD_MAX) {
+            if (bw >= 1 && bw <= BAND_WIDE && sz <= BAND_ORD_MAX) {
                 D->root[r] = -10 - ncomp_band++;          // marks a band component
+                BandSet& B = sets[bw > BAND_MAX];
                 const int m = band_split_point(sz, bw);
                 if (m > 0) {
                     // bodies [0, m + bw) forward, [m, sz) from the far end
-                    const int ct = band_sub(ord.data(), m + bw, bw);
+                    const int ct = band_sub(B, ord.data(), m + bw, bw);
                     std::vector<int> rev(ord.rbegin(), ord.rend() - m);
-                    const int cb = band_sub(rev.data(), sz - m, bw);
-                    band_jobs.insert(band_jobs.end(), {ct, cb, m});
+                    const int cb = band_sub(B, rev.data(), sz - m, bw);
+                    B.jobs.insert(B.jobs.end(), {ct, cb, m});
                 } else {
-                    const int ct = band_sub(ord.data(), sz, bw);
-                    band_jobs.insert(band_jobs.end(), {ct, -1, sz});
+                    const int ct = band_sub(B, ord.data(), sz, bw);
+                    B.jobs.insert(B.jobs.end(), {ct, -1, sz});
                 }
             }
         }
@@ -1085,63 +1192,72 @@ static int dense_solve_t(Engine* E, int* iters, int* fallback) {
             h_blocal[b] = D->fill[nsmall + m]++;
         }
     }
-    // band components: cptr | bandwidth | bodies in order
-    int* h_bcptr = h_sbody + small_bodies;
-    int* h_bbw = h_bcptr + nband + 1;
-    int* h_bord = h_bbw + nband;
-    for (int c = 0; c <= nband; c++) h_bcptr[c] = band_cptr[c];
-    for (int c = 0; c < nband; c++) h_bbw[c] = band_bw[c];
-    for (size_t i = 0; i < band_order.size(); i++) h_bord[i] = band_order[i];
-    int* h_pcomp = h_bord + band_order.size();
-    for (int c = 0; c < nband; c++)
-        for (int q = band_cptr[c]; q < band_cptr[c + 1]; q++) h_pcomp[q] = c;
-    int* h_jobs = h_pcomp + band_order.size();
-    for (size_t i = 0; i < band_jobs.size(); i++) h_jobs[i] = band_jobs[i];
-    const size_t nints = 2 * (size_t)nb + nsmall + 1 + small_bodies + 2 * (size_t)nband + 1 + 2 * band_order.size() +
-                         band_jobs.size();
+    // band components of each kernel: cptr | bandwidth | bodies in order |
+    // component of each position | jobs, and the block offsets
+    int* at = h_sbody + small_bodies;
+    int* band_maps[2] = {nullptr, nullptr};
+    long long* loff_at = D->loff_h;
+    for (int q = 0; q < 2; q++) {
+        const BandSet& B = sets[q];
+        band_maps[q] = at;
+        auto put = [&](const std::vector<int>& v) { at = std::copy(v.begin(), v.end(), at); };
+        put(B.cptr); put(B.bw); put(B.order);
+        for (size_t c = 0; c < B.bw.size(); c++) at = std::fill_n(at, B.cptr[c + 1] - B.cptr[c], (int)c);
+        put(B.jobs);
+        loff_at = std::copy(B.loff.begin(), B.loff.end(), loff_at);
+    }
+    const size_t nints = at - h;
     CUDA_TRY(cudaMemcpyAsync(D->imap_d, h, sizeof(int) * nints, cudaMemcpyHostToDevice, st));
     const int* d_bmap = D->imap_d; const int* d_blocal = D->imap_d + nb;
     const int* d_sptr = D->imap_d + 2 * nb; const int* d_sbody = d_sptr + nsmall + 1;
     CUDA_TRY(cudaMemsetAsync(D->info, 0, sizeof(int), st));      // status of the band and small kernels
-    if (nband > 0) {
-        const int* d_bcptr = d_sbody + small_bodies;
-        const int* d_bbw = d_bcptr + nband + 1;
-        const int* d_bord = d_bbw + nband;
-        size_t need = ((size_t)lblocks * 144 + 12 * band_order.size()) * sizeof(double);
+    if (nsub > 0) {
+        size_t doubles[2];
+        for (int q = 0; q < 2; q++) doubles[q] = (size_t)sets[q].blocks * 144 + 12 * sets[q].order.size();
+        const size_t need = (doubles[0] + doubles[1]) * sizeof(double);
         if (need > D->Lg_bytes) {
             if (D->Lg) cudaFree(D->Lg);
             if (D->Ab) cudaFree(D->Ab);
-            D->Ab = nullptr;
+            D->Lg = nullptr; D->Ab = nullptr;
             D->Lg_bytes = std::max(2 * need, (size_t)1 << 20);
             if (cudaMalloc(&D->Lg, D->Lg_bytes) != cudaSuccess || cudaMalloc(&D->Ab, D->Lg_bytes) != cudaSuccess) {
                 D->Lg_bytes = 0;
                 return E->fail(ABD_ERR_CUDA, "cudaMalloc band factors");
             }
         }
-        CUDA_TRY(cudaMemcpyAsync(D->loff_d, D->loff_h, sizeof(long long) * nband, cudaMemcpyHostToDevice, st));
-        const size_t smem = (size_t)band_smem_doubles() * sizeof(double);
-        if (!D->band_smem_set) {
-            CUDA_TRY(cudaFuncSetAttribute(k_band_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-            D->band_smem_set = true;
-        }
-        const int* d_pcomp = d_bord + band_order.size();
-        const int* d_jobs = d_pcomp + band_order.size();
-        const int npos = (int)band_order.size(), njobs = (int)band_jobs.size() / 3;
-        k_band_gather<T><<<grid_for(32L * npos * BAND_W), 256, 0, st>>>(npos, d_pcomp, d_bcptr, d_bord, d_bbw, D->loff_d,
-                                                                       E->row_ptr, E->bcol, (const T*)E->vals, (double*)D->Ab);
-        E->launches++;
+        CUDA_TRY(cudaMemcpyAsync(D->loff_d, D->loff_h, sizeof(long long) * nsub, cudaMemcpyHostToDevice, st));
         int ph = phase_begin(E, PH_BAND);
-        // one cluster of two CTAs per job
-        k_band_solve<<<2 * njobs, BAND_THREADS, smem, st>>>(njobs, d_jobs, d_bcptr, d_bord, d_bbw, D->loff_d,
-                                                            (const double*)D->Ab, lblocks, E->g, (double*)D->Lg, E->du,
-                                                            D->info);
-        // per component: band blocks read, factor written and read back,
-        // g read, y and du written and read
         double bytes = 0;
-        for (int c = 0; c < nband; c++)
-            bytes += (band_cptr[c + 1] - band_cptr[c]) * ((band_bw[c] + 1) * 144.0 * sizeof(double) * 3 + 96.0 * 4);
+        for (int q = 0; q < 2; q++) {
+            const BandSet& B = sets[q];
+            const int n = (int)B.bw.size(), npos = (int)B.order.size(), njobs = (int)B.jobs.size() / 3;
+            if (n == 0) continue;
+            const int* d_cptr = D->imap_d + (band_maps[q] - h);
+            const int* d_bw = d_cptr + n + 1;
+            const int* d_ord = d_bw + n;
+            const int* d_pcomp = d_ord + npos;
+            const int* d_jobs = d_pcomp + npos;
+            const long long* d_loff = D->loff_d + (q ? sets[0].bw.size() : 0);
+            double* Ab = (double*)D->Ab + (q ? doubles[0] : 0);
+            double* Lg = (double*)D->Lg + (q ? doubles[0] : 0);
+            auto kernel = q ? k_band_solve<BAND_WIDE + 1, sizeof(T) == 4> : k_band_solve<BAND_W, sizeof(T) == 4>;
+            const size_t smem = (size_t)band_smem_doubles(B.stride) * sizeof(double);
+            if (!D->band_smem_set[q][sizeof(T) == 8]) {
+                CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+                D->band_smem_set[q][sizeof(T) == 8] = true;
+            }
+            k_band_gather<T><<<grid_for(32L * npos * B.stride), 256, 0, st>>>(B.stride, npos, d_pcomp, d_cptr, d_ord, d_bw, d_loff,
+                                                                             E->row_ptr, E->bcol, (const T*)E->vals, Ab);
+            // one cluster of two CTAs per job
+            kernel<<<2 * njobs, BAND_THREADS, smem, st>>>(njobs, d_jobs, d_cptr, d_ord, d_bw, d_loff, Ab, B.blocks, E->g, Lg,
+                                                          E->du, D->info);
+            E->launches += 2;
+            // per component: band blocks read, factor written and read back,
+            // g read, y and du written and read
+            for (int c = 0; c < n; c++)
+                bytes += (B.cptr[c + 1] - B.cptr[c]) * ((B.bw[c] + 1) * 144.0 * sizeof(double) * 3 + 96.0 * 4);
+        }
         phase_end(E, ph, bytes);
-        E->launches++;
     }
     if (nsmall > 0) {
         size_t smem = ((size_t)nmax_small * (nmax_small + 1) + nmax_small) * sizeof(T);

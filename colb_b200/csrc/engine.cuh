@@ -51,25 +51,36 @@ DV uint32_t cell_hash(int scene, int cx, int cy, int cz) {
            ((uint32_t)scene * 2654435761u);
 }
 
+// The cells that hold every stored item whose box can overlap [qlo, qhi]:
+// c0 <= c <= c1 per axis.  False: visit nothing.  Non-finite boxes (a diverged
+// state) visit nothing; the Newton loop's NaN check reports them.  The cell
+// edge h bounds every box extent, so a finite query spans at most 3 cells per
+// axis.
+DV bool grid_range(float h, float4 qlo, float4 qhi, int (&c0)[3], int (&c1)[3]) {
+    if (!(h > 0.f && h < 3.0e38f)) return false;
+    if (!(isfinite(qlo.x) && isfinite(qlo.y) && isfinite(qlo.z) && isfinite(qhi.x) && isfinite(qhi.y) && isfinite(qhi.z))) return false;
+    float fx0 = floorf((qlo.x - h) / h), fx1 = floorf(qhi.x / h);
+    float fy0 = floorf((qlo.y - h) / h), fy1 = floorf(qhi.y / h);
+    float fz0 = floorf((qlo.z - h) / h), fz1 = floorf(qhi.z / h);
+    if (fx1 - fx0 > 4.f || fy1 - fy0 > 4.f || fz1 - fz0 > 4.f) return false;
+    if (fabsf(fx0) > 1.0e9f || fabsf(fy0) > 1.0e9f || fabsf(fz0) > 1.0e9f) return false;
+    c0[0] = (int)fx0; c1[0] = (int)fx1; c0[1] = (int)fy0; c1[1] = (int)fy1; c0[2] = (int)fz0; c1[2] = (int)fz1;
+    return true;
+}
+DV bool boxes_overlap(float4 lo, float4 hi, float4 qlo, float4 qhi) {
+    return !(lo.x > qhi.x || hi.x < qlo.x || lo.y > qhi.y || hi.y < qlo.y || lo.z > qhi.z || hi.z < qlo.z);
+}
+
 // Visit every stored item whose box overlaps [qlo,qhi] in the same scene,
 // each exactly once.
 template <class F>
 DV void grid_visit(const GridView& G, float4 qlo, float4 qhi, int scene, F&& visit) {
     float h = *G.cell;
-    // non-finite boxes (a diverged state) visit nothing; the Newton loop's
-    // NaN check reports them.  The cell edge bounds every box extent, so a
-    // finite query spans at most 3 cells per axis.
-    if (!(h > 0.f && h < 3.0e38f)) return;
-    if (!(isfinite(qlo.x) && isfinite(qlo.y) && isfinite(qlo.z) && isfinite(qhi.x) && isfinite(qhi.y) && isfinite(qhi.z))) return;
-    float fx0 = floorf((qlo.x - h) / h), fx1 = floorf(qhi.x / h);
-    float fy0 = floorf((qlo.y - h) / h), fy1 = floorf(qhi.y / h);
-    float fz0 = floorf((qlo.z - h) / h), fz1 = floorf(qhi.z / h);
-    if (fx1 - fx0 > 4.f || fy1 - fy0 > 4.f || fz1 - fz0 > 4.f) return;
-    if (fabsf(fx0) > 1.0e9f || fabsf(fy0) > 1.0e9f || fabsf(fz0) > 1.0e9f) return;
-    int x0 = (int)fx0, x1 = (int)fx1, y0 = (int)fy0, y1 = (int)fy1, z0 = (int)fz0, z1 = (int)fz1;
-    for (int cz = z0; cz <= z1; cz++)
-        for (int cy = y0; cy <= y1; cy++)
-            for (int cx = x0; cx <= x1; cx++) {
+    int c0[3], c1[3];
+    if (!grid_range(h, qlo, qhi, c0, c1)) return;
+    for (int cz = c0[2]; cz <= c1[2]; cz++)
+        for (int cy = c0[1]; cy <= c1[1]; cy++)
+            for (int cx = c0[0]; cx <= c1[0]; cx++) {
                 uint32_t key = cell_hash(scene, cx, cy, cz) & G.mask;
                 int b = G.bstart[key];
                 if (b < 0) continue;
@@ -79,8 +90,7 @@ DV void grid_visit(const GridView& G, float4 qlo, float4 qhi, int scene, F&& vis
                     if (G.scene && G.scene[j] != scene) continue;
                     float4 lo = G.lo[j];
                     if ((int)floorf(lo.x / h) != cx || (int)floorf(lo.y / h) != cy || (int)floorf(lo.z / h) != cz) continue;
-                    float4 hi = G.hi[j];
-                    if (lo.x > qhi.x || hi.x < qlo.x || lo.y > qhi.y || hi.y < qlo.y || lo.z > qhi.z || hi.z < qlo.z) continue;
+                    if (!boxes_overlap(lo, G.hi[j], qlo, qhi)) continue;
                     visit(j);
                 }
             }

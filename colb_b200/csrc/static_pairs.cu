@@ -9,9 +9,9 @@
 // keys, buckets, per-edge counts, radix-sort and scan scratch) lives in the
 // file-scope __device__ arrays below, sized for ABD_STATIC_MAX_EDGES edges.
 // Every GPU that loads the library holds these arrays until the process
-// exits: boxes 2 MiB, grid keys and values 1 MiB, buckets 1 MiB, per-edge
-// counts and offsets 0.5 MiB, sort and scan scratch 4 MiB, about 8.5 MiB in
-// all.
+// exits: boxes 4 MiB (by edge and by cell), grid keys 0.5 MiB, buckets 1 MiB,
+// per-edge counts, offsets and list positions 0.75 MiB, partner lists 4 MiB,
+// scan scratch 0.25 MiB, about 10.5 MiB in all.
 //
 // Host code must not pass the arrays' names to a kernel: in host code a
 // __device__ symbol names a host-side stand-in, not device memory.  The
@@ -32,19 +32,20 @@ std::string& abd_global_error();   // capi.cu: the message abd_last_error(NULL) 
 
 #define ST_MAXE ABD_STATIC_MAX_EDGES
 #define ST_H (2 * ST_MAXE)
-#define ST_CUB_BYTES (4 << 20)
+#define ST_CUB_BYTES (256 << 10)
+#define ST_POOL (1 << 20)                // partners that the lists of all edges hold
+#define ST_LIST 96                       // partners of one edge that a list holds
 
-static __device__ __align__(256) float4 g_st_lo[ST_MAXE];
-static __device__ __align__(256) float4 g_st_hi[ST_MAXE];
-static __device__ __align__(256) uint32_t g_st_keys[2 * ST_MAXE];
-static __device__ __align__(256) int g_st_vals[2 * ST_MAXE];
-static __device__ __align__(256) int g_st_bucket[2 * ST_H];
-static __device__ __align__(256) int g_st_count[2 * (ST_MAXE + 1) + 4];   // counts, offsets, bad-edge flag
-static __device__ __align__(256) float g_st_cell[4];
+static __device__ __align__(256) float4 g_st_box[4 * ST_MAXE];               // by edge: lo, hi; by cell: lo, hi
+static __device__ __align__(256) uint32_t g_st_keys[2 * ST_MAXE];            // bucket, place in it
+static __device__ __align__(256) int g_st_bucket[2 * (ST_H + 1) + 4];        // counts and flags (StaticFlags), starts
+static __device__ __align__(256) int g_st_count[3 * (ST_MAXE + 1)];          // pairs, offsets, list positions
+static __device__ __align__(256) int g_st_pool[ST_POOL];
 static __device__ __align__(256) unsigned char g_st_cub[ST_CUB_BYTES];
 
+struct StaticFlags { float cell; int bad; int pooled; int pad; };            // cell edge; bad edge index; pool entries taken
 struct StaticScratch {
-    float4* lo; float4* hi; uint32_t* keys; int* vals; int* bucket; int* count; float* cell; void* cub;
+    float4* box; uint32_t* keys; int* bucket; int* count; int* pool; void* cub;
     bool ready;
 };
 static StaticScratch g_scratch[64];
@@ -56,10 +57,9 @@ static int scratch_for_device(int dev, StaticScratch** out, std::string& err) {
     StaticScratch& S = g_scratch[dev];
     if (!S.ready) {
         struct { void** p; const void* sym; } t[] = {
-            {(void**)&S.lo, (const void*)&g_st_lo}, {(void**)&S.hi, (const void*)&g_st_hi},
-            {(void**)&S.keys, (const void*)&g_st_keys}, {(void**)&S.vals, (const void*)&g_st_vals},
+            {(void**)&S.box, (const void*)&g_st_box}, {(void**)&S.keys, (const void*)&g_st_keys},
             {(void**)&S.bucket, (const void*)&g_st_bucket}, {(void**)&S.count, (const void*)&g_st_count},
-            {(void**)&S.cell, (const void*)&g_st_cell}, {(void**)&S.cub, (const void*)&g_st_cub}};
+            {(void**)&S.pool, (const void*)&g_st_pool}, {(void**)&S.cub, (const void*)&g_st_cub}};
         for (auto& e : t) {
             cudaError_t rc = cudaGetSymbolAddress(e.p, e.sym);
             if (rc != cudaSuccess) {
@@ -73,12 +73,15 @@ static int scratch_for_device(int dev, StaticScratch** out, std::string& err) {
     return ABD_OK;
 }
 
-// boxes of the float32 copies of the endpoints (contact.py:150-154), padded
-__global__ void k_st_boxes(int ne, const double* __restrict__ x, const int* __restrict__ edges, float pad,
-                           float4* lo, float4* hi, float* cell) {
+// boxes of the float32 copies of the endpoints (contact.py:150-154), padded.
+// Every edge index must name a vertex of x: one that does not sets F->bad, and
+// the kernels after this one do nothing.
+__global__ void k_st_boxes(int ne, int nv, const double* __restrict__ x, const int* __restrict__ edges, float pad,
+                           float4* lo, float4* hi, StaticFlags* F) {
     float ext = 0.f;
     GS_LOOP(e, ne) {
         int a = edges[2*e], b = edges[2*e+1];
+        if ((unsigned)a >= (unsigned)nv || (unsigned)b >= (unsigned)nv) { F->bad = 1; continue; }
         float l[3], h[3];
 #pragma unroll
         for (int k = 0; k < 3; k++) {
@@ -89,75 +92,201 @@ __global__ void k_st_boxes(int ne, const double* __restrict__ x, const int* __re
         ext = fmaxf(ext, fmaxf(h[0] - l[0], fmaxf(h[1] - l[1], h[2] - l[2])));
     }
     for (int o = 16; o > 0; o >>= 1) ext = fmaxf(ext, __shfl_xor_sync(0xffffffffu, ext, o));
-    if ((threadIdx.x & 31) == 0 && ext > 0.f) atomic_max_pos(cell, ext);
+    if ((threadIdx.x & 31) == 0 && ext > 0.f) atomic_max_pos(&F->cell, ext);
 }
-__global__ void k_st_keys(int n, const float4* __restrict__ lo, const float* cell, uint32_t mask, uint32_t* keys, int* vals) {
-    float h = fmaxf(*cell, 1e-6f);
+// The edges are put in order of their buckets by counting: an edge's place in
+// its bucket is the count it found there (k_st_keys), a bucket's start the sum
+// of the counts below it, and k_st_fill copies the boxes to their places, so a
+// query reads a bucket's boxes from consecutive addresses.  The order within a
+// bucket is not fixed; the order of the results does not depend on it.  (A
+// radix sort of the keys took 45 us for 55,296 edges.)
+__global__ void k_st_keys(int n, const float4* __restrict__ lo, const StaticFlags* F, uint32_t mask, uint32_t* key,
+                          uint32_t* place, int* bucket) {
+    if (F->bad) return;
+    float h = fmaxf(F->cell, 1e-6f);
     GS_LOOP(i, n) {
         float4 l = lo[i];
-        keys[i] = cell_hash(0, (int)floorf(l.x / h), (int)floorf(l.y / h), (int)floorf(l.z / h)) & mask;
-        vals[i] = (int)i;
+        uint32_t k = cell_hash(0, (int)floorf(l.x / h), (int)floorf(l.y / h), (int)floorf(l.z / h)) & mask;
+        key[i] = k;
+        place[i] = atomicAdd(bucket + k, 1);
     }
 }
-__global__ void k_st_ranges(int n, const uint32_t* __restrict__ keys, int* bstart, int* bend) {
+// boxes in bucket order, the edge in lo's fourth word
+__global__ void k_st_fill(int n, const float4* __restrict__ lo, const float4* __restrict__ hi, const StaticFlags* F,
+                          const uint32_t* __restrict__ key, const uint32_t* __restrict__ place,
+                          const int* __restrict__ start, float4* lo_s, float4* hi_s) {
+    if (F->bad) return;
     GS_LOOP(i, n) {
-        uint32_t k = keys[i];
-        if (i == 0 || keys[i-1] != k) bstart[k] = (int)i;
-        if (i == n - 1 || keys[i+1] != k) bend[k] = (int)i + 1;
+        int at = start[key[i]] + (int)place[i];
+        float4 l = lo[i];
+        l.w = __int_as_float((int)i);
+        lo_s[at] = l; hi_s[at] = hi[i];
     }
 }
-// mode 0: count per edge; mode 1: write vertex quadruples, sorted by
-// partner, the rows that fit below cap (an edge whose rows cross cap keeps
-// the ones it visited first, so on overflow the rows are not the first cap
-// rows of the complete sorted list)
-__global__ void k_st_pairs(int ne, GridView GV, const double* __restrict__ x, const int* __restrict__ edges,
-                           const float4* __restrict__ qlo, const float4* __restrict__ qhi, double cand, int mode,
-                           int* count, const int* off, int* out4, int cap) {
-    float fc = __double2float_rn(cand);
-    GS_LOOP(i, ne) {
-        int ii = (int)i;
-        int a0 = edges[2*i], a1 = edges[2*i+1];
-        float p1[3], q1[3];
-        for (int k = 0; k < 3; k++) { p1[k] = __double2float_rn(x[3*a0+k]); q1[k] = __double2float_rn(x[3*a1+k]); }
-        int c = 0, base = mode == 1 ? off[i] : 0;
-        grid_visit(GV, qlo[i], qhi[i], 0, [&](int j) {
-            if (j <= ii) return;
-            int b0 = edges[2*j], b1 = edges[2*j+1];
-            if (a0 == b0 || a0 == b1 || a1 == b0 || a1 == b1) return;
-            float p2[3], q2[3];
-            for (int k = 0; k < 3; k++) { p2[k] = __double2float_rn(x[3*b0+k]); q2[k] = __double2float_rn(x[3*b1+k]); }
-            float s, t, d;
-            seg_seg_f32(p1, q1, p2, q2, 1e-6f, s, t, d);
-            if (!(d < fc)) return;
-            if (mode == 1) {
-                // the partner edge index goes in slot 2 until the segment is sorted
-                int at = base + c;
-                if ((unsigned)at < (unsigned)cap) { out4[4*at] = a0; out4[4*at+1] = a1; out4[4*at+2] = j; out4[4*at+3] = -1; }
+
+struct StaticGrid {
+    const float4 *lo, *hi;               // by edge
+    const float4 *lo_s, *hi_s;           // by bucket
+    const int* start;                    // bucket k: [start[k], start[k + 1])
+    uint32_t mask;
+    const double* x; const int* edges;
+    float cand;
+};
+// One warp visits the partners j > i of edge i closer than cand: emit(found, j)
+// is called by all lanes together, with the lane's j where found.  The lanes
+// look up 32 cells at once and then take the items of all of them side by side
+// (a lane finds the cell of its item by bisecting the running sums), and the
+// boxes that overlap wait in `queue` (64 ints of the warp's shared memory)
+// until 32 segment distances can be computed at once.
+template <class F>
+DV void st_visit(const StaticGrid& G, float h, int i, int* queue, F&& emit) {
+    const int lane = threadIdx.x & 31;
+    const float4 qlo = G.lo[i], qhi = G.hi[i];
+    const int a0 = G.edges[2*i], a1 = G.edges[2*i+1];
+    int c0[3], c1[3];
+    if (!grid_range(h, qlo, qhi, c0, c1)) return;
+    const int nx = c1[0] - c0[0] + 1, ny = c1[1] - c0[1] + 1, ncell = nx * ny * (c1[2] - c0[2] + 1);
+    float p1[3], q1[3];
+    for (int k = 0; k < 3; k++) { p1[k] = __double2float_rn(G.x[3*a0+k]); q1[k] = __double2float_rn(G.x[3*a1+k]); }
+    int queued = 0;
+    auto flush = [&](int n) {            // the first n <= 32 of the queue
+        bool found = lane < n;
+        int j = found ? queue[lane] : 0;
+        if (found) {
+            int b0 = G.edges[2*j], b1 = G.edges[2*j+1];
+            found = !(a0 == b0 || a0 == b1 || a1 == b0 || a1 == b1);
+            if (found) {
+                float p2[3], q2[3];
+                for (int k = 0; k < 3; k++) { p2[k] = __double2float_rn(G.x[3*b0+k]); q2[k] = __double2float_rn(G.x[3*b1+k]); }
+                float s, t, d;
+                seg_seg_f32(p1, q1, p2, q2, 1e-6f, s, t, d);
+                found = d < G.cand;
             }
-            c++;
-        });
-        if (mode == 0) { count[i] = c; continue; }
-        // order this edge's pairs by partner edge index, as the handle-based
-        // detection does, then expand partners to their vertex ids
-        int lo = base, hi = min(base + c, cap);
-        for (int k = lo + 1; k < hi; k++) {
-            int v2 = out4[4*k+2];
-            int m = k - 1;
-            while (m >= lo && out4[4*m+2] > v2) { out4[4*(m+1)+2] = out4[4*m+2]; m--; }
-            out4[4*(m+1)+2] = v2;
         }
-        for (int k = lo; k < hi; k++) {
-            int j = out4[4*k+2];
-            out4[4*k+2] = edges[2*j]; out4[4*k+3] = edges[2*j+1];
+        emit(found, j);
+        __syncwarp();
+    };
+    for (int cb = 0; cb < ncell; cb += 32) {
+        int cell = cb + lane, b = 0, n = 0;
+        const int cx = c0[0] + cell % nx, cy = c0[1] + cell / nx % ny, cz = c0[2] + cell / (nx * ny);
+        if (cell < ncell) {
+            const uint32_t key = cell_hash(0, cx, cy, cz) & G.mask;
+            b = G.start[key]; n = G.start[key + 1] - b;
+        }
+        int sum = n;                     // items of this lane's cell and the ones before it
+        for (int o = 1; o < 32; o <<= 1) { int v = __shfl_up_sync(0xffffffffu, sum, o); if (lane >= o) sum += v; }
+        const int total = __shfl_sync(0xffffffffu, sum, 31);
+        for (int f0 = 0; f0 < total; f0 += 32) {
+            const int f = f0 + lane;
+            int c = 0;                   // the first lane whose sum exceeds f
+            for (int o = 16; o > 0; o >>= 1) c += __shfl_sync(0xffffffffu, sum, c + o - 1) <= f ? o : 0;
+            const int at = __shfl_sync(0xffffffffu, b + n - sum, c) + f;
+            const int kx = __shfl_sync(0xffffffffu, cx, c), ky = __shfl_sync(0xffffffffu, cy, c), kz = __shfl_sync(0xffffffffu, cz, c);
+            bool in = f < total;
+            int j = 0;
+            if (in) {
+                const float4 lo = G.lo_s[at];
+                j = __float_as_int(lo.w);
+                // a bucket can hold other cells' items; they are visited from their own cell
+                in = j > i && boxes_overlap(lo, G.hi_s[at], qlo, qhi) && (int)floorf(lo.x / h) == kx &&
+                     (int)floorf(lo.y / h) == ky && (int)floorf(lo.z / h) == kz;
+            }
+            const unsigned m = __ballot_sync(0xffffffffu, in);
+            if (in) queue[queued + __popc(m & ((1u << lane) - 1))] = j;
+            __syncwarp();
+            queued += __popc(m);
+            if (queued >= 32) {
+                flush(32);
+                queued -= 32;
+                const int v = lane < queued ? queue[32 + lane] : 0;
+                __syncwarp();
+                if (lane < queued) queue[lane] = v;
+                __syncwarp();
+            }
         }
     }
+    if (queued > 0) flush(queued);
 }
-// every edge index must name a vertex of x
-__global__ void k_st_check(int ne, const int* __restrict__ edges, int nv, int* bad) {
-    GS_LOOP(i, 2L * ne) { int v = edges[i]; if (v < 0 || v >= nv) *bad = 1; }
+// Counts each edge's pairs and keeps its partners, in order, at pool[at[i]].  at[i] = -1:
+// more partners than ST_LIST or than the pool has room for (k_st_write visits again).  One warp
+// per edge: with one thread per edge, a count pass and a write pass of the
+// same walk took 609 us each for 55,296 edges (245 boxes and 13 distances per
+// edge); this pass takes 117 us, the write 17.
+__global__ void __launch_bounds__(256) k_st_find(int ne, StaticGrid G, StaticFlags* F, int* count, int* at, int* pool) {
+    __shared__ int s_queue[8][64], s_list[8][ST_LIST];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    int* list = s_list[w];
+    if (F->bad) { if (threadIdx.x == 0 && blockIdx.x == 0) count[ne] = 0; return; }
+    const float h = F->cell;
+    for (int i = blockIdx.x * 8 + w; i <= ne; i += gridDim.x * 8) {
+        if (i == ne) { if (lane == 0) count[ne] = 0; break; }
+        int c = 0;
+        st_visit(G, h, i, s_queue[w], [&](bool found, int j) {
+            const unsigned m = __ballot_sync(0xffffffffu, found);
+            const int k = c + __popc(m & ((1u << lane) - 1));
+            if (found && k < ST_LIST) list[k] = j;
+            c += __popc(m);
+        });
+        __syncwarp();
+        int base = -1;
+        if (lane == 0) {
+            count[i] = c;
+            if (c > 0 && c <= ST_LIST) {
+                base = atomicAdd(&F->pooled, c);
+                if (base + c > ST_POOL) base = -1;
+            }
+            at[i] = base;
+        }
+        base = __shfl_sync(0xffffffffu, base, 0);
+        if (base >= 0)
+            for (int k = lane; k < c; k += 32) {
+                const int j = list[k];
+                int rank = 0;
+                for (int l = 0; l < c; l++) rank += list[l] < j;
+                pool[base + rank] = j;
+            }
+        __syncwarp();
+    }
 }
-__global__ void k_st_total(const int* off, int ne, int* n_out) {
+// Writes vertex quadruples, by edge and partner, the rows that fit below cap.
+// An edge without a list (see k_st_find) visits its partners again and
+// orders them where they are written; one whose rows cross cap then keeps the
+// ones it visited first.
+__global__ void __launch_bounds__(256) k_st_write(int ne, StaticGrid G, const StaticFlags* F, const int* __restrict__ count,
+                                                  const int* __restrict__ off, const int* __restrict__ at,
+                                                  const int* __restrict__ pool, int* out4, int cap, int* n_out) {
+    __shared__ int s_queue[8][64];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    if (F->bad) return;
+    const float h = F->cell;
     if (threadIdx.x == 0 && blockIdx.x == 0) *n_out = off[ne];
+    for (int i = blockIdx.x * 8 + w; i < ne; i += gridDim.x * 8) {
+        const int c = count[i], base = off[i], from = at[i];
+        if (c == 0 || base >= cap) continue;
+        const int rows = min(c, cap - base);
+        if (from < 0) {
+            int k0 = base;
+            st_visit(G, h, i, s_queue[w], [&](bool found, int j) {
+                const unsigned m = __ballot_sync(0xffffffffu, found);
+                const int k = k0 + __popc(m & ((1u << lane) - 1));
+                if (found && k < cap) out4[4L*k+2] = j;
+                k0 += __popc(m);
+            });
+            __syncwarp();
+            if (lane == 0)
+                for (int k = base + 1; k < base + rows; k++) {
+                    int j = out4[4L*k+2], m = k - 1;
+                    while (m >= base && out4[4L*m+2] > j) { out4[4L*(m+1)+2] = out4[4L*m+2]; m--; }
+                    out4[4L*(m+1)+2] = j;
+                }
+            __syncwarp();
+        }
+        for (int k = lane; k < rows; k += 32) {
+            int* o = out4 + 4L * (base + k);
+            const int j = from < 0 ? o[2] : pool[from + k];
+            o[0] = G.edges[2*i]; o[1] = G.edges[2*i+1]; o[2] = G.edges[2*j]; o[3] = G.edges[2*j+1];
+        }
+    }
 }
 
 extern "C" int abd_ee_pairs_static(const double* x_dev, const int32_t* edges_dev, int32_t n_verts, int32_t n_edges,
@@ -176,57 +305,47 @@ extern "C" int abd_ee_pairs_static(const double* x_dev, const int32_t* edges_dev
     int rc = scratch_for_device(dev, &S, err);
     if (rc) return rc;
     cudaStream_t s = (cudaStream_t)stream_ptr;
-    // clear what the previous call left behind
-    float* cell = S->cell;
-    int* bad_edge = S->count + 2 * (ST_MAXE + 1);
-    if (cudaMemsetAsync(cell, 0, sizeof(float), s) != cudaSuccess ||
-        cudaMemsetAsync(bad_edge, 0, sizeof(int), s) != cudaSuccess ||
+    if (n_edges < 2) {
+        if (cudaMemsetAsync(n_pairs_dev, 0, sizeof(int32_t), s) != cudaSuccess) { err = "abd_ee_pairs_static: cudaMemsetAsync failed"; return ABD_ERR_CUDA; }
+        return cudaStreamSynchronize(s) == cudaSuccess ? ABD_OK : ABD_ERR_CUDA;
+    }
+    int H = 64; while (H < 2 * n_edges) H <<= 1;
+    float pad = (float)(0.5 * cand_dist * (1.0 + 1e-6) + 1e-7);
+    float4 *lo = S->box, *hi = lo + ST_MAXE, *lo_s = hi + ST_MAXE, *hi_s = lo_s + ST_MAXE;
+    uint32_t *key = S->keys, *place = key + ST_MAXE;
+    StaticFlags* F = (StaticFlags*)S->bucket;
+    int *bcount = S->bucket + 4, *bstart = bcount + ST_H + 1;
+    int *count = S->count, *off = count + ST_MAXE + 1, *at = off + ST_MAXE + 1;
+    size_t need = 0, need2 = 0;
+    cub::DeviceScan::ExclusiveSum(nullptr, need, bcount, bstart, H + 1, s);
+    cub::DeviceScan::ExclusiveSum(nullptr, need2, count, off, n_edges + 1, s);
+    if (need > ST_CUB_BYTES || need2 > ST_CUB_BYTES) { err = "abd_ee_pairs_static: scan scratch exceeds the static size"; return ABD_ERR_INVALID_ARG; }
+    // clear what the previous call left behind: the flags and the bucket counts, one range
+    if (cudaMemsetAsync(F, 0, sizeof(StaticFlags) + sizeof(int) * (H + 1), s) != cudaSuccess ||
         cudaMemsetAsync(n_pairs_dev, 0, sizeof(int32_t), s) != cudaSuccess) {
         err = "abd_ee_pairs_static: cudaMemsetAsync failed"; return ABD_ERR_CUDA;
     }
-    if (n_edges < 2) return cudaStreamSynchronize(s) == cudaSuccess ? ABD_OK : ABD_ERR_CUDA;
-    {
-        int bad = 0;
-        k_st_check<<<grid_for(2L * n_edges), 256, 0, s>>>(n_edges, edges_dev, n_verts, bad_edge);
-        if (cudaMemcpyAsync(&bad, bad_edge, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
-            cudaStreamSynchronize(s) != cudaSuccess) { err = "abd_ee_pairs_static: CUDA error"; return ABD_ERR_CUDA; }
-        if (bad) { err = "abd_ee_pairs_static: an edge index is outside [0, n_verts)"; return ABD_ERR_INVALID_ARG; }
+    k_st_boxes<<<grid_for(n_edges), 256, 0, s>>>(n_edges, n_verts, x_dev, edges_dev, pad, lo, hi, F);
+    k_st_keys<<<grid_for(n_edges), 256, 0, s>>>(n_edges, lo, F, (uint32_t)(H - 1), key, place, bcount);
+    if (cub::DeviceScan::ExclusiveSum(S->cub, need, bcount, bstart, H + 1, s) != cudaSuccess) {
+        err = "abd_ee_pairs_static: scan failed"; return ABD_ERR_CUDA;
     }
-    int H = 64; while (H < 2 * n_edges) H <<= 1;
-    int bits = 0; while ((1 << bits) < H) bits++;
-    float pad = (float)(0.5 * cand_dist * (1.0 + 1e-6) + 1e-7);
-    uint32_t* keys = S->keys; uint32_t* keys_s = S->keys + ST_MAXE;
-    int* vals = S->vals; int* vals_s = S->vals + ST_MAXE;
-    int* bstart = S->bucket; int* bend = S->bucket + ST_H;
-    int* count = S->count; int* off = S->count + (ST_MAXE + 1);
-    k_st_boxes<<<grid_for(n_edges), 256, 0, s>>>(n_edges, x_dev, edges_dev, pad, S->lo, S->hi, cell);
-    k_st_keys<<<grid_for(n_edges), 256, 0, s>>>(n_edges, S->lo, cell, (uint32_t)(H - 1), keys, vals);
-    size_t need = 0;
-    cub::DeviceRadixSort::SortPairs(nullptr, need, keys, keys_s, vals, vals_s, n_edges, 0, bits, s);
-    size_t need2 = 0;
-    cub::DeviceScan::ExclusiveSum(nullptr, need2, count, off, n_edges + 1, s);
-    if (need > ST_CUB_BYTES || need2 > ST_CUB_BYTES) { err = "abd_ee_pairs_static: sort scratch exceeds the static size"; return ABD_ERR_INVALID_ARG; }
-    if (cub::DeviceRadixSort::SortPairs(S->cub, need, keys, keys_s, vals, vals_s, n_edges, 0, bits, s) != cudaSuccess) {
-        err = "abd_ee_pairs_static: radix sort failed"; return ABD_ERR_CUDA;
-    }
-    if (cudaMemsetAsync(bstart, 0xFF, sizeof(int) * H, s) != cudaSuccess) { err = "abd_ee_pairs_static: memset"; return ABD_ERR_CUDA; }
-    k_st_ranges<<<grid_for(n_edges), 256, 0, s>>>(n_edges, keys_s, bstart, bend);
-    GridView GV{S->lo, S->hi, nullptr, cell, vals_s, bstart, bend, (uint32_t)(H - 1)};
-    k_st_pairs<<<grid_for(n_edges, 128), 128, 0, s>>>(n_edges, GV, x_dev, edges_dev, S->lo, S->hi, cand_dist, 0, count,
-                                                      nullptr, pairs_dev, cap);
-    if (cudaMemsetAsync(count + n_edges, 0, sizeof(int), s) != cudaSuccess) { err = "abd_ee_pairs_static: memset"; return ABD_ERR_CUDA; }
+    k_st_fill<<<grid_for(n_edges), 256, 0, s>>>(n_edges, lo, hi, F, key, place, bstart, lo_s, hi_s);
+    StaticGrid G{lo, hi, lo_s, hi_s, bstart, (uint32_t)(H - 1), x_dev, edges_dev, (float)cand_dist};
+    k_st_find<<<grid_for(32L * n_edges), 256, 0, s>>>(n_edges, G, F, count, at, S->pool);
     if (cub::DeviceScan::ExclusiveSum(S->cub, need2, count, off, n_edges + 1, s) != cudaSuccess) {
         err = "abd_ee_pairs_static: scan failed"; return ABD_ERR_CUDA;
     }
-    k_st_pairs<<<grid_for(n_edges, 128), 128, 0, s>>>(n_edges, GV, x_dev, edges_dev, S->lo, S->hi, cand_dist, 1, count,
-                                                      off, pairs_dev, cap);
-    k_st_total<<<1, 32, 0, s>>>(off, n_edges, n_pairs_dev);
+    k_st_write<<<grid_for(32L * n_edges), 256, 0, s>>>(n_edges, G, F, count, off, at, S->pool, pairs_dev, cap, n_pairs_dev);
+    int bad = 0;
+    if (cudaMemcpyAsync(&bad, &F->bad, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess) { err = "abd_ee_pairs_static: CUDA error"; return ABD_ERR_CUDA; }
     int n = 0;
     if (cudaMemcpyAsync(&n, n_pairs_dev, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
         cudaStreamSynchronize(s) != cudaSuccess) {
         err = std::string("abd_ee_pairs_static: ") + cudaGetErrorString(cudaGetLastError());
         return ABD_ERR_CUDA;
     }
+    if (bad) { err = "abd_ee_pairs_static: an edge index is outside [0, n_verts)"; return ABD_ERR_INVALID_ARG; }
     if (n > cap) { err = "abd_ee_pairs_static: more pairs than cap (the count is in *n_pairs_dev)"; return ABD_ERR_CONTACT_OVERFLOW; }
     return ABD_OK;
 }

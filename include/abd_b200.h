@@ -343,7 +343,7 @@ int abd_get_timing(AbdHandle* h, double* ms, int64_t* launches, double* bytes);
  * quadruples (a1, a2, b1, b2), but takes DEVICE pointers: x_dev (n_verts*3
  * doubles), edges_dev (n_edges*2 ints), pairs_dev (cap*4 ints) and
  * n_pairs_dev (one int).  All scratch lives in static device arrays of the
- * library (about 8.5 MiB per GPU, held until exit) sized for
+ * library (about 10.5 MiB per GPU, held until exit) sized for
  * ABD_STATIC_MAX_EDGES edges; larger inputs are rejected with
  * ABD_ERR_INVALID_ARG.  The first call on each device looks those arrays up
  * and caches their addresses (make it before any stream capture; after a

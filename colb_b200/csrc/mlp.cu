@@ -2,7 +2,7 @@
 // reference): 48 -> 256 -> 256 -> 256 -> 12, GELU, BF16 weights and
 // activations, FP32 accumulation.
 //
-// Inference (every step of warm_start 3): one CTA of 4 warps runs 128 bodies
+// Inference (every step of warm_start 3): one CTA of 16 warps runs 128 bodies
 // through all four layers.  Layer weights are stored once in the UMMA
 // canonical K-major layout (8x8 core matrices, no swizzle) and copied into
 // shared memory with one bulk asynchronous copy per layer; the activations
@@ -34,7 +34,7 @@ static_assert(NPARAM == ABD_MLP_NPARAM, "parameter count");
 constexpr int PW1 = 0, PW2 = PW1 + MH * K1 * 2, PW3 = PW2 + MH * MH * 2, PW4 = PW3 + MH * MH * 2, PTOT = PW4 + NO * MH * 2;
 // shared memory of the inference kernel
 constexpr int S_A = 0, S_W = S_A + 128 * MH * 2, S_BAR = S_W + MH * MH * 2, S_TM = S_BAR + 16, S_TOT = S_TM + 16;
-constexpr int NTHR = 128;
+constexpr int NTHR = 512;
 constexpr long WAIT_LIMIT = 1L << 22;
 
 // element index of (r, k) in a K-major canonical tile with K columns
@@ -120,7 +120,10 @@ DV void tmem_ld16(uint32_t taddr, float* v) {
     for (int i = 0; i < 16; i++) v[i] = __uint_as_float(r[i]);
 }
 
-// Y[n][12] = net((X - mean) / std) * ystd + ymean, 128 rows per CTA.
+// Y[n][12] = net((X - mean) / std) * ystd + ymean, 128 rows per CTA.  One CTA
+// fits an SM (operands and weights take 200 KB), and the epilogues (GELU of
+// 128 x 256 values per layer) bound it, so 16 warps share them: 50,021 rows
+// take 84 us, with four warps 105.
 __global__ void __launch_bounds__(NTHR, 1) k_mlp_infer(int n, const float* __restrict__ X, const float* __restrict__ norm,
                                                       const uint8_t* __restrict__ wpack, const float* __restrict__ bias,
                                                       float* __restrict__ Y, int* err) {
@@ -152,8 +155,8 @@ __global__ void __launch_bounds__(NTHR, 1) k_mlp_infer(int n, const float* __res
 
     // layer-1 operand: normalised inputs of this CTA's rows, BF16, K = 64
     {
-        int r = tid, gr = row0 + r;
-        for (int k0 = 0; k0 < K1; k0 += 8) {
+        const int r = tid & 127, gr = row0 + r;
+        for (int k0 = (tid >> 7) * 8; k0 < K1; k0 += NTHR / 128 * 8) {
             __align__(16) __nv_bfloat16 v[8];
 #pragma unroll
             for (int j = 0; j < 8; j++) {
@@ -194,10 +197,13 @@ __global__ void __launch_bounds__(NTHR, 1) k_mlp_infer(int n, const float* __res
         __syncthreads();
         if (status) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const int r = warp * 32 + lane, gr = row0 + r;
-        const uint32_t trow = tmem + ((uint32_t)(warp * 32) << 16);
+        // a warp reads the tensor-memory rows of its place among four; the four
+        // groups of four warps take a quarter of the columns each
+        const int r = (warp & 3) * 32 + lane, gr = row0 + r, part = warp >> 2;
+        const uint32_t trow = tmem + ((uint32_t)((warp & 3) * 32) << 16);
         if (l < 3) {
-            for (int c0 = 0; c0 < N; c0 += 32) {
+            const int cols = N / (NTHR / 128);
+            for (int c0 = part * cols; c0 < (part + 1) * cols; c0 += 32) {
                 float v[32];
                 tmem_ld32(trow + c0, v);
 #pragma unroll
@@ -208,7 +214,7 @@ __global__ void __launch_bounds__(NTHR, 1) k_mlp_infer(int n, const float* __res
                     *reinterpret_cast<uint4*>(sA + canon(r, c0 + j0, MH)) = *reinterpret_cast<const uint4*>(h);
                 }
             }
-        } else {
+        } else if (part == 0) {
             float v[16];
             tmem_ld16(trow, v);
             if (gr < n) {
@@ -664,12 +670,16 @@ struct MlpDev {
     float* y = nullptr; int ycap = 0;
     float* feat = nullptr;
     int* err = nullptr;
+    float* io = nullptr; int iocap = 0;      // rows in and out of abd_mlp_forward
 };
+// rows that abd_mlp_forward takes at once, and so the most it keeps room for
+// (15 MB); more rows than that hide the copies' fixed costs anyway
+constexpr int MLP_SLAB = 65536;
 
 void eng_mlp_free(Engine* E) {
     MlpDev* M = reinterpret_cast<MlpDev*>(E->mlp);
     if (!M) return;
-    void* ps[] = {M->pack, M->bias, M->norm, M->y, M->feat, M->err};
+    void* ps[] = {M->pack, M->bias, M->norm, M->y, M->feat, M->err, M->io};
     for (void* p : ps) if (p) cudaFree(p);
     delete M;
     E->mlp = nullptr;
@@ -684,20 +694,10 @@ static int mlp_infer(Engine* E, const float* X, int n, float* Y) {
         attr_set[dev] = true;
     }
     if (n <= 0) return ABD_OK;
-    CUDA_TRY(cudaMemsetAsync(M->err, 0, sizeof(int), E->stream));
     k_mlp_infer<<<(n + 127) / 128, NTHR, S_TOT, E->stream>>>(n, X, M->norm, M->pack, M->bias, Y, M->err);
     E->launches++;
     return ABD_OK;
 }
-static int mlp_check(Engine* E) {
-    MlpDev* M = reinterpret_cast<MlpDev*>(E->mlp);
-    int h = 0;
-    CUDA_TRY(cudaMemcpyAsync(&h, M->err, sizeof(int), cudaMemcpyDeviceToHost, E->stream));
-    CUDA_TRY(eng_stream_sync(E));
-    if (h) return E->fail(ABD_ERR_CUDA, "mlp inference: a wait ran out");
-    return ABD_OK;
-}
-
 // learned increment: ws = inertial increment + dt * (body frame -> world) y
 __global__ void k_ws_learned(int nb, const double* __restrict__ st, const float* __restrict__ y,
                              const double* __restrict__ mass, double dt, double g0, double g1, double g2, double* ws) {
@@ -765,6 +765,7 @@ extern "C" int abd_set_mlp(AbdHandle* h, const float* params, const float* norm)
     float* P = nullptr;
     if (cudaMalloc(&P, sizeof(float) * NPARAM) != cudaSuccess) return E->fail(ABD_ERR_CUDA, "cudaMalloc params");
     cudaError_t e = cudaMemcpyAsync(P, params, sizeof(float) * NPARAM, cudaMemcpyHostToDevice, E->stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(M->err, 0, sizeof(int), E->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(M->norm, norm, sizeof(float) * ABD_MLP_NNORM, cudaMemcpyHostToDevice, E->stream);
     if (e == cudaSuccess) {
         k_mlp_pack<<<grid_for((long)MH * MH), 256, 0, E->stream>>>(P, reinterpret_cast<__nv_bfloat16*>(M->pack), M->bias);
@@ -782,23 +783,36 @@ extern "C" int abd_mlp_forward(AbdHandle* h, const float* x, int32_t n, float* y
     if (n < 0 || (n > 0 && (!x || !y))) return E->fail(ABD_ERR_INVALID_ARG, "abd_mlp_forward: bad arguments");
     if (n == 0) return ABD_OK;
     if (cudaSetDevice(E->device) != cudaSuccess) return E->fail(ABD_ERR_CUDA, "cudaSetDevice");
-    float *dx = nullptr, *dy = nullptr;
-    if (cudaMalloc(&dx, sizeof(float) * MI * (size_t)n) != cudaSuccess || cudaMalloc(&dy, sizeof(float) * MO * (size_t)n) != cudaSuccess) {
-        cudaFree(dx);
-        return E->fail(ABD_ERR_CUDA, "cudaMalloc mlp io");
+    MlpDev* M = reinterpret_cast<MlpDev*>(E->mlp);
+    // two buffers kept for the next call: allocating and freeing them on each
+    // call took 1,280 of 2,290 us for 50,021 rows
+    const int rows = n < MLP_SLAB ? n : MLP_SLAB;
+    if (rows > M->iocap) {
+        if (M->io) { CUDA_TRY(eng_stream_sync(E)); cudaFree(M->io); }
+        M->io = nullptr; M->iocap = 0;
+        if (cudaMalloc(&M->io, sizeof(float) * (MI + MO) * (size_t)rows) != cudaSuccess) {
+            M->io = nullptr;
+            return E->fail(ABD_ERR_CUDA, "cudaMalloc mlp io");
+        }
+        M->iocap = rows;
     }
-    int rc = ABD_OK;
-    cudaError_t e = cudaMemcpyAsync(dx, x, sizeof(float) * MI * (size_t)n, cudaMemcpyHostToDevice, E->stream);
-    if (e != cudaSuccess) rc = E->fail(ABD_ERR_CUDA, "abd_mlp_forward: copy in");
-    if (!rc) rc = mlp_infer(E, dx, n, dy);
-    if (!rc) rc = mlp_check(E);
-    if (!rc) {
-        e = cudaMemcpyAsync(y, dy, sizeof(float) * MO * (size_t)n, cudaMemcpyDeviceToHost, E->stream);
-        if (e == cudaSuccess) e = eng_stream_sync(E);
-        if (e != cudaSuccess) rc = E->fail(ABD_ERR_CUDA, "abd_mlp_forward: copy out");
+    float *dx = M->io, *dy = M->io + (size_t)MI * M->iocap;
+    int flag = 0;
+    CUDA_TRY(cudaMemsetAsync(M->err, 0, sizeof(int), E->stream));
+    for (int r = 0; r < n; r += rows) {
+        const int k = n - r < rows ? n - r : rows;
+        if (cudaMemcpyAsync(dx, x + (size_t)MI * r, sizeof(float) * MI * (size_t)k, cudaMemcpyHostToDevice, E->stream) != cudaSuccess)
+            return E->fail(ABD_ERR_CUDA, "abd_mlp_forward: copy in");
+        int rc = mlp_infer(E, dx, k, dy);
+        if (rc) return rc;
+        if (cudaMemcpyAsync(y + (size_t)MO * r, dy, sizeof(float) * MO * (size_t)k, cudaMemcpyDeviceToHost, E->stream) != cudaSuccess)
+            return E->fail(ABD_ERR_CUDA, "abd_mlp_forward: copy out");
     }
-    cudaFree(dx); cudaFree(dy);
-    return rc;
+    cudaError_t e = cudaMemcpyAsync(&flag, M->err, sizeof(int), cudaMemcpyDeviceToHost, E->stream);
+    if (e == cudaSuccess) e = eng_stream_sync(E);
+    if (e != cudaSuccess) return E->fail(ABD_ERR_CUDA, "abd_mlp_forward: copy out");
+    if (flag) return E->fail(ABD_ERR_CUDA, "mlp inference: a wait ran out");
+    return ABD_OK;
 }
 
 // ------------------------------------------------------------------ trainer

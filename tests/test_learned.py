@@ -62,6 +62,24 @@ def test_mlp_tensor_core_forward_matches_oracle(chain_scene):
 
 
 @pytest.mark.gpu
+def test_mlp_forward_does_not_depend_on_how_rows_are_cut(chain_scene):
+    """Rows are independent: a call over more rows than the kept buffers hold,
+    and calls after a larger or a smaller one, give each row the value that it
+    gets alone in a short call, bit for bit."""
+    from colb_b200 import params as P
+    from colb_b200.engine import Engine
+    rng = np.random.default_rng(4)
+    e = Engine(P.reference_params(), chain_scene)
+    e.set_mlp(LO.init_params(2), _norm(rng))
+    x = rng.normal(size=(2 * 65536 + 5, 48)).astype(np.float32)
+    first = e.mlp_forward(x[:3])
+    y = e.mlp_forward(x)
+    assert np.array_equal(y[:3], first)
+    for a, b in ((0, 65536), (65535, 65537), (65536, 2 * 65536), (2 * 65536, 2 * 65536 + 5), (100, 229)):
+        assert np.array_equal(e.mlp_forward(x[a:b]), y[a:b]), (a, b)
+
+
+@pytest.mark.gpu
 def test_trainer_gradient_matches_oracle():
     from colb_b200.engine import Trainer
     rng = np.random.default_rng(4)

@@ -13,6 +13,7 @@
 // product uses width-16 shuffles.  Block values are column-major inside a
 // block, so at fixed column the 12 lanes read 12 consecutive values.
 #include "engine.cuh"
+#include <algorithm>
 
 #define CHECK_EVERY 8
 
@@ -277,6 +278,164 @@ __global__ void k_bi_e(KrylovArgs<T> A, int k, T* x, T* r, const T* __restrict__
     }
 }
 
+// ------------------------------------------------------------------ BiCGSTAB, one cluster per scene
+// A scene of up to KS_MAX bodies is solved by one launch: a cluster of C CTAs
+// holds its rows, 16 lanes per body as above, with the body's part of every
+// vector in the lanes' registers and the matrix blocks in shared memory as far as they fit.
+// What crosses CTAs goes through distributed shared memory: the SpMV's input
+// vector, of which every CTA keeps a copy, and each warp's part of the dot
+// products, which every warp adds up in the same order, so all threads agree
+// on the scalars and on the end of the iterations without the host.  Each of
+// the five steps of an iteration ends at a cluster barrier; the barriers, the
+// sums after them and the two SpMVs bound it.  The steps and their rounding are
+// k_bi_a .. k_bi_e's; sums are in a fixed order here, by atomics there.
+// 144 links in contact: 59 us per solve; in launches, 12 iterations and the
+// checks by the host took 290 us of kernels and as much again between them.
+// Larger scenes keep the launches: one CTA per SM of a cluster would read
+// their blocks from L2 with 8 of the 148 SMs.
+constexpr int KS_CL = 8;                     // CTAs of a cluster at most
+constexpr int KS_MAX = KS_CL * 32;           // bodies of a scene: 32 per CTA of 512 threads
+constexpr int KS_DOTS = 6;                   // rh.v, s.s, t.s, t.t, rho, r.r
+constexpr int KS_SMEM = 200 << 10;           // dynamic shared memory at most
+
+DV void ks_cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+}
+// address of `p` (this CTA's shared memory) in CTA `rank` of the cluster
+DV uint32_t ks_remote(const void* p, int rank) {
+    uint32_t a;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank));
+    return a;
+}
+DV void ks_store(uint32_t a, double v) { asm volatile("st.shared::cluster.f64 [%0], %1;" :: "r"(a), "d"(v) : "memory"); }
+DV void ks_store(uint32_t a, float v) { asm volatile("st.shared::cluster.f32 [%0], %1;" :: "r"(a), "f"(v) : "memory"); }
+
+template <class T>
+inline size_t ks_smem(int bodies, int blocks) {
+    return sizeof(double) * KS_DOTS * KS_CL * 16 + sizeof(T) * 12 * (size_t)bodies + (sizeof(T) * 144 + sizeof(int)) * (size_t)blocks;
+}
+// bodies: capacity of the shared input vector; blocks: of the shared matrix blocks
+template <class T>
+__global__ void __launch_bounds__(512, 1)
+k_bi_scene(KrylovArgs<T> A, int bodies, int blocks, const int* __restrict__ body_begin, const double* __restrict__ g,
+           double* du, int* kiter, int* active) {
+    extern __shared__ __align__(16) unsigned char ks_raw[];
+    double* part = reinterpret_cast<double*>(ks_raw);                 // [KS_DOTS][C * warps]
+    T* xs = reinterpret_cast<T*>(part + KS_DOTS * KS_CL * 16);        // [bodies][12]
+    T* blk = xs + 12 * (size_t)bodies;                                // [blocks][144]
+    int* col = reinterpret_cast<int*>(blk + 144 * (size_t)blocks);    // [blocks]
+    uint32_t C, c;
+    asm("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(C));
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(c));
+    const int s = blockIdx.x / C, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5, nslot = C * nw;
+    const int first = body_begin[s], n = body_begin[s + 1] - first, per = (n + (int)C - 1) / (int)C;
+    const int l = threadIdx.x % HALF, local = (int)c * per + (int)threadIdx.x / HALF;
+    const bool has = (int)threadIdx.x / HALF < per && local < n;
+    const bool on = has && l < 12;
+    const int b = first + (has ? local : 0);
+    const long i = 12L * b + (l < 12 ? l : 0);
+    if (A.ndone[s] || A.kdone[s]) {                                   // the whole cluster
+        if (on) du[i] = 0.0;
+        return;
+    }
+    const int r0 = min((int)c * per, n), r1 = min(r0 + per, n);
+    const int k0 = A.row_ptr[first + r0], nblk = A.row_ptr[first + r1] - k0;
+    const bool cached = nblk <= blocks;
+    if (cached) {
+        for (long e = threadIdx.x; e < 144L * nblk; e += blockDim.x) blk[e] = A.vals[144L * k0 + e];
+        for (int e = threadIdx.x; e < nblk; e += blockDim.x) col[e] = A.bcol[k0 + e] - first;
+    }
+    const int q0 = has ? A.row_ptr[b] : 0, q1 = has ? A.row_ptr[b + 1] : 0;
+    T d[12];                                                          // row l of the body's inverse diagonal block
+#pragma unroll
+    for (int j = 0; j < 12; j++) d[j] = on ? A.dinv[144L * b + j * 12 + l] : (T)0;
+    auto precond = [&](double own) {
+        double a0 = 0, a1 = 0;
+#pragma unroll
+        for (int j = 0; j < 12; j += 2) {
+            a0 += (double)d[j] * __shfl_sync(0xffffffffu, own, j, HALF);
+            a1 += (double)d[j + 1] * __shfl_sync(0xffffffffu, own, j + 1, HALF);
+        }
+        return a0 + a1;
+    };
+    auto publish = [&](T v) {
+        if (!on) return;
+        for (int r = 0; r < (int)C; r++) ks_store(ks_remote(xs + 12 * local + l, r), v);
+    };
+    auto block_mv = [&](const T* V, const T* x, double (&acc)[3]) {
+#pragma unroll
+        for (int j = 0; j < 12; j++) acc[j % 3] += (double)V[j * 12] * (double)x[j];
+    };
+    auto spmv = [&]() {
+        double acc[3] = {0, 0, 0};
+        if (on) {
+            if (cached) for (int q = q0; q < q1; q++) block_mv(blk + 144 * (q - k0) + l, xs + 12 * col[q - k0], acc);
+            else for (int q = q0; q < q1; q++) block_mv(A.vals + 144L * q + l, xs + 12 * (A.bcol[q] - first), acc);
+        }
+        return acc[0] + acc[1] + acc[2];
+    };
+    auto add = [&](int dot, double v) {                               // this warp's part, to every CTA
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        if (lane < (int)C) ks_store(ks_remote(part + dot * nslot + (int)c * nw + warp, lane), v);
+    };
+    auto total = [&](int dot) {
+        double v = 0;
+        for (int e = lane; e < nslot; e += 32) v += part[dot * nslot + e];
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        return v;
+    };
+    T x = (T)0, r = (T)(on ? g[i] : 0.0), p = (T)0, v = (T)0;
+    const T rh = r;
+    ks_cluster_sync();                                                // every CTA runs; its blocks are in place
+    { const double rv = on ? g[i] : 0.0; add(4, rv * rv); }
+    ks_cluster_sync();
+    double rho = total(4), rr = rho, run_rho = 0, run_al = 0, run_om = 0;
+    const double bb = rho;
+    int k = 0;
+#pragma unroll 1
+    for (; k < A.maxit; k++) {
+        if (!(rr > A.tol2 * bb) || (k > 0 && !(run_rho != 0.0 && run_om != 0.0))) break;
+        const double beta = k == 0 ? 0.0 : (rho / run_rho) * (run_al / run_om);
+        const double pn = (double)r + beta * ((double)p - run_om * (double)v);
+        p = (T)pn;
+        const T y = (T)precond(pn);
+        publish(y);
+        ks_cluster_sync();
+        double o = spmv();
+        v = (T)o;
+        add(0, (double)rh * o);
+        ks_cluster_sync();
+        const double rv = total(0), alpha = rv != 0.0 ? rho / rv : 0.0;
+        x = (T)((double)x + alpha * (double)y);
+        const double sn = (double)r - alpha * (double)v;
+        const T sv = (T)sn, z = (T)precond(sn);
+        publish(z);
+        add(1, sn * sn);
+        ks_cluster_sync();
+        const double ss = total(1);
+        o = spmv();
+        add(2, (double)sv * o);
+        add(3, o * o);
+        ks_cluster_sync();
+        const double ts = total(2), tt = total(3);
+        const double omega = (ss <= A.tol2 * bb || !(tt > 0)) ? 0.0 : ts / tt;
+        x = (T)((double)x + omega * (double)z);
+        const double rn = (double)sv - omega * (double)(T)o;
+        r = (T)rn;
+        add(4, (double)rh * rn);
+        add(5, rn * rn);
+        run_rho = rho; run_al = alpha; run_om = omega;
+        ks_cluster_sync();
+        rho = total(4); rr = total(5);
+    }
+    if (on) du[i] = (double)x;
+    if (c == 0 && threadIdx.x == 0) {
+        kiter[s] = k;
+        if (rr > A.tol2 * bb && run_rho != 0.0 && run_om != 0.0) atomicAdd(active, 1);
+    }
+}
+
 // number of scenes still iterating
 // PCG (bicg = 0): a scene stays alive while its last p.Ap > 0.
 // BiCGSTAB (bicg = 1): while its running rho and omega are non-zero (rho may
@@ -314,6 +473,34 @@ static int solve_t(Engine* E, int* iters) {
     int* kiter = E->sci + SI_KITER * ns;
     CUDA_TRY(cudaMemsetAsync(kdone, 0, sizeof(int) * ns, st));
     CUDA_TRY(cudaMemsetAsync(kiter, 0, sizeof(int) * ns, st));
+    int most = 0;                          // bodies of the largest scene
+    for (int s = 0; s < ns; s++) most = std::max(most, E->h_body_begin[s + 1] - E->h_body_begin[s]);
+    if (E->krylov_kind == ABD_SOLVER_BICGSTAB && most <= KS_MAX && A.maxit > 0) {
+        int C = 1;                         // the smallest cluster with 16 bodies per CTA, or the largest
+        while (C < KS_CL && most > 16 * C) C *= 2;
+        const int per = (most + C - 1) / C;
+        // room for all of a CTA's blocks when it has at most twice the mean
+        const long want = 2L * E->nnzb_host / ((long)ns * C) + 16, fit = (KS_SMEM - (long)ks_smem<T>(most, 0)) / (long)(sizeof(T) * 144 + 4);
+        const int blocks = (int)std::min(want, fit);
+        const size_t smem = ks_smem<T>(most, blocks);
+        CUDA_TRY(cudaFuncSetAttribute(k_bi_scene<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, KS_SMEM));
+        CUDA_TRY(cudaMemsetAsync(&E->dcnt->krylov_active, 0, sizeof(int), st));
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)ns * C); cfg.blockDim = dim3(32 * ((per + 1) / 2)); cfg.dynamicSmemBytes = smem; cfg.stream = st;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = C; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+        cfg.attrs = at; cfg.numAttrs = 1;
+        CUDA_TRY(cudaLaunchKernelEx(&cfg, k_bi_scene<T>, A, most, blocks, (const int*)E->sc_body_begin, (const double*)E->g, E->du,
+                                    kiter, &E->dcnt->krylov_active));
+        E->launches++;
+        CUDA_TRY(cudaMemcpyAsync(E->hsci, kiter, sizeof(int) * ns, cudaMemcpyDeviceToHost, st));
+        int rc = eng_sync_counters(E);
+        if (rc) return rc;
+        if (E->hcnt->krylov_active > 0) E->solver_capped++;
+        *iters = *std::max_element(E->hsci, E->hsci + ns);
+        return ABD_OK;
+    }
     // zero all rings
     CUDA_TRY(cudaMemsetAsync(E->scd + SD_BB * ns, 0, sizeof(double) * ns * (SD_COUNT - SD_BB), st));
     int bicg = E->krylov_kind == ABD_SOLVER_BICGSTAB;

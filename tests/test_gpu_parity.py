@@ -297,3 +297,44 @@ def test_body_pair_candidates_equal_grid_at_cluster_edges(nu, nv, cand):
         got.append((quads, kinds))
     assert len(got[0][0]) > 0
     assert np.array_equal(got[0][0], got[1][0]) and np.array_equal(got[0][1], got[1][1])
+
+
+def _links(scene, state, n):
+    """The first n links of copies of the chain scene, the copies 100 apart."""
+    nb, nv = len(scene["mass"]), len(scene["xbar"])
+    parts = {k: [] for k in ("xbar", "vert_body", "edges", "mass", "inertia_J", "state")}
+    for c in range((n + nb - 1) // nb):
+        m = min(nb, n - c * nb)
+        v = int((scene["vert_body"] < m).sum())
+        st = state[:m].copy()
+        st[:, [S.ST_NOW, S.ST_NXT]] += 100.0 * c
+        for key, a in (("xbar", scene["xbar"][:v]), ("vert_body", scene["vert_body"][:v] + c * nb),
+                       ("edges", scene["edges"][(scene["edges"] < v).all(1)] + c * nv), ("mass", scene["mass"][:m]),
+                       ("inertia_J", scene["inertia_J"][:m]), ("state", st)):
+            parts[key].append(a)
+    return dict(scene, **{k: np.concatenate(v) for k, v in parts.items()})
+
+
+@pytest.mark.parametrize("sizes", [(1,), (2,), (16,), (17,), (33,), (65,), (144,), (256,), (257,), (144,) + 20 * (1,)])
+@pytest.mark.parametrize("precision", [0, 1])
+def test_bicgstab_by_scene_size(chain_scene, chain_pairs, sizes, precision):
+    """BiCGSTAB in one cluster per scene (1 to 8 thread blocks, one to 32 bodies
+    in a block, blocks that keep their part of the matrix and, with many small
+    scenes beside a large one, blocks that do not) and in separate launches
+    (257 bodies), against a dense solve: the error is at most the residual's
+    bound plus the rounding of the stored vectors, times the condition number."""
+    tol, eps = (1e-12, 2.2e-16) if precision == 0 else (1e-6, 1.2e-7)
+    scenes = [_links(chain_scene, chain_pairs["states"][1], n) for n in sizes]
+    e = Engine(P.reference_params(linear_solver=0, lin_tol=tol, hess_mode=1, precision=precision), scenes)
+    g, H = e.assemble()
+    du, it = e.solve()
+    assert it > 0
+    at = 0
+    for n in sizes:
+        k = slice(12 * at, 12 * (at + n))
+        at += n
+        A, b = H[k, k], g[k]
+        d = 1.0 / np.sqrt(np.diag(A))
+        ref = np.linalg.solve(A, b)
+        kappa = np.linalg.cond(A * d[:, None] * d)
+        assert np.linalg.norm((du[k] - ref) / d) <= (tol + 50 * eps) * kappa * np.linalg.norm(ref / d), (n, kappa)

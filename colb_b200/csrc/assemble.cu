@@ -16,6 +16,7 @@
 // atomics.
 #include "contact.cuh"
 #include "contact_hess.cuh"
+#include "block_inverse.cuh"
 #include <cub/cub.cuh>
 
 Geo eng_geo(Engine* E);
@@ -24,14 +25,22 @@ DV int stencil_np(int type) { return type == T_PP ? 2 : (type == T_PE ? 3 : (typ
 DV int other_vertex(int type, int4 s) { return type == T_EE ? s.z : (type == T_PG ? s.x : s.y); }
 
 // ---------------------------------------------------------- prepare + keys
-// Contacts [0, n_total) (the device count); with nkey_pairs > n_total the key
+// Pattern of the block rows as bits: row b has `words` words, bit c for
+// body c of its scene (null: the keys below instead).  k_bit_rows clears what it reads.
+struct BitRows { uint32_t* bits; int words; const int* bscene; const int* sc_body_begin; };
+DV void set_bit(const BitRows& B, int r, int c) {
+    uint32_t* w = B.bits + (long)r * B.words + (c >> 5);
+    const uint32_t m = 1u << (c & 31);
+    if (!(*(volatile uint32_t*)w & m)) atomicOr(w, m);
+}
+// Contacts [0, n_total) (the device count, at most cap); with nkey_pairs > n_total the key
 // pairs of the slots up to nkey_pairs are sentinels (~0), so a sort sized
 // before the count is known sees only real keys and sentinels.
 __global__ void k_contact_prepare(const Counters* cnt, const int4* __restrict__ contacts, Geo G, int f32, double dhat,
-                                  int nb, int4* cst, int* ctype, double* cxb, int2* cbody,
-                                  unsigned long long* keys, int* n_active, int nkey_pairs) {
-    int n = cnt->n_total;
-    GS_LOOP(c, nkey_pairs) {
+                                  int nb, int cap, int4* cst, int* ctype, double* cxb, int2* cbody,
+                                  unsigned long long* keys, BitRows B, int* n_active, int nkey_pairs) {
+    int n = min(cnt->n_total, cap);
+    if (!B.bits) GS_LOOP(c, nkey_pairs) {
         if (c >= n) { keys[nb + 2*c] = ~0ull; keys[nb + 2*c + 1] = ~0ull; }
     }
     GS_LOOP(c, n) {
@@ -44,14 +53,99 @@ __global__ void k_contact_prepare(const Counters* cnt, const int4* __restrict__ 
             int b1 = G.vbody[other_vertex(type, stv)];
             cbody[c] = make_int2(b0, b1);
             if (b0 != b1 && G.mass[b0] > 0.0 && G.mass[b1] > 0.0) {
+                if (B.bits) {
+                    const int f = B.sc_body_begin[B.bscene[b0]];
+                    set_bit(B, b0, b1 - f); set_bit(B, b1, b0 - f);
+                }
                 k0 = (unsigned long long)b0 * nb + b1;
                 k1 = (unsigned long long)b1 * nb + b0;
             }
             atomicAdd(n_active, 1);
         }
         cst[c] = stv; ctype[c] = act ? type : -1; cxb[c] = xb;
-        keys[nb + 2*c] = k0; keys[nb + 2*c + 1] = k1;
+        if (!B.bits) { keys[nb + 2*c] = k0; keys[nb + 2*c + 1] = k1; }
     }
+}
+// Block rows from the bits, by one block: each row's count, their running
+// sums, then the columns (ascending, so this is the order a sort of the keys
+// gives).  A row is read by `lanes` threads, a power of two up to a warp, one
+// word each.  The bits and the contact count are cleared for the next
+// assembly, and what the host's component analysis reads is written to its pinned
+// memory from here.  Replaces clearing, diagonal keys, a radix sort, the
+// removal of doubles, the rows and three copies: FIGB.
+struct BitHost { int* row; int* col; int* done; Counters* cnt; };      // null: not wanted
+__global__ void __launch_bounds__(1024) k_bit_rows(int nb, int bound, BitRows B, int lanes, int* row_ptr, int* bcol,
+                                                   Counters* cnt, int ns, const int* done, BitHost H) {
+    __shared__ int s_sum[32];
+    __shared__ int s_total;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, sub = tid & (lanes - 1);
+    const unsigned group = lanes == 32 ? 0xffffffffu : ((1u << lanes) - 1) << (lane & ~(lanes - 1));
+#pragma unroll 4
+    for (int r = tid / lanes; r < nb; r += 1024 / lanes) {
+        const int self = r - B.sc_body_begin[B.bscene[r]];
+        int n = 0;
+        for (int w = sub; w < B.words; w += lanes) {
+            uint32_t v = B.bits[(long)r * B.words + w];
+            if (w == self >> 5) v |= 1u << (self & 31);
+            n += __popc(v);
+        }
+        for (int o = lanes / 2; o > 0; o >>= 1) n += __shfl_xor_sync(group, n, o);
+        if (sub == 0) row_ptr[r] = n;
+    }
+    __syncthreads();
+    // exclusive sums, each thread over a run of rows
+    const int per = (nb + 1023) / 1024, r0 = min(tid * per, nb), r1 = min(r0 + per, nb);
+    int mine = 0;
+    for (int r = r0; r < r1; r++) mine += row_ptr[r];
+    int incl = mine;
+    for (int o = 1; o < 32; o <<= 1) { int v = __shfl_up_sync(0xffffffffu, incl, o); if (lane >= o) incl += v; }
+    if (lane == 31) s_sum[warp] = incl;
+    __syncthreads();
+    if (warp == 0) {
+        int v = s_sum[lane];
+        for (int o = 1; o < 32; o <<= 1) { int u = __shfl_up_sync(0xffffffffu, v, o); if (lane >= o) v += u; }
+        if (lane == 31) s_total = v;
+        s_sum[lane] = v - s_sum[lane];
+    }
+    __syncthreads();
+    for (int r = r0, at = s_sum[warp] + incl - mine; r < r1; r++) { const int n = row_ptr[r]; row_ptr[r] = at; at += n; }
+    if (tid == 0) {
+        row_ptr[nb] = s_total;
+        cnt->nnzb = cnt->nkeys = s_total;
+        cnt->n_active = cnt->act; cnt->act = 0;
+    }
+    __syncthreads();
+#pragma unroll 2
+    for (int r = tid / lanes; r < nb; r += 1024 / lanes) {
+        const int first = B.sc_body_begin[B.bscene[r]], self = r - first;
+        int base = row_ptr[r];
+        for (int w0 = 0; w0 < B.words; w0 += lanes) {
+            const int w = w0 + sub;
+            uint32_t v = 0;
+            if (w < B.words) {
+                uint32_t* p = B.bits + (long)r * B.words + w;
+                v = *p;
+                if (v) *p = 0;
+                if (w == self >> 5) v |= 1u << (self & 31);
+            }
+            int n = __popc(v), sum = n;
+            for (int o = 1; o < lanes; o <<= 1) { int u = __shfl_up_sync(group, sum, o, lanes); if (sub >= o) sum += u; }
+            for (int at = base + sum - n; v; v &= v - 1, at++) {
+                if (at >= bound) break;              // a count beyond the host's guess: it will assemble again
+                bcol[at] = first + 32 * w + __ffs(v) - 1;
+            }
+            base += __shfl_sync(group, sum, lanes - 1, lanes);
+        }
+    }
+    __syncthreads();
+    // whole lines at a time: single words took 60 us for 4,096 rows
+    if (H.row) {
+        const int m = min(s_total, bound);
+        for (int i = tid; i <= nb; i += 1024) H.row[i] = row_ptr[i];
+        for (int i = tid; i < m; i += 1024) H.col[i] = bcol[i];
+    }
+    if (H.done) for (int s = tid; s < ns; s += 1024) H.done[s] = done[s];
+    if (H.cnt) for (int i = tid; i < (int)(sizeof(Counters) / sizeof(int)); i += 1024) ((int*)H.cnt)[i] = ((const int*)cnt)[i];
 }
 __global__ void k_diag_keys(int nb, unsigned long long* keys) {
     GS_LOOP(b, nb) keys[b] = (unsigned long long)b * nb + b;
@@ -70,16 +164,11 @@ __global__ void k_block_rows(int nb, const unsigned long long* __restrict__ ukey
 }
 
 
-template <class T>
-__global__ void k_zero_vals(const Counters* cnt, T* vals) {
-    long n = (long)cnt->nnzb * 144;
-    GS_LOOP(i, n) vals[i] = (T)0;
-}
-
 // ---------------------------------------------------- inertia + ortho (abd.py:108-149)
 // One warp per body: gradient by lanes 0..11, the 9x9 orthogonality Hessian
 // (scaled by dt^2) built lane-parallel in shared memory, projected to PSD
 // when requested, and written with the mass terms into the diagonal block.
+// The warp also clears the row's other blocks for the contacts.
 #define BA_WARPS 4
 template <class T>
 __global__ void __launch_bounds__(32 * BA_WARPS) k_body_assemble(int nb, const double* __restrict__ st,
@@ -94,6 +183,8 @@ __global__ void __launch_bounds__(32 * BA_WARPS) k_body_assemble(int nb, const d
         int bi = find_block(row_ptr, bcol, b, b);
         if (bi < 0) continue;                              // every row holds its diagonal key
         T* V = vals + (long)bi * 144;
+        for (int k = row_ptr[b]; k < row_ptr[b + 1]; k++)
+            if (k != bi) for (int e = lane; e < 144; e += 32) vals[(long)k * 144 + e] = (T)0;
         double* g = grad + 12L * b;
         double m = mass[b];
         if (!(m > 0.0)) {
@@ -257,8 +348,9 @@ __global__ void __launch_bounds__(32 * CAW) k_contact_assemble(const Counters* c
 }
 
 // ---------------------------------------------------- block-Jacobi inverse
-// One warp per body: Gauss-Jordan with partial pivoting on [D | I] in shared
-// memory, lanes owning the 24 columns.  A singular block gives the identity.
+// One warp per body; a singular block gives the identity.  The Krylov solves'
+// preconditioner and the increment of a body that the mixed-precision guard
+// replaces; the direct solve inverts the blocks of single bodies itself.
 #define BI_WARPS 4
 template <class T>
 __global__ void __launch_bounds__(32 * BI_WARPS) k_block_inverse(int nb, const int* __restrict__ row_ptr,
@@ -269,41 +361,7 @@ __global__ void __launch_bounds__(32 * BI_WARPS) k_block_inverse(int nb, const i
     for (int b = blockIdx.x * BI_WARPS + w; b < nb; b += gridDim.x * BI_WARPS) {
         int bi = find_block(row_ptr, bcol, b, b);
         if (bi < 0) continue;
-        const T* V = vals + (long)bi * 144;
-        for (int e = lane; e < 288; e += 32) {
-            int r = e / 24, c = e % 24;
-            M[r][c] = c < 12 ? (double)V[c*12 + r] : (c - 12 == r ? 1.0 : 0.0);
-        }
-        __syncwarp();
-        bool ok = true;
-        for (int c = 0; c < 12; c++) {
-            // first row of largest magnitude in column c at or below the diagonal
-            double best = lane >= c && lane < 12 ? fabs(M[lane][c]) : -1.0;
-            int p = lane;
-            for (int o = 16; o > 0; o >>= 1) {
-                double ob = __shfl_xor_sync(0xffffffffu, best, o);
-                int op = __shfl_xor_sync(0xffffffffu, p, o);
-                if (ob > best || (ob == best && op < p)) { best = ob; p = op; }
-            }
-            if (M[p][c] == 0.0) { ok = false; break; }
-            if (p != c && lane < 24) { double t = M[p][lane]; M[p][lane] = M[c][lane]; M[c][lane] = t; }
-            __syncwarp();
-            double iv = 1.0 / M[c][c];
-            __syncwarp();
-            if (lane < 24) M[c][lane] *= iv;
-            __syncwarp();
-            double f[12];
-#pragma unroll
-            for (int r = 0; r < 12; r++) f[r] = M[r][c];
-            __syncwarp();
-            if (lane < 24) {
-                double mc = M[c][lane];
-#pragma unroll
-                for (int r = 0; r < 12; r++)
-                    if (r != c && f[r] != 0.0) M[r][lane] -= f[r] * mc;
-            }
-            __syncwarp();
-        }
+        const bool ok = block_inverse_warp<T>(vals + (long)bi * 144, M, lane);
         T* D = dinv + (long)b * 144;
         for (int e = lane; e < 144; e += 32) {
             int c = e / 12, r = e % 12;
@@ -312,17 +370,14 @@ __global__ void __launch_bounds__(32 * BI_WARPS) k_block_inverse(int nb, const i
         __syncwarp();
     }
 }
-
-// per-scene ||g||^2
-__global__ void k_grad_norm(int nb, const double* __restrict__ g, const int* __restrict__ bscene, double* gg) {
-    long n = 12L * nb;
-    for (long base = (long)blockIdx.x * blockDim.x; base < n; base += (long)gridDim.x * blockDim.x) {
-        long i = base + threadIdx.x;
-        bool valid = i < n;
-        int s = valid ? bscene[i / 12] : 0;
-        double v = valid ? g[i] * g[i] : 0.0;
-        warp_reduce_add(gg, s, v, valid);
-    }
+int eng_block_inverse(Engine* E) {
+    const int nb = E->nb, grid = grid_for(32L * nb, 32 * BI_WARPS);
+    int ph = phase_begin(E, PH_ASM_INV);
+    if (E->mixed) k_block_inverse<float><<<grid, 32 * BI_WARPS, 0, E->stream>>>(nb, E->row_ptr, E->bcol, (const float*)E->vals, (float*)E->dinv);
+    else k_block_inverse<double><<<grid, 32 * BI_WARPS, 0, E->stream>>>(nb, E->row_ptr, E->bcol, (const double*)E->vals, (double*)E->dinv);
+    phase_end(E, ph, 0);
+    E->launches++;
+    return ABD_OK;
 }
 
 // waits for the copy the last assembly queued (counters, block keys, done
@@ -341,6 +396,14 @@ int eng_sync_counters(Engine* E) {
     int rc = eng_asm_wait(E);
     if (rc) return rc;
     CUDA_TRY(cudaMemcpyAsync(E->hcnt, E->dcnt, sizeof(Counters), cudaMemcpyDeviceToHost, E->stream));
+    CUDA_TRY(eng_stream_sync(E));
+    return ABD_OK;
+}
+
+// the counters that the last kernel queued left in pinned memory
+// (k_bit_rows run ahead), or a copy of them
+int eng_sync_ahead(Engine* E) {
+    if (!(E->keys_ahead && E->row_bits)) return eng_sync_counters(E);
     CUDA_TRY(eng_stream_sync(E));
     return ABD_OK;
 }
@@ -392,11 +455,49 @@ static int asm_keys(Engine* E, bool ahead, long long& bound) {
     // plus the sentinel
     bound = std::min<long long>(nkeys, E->dense_blocks) + 1;
     if (bound > E->blk_cap) { if ((rc = eng_grow_blocks(E, (int)bound))) return rc; }
-    CUDA_TRY(cudaMemsetAsync(&E->dcnt->n_active, 0, sizeof(int), s));
-    k_diag_keys<<<grid_for(nb), 256, 0, s>>>(nb, E->keys);
-    k_contact_prepare<<<grid_for(n > 0 ? n : 1, 128), 128, 0, s>>>(E->dcnt, E->contacts, G, P.ee_f32, P.dhat, nb, E->cst,
-                                                                   E->ctype, E->cxb, E->cbody, E->keys, &E->dcnt->n_active,
+    const int ls = E->P.linear_solver;
+    const bool direct = ls == ABD_SOLVER_AUTO || ls == ABD_SOLVER_DIRECT;
+    if (direct) {
+        // rows and columns, or keys of two words
+        const int words = E->row_bits ? nb + 1 + (int)bound : 2 * nkeys;
+        if (words > E->h_pattern_cap) {
+            if (E->h_pattern) { CUDA_TRY(eng_stream_sync(E)); cudaFreeHost(E->h_pattern); }
+            E->h_pattern = nullptr; E->h_pattern_cap = 0;
+            const int cap = words + words / 2 + 2048;
+            if (cudaMallocHost(&E->h_pattern, sizeof(int) * cap) != cudaSuccess)
+                return E->fail(ABD_ERR_CUDA, "cudaMallocHost block pattern");
+            E->h_pattern_cap = cap;
+        }
+        if (!E->h_done && cudaMallocHost(&E->h_done, sizeof(int) * E->ns) != cudaSuccess) {
+            E->h_done = nullptr;
+            return E->fail(ABD_ERR_CUDA, "cudaMallocHost done flags");
+        }
+    }
+    E->keys_host = false;
+    E->asm_direct = direct;
+    const BitRows B{E->row_bits, E->row_words, E->bscene, E->sc_body_begin};
+    int* n_active = B.bits ? &E->dcnt->act : &E->dcnt->n_active;
+    if (!B.bits) {
+        CUDA_TRY(cudaMemsetAsync(n_active, 0, sizeof(int), s));
+        k_diag_keys<<<grid_for(nb), 256, 0, s>>>(nb, E->keys);
+    }
+    k_contact_prepare<<<grid_for(n > 0 ? n : 1, 128), 128, 0, s>>>(E->dcnt, E->contacts, G, P.ee_f32, P.dhat, nb, E->cap, E->cst,
+                                                                   E->ctype, E->cxb, E->cbody, E->keys, B, n_active,
                                                                    ahead ? n : 0);
+    if (B.bits) {
+        int lanes = 1;
+        while (lanes < 32 && lanes < B.words) lanes *= 2;
+        BitHost H{nullptr, nullptr, nullptr, E->hcnt};
+        if (direct) { H.row = E->h_pattern; H.col = E->h_pattern + nb + 1; H.done = E->h_done; }
+        k_bit_rows<<<1, 1024, 0, s>>>(nb, (int)bound, B, lanes, E->row_ptr, E->bcol, E->dcnt, E->ns,
+                                      E->sci + SI_DONE * E->ns, H);
+        E->launches += 2;
+        if (!ahead) {
+            CUDA_TRY(cudaEventRecord(E->ev_asm, s));
+            E->asm_pending = true;
+        }
+        return ABD_OK;
+    }
     int bits = 1;
     while (bits < 64 && ((unsigned long long)nb * nb) >> bits) bits++;
     size_t bytes = E->cub_bytes;
@@ -405,26 +506,10 @@ static int asm_keys(Engine* E, bool ahead, long long& bound) {
     int* n_unique = &E->dcnt->nkeys;
     CUDA_TRY(cub::DeviceSelect::Unique(E->cub_tmp, bytes, E->keys_s, E->ukeys, n_unique, nkeys, s));
     E->launches += 4;
-    E->keys_host = false;
-    const int ls = E->P.linear_solver;
-    const bool direct = ls == ABD_SOLVER_AUTO || ls == ABD_SOLVER_DIRECT;
     if (direct) {
-        if (nkeys > E->h_ukeys_cap) {
-            if (E->h_ukeys) cudaFreeHost(E->h_ukeys);
-            E->h_ukeys = nullptr; E->h_ukeys_cap = 0;
-            int cap = nkeys + nkeys / 2 + 1024;
-            if (cudaMallocHost(&E->h_ukeys, sizeof(unsigned long long) * cap) != cudaSuccess)
-                return E->fail(ABD_ERR_CUDA, "cudaMallocHost block keys");
-            E->h_ukeys_cap = cap;
-        }
-        if (!E->h_done && cudaMallocHost(&E->h_done, sizeof(int) * E->ns) != cudaSuccess) {
-            E->h_done = nullptr;
-            return E->fail(ABD_ERR_CUDA, "cudaMallocHost done flags");
-        }
-        CUDA_TRY(cudaMemcpyAsync(E->h_ukeys, E->ukeys, sizeof(unsigned long long) * nkeys, cudaMemcpyDeviceToHost, s));
+        CUDA_TRY(cudaMemcpyAsync(E->h_pattern, E->ukeys, sizeof(unsigned long long) * nkeys, cudaMemcpyDeviceToHost, s));
         CUDA_TRY(cudaMemcpyAsync(E->h_done, E->sci + SI_DONE * E->ns, sizeof(int) * E->ns, cudaMemcpyDeviceToHost, s));
     }
-    E->asm_direct = direct;
     if (!ahead) {
         CUDA_TRY(cudaMemcpyAsync(E->hcnt, E->dcnt, sizeof(Counters), cudaMemcpyDeviceToHost, s));
         CUDA_TRY(cudaEventRecord(E->ev_asm, s));
@@ -470,23 +555,22 @@ int eng_assemble(Engine* E) {
     } else if ((rc = asm_keys(E, false, bound))) {
         return rc;
     }
-    int* n_unique = &E->dcnt->nkeys;
-    const long nnzb = bound;     // launch bound; the kernels read the count from the device
-    k_block_rows<<<grid_for(nnzb), 256, 0, s>>>(nb, E->ukeys, n_unique, E->row_ptr, E->bcol, E->dcnt);
+    if (!E->row_bits) {
+        // launch bound; the kernel reads the count from the device
+        k_block_rows<<<grid_for(bound), 256, 0, s>>>(nb, E->ukeys, &E->dcnt->nkeys, E->row_ptr, E->bcol, E->dcnt);
+        E->launches++;
+    }
     phase_end(E, ph, 0);
     double sc = P.kappa * P.dt * P.dt;
     if (E->mixed) {
         float* V = (float*)E->vals;
-        k_zero_vals<float><<<grid_for((long)nnzb * 144), 256, 0, s>>>(E->dcnt, V);
         k_body_assemble<float><<<grid_for(32L * nb, 32 * BA_WARPS), 32 * BA_WARPS, 0, s>>>(nb, E->st, E->mass, E->J, P.dt, P.gravity[0], P.gravity[1], P.gravity[2],
                                                                P.k_ortho, P.hess_mode == ABD_HESS_PROJECTED, P.pinned_diag,
                                                                E->row_ptr, E->bcol, V, E->g);
         if (n > 0)
             launch_contact_assemble<float>(E, n, G, sc, V);
-        k_block_inverse<float><<<grid_for(32L * nb, 32 * BI_WARPS), 32 * BI_WARPS, 0, s>>>(nb, E->row_ptr, E->bcol, V, (float*)E->dinv);
     } else {
         double* V = (double*)E->vals;
-        k_zero_vals<double><<<grid_for((long)nnzb * 144), 256, 0, s>>>(E->dcnt, V);
         int p1 = phase_begin(E, PH_ASM_BODY);
         k_body_assemble<double><<<grid_for(32L * nb, 32 * BA_WARPS), 32 * BA_WARPS, 0, s>>>(nb, E->st, E->mass, E->J, P.dt, P.gravity[0], P.gravity[1], P.gravity[2],
                                                                 P.k_ortho, P.hess_mode == ABD_HESS_PROJECTED, P.pinned_diag,
@@ -499,13 +583,7 @@ int eng_assemble(Engine* E) {
         // per candidate: type; per active contact: stencil, barrier argument,
         // 4 positions + 4 rest positions, 4 body blocks and the gradient rows
         phase_end(E, p2, 4.0 * n + E->hcnt->n_active * (16.0 + 8.0 + 96.0 + 96.0 + 4 * 1152.0 + 384.0));
-        int p3 = phase_begin(E, PH_ASM_INV);
-        k_block_inverse<double><<<grid_for(32L * nb, 32 * BI_WARPS), 32 * BI_WARPS, 0, s>>>(nb, E->row_ptr, E->bcol, V, (double*)E->dinv);
-        phase_end(E, p3, 0);
     }
-    double* gg = E->scd + SD_GG * E->ns;
-    CUDA_TRY(cudaMemsetAsync(gg, 0, sizeof(double) * E->ns, s));
-    k_grad_norm<<<grid_for(12L * nb), 256, 0, s>>>(nb, E->g, E->bscene, gg);
-    E->launches += 6 + (n > 0);
+    E->launches += 1 + (n > 0);
     return ABD_OK;
 }

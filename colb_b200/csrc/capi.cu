@@ -124,6 +124,13 @@ int eng_alloc(Engine* E) {
     cudaMemsetAsync(E->sw_nee, 0, sizeof(int), E->stream);
     cudaMemsetAsync(E->zero_ns, 0, sizeof(int) * ns, E->stream);
     DALLOC(E->row_ptr, nb + 1);
+    int most = 0;
+    for (int i = 0; i < ns; i++) most = std::max(most, E->h_body_begin[i + 1] - E->h_body_begin[i]);
+    E->row_words = (most + 31) / 32;
+    if ((long)nb * E->row_words <= ROW_BITS_MAX) {
+        DALLOC(E->row_bits, (size_t)nb * E->row_words);
+        cudaMemsetAsync(E->row_bits, 0, sizeof(uint32_t) * nb * E->row_words, E->stream);
+    }
     E->blk_cap = 0;
     if ((rc = eng_grow_blocks(E, nb + std::min(2 * E->cap, 8 * nb + 1024)))) return rc;
     size_t es = E->mixed ? sizeof(float) : sizeof(double);
@@ -156,12 +163,12 @@ void eng_free(Engine* E) {
     for (void* p : bd) if (p) cudaFree(p);
     grid_free(E->gee); grid_free(E->gpt);
     if (E->st_in) cudaFree(E->st_in);
-    if (E->h_ukeys) cudaFreeHost(E->h_ukeys);
+    if (E->h_pattern) cudaFreeHost(E->h_pattern);
     if (E->h_done) cudaFreeHost(E->h_done);
     void* ps[] = {E->xbar, E->vbody, E->vscene, E->bscene, E->edges, E->tris, E->mass, E->J, E->planes, E->plane_scene,
                   E->sc_plane_begin, E->sc_body_begin, E->edge_scene, E->tri_scene, E->st, E->backup, E->du, E->g, E->x,
                   E->xf, E->pv, E->ws, E->contacts, E->cst, E->ctype, E->cxb, E->cbody, E->cblk, E->keys, E->keys_s,
-                  E->ukeys, E->row_ptr, E->bcol, E->vals, E->dinv, E->scd, E->sci, E->cub_tmp, E->dcnt, E->prof_d,
+                  E->ukeys, E->row_bits, E->row_ptr, E->bcol, E->vals, E->dinv, E->scd, E->sci, E->cub_tmp, E->dcnt, E->prof_d,
                   E->sw, E->sw_flag, E->sw_off, E->pmag, E->vchunk, E->zero_int, E->zero_ns, E->sw_nee};
     for (void* p : ps) if (p) cudaFree(p);
     for (int i = 0; i < 10; i++) if (E->kv[i]) cudaFree(E->kv[i]);

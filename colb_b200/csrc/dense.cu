@@ -19,6 +19,7 @@
 // Mixed precision factors its FP32 blocks in FP64 on the band path, in FP32 on
 // the others.
 #include "engine.cuh"
+#include "block_inverse.cuh"
 #include <cstring>
 #include <cusolverDn.h>
 #include <algorithm>
@@ -56,26 +57,35 @@ __global__ void k_rhs_gather(int nb, const double* __restrict__ g, const int* __
         if (c >= 0) x[comp_rhs[c] + 12L * blocal[b] + i % 12] = (T)g[i];
     }
 }
-// du of every body: large components from their dense solution, single
-// bodies from their 12x12 block inverse (column-major); bodies of small
+// du of every body, one warp each: large components from their dense solution, single
+// bodies through the inverse of their 12x12 block; bodies of small
 // components (bcomp -2) and band components (-3) were written by
-// k_small_solve / k_band_solve
+// k_small_solve / k_band_solve.  (The inverses of all bodies, single or not, in
+// a launch of their own took 12 us for 256 bodies and 39 for 4,096.)
+constexpr int DU_WARPS = 4;
 template <class T>
-__global__ void k_du_scatter(int nb, const double* __restrict__ g, const int* __restrict__ bcomp,
+__global__ void __launch_bounds__(32 * DU_WARPS) k_du_scatter(int nb, const double* __restrict__ g, const int* __restrict__ bcomp,
                              const int* __restrict__ blocal, const long long* __restrict__ comp_rhs,
-                             const T* __restrict__ x, const T* __restrict__ dinv, const int* __restrict__ bscene,
+                             const T* __restrict__ x, const int* __restrict__ row_ptr, const int* __restrict__ bcol,
+                             const T* __restrict__ vals, const int* __restrict__ bscene,
                              const int* __restrict__ ndone, double* du) {
-    GS_LOOP(i, 12L * nb) {
-        int b = (int)(i / 12), r = (int)(i % 12);
-        if (ndone[bscene[b]]) continue;
-        int c = bcomp[b];
-        if (c <= -2) continue;
-        if (c >= 0) { du[i] = (double)x[comp_rhs[c] + 12L * blocal[b] + r]; continue; }
-        const T* D = dinv + 144L * b;
-        double acc = 0;
+    __shared__ double sM[DU_WARPS][12][25];
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    double (*M)[25] = sM[w];
+    for (int b = blockIdx.x * DU_WARPS + w; b < nb; b += gridDim.x * DU_WARPS) {
+        const int c = bcomp[b];
+        if (c <= -2 || ndone[bscene[b]]) continue;
+        if (c >= 0) { if (lane < 12) du[12L * b + lane] = (double)x[comp_rhs[c] + 12L * blocal[b] + lane]; continue; }
+        const int bi = find_block(row_ptr, bcol, b, b);
+        const bool ok = block_inverse_warp<T>(vals + (long)bi * 144, M, lane);
+        if (lane < 12) {
+            double acc = 0;
 #pragma unroll
-        for (int k = 0; k < 12; k++) acc += (double)D[k * 12 + r] * g[12L * b + k];
-        du[i] = acc;
+            for (int k = 0; k < 12; k++)
+                acc += (double)(T)(ok ? M[lane][12 + k] : (lane == k ? 1.0 : 0.0)) * g[12L * b + k];
+            du[12L * b + lane] = acc;
+        }
+        __syncwarp();
     }
 }
 
@@ -897,8 +907,8 @@ struct DenseState {
     void* Lg = nullptr; size_t Lg_bytes = 0;         // band factors
     void* Ab = nullptr;                              // band blocks gathered in component order (Lg_bytes)
     std::vector<unsigned long long> keys;
-    std::vector<int> done, parent, size, root, bmap, fill;
-    std::vector<int> adj_ptr, adj, pos, deg, members, mptr, bfs;
+    std::vector<int> done, rp, col, act, parent, size, root, fill;
+    std::vector<int> pos, members, mptr;
     bool smem_set[2] = {false, false};
     bool band_smem_set[2][2] = {};
 };
@@ -1017,79 +1027,83 @@ static int dense_solve_t(Engine* E, int* iters, int* fallback) {
     cudaStream_t st = E->stream;
     const int* ndone = E->sci + SI_DONE * E->ns;
     const int nb = E->nb;
-    // block pattern and done flags to the host (already there when the
-    // assembly copied them within its sync)
+    // block pattern and done flags on the host (already there when the
+    // assembly sent them): rows and columns, made from the keys where the
+    // assembly sorted keys
     const int nk = E->nnzb_host;
-    D->keys.resize(std::max(nk, 1));
-    D->done.resize(E->ns);
-    if (E->keys_host && nk <= E->h_ukeys_cap) {
-        if (nk > 0) memcpy(D->keys.data(), E->h_ukeys, sizeof(unsigned long long) * nk);
-        memcpy(D->done.data(), E->h_done, sizeof(int) * E->ns);
+    const int* rp; const int* col;
+    const int* done;
+    if (E->keys_host && E->row_bits) {
+        rp = E->h_pattern; col = rp + nb + 1; done = E->h_done;
     } else {
-        if (nk > 0) CUDA_TRY(cudaMemcpyAsync(D->keys.data(), E->ukeys, sizeof(unsigned long long) * nk, cudaMemcpyDeviceToHost, st));
-        CUDA_TRY(cudaMemcpyAsync(D->done.data(), ndone, sizeof(int) * E->ns, cudaMemcpyDeviceToHost, st));
-        CUDA_TRY(eng_stream_sync(E));
+        D->done.resize(E->ns);
+        D->rp.assign(nb + 1, 0);
+        D->col.resize(std::max(nk, 1));
+        if (E->row_bits) {
+            CUDA_TRY(cudaMemcpyAsync(D->rp.data(), E->row_ptr, sizeof(int) * (nb + 1), cudaMemcpyDeviceToHost, st));
+            CUDA_TRY(cudaMemcpyAsync(D->col.data(), E->bcol, sizeof(int) * nk, cudaMemcpyDeviceToHost, st));
+            CUDA_TRY(cudaMemcpyAsync(D->done.data(), ndone, sizeof(int) * E->ns, cudaMemcpyDeviceToHost, st));
+            CUDA_TRY(eng_stream_sync(E));
+        } else {
+            D->keys.resize(std::max(nk, 1));
+            if (E->keys_host && 2LL * nk <= E->h_pattern_cap) {
+                if (nk > 0) memcpy(D->keys.data(), E->h_pattern, sizeof(unsigned long long) * nk);
+                memcpy(D->done.data(), E->h_done, sizeof(int) * E->ns);
+            } else {
+                if (nk > 0) CUDA_TRY(cudaMemcpyAsync(D->keys.data(), E->ukeys, sizeof(unsigned long long) * nk, cudaMemcpyDeviceToHost, st));
+                CUDA_TRY(cudaMemcpyAsync(D->done.data(), ndone, sizeof(int) * E->ns, cudaMemcpyDeviceToHost, st));
+                CUDA_TRY(eng_stream_sync(E));
+            }
+            int m = 0;
+            for (int k = 0; k < nk; k++) {           // sorted
+                const unsigned long long key = D->keys[k];
+                if (key == ~0ull) continue;
+                D->rp[key / nb + 1]++;
+                D->col[m++] = (int)(key % nb);
+            }
+            for (int b = 0; b < nb; b++) D->rp[b + 1] += D->rp[b];
+        }
+        rp = D->rp.data(); col = D->col.data(); done = D->done.data();
     }
     E->keys_host = false;
-    // union-find over bodies, joined by off-diagonal blocks
+    // bodies coupled to others, of the scenes still iterating: all that the
+    // analysis looks at (a batch has thousands of bodies that touch nothing)
+    std::vector<int>& act = D->act;
+    act.clear();
+    for (int b = 0; b < nb; b++) if (rp[b + 1] - rp[b] > 1 && !done[E->h_bscene[b]]) act.push_back(b);
+    // union-find, joined by off-diagonal blocks; a root is its component's first body
     std::vector<int>& parent = D->parent;
-    parent.resize(nb);
-    for (int b = 0; b < nb; b++) parent[b] = b;
+    parent.resize(nb); D->size.resize(nb); D->pos.resize(nb); D->root.resize(nb); D->mptr.resize(nb);
+    for (int b : act) { parent[b] = b; D->size[b] = 0; D->pos[b] = -1; D->root[b] = -1; }
     auto find = [&](int x) { while (parent[x] != x) { parent[x] = parent[parent[x]]; x = parent[x]; } return x; };
-    for (int k = 0; k < nk; k++) {
-        unsigned long long key = D->keys[k];
-        if (key == ~0ull) continue;
-        int r = (int)(key / nb), c = (int)(key % nb);
-        if (r == c) continue;
-        int a = find(r), b2 = find(c);
-        if (a != b2) { if (a < b2) parent[b2] = a; else parent[a] = b2; }
-    }
-    D->size.assign(nb, 0);
-    for (int b = 0; b < nb; b++) D->size[find(b)]++;
-    const bool projected = E->P.hess_mode == ABD_HESS_PROJECTED;
-    // body adjacency (off-diagonal blocks, both directions are stored)
-    D->adj_ptr.assign(nb + 1, 0);
-    for (int k = 0; k < nk; k++) {
-        unsigned long long key = D->keys[k];
-        if (key == ~0ull) continue;
-        int r = (int)(key / nb), c = (int)(key % nb);
-        if (r != c) D->adj_ptr[r + 1]++;
-    }
-    for (int b = 0; b < nb; b++) D->adj_ptr[b + 1] += D->adj_ptr[b];
-    D->adj.resize(std::max(D->adj_ptr[nb], 1));
-    {
-        std::vector<int> at(D->adj_ptr.begin(), D->adj_ptr.end() - 1);
-        for (int k = 0; k < nk; k++) {           // keys are sorted: neighbours ascending
-            unsigned long long key = D->keys[k];
-            if (key == ~0ull) continue;
-            int r = (int)(key / nb), c = (int)(key % nb);
-            if (r != c) D->adj[at[r]++] = c;
+    for (int r : act)
+        for (int e = rp[r]; e < rp[r + 1] && col[e] < r; e++) {      // columns ascend, both directions are stored
+            int a = find(r), b2 = find(col[e]);
+            if (a != b2) { if (a < b2) parent[b2] = a; else parent[a] = b2; }
         }
-    }
-    // members of every multi-body component of a scene still iterating
-    D->mptr.assign(nb + 1, 0);
-    for (int b = 0; b < nb; b++) { int r = find(b); if (D->size[r] >= 2 && !D->done[E->h_bscene[b]]) D->mptr[r + 1]++; }
-    for (int b = 0; b < nb; b++) D->mptr[b + 1] += D->mptr[b];
-    D->members.resize(std::max(D->mptr[nb], 1));
+    for (int b : act) D->size[find(b)]++;
+    const bool projected = E->P.hess_mode == ABD_HESS_PROJECTED;
+    // members of every component, ascending
+    D->members.resize(std::max<size_t>(act.size(), 1));
     {
-        std::vector<int> at(D->mptr.begin(), D->mptr.end() - 1);
-        for (int b = 0; b < nb; b++) { int r = find(b); if (D->size[r] >= 2 && !D->done[E->h_bscene[b]]) D->members[at[r]++] = b; }
+        int at = 0;
+        for (int b : act) if (parent[b] == b) { D->mptr[b] = at; at += D->size[b]; D->size[b] = 0; }
+        for (int b : act) { int r = find(b); D->members[D->mptr[r] + D->size[r]++] = b; }
     }
     // reverse Cuthill-McKee order of a component (BFS from a minimum-degree
     // body, neighbours by ascending degree, reversed) and its body bandwidth
-    D->pos.assign(nb, -1);
+    std::vector<int> nb_;
     auto rcm = [&](int r, std::vector<int>& out) {
         const int* m = D->members.data() + D->mptr[r];
-        int n = D->mptr[r + 1] - D->mptr[r];
-        auto degree = [&](int b) { return D->adj_ptr[b + 1] - D->adj_ptr[b]; };
+        int n = D->size[r];
+        auto degree = [&](int b) { return rp[b + 1] - rp[b]; };
         int start = m[0];
         for (int i = 1; i < n; i++) if (degree(m[i]) < degree(start)) start = m[i];
         out.clear(); out.push_back(start); D->pos[start] = 0;
-        std::vector<int> nb_;
         for (size_t h = 0; h < out.size(); h++) {
             int u = out[h];
             nb_.clear();
-            for (int e = D->adj_ptr[u]; e < D->adj_ptr[u + 1]; e++) if (D->pos[D->adj[e]] < 0) nb_.push_back(D->adj[e]);
+            for (int e = rp[u]; e < rp[u + 1]; e++) if (D->pos[col[e]] < 0) nb_.push_back(col[e]);
             std::sort(nb_.begin(), nb_.end(), [&](int a, int b) { return degree(a) != degree(b) ? degree(a) < degree(b) : a < b; });
             for (int v : nb_) if (D->pos[v] < 0) { D->pos[v] = 0; out.push_back(v); }
         }
@@ -1097,14 +1111,16 @@ static int dense_solve_t(Engine* E, int* iters, int* fallback) {
         for (int i = 0; i < (int)out.size(); i++) D->pos[out[i]] = i;
         int bw = 0;
         for (int u : out)
-            for (int e = D->adj_ptr[u]; e < D->adj_ptr[u + 1]; e++) bw = std::max(bw, std::abs(D->pos[u] - D->pos[D->adj[e]]));
+            for (int e = rp[u]; e < rp[u + 1]; e++) bw = std::max(bw, std::abs(D->pos[u] - D->pos[col[e]]));
         return bw;
     };
     // components of scenes still iterating: band components (one CTA each,
     // Cholesky), small ones (one CTA each, dense in shared memory) and large
     // ones (cuSOLVER)
-    D->root.assign(nb, -1);
-    D->bmap.assign(nb, -1);
+    int* h = D->imap_h;
+    int* h_bmap = h; int* h_blocal = h + nb;
+    std::fill_n(h_bmap, nb, -1);
+    std::fill_n(h_blocal, nb, 0);
     std::vector<int> small_root, large_n, ord;
     std::vector<long long> large_off, large_rhs;
     long long aoff = 0, roff = 0;
@@ -1126,9 +1142,8 @@ static int dense_solve_t(Engine* E, int* iters, int* fallback) {
         nsub++;
         return (int)B.bw.size() - 1;
     };
-    for (int b = 0; b < nb; b++) {
+    for (int b : act) {
         int r = find(b), sz = D->size[r];
-        if (sz < 2 || D->done[E->h_bscene[b]]) continue;
         // the band path takes every component of body bandwidth <= BAND_WIDE
         // of a projected Hessian, large ones split between the two CTAs of a
         // cluster, and cuSOLVER only wider ones
@@ -1150,7 +1165,7 @@ static int dense_solve_t(Engine* E, int* iters, int* fallback) {
                 }
             }
         }
-        if (D->root[r] <= -10) { D->bmap[b] = -3; continue; }
+        if (D->root[r] <= -10) { h_bmap[b] = -3; continue; }
         if (D->root[r] < 0) {
             if (sz <= SMALL_MAX_BODIES) {
                 D->root[r] = (int)small_root.size();
@@ -1165,8 +1180,8 @@ static int dense_solve_t(Engine* E, int* iters, int* fallback) {
                 nmax_large = std::max(nmax_large, n);
             }
         }
-        if (sz <= SMALL_MAX_BODIES) { D->bmap[b] = -2; small_bodies++; }
-        else D->bmap[b] = D->root[r];
+        if (sz <= SMALL_MAX_BODIES) { h_bmap[b] = -2; small_bodies++; }
+        else h_bmap[b] = D->root[r];
     }
     const int nsmall = (int)small_root.size(), nlarge = (int)large_n.size();
     E->comp_band += ncomp_band; E->comp_small += nsmall; E->comp_large += nlarge;
@@ -1174,15 +1189,12 @@ static int dense_solve_t(Engine* E, int* iters, int* fallback) {
     if (aoff * (long long)sizeof(T) > (4LL << 30)) { *fallback = 1; E->krylov_fallbacks++; return ABD_OK; }
     // local body index inside its component (body order) and the small
     // components' body lists, packed into one upload
-    int* h = D->imap_h;
-    int* h_bmap = h; int* h_blocal = h + nb; int* h_sptr = h + 2 * nb; int* h_sbody = h_sptr + nsmall + 1;
+    int* h_sptr = h + 2 * nb; int* h_sbody = h_sptr + nsmall + 1;
     D->fill.assign(nsmall + nlarge, 0);
     h_sptr[0] = 0;
     for (int c = 0; c < nsmall; c++) h_sptr[c + 1] = h_sptr[c] + D->size[small_root[c]];
-    for (int b = 0; b < nb; b++) {
-        int m = D->bmap[b];
-        h_bmap[b] = m;
-        h_blocal[b] = 0;
+    for (int b : act) {
+        int m = h_bmap[b];
         if (m == -2) {
             int c = D->root[find(b)];
             int l = D->fill[c]++;
@@ -1312,8 +1324,8 @@ static int dense_solve_t(Engine* E, int* iters, int* fallback) {
             if (use_lu[c] && lu_solve<T>(D, large_n[c], A + large_off[c], x + large_rhs[c], work, D->info + 2 + 2 * c) != CUSOLVER_STATUS_SUCCESS)
                 return E->fail(ABD_ERR_CUDA, "cusolver getrf/getrs");
     }
-    k_du_scatter<T><<<grid_for(12L * nb), 256, 0, st>>>(nb, E->g, d_bmap, d_blocal, nlarge ? D->comp_d + nlarge : nullptr, x,
-                                                       (const T*)E->dinv, E->bscene, ndone, E->du);
+    k_du_scatter<T><<<grid_for(32L * nb, 32 * DU_WARPS), 32 * DU_WARPS, 0, st>>>(nb, E->g, d_bmap, d_blocal,
+        nlarge ? D->comp_d + nlarge : nullptr, x, E->row_ptr, E->bcol, (const T*)E->vals, E->bscene, ndone, E->du);
     E->launches++;
     *iters = 1;
     return ABD_OK;

@@ -104,10 +104,15 @@ struct Counters {
     int nkeys, grp_fail, ls_trials, ls_nsw;   // ls_*: trial count and list length of a graph line search
     int n_sw, n_sw_ee, sw_overflow, pos_changed;   // pos_changed: abd_set_state moved a body
     int du_guard;                                  // mixed-precision increments replaced (du_guard)
+    int act;                                       // active contacts counted so far (assembly by row bits)
     int ticket;                                    // blocks that have finished the current search kernel
     alignas(8) int bp[8];                          // host only: counts of a body-pair build (bpair.cu)
 };
 #define DETECT_COUNTER_BYTES (5 * sizeof(int))   // n_ee .. overflow
+
+// words of the block rows' bit pattern at most: one block reads them all, and
+// FIGW
+constexpr long ROW_BITS_MAX = 1 << 16;
 
 struct Engine {
     AbdParams P;
@@ -162,7 +167,7 @@ struct Engine {
     int* sw_nee = nullptr;         // device copy of the list's EE count (the list filter reads it)
     // block keys and done flags of the last assembly, copied to pinned host
     // memory in the assembly's own sync for the direct solver's analysis
-    unsigned long long* h_ukeys = nullptr; int h_ukeys_cap = 0; int* h_done = nullptr; bool keys_host = false;
+    int* h_pattern = nullptr; int h_pattern_cap = 0; int* h_done = nullptr; bool keys_host = false;
     int* sw_flag = nullptr; int* sw_off = nullptr;
     int4* vchunk = nullptr; int nvchunk = 0;       // runs of <= VCHUNK vertices of one body {body, first, count, first run}
     bool x_fresh = false;          // x and xf are the vertices of st's nxt state
@@ -173,6 +178,7 @@ struct Engine {
     // block matrix
     unsigned long long* keys = nullptr; unsigned long long* keys_s = nullptr; unsigned long long* ukeys = nullptr;
     int blk_cap = 0;
+    uint32_t* row_bits = nullptr; int row_words = 0;   // pattern of the block rows (assemble.cu), null: too large
     int nnzb_host = 0;             // block count of the last assembly (host copy)
     long long dense_blocks = 0;    // sum over scenes of n_bodies^2: no assembly has more blocks
     // the assembly's counters and block keys travel to the host behind
@@ -321,6 +327,7 @@ int eng_intersections(Engine* E, int* count);
 int eng_sync_counters(Engine* E);
 int eng_asm_wait(Engine* E);                           // counters and block keys of the last assembly on the host
 int eng_assemble_keys_ahead(Engine* E);               // the next iterate's block keys, before the iteration's sync
+int eng_sync_ahead(Engine* E);                        // the sync after eng_assemble_keys_ahead
 void eng_keys_ahead_synced(Engine* E);                // after that sync: keys on the host unless the detection overflowed
 int eng_grid_build(Engine* E, Grid& G);
 GridView eng_view(const Grid& G);

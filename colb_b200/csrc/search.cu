@@ -50,8 +50,9 @@ struct LsGrid { int bodies, pairs, chunks, group; int total() const { return bod
 // large batches, where most chunks belong to scenes that have converged
 inline int chunk_group(int nchunks, int warps) { return std::min(32, std::max(1, (nchunks + warps - 1) / warps)); }
 
-__global__ void k_ls_zero(int n, double* toi, double* e0, double* e0n) {
+__global__ void k_ls_zero(int n, double* toi, double* e0, double* e0n, int ns, double* gg) {
     GS_LOOP(i, n) { toi[i] = 1.0; e0[i] = 0.0; e0n[i] = 0.0; }
+    GS_LOOP(i, ns) gg[i] = 0.0;
 }
 
 struct LsArgs {
@@ -59,6 +60,7 @@ struct LsArgs {
     const int4* list; const int4* chunks; int nchunks;
     Geo G; const double* p;                      // geometry at the current positions, displacement of the step
     const double* st; const double* J; double* backup;
+    const double* g; const int* bscene; double* gg;   // gradient, and its squared norm per scene
     const int* unit; const int* skip;            // unit of a body; units left alone
     BodyTerms B; PairTerms T; StepBoxes box; int npl;
     int ccd; double ccd_scale; int ccd_it;
@@ -86,6 +88,14 @@ DV void ls_terms(const LsArgs& A, const LsGrid& g, int* capped) {
             }
             warp_reduce_add(A.E, u, e, valid);
             warp_reduce_add(A.En, u, en, valid);
+            if (BEGIN) {
+                double n2 = 0;
+                if (b < A.nb) {
+#pragma unroll
+                    for (int k = 0; k < 12; k++) n2 += A.g[12 * b + k] * A.g[12 * b + k];
+                }
+                warp_reduce_add(A.gg, b < A.nb ? A.bscene[b] : 0, n2, b < A.nb);
+            }
         }
     } else if ((int)blockIdx.x < g.bodies + g.pairs) {
         const int n = A.n_dev ? *A.n_dev : A.n;
@@ -300,7 +310,8 @@ int eng_ls_begin(Engine* E, const LsUnits& U, const int* udone) {
     int rc = eng_transform(E);
     if (rc) return rc;
     LsArgs A = ls_args(E, U, udone, SD_E0);
-    k_ls_zero<<<grid_for(U.n), 256, 0, s>>>(U.n, A.toi, A.E, A.En);
+    A.g = E->g; A.bscene = E->bscene; A.gg = E->scd + SD_GG * E->ns;
+    k_ls_zero<<<grid_for(std::max(U.n, E->ns)), 256, 0, s>>>(U.n, A.toi, A.E, A.En, E->ns, A.gg);
     const int threads = TUNE_THREADS[tune_begin(E, TK_LIST_ENERGY, 3, 1)];
     const LsGrid g = ls_grid(E, threads, E->n_sw);
     k_ls_begin<<<g.total(), threads, 0, s>>>(A, g, U.n, udone, U.i + SI_ACC * U.n, U.d + SD_ALPHA * U.n, U.i + SI_STALL * U.n,

@@ -643,7 +643,10 @@ static int du_guard(Engine* E, bool inject) {
     return ABD_OK;
 }
 static int solve_any(Engine* E, int* iters);
+int eng_block_inverse(Engine* E);
 int eng_solve(Engine* E, int* iters, bool first_iter) {
+    // the guard's increment, and the Krylov solves' preconditioner
+    if (E->mixed) { int rc = eng_block_inverse(E); if (rc) return rc; }
     int rc = solve_any(E, iters);
     if (rc || !E->mixed) return rc;
     return du_guard(E, first_iter && (E->P.test_inject & ABD_INJECT_DU_NONFINITE));
@@ -659,6 +662,7 @@ static int solve_any(Engine* E, int* iters) {
         // too many large components for one factorization each
         kind = E->P.hess_mode == ABD_HESS_PROJECTED ? ABD_SOLVER_PCG : ABD_SOLVER_BICGSTAB;
     }
+    if (!E->mixed) { int rc = eng_block_inverse(E); if (rc) return rc; }
     KrylovKind kk(E, kind);
     if (E->mixed) return solve_t<float>(E, iters);
     return solve_t<double>(E, iters);

@@ -333,7 +333,7 @@ int eng_step(Engine* E, int n_steps, AbdStepStats* stats) {
                 // brings them to the direct solver too
                 if ((rc = eng_assemble_keys_ahead(E))) return rc;
             }
-            if ((rc = eng_sync_counters(E))) return rc;
+            if ((rc = eng_sync_ahead(E))) return rc;
             eng_keys_ahead_synced(E);
             detected_ahead = ahead;
             if (graph_ran) {

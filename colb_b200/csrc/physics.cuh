@@ -94,6 +94,7 @@ DV double ortho_hess(const double* q, double k, int i, int j, int r, int c) {
 // a vanishing singular value's u completed by a cross product.
 DV void svd3(const double* A, double* U, double* s, double* V) {
     double S[9];
+#pragma unroll
     for (int i = 0; i < 3; i++)
         for (int j = 0; j < 3; j++) S[3*i+j] = A[i] * A[j] + A[3+i] * A[3+j] + A[6+i] * A[6+j];
     for (int i = 0; i < 9; i++) V[i] = (i % 4 == 0) ? 1.0 : 0.0;
@@ -101,6 +102,7 @@ DV void svd3(const double* A, double* U, double* s, double* V) {
     for (int sweep = 0; sweep < 16; sweep++) {
         double off = S[1] * S[1] + S[2] * S[2] + S[5] * S[5];
         if (!(off > 1e-34 * tr * tr)) break;
+#pragma unroll
         for (int pq = 0; pq < 3; pq++) {
             int p = pq == 2 ? 1 : 0, q = pq == 0 ? 1 : 2;
             double apq = S[3*p+q];
@@ -126,11 +128,13 @@ DV void svd3(const double* A, double* U, double* s, double* V) {
     double smax = 0;
     for (int i = 0; i < 3; i++) { s[i] = sqrt(fmax(S[4*i], 0.0)); smax = fmax(smax, s[i]); }
     bool ok[3];
+#pragma unroll
     for (int i = 0; i < 3; i++) {
         ok[i] = s[i] > 1e-12 * smax && s[i] > 0.0;
         for (int r = 0; r < 3; r++)
             U[3*r+i] = ok[i] ? (A[3*r] * V[i] + A[3*r+1] * V[3+i] + A[3*r+2] * V[6+i]) / s[i] : 0.0;
     }
+#pragma unroll
     for (int i = 0; i < 3; i++) {
         if (ok[i]) continue;
         int j = (i + 1) % 3, k = (i + 2) % 3;
@@ -152,35 +156,39 @@ DV void svd3(const double* A, double* U, double* s, double* V) {
 //   U e_i e_i^T V^T                       12 s_i^2 - 4
 //   U (e_i e_j^T + e_j e_i^T) V^T / sqrt2   4 (s_i^2 + s_i s_j + s_j^2 - 1)
 //   U (e_i e_j^T - e_j e_i^T) V^T / sqrt2   4 (s_i^2 - s_i s_j + s_j^2 - 1)
-// (times k).  Each lane of a warp writes its entries of out (ld 12) times
-// scale; all 32 lanes call it.
-DV void ortho_hess_psd_warp(const double* q, double scale, double* out, int lane) {
-    double U[9], s[3], V[9];
-    svd3(q, U, s, V);
-    double lam[9], vec[9][9];
-    int m = 0;
+// (times k).  usv holds U, V (row-major) and s; vec is 81 doubles of scratch.
+// The lanes of a warp build the nine eigenvectors and then the entries of out
+// (ld 12) times scale; all 32 call it.
+struct OrthoSvd { double U[9], V[9], s[3]; };
+DV void ortho_hess_psd_warp(const OrthoSvd& usv, double scale, double* vec, double* out, int lane) {
     const double r2 = 0.70710678118654752440;
-    for (int i = 0; i < 3; i++, m++) {
-        lam[m] = 12.0 * s[i] * s[i] - 4.0;
-        for (int r = 0; r < 3; r++)
-            for (int c = 0; c < 3; c++) vec[m][3*r+c] = U[3*r+i] * V[3*c+i];
-    }
-    for (int i = 0; i < 3; i++)
-        for (int j = i + 1; j < 3; j++) {
-            lam[m] = 4.0 * (s[i] * s[i] + s[i] * s[j] + s[j] * s[j] - 1.0);
-            lam[m + 1] = 4.0 * (s[i] * s[i] - s[i] * s[j] + s[j] * s[j] - 1.0);
-            for (int r = 0; r < 3; r++)
-                for (int c = 0; c < 3; c++) {
-                    double a = U[3*r+i] * V[3*c+j], b = U[3*r+j] * V[3*c+i];
-                    vec[m][3*r+c] = (a + b) * r2;
-                    vec[m + 1][3*r+c] = (a - b) * r2;
-                }
-            m += 2;
+    const double *U = usv.U, *V = usv.V, *s = usv.s;
+    for (int e = lane; e < 81; e += 32) {
+        const int m = e / 9, r = e % 9 / 3, c = e % 3;
+        double v;
+        if (m < 3) v = U[3*r+m] * V[3*c+m];
+        else {
+            const int pr = (m - 3) >> 1, i = pr == 2 ? 1 : 0, j = pr == 0 ? 1 : 2;
+            const double a = U[3*r+i] * V[3*c+j], b = U[3*r+j] * V[3*c+i];
+            v = ((m - 3) & 1 ? a - b : a + b) * r2;
         }
+        vec[e] = v;
+    }
+    double lam[9];
+#pragma unroll
+    for (int i = 0; i < 3; i++) lam[i] = 12.0 * s[i] * s[i] - 4.0;
+#pragma unroll
+    for (int pr = 0; pr < 3; pr++) {
+        const int i = pr == 2 ? 1 : 0, j = pr == 0 ? 1 : 2;
+        lam[3 + 2 * pr] = 4.0 * (s[i] * s[i] + s[i] * s[j] + s[j] * s[j] - 1.0);
+        lam[4 + 2 * pr] = 4.0 * (s[i] * s[i] - s[i] * s[j] + s[j] * s[j] - 1.0);
+    }
+    __syncwarp();
     for (int e = lane; e < 81; e += 32) {
         int a = e / 9, b = e % 9;
         double acc = 0;
-        for (int k = 0; k < 9; k++) if (lam[k] > 0) acc += lam[k] * vec[k][a] * vec[k][b];
+#pragma unroll
+        for (int k = 0; k < 9; k++) if (lam[k] > 0) acc += lam[k] * vec[9*k+a] * vec[9*k+b];
         out[a * 12 + b] = acc * scale;
     }
 }

@@ -66,3 +66,17 @@ DV void atomic_min_pos(double* addr, double v) {
 DV void atomic_max_pos(float* addr, float v) {
     atomicMax(reinterpret_cast<int*>(addr), __float_as_int(v));
 }
+
+// The block that finishes last returns true in every thread.  Blocks publish
+// their atomics before they take a ticket, and the last one resets it.
+DV bool last_block(int* ticket) {
+    __shared__ int last;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        last = atomicAdd(ticket, 1) == (int)gridDim.x - 1;
+        if (last) { *ticket = 0; __threadfence(); }
+    }
+    __syncthreads();
+    return last;
+}

@@ -216,42 +216,139 @@ __global__ void k_pt_pairs(int nv, GridView GV, Geo G, const float4* __restrict_
     }
 }
 
-// half-space candidates: per vertex over its scene's planes
-__global__ void k_pg_pairs(int nv, Geo G, const int* __restrict__ vscene, double filt, int mode,
-                           int* qcount, const int* qoff, const Counters* cnt, int cap, int4* out, int* overflow) {
-    GS_LOOP(v, nv) {
-        int s = vscene[v];
-        int p0 = G.sc_plane_begin[s], p1 = G.sc_plane_begin[s+1];
-        int c = 0, base = 0;
-        if (mode == 1) base = cnt->n_ee + cnt->n_pt + qoff[v];
-        for (int pl = p0; pl < p1; pl++) {
-            const double* n = G.planes + 4*pl;
-            double d = n[0] * G.x[3*v] + n[1] * G.x[3*v+1] + n[2] * G.x[3*v+2] - n[3];
-            if (!(d < filt)) continue;
-            if (mode == 1) {
-                int at = base + c;
-                if ((unsigned)at < (unsigned)cap) out[at] = make_int4(ABD_CONTACT_PG, (int)v, pl, 0);
-                else *overflow = 1;
-            }
-            c++;
-        }
-        if (mode == 0) qcount[v] = c;
-    }
-}
-
 __global__ void k_store_count(const int* qoff, int n, int slot, Counters* cnt) {
     if (threadIdx.x == 0 && blockIdx.x == 0) {
         int v = qoff[n];
         if (slot == 0) cnt->n_ee = v;
-        else if (slot == 1) cnt->n_pt = v;
-        else cnt->n_pg = v;
+        else cnt->n_pt = v;
     }
 }
-__global__ void k_finalize_counts(Counters* cnt, int cap) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        int n = cnt->n_ee + cnt->n_pt + cnt->n_pg;
-        cnt->n_total = n;
-        if (n > cap) cnt->overflow = 1;
+
+// ------------------------------------------------------------------ ordered filter
+// The candidates that survive among the listed pairs (EE, then PT) and then
+// those of the vertices near a half-space (by vertex, then plane), in order
+// and in two launches.  k_filter_count tests every item: a tile of pairs per
+// block, whose survivors it keeps as bits, or a tile of vertices; the block
+// that finishes last turns the tiles' counts into places and sets the
+// counters.  k_filter_write copies the survivors of its tile there; most
+// tiles have none.  (Flags, a scan and a copy per kind with their clears took eight
+// nodes of an iteration: eight cubes 31 -> 12 us with the gaps, the resting 16 x 16
+// net 28 -> 13, 512 scenes of 1.6 million vertices 48 -> 30.)
+constexpr int FL_THREADS = 256;
+constexpr int FL_VERTS = 4 * FL_THREADS;         // vertices of a tile
+struct FilterArgs {
+    int n; const int4* list; int f32, self_contact;  // listed pairs; n < 0: EE and PT are counted already
+    int list_tiles, vert_tiles;
+    int nv; const int* vscene; double filt;
+    Geo G;
+    uint32_t* keep;                              // survivors of the list, a bit each
+    int *list_at, *ee, *vert_at;                 // per tile: count, then place; EE survivors
+    int4* out; int cap; Counters* cnt;
+};
+DV int pg_count(const FilterArgs& A, int v) {
+    const int s = A.vscene[v], p1 = A.G.sc_plane_begin[s + 1];
+    int c = 0;
+    for (int pl = A.G.sc_plane_begin[s]; pl < p1; pl++) {
+        const double* n = A.G.planes + 4*pl;
+        const double d = n[0] * A.G.x[3*v] + n[1] * A.G.x[3*v+1] + n[2] * A.G.x[3*v+2] - n[3];
+        c += d < A.filt;
+    }
+    return c;
+}
+// exclusive sum over the block's threads and the block's total; every thread calls it
+DV int block_scan(int v, int* sh, int& total) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    int incl = v;
+    for (int o = 1; o < 32; o <<= 1) { int u = __shfl_up_sync(0xffffffffu, incl, o); if (lane >= o) incl += u; }
+    __syncthreads();                             // sh is free
+    if (lane == 31) sh[w] = incl;
+    __syncthreads();
+    int before = 0;
+    total = 0;
+    for (int k = 0; k < FL_THREADS / 32; k++) { if (k < w) before += sh[k]; total += sh[k]; }
+    return before + incl - v;
+}
+// counts at `at` (of other blocks) to places from `base` on; returns the end
+DV int places(int* at, int n, int base, int* sh) {
+    for (int t = 0; t < n; t += FL_THREADS) {
+        const int k = t + threadIdx.x;
+        int total, e = block_scan(k < n ? __ldcg(at + k) : 0, sh, total);
+        if (k < n) at[k] = base + e;
+        base += total;
+    }
+    return base;
+}
+__global__ void __launch_bounds__(FL_THREADS) k_filter_count(FilterArgs A) {
+    __shared__ int sh[FL_THREADS / 32];
+    const int tile = blockIdx.x, tid = threadIdx.x;
+    if (tile < A.list_tiles) {
+        const int c = tile * FL_THREADS + tid;
+        bool keep = false, ee = false;
+        if (c < A.n) {
+            const int4 C = A.list[c];
+            ee = C.x == ABD_CONTACT_EE;
+            if (ee) { double s, t, d; keep = ee_test(A.G, C.y, C.z, A.f32, A.self_contact, A.filt, s, t, d); }
+            else keep = pt_test(A.G, C.y, C.z, A.self_contact, A.filt);
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, keep);
+        if ((tid & 31) == 0 && c < A.n) A.keep[c >> 5] = m;
+        const int kept = __syncthreads_count(keep), kept_ee = __syncthreads_count(keep && ee);
+        if (tid == 0) { A.list_at[tile] = kept; A.ee[tile] = kept_ee; }
+    } else if (tile < A.list_tiles + A.vert_tiles) {
+        const int v0 = (tile - A.list_tiles) * FL_VERTS + tid;
+        int c = 0;
+#pragma unroll
+        for (int j = 0; j < FL_VERTS / FL_THREADS; j++) { const int v = v0 + j * FL_THREADS; if (v < A.nv) c += pg_count(A, v); }
+        int total;
+        block_scan(c, sh, total);
+        if (tid == 0) A.vert_at[tile - A.list_tiles] = total;
+    }
+    if (!last_block(&A.cnt->ticket)) return;
+    int n_ee = 0, base = 0;
+    if (A.n < 0) base = A.cnt->n_ee + A.cnt->n_pt;
+    else {
+        int e = 0;
+        for (int k = tid; k < A.list_tiles; k += FL_THREADS) e += __ldcg(A.ee + k);
+        block_scan(e, sh, n_ee);
+        base = places(A.list_at, A.list_tiles, 0, sh);
+    }
+    const int end = places(A.vert_at, A.vert_tiles, base, sh);
+    if (tid == 0) {
+        if (A.n >= 0) { A.cnt->n_ee = n_ee; A.cnt->n_pt = base - n_ee; A.cnt->overflow = 0; }
+        A.cnt->n_pg = end - base;
+        A.cnt->n_total = end;
+        if (end > A.cap) A.cnt->overflow = 1;
+    }
+}
+__global__ void __launch_bounds__(FL_THREADS) k_filter_write(FilterArgs A) {
+    __shared__ int sh[FL_THREADS / 32];
+    const int tile = blockIdx.x, tid = threadIdx.x;
+    if (tile < A.list_tiles) {
+        const int c = tile * FL_THREADS + tid, w0 = tile * (FL_THREADS / 32), nw = (A.n + 31) / 32;
+        const unsigned m = c < A.n ? A.keep[c >> 5] : 0;
+        if (!(m >> (tid & 31) & 1)) return;
+        int at = A.list_at[tile] + __popc(m & ((1u << (tid & 31)) - 1));
+        for (int w = w0; w < (c >> 5) && w < nw; w++) at += __popc(A.keep[w]);
+        if ((unsigned)at < (unsigned)A.cap) A.out[at] = A.list[c];
+        return;
+    }
+    const int t = tile - A.list_tiles;
+    int base = A.vert_at[t];
+    const int end = t + 1 < A.vert_tiles ? A.vert_at[t + 1] : A.cnt->n_total;
+    if (base == end) return;
+    for (int j = 0; j < FL_VERTS / FL_THREADS; j++) {
+        const int v = t * FL_VERTS + j * FL_THREADS + tid;
+        int total, at = base + block_scan(v < A.nv ? pg_count(A, v) : 0, sh, total);
+        base += total;
+        if (v >= A.nv) continue;
+        const int s = A.vscene[v], p1 = A.G.sc_plane_begin[s + 1];
+        for (int pl = A.G.sc_plane_begin[s]; pl < p1; pl++) {
+            const double* n = A.G.planes + 4*pl;
+            const double d = n[0] * A.G.x[3*v] + n[1] * A.G.x[3*v+1] + n[2] * A.G.x[3*v+2] - n[3];
+            if (!(d < A.filt)) continue;
+            if ((unsigned)at < (unsigned)A.cap) A.out[at] = make_int4(ABD_CONTACT_PG, v, pl, 0);
+            at++;
+        }
     }
 }
 
@@ -322,25 +419,24 @@ int eng_detect(Engine* E, double filt) {
     return eng_pg_candidates(E, filt);
 }
 
-// half-space candidates appended after EE and PT, then the total
-int eng_pg_candidates(Engine* E, double filt) {
-    cudaStream_t s = E->stream;
-    int rc;
-    if (E->npl > 0) {
-        Geo G = geo(E);
-        // reuse the PT query buffers for the per-vertex plane counts
-        int* qc = E->gpt.qcount; int* qo = E->gpt.qoff;
-        k_pg_pairs<<<grid_for(E->nv), 256, 0, s>>>(E->nv, G, E->vscene, filt, 0, qc, nullptr, E->dcnt, E->cap, E->contacts, &E->dcnt->overflow);
-        CUDA_TRY(cudaMemsetAsync(qc + E->nv, 0, sizeof(int), s));
-        if ((rc = scan_counts(E, qc, qo, E->nv))) return rc;
-        k_store_count<<<1, 32, 0, s>>>(qo, E->nv, 2, E->dcnt);
-        k_pg_pairs<<<grid_for(E->nv), 256, 0, s>>>(E->nv, G, E->vscene, filt, 1, qc, qo, E->dcnt, E->cap, E->contacts, &E->dcnt->overflow);
-        E->launches += 3;
-    }
-    k_finalize_counts<<<1, 32, 0, s>>>(E->dcnt, E->cap);
-    E->launches++;
+int eng_filter(Engine* E, int n_list, double filt) {
+    FilterArgs A;
+    A.n = n_list; A.list = E->sw; A.f32 = E->P.ee_f32; A.self_contact = E->P.self_contact;
+    A.list_tiles = n_list > 0 ? (n_list + FL_THREADS - 1) / FL_THREADS : 0;
+    A.vert_tiles = E->npl > 0 ? (E->nv + FL_VERTS - 1) / FL_VERTS : 0;
+    A.nv = E->nv; A.vscene = E->vscene; A.filt = filt; A.G = geo(E);
+    A.keep = (uint32_t*)E->sw_flag; A.list_at = E->sw_off; A.ee = E->sw_off + A.list_tiles;
+    A.vert_at = E->gpt.qoff;                     // the PT query's, free here
+    A.out = E->contacts; A.cap = E->cap; A.cnt = E->dcnt;
+    const int tiles = A.list_tiles + A.vert_tiles;
+    k_filter_count<<<std::max(tiles, 1), FL_THREADS, 0, E->stream>>>(A);
+    if (tiles > 0) k_filter_write<<<tiles, FL_THREADS, 0, E->stream>>>(A);
+    E->launches += 1 + (tiles > 0);
     return ABD_OK;
 }
+
+// half-space candidates appended after EE and PT, then the total
+int eng_pg_candidates(Engine* E, double filt) { return eng_filter(E, -1, filt); }
 
 // ------------------------------------------------------------------ energies
 __global__ void k_body_energy(int nb, const double* __restrict__ st, const double* __restrict__ mass,

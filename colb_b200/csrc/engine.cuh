@@ -328,6 +328,7 @@ int eng_intersections(Engine* E, int* count);
 int eng_sync_counters(Engine* E);
 int eng_asm_wait(Engine* E);                           // counters and block keys of the last assembly on the host
 int eng_assemble_keys_ahead(Engine* E);               // the next iterate's block keys, before the iteration's sync
+int eng_filter(Engine* E, int n_list, double filt);   // candidates of the swept list (n_list >= 0) and of the half-spaces
 int eng_sync_ahead(Engine* E);                        // the sync after eng_assemble_keys_ahead
 void eng_keys_ahead_synced(Engine* E);                // after that sync: keys on the host unless the detection overflowed
 int eng_grid_build(Engine* E, Grid& G);

@@ -30,19 +30,6 @@ DV void box_plane(float4 lo, float4 hi, const double* n, double& dmin, double& d
     dmin = fmin(a0, a1) + fmin(b0, b1) + fmin(c0, c1) - n[3];
     dmax = fmax(a0, a1) + fmax(b0, b1) + fmax(c0, c1) - n[3];
 }
-// The block that finishes last returns true in every thread.  Blocks publish
-// their atomics before they take a ticket, and the last one resets it.
-DV bool last_block(int* ticket) {
-    __shared__ int last;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        last = atomicAdd(ticket, 1) == (int)gridDim.x - 1;
-        if (last) { *ticket = 0; __threadfence(); }
-    }
-    __syncthreads();
-    return last;
-}
 // grid split over the three kinds of work; a warp looks at `group` chunks at
 // once and then works on the live ones
 struct LsGrid { int bodies, pairs, chunks, group; int total() const { return bodies + pairs + chunks; } };

@@ -305,49 +305,11 @@ int eng_energy_candidates(Engine* E, int slot, const int* skip) {
 }
 
 // ------------------------------------------------------------------ detection from the list
-__global__ void k_list_flags(int n, const int4* __restrict__ list, Geo G, int f32, int self_contact, double cand,
-                             int* flag) {
-    GS_LOOP(c, n) {
-        int4 C = list[c];
-        bool keep;
-        if (C.x == ABD_CONTACT_EE) { double s, t, d; keep = ee_test(G, C.y, C.z, f32, self_contact, cand, s, t, d); }
-        else keep = pt_test(G, C.y, C.z, self_contact, cand);
-        flag[c] = keep ? 1 : 0;
-    }
-}
-__global__ void k_list_scatter(int n, const int4* __restrict__ list, const int* __restrict__ flag, const int* __restrict__ off,
-                               int4* out, const int* __restrict__ n_ee_dev, Counters* cnt, int cap) {
-    const int n_ee_list = *n_ee_dev;
-    GS_LOOP(c, n) {
-        if (flag[c]) { int at = off[c]; if ((unsigned)at < (unsigned)cap) out[at] = list[c]; }
-    }
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        cnt->n_ee = off[n_ee_list];
-        cnt->n_pt = off[n] - off[n_ee_list];
-    }
-}
-
-int eng_pg_candidates(Engine* E, double filt);
-
 // candidate list at the current nxt state from the swept list; the list
 // must cover the current positions (built for the step that led here)
 int eng_detect_list(Engine* E) {
-    cudaStream_t s = E->stream;
     const AbdParams& P = E->P;
     int rc = eng_transform(E);
     if (rc) return rc;
-    CUDA_TRY(cudaMemsetAsync(E->dcnt, 0, DETECT_COUNTER_BYTES, s));
-    int n = E->n_sw;
-    if (n > 0) {
-        Geo G = eng_geo(E);
-        int* flag = E->sw_flag;
-        int* off = E->sw_off;
-        k_list_flags<<<grid_for(n), 256, 0, s>>>(n, E->sw, G, P.ee_f32, P.self_contact, P.cand_dist, flag);
-        CUDA_TRY(cudaMemsetAsync(flag + n, 0, sizeof(int), s));
-        size_t bytes = E->cub_bytes;
-        CUDA_TRY(cub::DeviceScan::ExclusiveSum(E->cub_tmp, bytes, flag, off, n + 1, s));
-        k_list_scatter<<<grid_for(n), 256, 0, s>>>(n, E->sw, flag, off, E->contacts, E->sw_nee, E->dcnt, E->cap);
-        E->launches += 3;
-    }
-    return eng_pg_candidates(E, P.cand_dist);
+    return eng_filter(E, E->n_sw, P.cand_dist);
 }

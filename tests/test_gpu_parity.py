@@ -338,3 +338,24 @@ def test_bicgstab_by_scene_size(chain_scene, chain_pairs, sizes, precision):
         ref = np.linalg.solve(A, b)
         kappa = np.linalg.cond(A * d[:, None] * d)
         assert np.linalg.norm((du[k] - ref) / d) <= (tol + 50 * eps) * kappa * np.linalg.norm(ref / d), (n, kappa)
+
+
+@pytest.mark.parametrize("nu,nv,bodies", [(3, 3, 1), (16, 16, 1), (31, 33, 1), (32, 32, 1), (25, 41, 1), (16, 8, 9), (32, 32, 3)])
+@pytest.mark.parametrize("broadphase", [1, 2])
+def test_half_space_candidates_at_tile_edges(nu, nv, bodies, broadphase):
+    """Bodies of 9 to 1,025 vertices (below, at and above the 1,024 vertices of
+    a block) that cross two half-spaces or none: by vertex, then plane."""
+    V, F = S.torus_mesh(1.0, 0.25, nu, nv)
+    rng = np.random.default_rng(nu + bodies)
+    sc = S.assemble_bodies([S._body(V, F, 1000.0, [4.0 * k, rng.uniform(-0.4, 0.4) + (5.0 if k % 3 == 1 else 0.0), 0.0],
+                                    S._rand_rotation(rng)) for k in range(bodies)],
+                           planes=[[0.0, 1.0, 0.0, -0.2], [0.6, 0.8, 0.0, 0.1]])
+    p = P.config_params(broadphase=broadphase)
+    e = Engine(p, sc)
+    x = e.vertices()
+    d = x @ np.array([[0.0, 1.0, 0.0], [0.6, 0.8, 0.0]]).T - np.array([-0.2, 0.1])
+    want = np.argwhere(d < p.cand_dist)
+    quads, kinds = e.pairs()
+    got = quads[kinds == 2][:, :2]
+    assert len(want) > 0 and np.array_equal(got, want)
+    assert np.all(np.diff(kinds) >= 0)

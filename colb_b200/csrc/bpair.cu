@@ -165,7 +165,8 @@ struct BpDisp {                                                      // dq null:
 };
 constexpr int BOX_THREADS = 128;
 __global__ void __launch_bounds__(BOX_THREADS) k_bp_boxes(int nb, const int* __restrict__ vbeg, const double* __restrict__ x,
-        BpDisp D, float pad, int keep, BpBoxes B) {
+        BpDisp D, float pad, int keep, BpBoxes B, int* cnt) {
+    if (blockIdx.x == 0 && threadIdx.x < 8) cnt[threadIdx.x] = 0;         // the build's counts
     __shared__ float4 slo[BOX_THREADS / 32], shi[BOX_THREADS / 32];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     for (int b = blockIdx.x; b < nb; b += gridDim.x) {
@@ -511,11 +512,14 @@ static int bp_reserve(Engine* E, int bp_need, long long item_need, int key_need)
     return ABD_OK;
 }
 
+// the counts to pinned host memory (a copy costs 6 us with its gap, this 3)
+__global__ void k_bp_send(const int* __restrict__ cnt, int* host) { if (threadIdx.x < 8) host[threadIdx.x] = cnt[threadIdx.x]; }
+
 // Build a sorted (kind, a, b) list of EE and PT candidates into `out`
 // (capacity *cap, grown through `grow`).  disp.dq null: static positions.
 // mode 0: swept list with limit lim; mode 1: detection with distance filt.
 // The list length comes back to the host; its EE count stays on the device
-// (copied to nee_dev when given; BpScratch::cnt[2] until the next build).
+// (BpScratch::cnt[2] until the next build).
 // Steps of the resting 16 x 16 net, one handle: 13.51 -> 11.85 ms per step, of
 // eight nets in one handle 24.5 -> 18.1 ms, against one block per body pair
 // with both bodies' primitives staged in shared memory (90 and 464 us per
@@ -523,7 +527,7 @@ static int bp_reserve(Engine* E, int bp_need, long long item_need, int key_need)
 // and a radix sort over 64 bits for every list (35 us for short ones, k_bp_rank
 // 12 us; the sort stays for longer lists, where counting is quadratic).
 static int bp_build(Engine* E, const BpDisp& disp, double lim, double filt, int mode, int4*& out, int& cap, int& n_out,
-                    int* nee_dev, int (*grow)(Engine*, int)) {
+                    int (*grow)(Engine*, int)) {
     cudaStream_t s = E->stream;
     const AbdParams& P = E->P;
     int rc;
@@ -536,10 +540,10 @@ static int bp_build(Engine* E, const BpDisp& disp, double lim, double filt, int 
     const int keep = mode == 0 && S->swept && E->sw_valid;
     S->swept = false;
     const int body_grid = std::min(E->nb, NUM_SMS * 16);
-    k_bp_boxes<<<body_grid, BOX_THREADS, 0, s>>>(E->nb, E->bd_vbeg, E->x, disp, pad, keep, S->B);
+    k_bp_boxes<<<body_grid, BOX_THREADS, 0, s>>>(E->nb, E->bd_vbeg, E->x, disp, pad, keep, S->B, S->cnt);
     E->launches++;
     for (int attempt = 0; attempt < 8; attempt++) {
-        CUDA_TRY(cudaMemsetAsync(S->cnt, 0, sizeof(int) * 8, s));
+        if (attempt > 0) CUDA_TRY(cudaMemsetAsync(S->cnt, 0, sizeof(int) * 8, s));
         k_body_pairs<<<grid_for(32L * E->nb), 256, 0, s>>>(E->nb, E->bscene, E->sc_body_begin, S->B.blo, S->B.bhi,
                                                             P.self_contact, S->bpairs, S->bp_cap, S->cnt, S->B.paired);
         k_bp_clboxes<<<body_grid, BOX_THREADS, 0, s>>>(E->nb, E->bd_vbeg, E->bd_ebeg, E->bd_tbeg, E->edges, E->tris, do_ee,
@@ -556,8 +560,8 @@ static int bp_build(Engine* E, const BpDisp& disp, double lim, double filt, int 
             E->launches += 2;
         };
         expand(0, INT_MAX);
-        E->launches += 2;
-        CUDA_TRY(cudaMemcpyAsync(E->hcnt->bp, S->cnt, sizeof(int) * 8, cudaMemcpyDeviceToHost, s));
+        k_bp_send<<<1, 32, 0, s>>>(S->cnt, E->hcnt->bp);
+        E->launches += 3;
         CUDA_TRY(eng_stream_sync(E));
         const int npairs = E->hcnt->bp[0];
         long long items;
@@ -576,7 +580,8 @@ static int bp_build(Engine* E, const BpDisp& disp, double lim, double filt, int 
             for (int q0 = 0; q0 < npairs; q0 += step) {
                 CUDA_TRY(cudaMemsetAsync(nitems, 0, sizeof(long long), s));
                 expand(q0, std::min(npairs, q0 + step));
-                CUDA_TRY(cudaMemcpyAsync(E->hcnt->bp, S->cnt, sizeof(int) * 8, cudaMemcpyDeviceToHost, s));
+                k_bp_send<<<1, 32, 0, s>>>(S->cnt, E->hcnt->bp);
+                E->launches++;
                 CUDA_TRY(eng_stream_sync(E));
                 memcpy(&items, E->hcnt->bp + 4, sizeof items);
                 if (items > S->item_cap) return E->fail(ABD_ERR_CONTACT_OVERFLOW, "body-pair broad phase: one body pair's cluster pairs do not fit");
@@ -597,7 +602,6 @@ static int bp_build(Engine* E, const BpDisp& disp, double lim, double filt, int 
             k_bp_decode<<<grid_for(n), 256, 0, s>>>(n, S->keys_s, out, S->cnt + 2);
             E->launches += 2;
         }
-        if (nee_dev) CUDA_TRY(cudaMemcpyAsync(nee_dev, S->cnt + 2, sizeof(int), cudaMemcpyDeviceToDevice, s));
         n_out = n;
         S->swept = mode == 0;
         return ABD_OK;
@@ -613,9 +617,9 @@ static int grow_ct(Engine* E, int need) { return eng_grow_contacts(E, need); }
 int eng_swept_bp(Engine* E, const double* dq, double sign, const int* done, double lim) {
     int n = 0;
     const BpDisp disp = {dq, sign, E->xbar, E->mass, E->bscene, done, E->pv, E->pmag};
-    int rc = bp_build(E, disp, lim, lim, 0, E->sw, E->sw_cap, n, E->sw_nee, grow_sw);
+    int rc = bp_build(E, disp, lim, lim, 0, E->sw, E->sw_cap, n, grow_sw);
     if (rc) return rc;
-    E->n_sw = n; E->n_sw_ee = -1; E->sw_valid = true;   // EE count on the device only (E->sw_nee)
+    E->n_sw = n; E->sw_valid = true;
     return ABD_OK;
 }
 
@@ -630,7 +634,7 @@ int eng_detect_bp(Engine* E, double filt) {
     CUDA_TRY(cudaMemsetAsync(E->dcnt, 0, DETECT_COUNTER_BYTES, E->stream));
     double lim = filt * (1.0 + 1e-6) + 1e-7;
     int n = 0;
-    if ((rc = bp_build(E, BpDisp{}, lim, filt, 1, E->contacts, E->cap, n, nullptr, grow_ct))) return rc;
+    if ((rc = bp_build(E, BpDisp{}, lim, filt, 1, E->contacts, E->cap, n, grow_ct))) return rc;
     k_bp_counts<<<1, 32, 0, E->stream>>>(E->dcnt, bps(E)->cnt + 2, n);
     E->launches++;
     return eng_pg_candidates(E, filt);

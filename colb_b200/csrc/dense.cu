@@ -900,10 +900,9 @@ struct DenseState {
     void* rhs = nullptr; size_t rhs_bytes = 0;
     void* work = nullptr; size_t work_bytes = 0; int work_n = 0;
     int* ipiv = nullptr;
-    int* info = nullptr;                             // [0] small-component status, then 2 per large component
+    int* info = nullptr;                             // 2 per large component, from [2] on
     long long* comp_d = nullptr;                     // per large component: offset | rhs offset | n
-    int* imap_d = nullptr; int* imap_h = nullptr;    // bmap | blocal | sptr | sbody | band cptr | bw | order
-    long long* loff_d = nullptr; long long* loff_h = nullptr;   // band factor offsets (blocks)
+    int* imap_d = nullptr; int* imap_h = nullptr;    // bmap | blocal | sptr | sbody | band maps | band factor offsets (blocks) | status
     void* Lg = nullptr; size_t Lg_bytes = 0;         // band factors
     void* Ab = nullptr;                              // band blocks gathered in component order (Lg_bytes)
     std::vector<unsigned long long> keys;
@@ -920,10 +919,9 @@ void eng_dense_free(Engine* E) {
     DenseState* D = ds_of(E);
     if (!D) return;
     if (D->h) cusolverDnDestroy(D->h);
-    void* ps[] = {D->A, D->rhs, D->work, D->ipiv, D->info, D->comp_d, D->imap_d, D->loff_d, D->Lg, D->Ab};
+    void* ps[] = {D->A, D->rhs, D->work, D->ipiv, D->info, D->comp_d, D->imap_d, D->Lg, D->Ab};
     for (void* p : ps) if (p) cudaFree(p);
     if (D->imap_h) cudaFreeHost(D->imap_h);
-    if (D->loff_h) cudaFreeHost(D->loff_h);
     delete D;
     E->dense_state = nullptr;
 }
@@ -946,11 +944,9 @@ static int dense_init(Engine* E) {
     cusolverDnSetStream(D->h, E->stream);
     // component maps, small-component lists, band sub-components (a split
     // component's separator appears in both halves) and band jobs
-    size_t ni = 12 * (size_t)E->nb + 32;
+    size_t ni = 14 * (size_t)E->nb + 40;
     if (cudaMalloc(&D->imap_d, sizeof(int) * ni) != cudaSuccess) return E->fail(ABD_ERR_CUDA, "cudaMalloc maps");
     if (cudaMallocHost(&D->imap_h, sizeof(int) * ni) != cudaSuccess) return E->fail(ABD_ERR_CUDA, "cudaMallocHost maps");
-    if (cudaMalloc(&D->loff_d, sizeof(long long) * (E->nb + 1)) != cudaSuccess) return E->fail(ABD_ERR_CUDA, "cudaMalloc band offsets");
-    if (cudaMallocHost(&D->loff_h, sizeof(long long) * (E->nb + 1)) != cudaSuccess) return E->fail(ABD_ERR_CUDA, "cudaMallocHost band offsets");
     if (cudaMalloc(&D->info, sizeof(int) * (2 * MAX_LARGE_COMPONENTS + 2)) != cudaSuccess) return E->fail(ABD_ERR_CUDA, "cudaMalloc info");
     if (cudaMalloc(&D->comp_d, sizeof(long long) * 3 * MAX_LARGE_COMPONENTS) != cudaSuccess) return E->fail(ABD_ERR_CUDA, "cudaMalloc comps");
     return ABD_OK;
@@ -1208,7 +1204,6 @@ static int dense_solve_t(Engine* E, int* iters, int* fallback) {
     // component of each position | jobs, and the block offsets
     int* at = h_sbody + small_bodies;
     int* band_maps[2] = {nullptr, nullptr};
-    long long* loff_at = D->loff_h;
     for (int q = 0; q < 2; q++) {
         const BandSet& B = sets[q];
         band_maps[q] = at;
@@ -1216,13 +1211,18 @@ static int dense_solve_t(Engine* E, int* iters, int* fallback) {
         put(B.cptr); put(B.bw); put(B.order);
         for (size_t c = 0; c < B.bw.size(); c++) at = std::fill_n(at, B.cptr[c + 1] - B.cptr[c], (int)c);
         put(B.jobs);
-        loff_at = std::copy(B.loff.begin(), B.loff.end(), loff_at);
     }
+    // the offsets behind them (8-byte aligned), and the status of the band and small kernels
+    if ((at - h) & 1) *at++ = 0;
+    const size_t loff_first = at - h;
+    for (int q = 0; q < 2; q++)
+        for (long long v : sets[q].loff) { memcpy(at, &v, sizeof v); at += 2; }
+    *at = 0;
+    int* d_status = D->imap_d + (at++ - h);
     const size_t nints = at - h;
     CUDA_TRY(cudaMemcpyAsync(D->imap_d, h, sizeof(int) * nints, cudaMemcpyHostToDevice, st));
     const int* d_bmap = D->imap_d; const int* d_blocal = D->imap_d + nb;
     const int* d_sptr = D->imap_d + 2 * nb; const int* d_sbody = d_sptr + nsmall + 1;
-    CUDA_TRY(cudaMemsetAsync(D->info, 0, sizeof(int), st));      // status of the band and small kernels
     if (nsub > 0) {
         size_t doubles[2];
         for (int q = 0; q < 2; q++) doubles[q] = (size_t)sets[q].blocks * 144 + 12 * sets[q].order.size();
@@ -1237,7 +1237,6 @@ static int dense_solve_t(Engine* E, int* iters, int* fallback) {
                 return E->fail(ABD_ERR_CUDA, "cudaMalloc band factors");
             }
         }
-        CUDA_TRY(cudaMemcpyAsync(D->loff_d, D->loff_h, sizeof(long long) * nsub, cudaMemcpyHostToDevice, st));
         int ph = phase_begin(E, PH_BAND);
         double bytes = 0;
         for (int q = 0; q < 2; q++) {
@@ -1249,7 +1248,7 @@ static int dense_solve_t(Engine* E, int* iters, int* fallback) {
             const int* d_ord = d_bw + n;
             const int* d_pcomp = d_ord + npos;
             const int* d_jobs = d_pcomp + npos;
-            const long long* d_loff = D->loff_d + (q ? sets[0].bw.size() : 0);
+            const long long* d_loff = reinterpret_cast<const long long*>(D->imap_d + loff_first) + (q ? sets[0].bw.size() : 0);
             double* Ab = (double*)D->Ab + (q ? doubles[0] : 0);
             double* Lg = (double*)D->Lg + (q ? doubles[0] : 0);
             auto kernel = q ? k_band_solve<BAND_WIDE + 1, sizeof(T) == 4> : k_band_solve<BAND_W, sizeof(T) == 4>;
@@ -1262,7 +1261,7 @@ static int dense_solve_t(Engine* E, int* iters, int* fallback) {
                                                                              E->row_ptr, E->bcol, (const T*)E->vals, Ab);
             // one cluster of two CTAs per job
             kernel<<<2 * njobs, BAND_THREADS, smem, st>>>(njobs, d_jobs, d_cptr, d_ord, d_bw, d_loff, Ab, B.blocks, E->g, Lg,
-                                                          E->du, D->info);
+                                                          E->du, d_status);
             E->launches += 2;
             // per component: band blocks read, factor written and read back,
             // g read, y and du written and read
@@ -1280,7 +1279,7 @@ static int dense_solve_t(Engine* E, int* iters, int* fallback) {
             D->smem_set[sizeof(T) == 8] = true;
         }
         k_small_solve<T><<<nsmall, SMALL_THREADS, smem, st>>>(nsmall, d_sptr, d_sbody, d_blocal, E->row_ptr, E->bcol,
-                                                              (const T*)E->vals, E->g, projected ? 1 : 0, E->du, D->info);
+                                                              (const T*)E->vals, E->g, projected ? 1 : 0, E->du, d_status);
         E->launches++;
     }
     T* x = nullptr;

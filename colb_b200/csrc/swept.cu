@@ -257,8 +257,6 @@ int eng_swept(Engine* E, const double* dq, double sign, const int* done) {
         if ((rc = eng_grow_swept(E, E->hcnt->n_sw))) return rc;
     }
     E->n_sw = E->hcnt->n_sw;
-    E->n_sw_ee = E->hcnt->n_sw_ee;
-    CUDA_TRY(cudaMemcpyAsync(E->sw_nee, &E->dcnt->n_sw_ee, sizeof(int), cudaMemcpyDeviceToDevice, s));
     E->sw_valid = true;
     return ABD_OK;
 }

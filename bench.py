@@ -483,8 +483,8 @@ def main():
     # reported separately as phases_ms_per_step.dense; the swept-candidate
     # phase brackets several kernels, a sort and a host read-back, so it
     # appears only in phases_ms_per_step)
-    kernel_names = {"asm_contact": "k_contact_assemble", "energy_list": "k_list_energy",
-                    "spmv": "k_pcg_spmv / k_bi_spmv", "energy_query": "k_ee/pt_energy", "band": "k_band_solve"}
+    kernel_names = {"asm_contact": "k_contact_assemble", "energy_list": "k_ls_energy",
+                    "spmv": "k_bi_scene / k_pcg_spmv / k_bi_spmv", "energy_query": "k_ee/pt_energy", "band": "k_band_solve"}
     dom = max(kernel_names, key=lambda k: ph[k]["ms"])
     avg_ms = ph[dom]["ms"] / max(1, ph[dom]["launches"])
     avg_bytes = ph[dom]["bytes"] / max(1, ph[dom]["launches"])

@@ -491,8 +491,10 @@ static int solve_t(Engine* E, int* iters) {
         at[0].id = cudaLaunchAttributeClusterDimension;
         at[0].val.clusterDim.x = C; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
         cfg.attrs = at; cfg.numAttrs = 1;
+        int ph = phase_begin(E, PH_SPMV);
         CUDA_TRY(cudaLaunchKernelEx(&cfg, k_bi_scene<T>, A, most, blocks, (const int*)E->sc_body_begin, (const double*)E->g, E->du,
                                     kiter, &E->dcnt->krylov_active));
+        phase_end(E, ph, (double)sizeof(T) * (144.0 * E->nnzb_host + 24.0 * nb));     // blocks and right-hand side in, du out
         E->launches++;
         CUDA_TRY(cudaMemcpyAsync(E->hsci, kiter, sizeof(int) * ns, cudaMemcpyDeviceToHost, st));
         int rc = eng_sync_counters(E);

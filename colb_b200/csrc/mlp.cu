@@ -19,6 +19,7 @@
 // BF16-rounded weights and activations like inference, MSE loss, backward
 // with straight-through rounding.
 #include "engine.cuh"
+#include <mutex>
 #include <cuda_bf16.h>
 
 namespace {
@@ -671,6 +672,7 @@ struct MlpDev {
     float* feat = nullptr;
     int* err = nullptr;
     float* io = nullptr; int iocap = 0;      // rows in and out of abd_mlp_forward
+    std::mutex io_mu;                        // one call at a time uses them
 };
 // rows that abd_mlp_forward takes at once, and so the most it keeps room for
 // (15 MB); more rows than that hide the copies' fixed costs anyway
@@ -784,6 +786,7 @@ extern "C" int abd_mlp_forward(AbdHandle* h, const float* x, int32_t n, float* y
     if (n == 0) return ABD_OK;
     if (cudaSetDevice(E->device) != cudaSuccess) return E->fail(ABD_ERR_CUDA, "cudaSetDevice");
     MlpDev* M = reinterpret_cast<MlpDev*>(E->mlp);
+    std::lock_guard<std::mutex> lock(M->io_mu);
     // two buffers kept for the next call: allocating and freeing them on each
     // call took 1,280 of 2,290 us for 50,021 rows
     const int rows = n < MLP_SLAB ? n : MLP_SLAB;

@@ -1,6 +1,6 @@
 // assemble.cu — gradient and block Hessian of the incremental potential.
 //
-//  inertia + orthogonality  abd.py:108-166, ortho.py:9-41 (one thread per body)
+//  inertia + orthogonality  abd.py:108-166, ortho.py:9-41 (one warp per body, one thread its SVD)
 //  barrier contacts ....... abd.py:198-571: classify each candidate into a
 //                           PP / PE / EE (or PT / PG) stencil, differentiate its
 //                           squared distance, chain through the barrier and map
@@ -10,8 +10,9 @@
 // The reference writes 64 triplets per contact into a COO array (with the
 // contact/inertia slot overlap at abd.py:111 vs :311) and converts the whole
 // array to BSR every iteration (abd.py:634).  Here the body-pair pattern is
-// built once per Newton iteration from the sorted contact list (radix sort +
-// unique of 64-bit body-pair keys into CSR of 12x12 blocks), and each active
+// built once per Newton iteration from bits that the contacts set (k_bit_rows:
+// CSR of 12x12 blocks; a radix sort of 64-bit body-pair keys where the bits
+// would take too many words), and each active
 // contact adds its four body blocks into that structure with FP64/FP32
 // atomics.
 #include "contact.cuh"

@@ -5,7 +5,7 @@
 // The system decouples into the connected components of the body graph whose
 // edges are the off-diagonal 12x12 blocks (two dynamic bodies joined by an
 // active contact).  A component is factored on its own:
-//   - one body: the 12x12 block inverse written by the assembly;
+//   - one body: the inverse of its 12x12 block (k_du_scatter);
 //   - Hessian projected to PSD and, in reverse Cuthill-McKee order, a body
 //     bandwidth of at most BAND_WIDE: a banded L D L^T with the active window in
 //     registers, all such components of bandwidth up to BAND_MAX in one launch

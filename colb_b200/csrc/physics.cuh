@@ -64,18 +64,6 @@ DV double ortho_noise(const double* q, double k) {
 DV double contact_noise(double sc, double b0, double b1, double x, double L, double mult) {
     return sc * (fabs(b0) + fabs(b1) * 8.0 * sqrt(fabs(x)) * L * mult);
 }
-DV void ortho_grad(const double* q, double k, double* g) {
-#pragma unroll
-    for (int i = 0; i < 3; i++) {
-        double gi0 = -q[3*i], gi1 = -q[3*i+1], gi2 = -q[3*i+2];
-#pragma unroll
-        for (int j = 0; j < 3; j++) {
-            double d = q[3*i] * q[3*j] + q[3*i+1] * q[3*j+1] + q[3*i+2] * q[3*j+2];
-            gi0 += d * q[3*j]; gi1 += d * q[3*j+1]; gi2 += d * q[3*j+2];
-        }
-        g[3*i] = gi0 * 4.0 * k; g[3*i+1] = gi1 * 4.0 * k; g[3*i+2] = gi2 * 4.0 * k;
-    }
-}
 // 3x3 block (i,j) of the ortho Hessian, entry (r,c)
 DV double ortho_hess(const double* q, double k, int i, int j, int r, int c) {
     double v;
@@ -307,136 +295,6 @@ DV double pt_dist2(const double* p, const double* a, const double* b, const doub
         default: return d2_pt_plane_val(P, A, B, Cc);
     }
 }
-
-// With derivatives.  Outputs: g (3*np), H ((3np)^2 row-major, ld = 3np).
-// Map from auxiliary vectors y to stencil points: C[point][aux] in {-1,0,1}.
-template <int NP, int NA>
-DV void map_aux(const signed char (&C)[NP][NA], const double* gy, const double* Hy, double* g, double* H) {
-    constexpr int NY = 3 * NA, NX = 3 * NP;
-#pragma unroll
-    for (int i = 0; i < NP; i++)
-#pragma unroll
-        for (int k = 0; k < 3; k++) {
-            double s = 0;
-#pragma unroll
-            for (int a = 0; a < NA; a++) s += C[i][a] * gy[3*a+k];
-            g[3*i+k] = s;
-        }
-#pragma unroll 1
-    for (int i = 0; i < NP; i++)
-#pragma unroll 1
-        for (int j = 0; j < NP; j++)
-#pragma unroll
-            for (int r = 0; r < 3; r++)
-#pragma unroll
-                for (int c = 0; c < 3; c++) {
-                    double s = 0;
-#pragma unroll
-                    for (int a = 0; a < NA; a++)
-#pragma unroll
-                        for (int b = 0; b < NA; b++)
-                            if (C[i][a] && C[j][b]) s += C[i][a] * C[j][b] * Hy[(3*a+r)*NY + 3*b+c];
-                    H[(3*i+r)*NX + 3*j+c] = s;
-                }
-}
-
-DV double d2_pp_full(d3 a, d3 b, double* g, double* H) {
-    d3 d = a - b;
-    g[0] = 2*d.x; g[1] = 2*d.y; g[2] = 2*d.z; g[3] = -2*d.x; g[4] = -2*d.y; g[5] = -2*d.z;
-#pragma unroll
-    for (int i = 0; i < 36; i++) H[i] = 0.0;
-#pragma unroll
-    for (int k = 0; k < 3; k++) { H[k*6+k] = 2; H[(3+k)*6+3+k] = 2; H[k*6+3+k] = -2; H[(3+k)*6+k] = -2; }
-    return dot(d, d);
-}
-
-DV double d2_pe_full(d3 p, d3 e0, d3 e1, double* g, double* H) {
-    d3 w = p - e0, e = e1 - e0;
-    double c = dot(w, e), s = dot(e, e), is = 1.0 / s;
-    double f = dot(w, w) - c * c * is;
-    double gy[6], Hy[36];
-    double W[3] = {w.x, w.y, w.z}, E[3] = {e.x, e.y, e.z};
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-        gy[k] = 2*W[k] - 2*c*is*E[k];
-        gy[3+k] = -2*c*is*W[k] + 2*c*c*is*is*E[k];
-    }
-#pragma unroll
-    for (int r = 0; r < 3; r++)
-#pragma unroll
-        for (int q = 0; q < 3; q++) {
-            double I = (r == q) ? 1.0 : 0.0;
-            Hy[r*6+q] = 2*I - 2*is*E[r]*E[q];
-            double we = -2*is*E[r]*W[q] - 2*c*is*I + 4*c*is*is*E[r]*E[q];
-            Hy[r*6+3+q] = we;
-            Hy[(3+q)*6+r] = we;
-            Hy[(3+r)*6+3+q] = -2*is*W[r]*W[q] + 4*c*is*is*(W[r]*E[q] + E[r]*W[q])
-                              - 8*c*c*is*is*is*E[r]*E[q] + 2*c*c*is*is*I;
-        }
-    const signed char C[3][2] = {{1, 0}, {-1, -1}, {0, 1}};
-    map_aux<3, 2>(C, gy, Hy, g, H);
-    return f;
-}
-
-DV void skew(d3 a, double* S) {
-    S[0] = 0;    S[1] = -a.z; S[2] = a.y;
-    S[3] = a.z;  S[4] = 0;    S[5] = -a.x;
-    S[6] = -a.y; S[7] = a.x;  S[8] = 0;
-}
-// f = (w.n)^2/(n.n), n = u x v; derivatives w.r.t. (w, u, v)
-DV double d2_wn_full(d3 w, d3 u, d3 v, double* gy, double* Hy) {
-    d3 n = cross(u, v);
-    double a = dot(w, n), b = dot(n, n), ib = 1.0 / b;
-    double f = a * a * ib;
-    d3 vw = cross(v, w), wu = cross(w, u), vn = cross(v, n), nu = cross(n, u);
-    double ga[9] = {n.x, n.y, n.z, vw.x, vw.y, vw.z, wu.x, wu.y, wu.z};
-    double gb[9] = {0, 0, 0, 2*vn.x, 2*vn.y, 2*vn.z, 2*nu.x, 2*nu.y, 2*nu.z};
-    double Su[9], Sv[9], Sw[9], Sn[9];
-    skew(u, Su); skew(v, Sv); skew(w, Sw); skew(n, Sn);
-    // Ha and Hb only have off-diagonal (w,u), (w,v), (u,v) and (u,u), (u,v), (v,v) blocks
-#pragma unroll
-    for (int i = 0; i < 9; i++) gy[i] = 2*a*ib*ga[i] - a*a*ib*ib*gb[i];
-    double c1 = 2*ib, c2 = 2*a*ib, c3 = 2*a*ib*ib, c4 = 2*a*a*ib*ib*ib, c5 = a*a*ib*ib;
-#pragma unroll 1
-    for (int i = 0; i < 9; i++)
-#pragma unroll
-        for (int j = 0; j < 9; j++) {
-            int bi = i / 3, bj = j / 3, r = i % 3, c = j % 3;
-            double ha = 0, hb = 0;
-            if (bi == 0 && bj == 1) ha = -Sv[3*r+c];
-            else if (bi == 1 && bj == 0) ha = -Sv[3*c+r];
-            else if (bi == 0 && bj == 2) ha = Su[3*r+c];
-            else if (bi == 2 && bj == 0) ha = Su[3*c+r];
-            else if (bi == 1 && bj == 2) ha = -Sw[3*r+c];
-            else if (bi == 2 && bj == 1) ha = -Sw[3*c+r];
-            if (bi == 1 && bj == 1) {          // 2 [v]x^T [v]x
-                double s = 0; for (int m = 0; m < 3; m++) s += Sv[3*m+r] * Sv[3*m+c]; hb = 2*s;
-            } else if (bi == 1 && bj == 2) {   // 2 [v]x [u]x - 2 [n]x
-                double s = 0; for (int m = 0; m < 3; m++) s += Sv[3*r+m] * Su[3*m+c]; hb = 2*s - 2*Sn[3*r+c];
-            } else if (bi == 2 && bj == 1) {   // 2 [u]x [v]x + 2 [n]x
-                double s = 0; for (int m = 0; m < 3; m++) s += Su[3*r+m] * Sv[3*m+c]; hb = 2*s + 2*Sn[3*r+c];
-            } else if (bi == 2 && bj == 2) {   // 2 [u]x^T [u]x
-                double s = 0; for (int m = 0; m < 3; m++) s += Su[3*m+r] * Su[3*m+c]; hb = 2*s;
-            }
-            Hy[i*9+j] = c1*ga[i]*ga[j] + c2*ha - c3*(ga[i]*gb[j] + gb[i]*ga[j]) + c4*gb[i]*gb[j] - c5*hb;
-        }
-    return f;
-}
-DV double d2_ee_line_full(d3 a0, d3 a1, d3 b0, d3 b1, double* g, double* H) {
-    double gy[9], Hy[81];
-    double f = d2_wn_full(a0 - b0, a1 - a0, b1 - b0, gy, Hy);
-    const signed char C[4][3] = {{1, -1, 0}, {0, 1, 0}, {-1, 0, -1}, {0, 0, 1}};
-    map_aux<4, 3>(C, gy, Hy, g, H);
-    return f;
-}
-DV double d2_pt_plane_full(d3 p, d3 t0, d3 t1, d3 t2, double* g, double* H) {
-    double gy[9], Hy[81];
-    double f = d2_wn_full(p - t0, t1 - t0, t2 - t0, gy, Hy);
-    const signed char C[4][3] = {{1, 0, 0}, {-1, -1, -1}, {0, 1, 0}, {0, 0, 1}};
-    map_aux<4, 3>(C, gy, Hy, g, H);
-    return f;
-}
-
 
 // ------------------------------------------------------------ additive CCD
 // kind 0: edge-edge (x0 x1 | x2 x3), kind 1: point-triangle (x0 | x1 x2 x3).

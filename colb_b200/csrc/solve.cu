@@ -6,7 +6,8 @@
 // reduced per scene, and each kernel recomputes the scene's scalars from
 // those sums, so an iteration needs no host round trip.  Converged scenes
 // stop updating.  The host checks the number of active scenes every
-// CHECK_EVERY iterations.
+// CHECK_EVERY iterations.  BiCGSTAB of scenes of up to KS_MAX bodies runs in
+// one launch (k_bi_scene).
 //
 // Thread mapping: 16 lanes per body row (lanes 0..11 own one DoF each), so
 // a body's 12 entries live in one half-warp and the 12x12 preconditioner

@@ -359,3 +359,28 @@ def test_half_space_candidates_at_tile_edges(nu, nv, bodies, broadphase):
     got = quads[kinds == 2][:, :2]
     assert len(want) > 0 and np.array_equal(got, want)
     assert np.all(np.diff(kinds) >= 0)
+
+
+@pytest.mark.parametrize("extra", [30, 400, 1500])
+@pytest.mark.parametrize("n", [3, 8])
+def test_block_pattern_by_handle_size(n, extra):
+    """The block pattern from row bits (one block, and a cluster of eight with
+    400 more bodies) and from sorted keys (1,500 more bodies): a net in contact
+    gets the gradient and the increment that it gets alone, up to the rounding
+    of sums in another order, times the condition number of the Jacobi-scaled
+    system for the increment (15 for 9 links; 1.4e9 for 64, where one rounding of the
+    entries moves it by 2e-8)."""
+    net = S.config2_chain_net(n=n, seed=2, pitch=1.5 - 5e-4)
+    p = P.config_params()
+    e = Engine(p, net)
+    g0, H = e.assemble()
+    d0, _ = e.solve()
+    e = Engine(p, [S.config5_pile(n=extra, seed=1), net])
+    g1 = e.assemble(dense=False)[0][-12 * n * n:]
+    d1 = e.solve()[0]
+    assert np.all(np.isfinite(d1))
+    d1 = d1[-12 * n * n:]
+    assert np.abs(g0 - g1).max() <= 1e-12 * np.abs(g0).max()
+    s = 1.0 / np.sqrt(np.diag(H))
+    kappa = np.linalg.cond(H * s[:, None] * s)
+    assert np.linalg.norm((d0 - d1) / s) <= 50 * 2.2e-16 * kappa * np.linalg.norm(d0 / s)

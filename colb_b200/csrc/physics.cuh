@@ -95,9 +95,11 @@ DV void svd3(const double* A, double* U, double* s, double* V) {
             int p = pq == 2 ? 1 : 0, q = pq == 0 ? 1 : 2;
             double apq = S[3*p+q];
             if (apq == 0.0) continue;
-            // tan of the rotation from d / (2 apq) = cot of twice its angle, one division and two roots
-            const double d = S[3*q+q] - S[3*p+p], g = 2 * apq;
-            const double t = (d >= 0 ? g : -g) / (fabs(d) + sqrt(d * d + g * g));
+            // cot of twice the angle, then its tangent: a quotient, so that neither a tiny apq beside equal
+            // diagonal entries nor large entries are squared out of range (a form without this division
+            // squares both, and with |apq| below 1e-162 gives a NaN rotation)
+            const double theta = (S[3*q+q] - S[3*p+p]) / (2 * apq);
+            const double t = (theta >= 0 ? 1.0 : -1.0) / (fabs(theta) + sqrt(theta * theta + 1));
             const double c = rsqrt(t * t + 1), sn = t * c;
             for (int k = 0; k < 3; k++) {          // S <- S R
                 double skp = S[3*k+p], skq = S[3*k+q];

@@ -78,14 +78,25 @@ __global__ void k_contact_prepare(const Counters* cnt, const int4* __restrict__ 
 // cubes: 7 us now; 10 for the 256 bodies of a net, 18 for 512 scenes of 10,801
 // bodies (one block for those: 69).
 constexpr int BR_CL = 8, BR_SPLIT = 4096;
+DV uint32_t br_cluster_blocks() { uint32_t n; asm("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(n)); return n; }
+DV uint32_t br_cluster_rank() { uint32_t r; asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
+DV void br_cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+DV void br_cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
+// v to `p` of this block's shared memory in block `rank` of the cluster
+DV void br_store(int* p, int rank, int v) {
+    uint32_t a;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank));
+    asm volatile("st.shared::cluster.u32 [%0], %1;" :: "r"(a), "r"(v) : "memory");
+}
 struct BitHost { int* row; int* col; int* done; Counters* cnt; };      // null: not wanted
 __global__ void __launch_bounds__(1024) k_bit_rows(int nb, int bound, BitRows B, int lanes, int* row_ptr, int* bcol,
                                                    Counters* cnt, int ns, const int* done, BitHost H) {
     __shared__ int s_sum[32], s_of[BR_CL];
     __shared__ int s_total;
-    uint32_t C, c;
-    asm("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(C));
-    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(c));
+    const uint32_t C = br_cluster_blocks(), c = br_cluster_rank();
+    // the other blocks' shared memory may be written once they all run: they
+    // meet here, and the wait comes after the rows are counted
+    if (C > 1) br_cluster_arrive();
     const int share = (nb + (int)C - 1) / (int)C, b0 = min((int)c * share, nb), b1 = min(b0 + share, nb);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, sub = tid & (lanes - 1);
     const unsigned group = lanes == 32 ? 0xffffffffu : ((1u << lanes) - 1) << (lane & ~(lanes - 1));
@@ -119,13 +130,10 @@ __global__ void __launch_bounds__(1024) k_bit_rows(int nb, int bound, BitRows B,
     __syncthreads();
     int before = 0, all = s_total;           // blocks of the rows of the cluster's earlier blocks, of all rows
     if (C > 1) {
-        if (tid < (int)C) {
-            uint32_t a;
-            asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((uint32_t)__cvta_generic_to_shared(&s_of[c])), "r"(tid));
-            asm volatile("st.shared::cluster.u32 [%0], %1;" :: "r"(a), "r"(s_total) : "memory");
-        }
-        asm volatile("barrier.cluster.arrive.release;" ::: "memory");
-        asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+        br_cluster_wait();
+        if (tid < (int)C) br_store(&s_of[c], tid, s_total);
+        br_cluster_arrive();
+        br_cluster_wait();
         all = 0;
         for (int k = 0; k < (int)C; k++) { if (k < (int)c) before += s_of[k]; all += s_of[k]; }
     }

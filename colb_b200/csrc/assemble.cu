@@ -401,6 +401,7 @@ __global__ void __launch_bounds__(32 * CAW) k_contact_assemble(const Counters* c
             }
             __syncwarp();
         }
+        __syncwarp();                 // the last types are read before the next contacts' are written
     }
 }
 

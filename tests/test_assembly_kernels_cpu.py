@@ -36,3 +36,21 @@ def test_block_rows_by_a_block_and_by_a_cluster(tmp_path):
     text = text.replace("__shared__ int s_total;", "int& s_total = s_of[BR_CL];")
     assert "__shared__" not in text
     _run(tmp_path, "bit_rows_test.cpp", "bit_rows.inc", text)
+
+
+@pytest.mark.skipif(shutil.which("g++") is None, reason="needs g++")
+def test_contact_assembly_over_several_groups_of_a_warp(tmp_path):
+    common, phys, eng = _source("common.cuh"), _source("physics.cuh"), _source("engine.cuh")
+    text = common[common.index("struct d3 {"):common.index("HD double comp(")]
+    text += "inline d3 ld3(const double* p) { return mk3(p[0], p[1], p[2]); }\n"
+    text += phys[phys.index("DV void barrier3("):phys.index("// ---------------------------------------------------------- orthogonality")]
+    text += eng[eng.index("DV int find_block("):eng.index("#define GS_LOOP")]
+    text += _source("contact_hess.cuh").replace("#pragma once", "").replace('#include "common.cuh"', "")
+    src = _source("assemble.cu")
+    text += src[src.index("DV int stencil_np("):src.index("DV int other_vertex(")]
+    text += src[src.index("constexpr int CA_PER = 8;"):src.index("// ---------------------------------------------------- block-Jacobi inverse")]
+    for plain in ("double m[CA_PER][15], frame[CA_PER][9], w[CA_PER][12], gd[CA_PER], J[4][4];", "int v[CA_PER][4], type[CA_PER];"):
+        kind, names = plain.split(" ", 1)
+        assert plain in text
+        text = text.replace(plain, f"Checked<{kind}> {names}")
+    _run(tmp_path, "contact_assemble_test.cpp", "contact_assemble.inc", text)

@@ -124,12 +124,14 @@ DV bool bp_pt_ok(const BpArgs& A, int pv, int t) {
     double L = (double)A.pmag[pv] + (double)fmaxf(A.pmag[a], fmaxf(A.pmag[b], A.pmag[c]));
     return d - L < A.lim;
 }
-// the hit counter stops growing once it passes the capacity (by at most the
-// threads in flight), so a pathological step (a displacement that makes every
+// the hit counter stops growing once it has passed the capacity (by at most
+// the threads in flight), so a pathological step (a displacement that makes every
 // primitive pair reachable) cannot wrap it; the host then grows the buffer a
-// bounded number of times and reports ABD_ERR_CONTACT_OVERFLOW
+// bounded number of times and reports ABD_ERR_CONTACT_OVERFLOW.  A counter that
+// only equals the capacity still counts: the first hit without a place must
+// show, or the host would take a list that lacks it for complete.
 DV void bp_emit(const BpArgs& A, int kind, int a, int b) {
-    if (*(volatile int*)A.count >= A.cap) return;
+    if (*(volatile int*)A.count > A.cap) return;
     int at = atomicAdd(A.count, 1);
     if ((unsigned)at < (unsigned)A.cap) A.out[at] = ((unsigned long long)kind << 62) | ((unsigned long long)a << 31) | (unsigned long long)b;
 }

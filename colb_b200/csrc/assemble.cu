@@ -517,11 +517,11 @@ static int asm_keys(Engine* E, bool ahead, long long& bound) {
     const bool direct = ls == ABD_SOLVER_AUTO || ls == ABD_SOLVER_DIRECT;
     if (direct) {
         // rows and columns, or keys of two words
-        const int words = E->row_bits ? nb + 1 + (int)bound : 2 * nkeys;
+        const long long words = E->row_bits ? nb + 1 + bound : 2LL * nkeys;
         if (words > E->h_pattern_cap) {
             if (E->h_pattern) { CUDA_TRY(eng_stream_sync(E)); cudaFreeHost(E->h_pattern); }
             E->h_pattern = nullptr; E->h_pattern_cap = 0;
-            const int cap = words + words / 2 + 2048;
+            const long long cap = words + words / 2 + 2048;
             if (cudaMallocHost(&E->h_pattern, sizeof(int) * cap) != cudaSuccess)
                 return E->fail(ABD_ERR_CUDA, "cudaMallocHost block pattern");
             E->h_pattern_cap = cap;

@@ -468,15 +468,16 @@ void eng_bp_free(Engine* E) {
 static int bp_reserve(Engine* E, int bp_need, long long item_need, int key_need) {
     BpScratch* S = bps(E);
     if (!S) {
-        S = new BpScratch(); E->bp_state = S;
+        S = new BpScratch();
         // one allocation for all boxes, flags and counters of the handle
         const size_t nb = E->nb, nv = E->nv;
         const size_t nc[3] = {nv / 32 + nb + 1, (size_t)E->ne / 32 + nb + 1, (size_t)E->nt / 32 + nb + 1};
         const size_t boxes = 2 * (nb + nv + nc[0] + nc[1] + nc[2]);
         if (cudaMalloc(&S->slab, sizeof(float4) * boxes + sizeof(int) * (8 + 3 * nb)) != cudaSuccess) {
-            S->slab = nullptr;
+            delete S;
             return E->fail(ABD_ERR_CUDA, "cudaMalloc body boxes");
         }
+        E->bp_state = S;
         float4* at = reinterpret_cast<float4*>(S->slab);
         auto take = [&](float4*& lo, float4*& hi, size_t n) { lo = at; hi = at + n; at += 2 * n; };
         take(S->B.blo, S->B.bhi, nb);
@@ -487,29 +488,36 @@ static int bp_reserve(Engine* E, int bp_need, long long item_need, int key_need)
     }
     // buffers in use by queued work are freed only after the stream drains
     if (bp_need > S->bp_cap || item_need > S->item_cap || key_need > S->key_cap) eng_stream_sync(E);
+    // half as much again; a list that does not fit is an overflow, which the
+    // swept list answers with a shorter step
+    auto more = [](long long need, long long extra, long long limit) { return std::min(need + need / 2 + extra, limit); };
     if (bp_need > S->bp_cap) {
-        if (S->bpairs) cudaFree(S->bpairs);
-        S->bpairs = nullptr;
-        S->bp_cap = bp_need + bp_need / 2 + 1024;
-        if (cudaMalloc(&S->bpairs, sizeof(int2) * S->bp_cap) != cudaSuccess) return E->fail(ABD_ERR_CUDA, "cudaMalloc body pairs");
+        const int cap = (int)more(bp_need, 1024, LIST_MAX);
+        if (bp_need > cap) return E->fail(ABD_ERR_CONTACT_OVERFLOW, "body pairs beyond the largest list");
+        Replacement R;
+        R.add(S->bpairs, cap);
+        if (!R.commit()) return E->fail(ABD_ERR_CONTACT_OVERFLOW, "body pairs do not fit in device memory");
+        S->bp_cap = cap;
     }
     if (item_need > S->item_cap) {
-        if (S->items) cudaFree(S->items);
-        S->items = nullptr;
-        S->item_cap = std::min(item_need + item_need / 2 + 4096, BP_ITEM_LIMIT);
-        if (cudaMalloc(&S->items, sizeof(int4) * (size_t)S->item_cap) != cudaSuccess) return E->fail(ABD_ERR_CUDA, "cudaMalloc cluster pairs");
+        const long long cap = more(item_need, 4096, BP_ITEM_LIMIT);
+        Replacement R;
+        R.add(S->items, cap);
+        if (!R.commit()) return E->fail(ABD_ERR_CONTACT_OVERFLOW, "cluster pairs do not fit in device memory");
+        S->item_cap = cap;
     }
     if (key_need > S->key_cap) {
-        if (S->keys) cudaFree(S->keys);
-        if (S->tmp) cudaFree(S->tmp);
-        S->keys = S->keys_s = nullptr; S->tmp = nullptr;
-        S->key_cap = key_need + key_need / 2 + 4096;
-        if (cudaMalloc(&S->keys, 2 * sizeof(unsigned long long) * S->key_cap) != cudaSuccess)
-            return E->fail(ABD_ERR_CUDA, "cudaMalloc pair keys");
-        S->keys_s = S->keys + S->key_cap;
-        S->tmp_bytes = 0;
-        cub::DeviceRadixSort::SortKeys(nullptr, S->tmp_bytes, S->keys, S->keys_s, S->key_cap);
-        if (cudaMalloc(&S->tmp, S->tmp_bytes) != cudaSuccess) return E->fail(ABD_ERR_CUDA, "cudaMalloc sort scratch");
+        const int cap = (int)more(key_need, 4096, LIST_MAX);
+        if (key_need > cap) return E->fail(ABD_ERR_CONTACT_OVERFLOW, "pairs beyond the largest list");
+        size_t tmp_bytes = 0;
+        cub::DeviceRadixSort::SortKeys(nullptr, tmp_bytes, S->keys, S->keys_s, cap);
+        Replacement R;
+        R.add(S->keys, 2 * (size_t)cap);
+        R.add_bytes(&S->tmp, tmp_bytes);
+        if (!R.commit()) return E->fail(ABD_ERR_CONTACT_OVERFLOW, "pair keys do not fit in device memory");
+        S->key_cap = cap;
+        S->keys_s = S->keys + cap;
+        S->tmp_bytes = tmp_bytes;
     }
     return ABD_OK;
 }

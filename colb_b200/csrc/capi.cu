@@ -45,9 +45,9 @@ static void grid_free(Grid& G) {
     G = Grid();
 }
 
-static size_t cub_need(Engine* E, int nkeys64) {
+static size_t cub_need(Engine* E, int sw_cap, int nkeys64) {
     size_t need = 0, b = 0;
-    cub::DeviceScan::ExclusiveSum(nullptr, b, (int*)nullptr, (int*)nullptr, E->sw_cap + 1);
+    cub::DeviceScan::ExclusiveSum(nullptr, b, (int*)nullptr, (int*)nullptr, sw_cap + 1);
     need = std::max(need, b);
     int nmax = std::max(std::max(E->ne, E->nt), 1);
     cub::DeviceRadixSort::SortPairs(nullptr, b, (uint32_t*)nullptr, (uint32_t*)nullptr, (int*)nullptr, (int*)nullptr, nmax);
@@ -62,50 +62,49 @@ static size_t cub_need(Engine* E, int nkeys64) {
 }
 
 int eng_grow_blocks(Engine* E, int need) {
-    int cap = std::max(need, 2 * E->blk_cap);
+    const int cap = std::max(need, (int)std::min(2LL * E->blk_cap, (long long)LIST_MAX));
     cudaStreamSynchronize(E->stream);
-    if (E->bcol) cudaFree(E->bcol);
-    if (E->vals) cudaFree(E->vals);
-    E->bcol = nullptr; E->vals = nullptr;
-    DALLOC(E->bcol, cap);
-    size_t es = E->mixed ? sizeof(float) : sizeof(double);
-    cudaError_t e = cudaMalloc(&E->vals, (size_t)cap * 144 * es);
-    if (e != cudaSuccess) return E->fail(ABD_ERR_CUDA, "cudaMalloc blocks");
+    Replacement R;
+    R.add(E->bcol, cap);
+    R.add_bytes(&E->vals, (size_t)cap * 144 * (E->mixed ? sizeof(float) : sizeof(double)));
+    if (!R.commit()) return E->fail(ABD_ERR_CUDA, "cudaMalloc blocks");
     E->blk_cap = cap;
     return ABD_OK;
 }
 
 int eng_grow_contacts(Engine* E, int need) {
-    int cap = std::max(need + need / 4 + 1024, 2 * E->cap);
+    // a key per body and two per contact are counted by an int
+    const int cap = grown_cap(need, E->cap, (LIST_MAX - E->nb) / 2), nkeys = E->nb + 2 * cap;
+    if (!cap) return E->fail(ABD_ERR_CONTACT_OVERFLOW, "contacts beyond the largest list");
     cudaStreamSynchronize(E->stream);
-    void* ps[] = {E->contacts, E->cst, E->ctype, E->cxb, E->cbody, E->keys, E->keys_s, E->ukeys, E->cub_tmp};
-    for (void* p : ps) if (p) cudaFree(p);
+    const size_t cub_bytes = cub_need(E, E->sw_cap, nkeys);
+    Replacement R;
+    R.add(E->contacts, cap); R.add(E->cst, cap); R.add(E->ctype, cap); R.add(E->cxb, cap); R.add(E->cbody, cap);
+    R.add(E->keys, nkeys); R.add(E->keys_s, nkeys); R.add(E->ukeys, nkeys);
+    R.add_bytes(&E->cub_tmp, cub_bytes);
+    if (!R.commit()) return E->fail(ABD_ERR_CONTACT_OVERFLOW, "contacts do not fit in device memory");
     E->cap = cap;
-    int nkeys = E->nb + 2 * cap;
-    DALLOC(E->contacts, cap); DALLOC(E->cst, cap); DALLOC(E->ctype, cap); DALLOC(E->cxb, cap); DALLOC(E->cbody, cap);
-    DALLOC(E->keys, nkeys); DALLOC(E->keys_s, nkeys); DALLOC(E->ukeys, nkeys);
-    E->cub_bytes = cub_need(E, nkeys);
-    cudaError_t e = cudaMalloc(&E->cub_tmp, E->cub_bytes);
-    if (e != cudaSuccess) return E->fail(ABD_ERR_CUDA, "cudaMalloc cub scratch");
+    E->cub_bytes = cub_bytes;
+    return ABD_OK;
+}
+
+int eng_grow_swept(Engine* E, int need) {
+    const int cap = grown_cap(need, E->sw_cap);
+    if (!cap) return E->fail(ABD_ERR_CONTACT_OVERFLOW, "swept pairs beyond the largest list");
+    cudaStreamSynchronize(E->stream);
+    const size_t cub_bytes = cub_need(E, cap, E->nb + 2 * E->cap);
+    Replacement R;
+    R.add(E->sw, cap); R.add(E->sw_flag, (size_t)cap + 1); R.add(E->sw_off, (size_t)cap + 1);
+    R.add_bytes(&E->cub_tmp, cub_bytes);
+    if (!R.commit()) return E->fail(ABD_ERR_CONTACT_OVERFLOW, "swept pairs do not fit in device memory");
+    E->sw_cap = cap;
+    E->cub_bytes = cub_bytes;
+    E->sw_valid = false;
     return ABD_OK;
 }
 
 bool eng_use_bp(const Engine* E) {
     return E->bd_ok && (E->P.broadphase == 2 || E->P.broadphase == 0);
-}
-
-int eng_grow_swept(Engine* E, int need) {
-    int cap = std::max(need + need / 4 + 1024, 2 * E->sw_cap);
-    cudaStreamSynchronize(E->stream);
-    void* ps[] = {E->sw, E->sw_flag, E->sw_off, E->cub_tmp};
-    for (void* p : ps) if (p) cudaFree(p);
-    E->sw = nullptr; E->sw_flag = nullptr; E->sw_off = nullptr; E->cub_tmp = nullptr;
-    E->sw_cap = cap;
-    DALLOC(E->sw, cap); DALLOC(E->sw_flag, cap + 1); DALLOC(E->sw_off, cap + 1);
-    E->cub_bytes = cub_need(E, E->nb + 2 * E->cap);
-    if (cudaMalloc(&E->cub_tmp, E->cub_bytes) != cudaSuccess) return E->fail(ABD_ERR_CUDA, "cudaMalloc cub scratch");
-    E->sw_valid = false;
-    return ABD_OK;
 }
 
 int eng_alloc(Engine* E) {
@@ -117,7 +116,7 @@ int eng_alloc(Engine* E) {
     DALLOC(E->x, 3L * nv); DALLOC(E->xf, nv); DALLOC(E->pv, 3L * nv); DALLOC(E->ws, 12L * nb);
     E->cap = 0;
     E->sw_cap = std::max(E->P.contact_capacity, 1024);
-    if ((rc = eng_grow_contacts(E, std::max(E->P.contact_capacity, 1024) * 4 / 5))) return rc;
+    if (eng_grow_contacts(E, (int)(std::max(E->P.contact_capacity, 1024) * 4LL / 5))) return E->fail(ABD_ERR_CUDA, "cudaMalloc contacts");
     DALLOC(E->sw, E->sw_cap); DALLOC(E->sw_flag, E->sw_cap + 1); DALLOC(E->sw_off, E->sw_cap + 1);
     DALLOC(E->pmag, nv); DALLOC(E->zero_int, 1); DALLOC(E->zero_ns, ns);
     cudaMemsetAsync(E->zero_int, 0, sizeof(int), E->stream);

@@ -940,15 +940,16 @@ static int dense_init(Engine* E) {
     if (E->dense_state) return ABD_OK;
     DenseState* D = new DenseState();
     E->dense_state = D;
-    if (cusolverDnCreate(&D->h) != CUSOLVER_STATUS_SUCCESS) return E->fail(ABD_ERR_CUDA, "cusolverDnCreate");
+    auto fails = [&](const char* what) { eng_dense_free(E); return E->fail(ABD_ERR_CUDA, what); };
+    if (cusolverDnCreate(&D->h) != CUSOLVER_STATUS_SUCCESS) return fails("cusolverDnCreate");
     cusolverDnSetStream(D->h, E->stream);
     // component maps, small-component lists, band sub-components (a split
     // component's separator appears in both halves) and band jobs
     size_t ni = 14 * (size_t)E->nb + 40;
-    if (cudaMalloc(&D->imap_d, sizeof(int) * ni) != cudaSuccess) return E->fail(ABD_ERR_CUDA, "cudaMalloc maps");
-    if (cudaMallocHost(&D->imap_h, sizeof(int) * ni) != cudaSuccess) return E->fail(ABD_ERR_CUDA, "cudaMallocHost maps");
-    if (cudaMalloc(&D->info, sizeof(int) * (2 * MAX_LARGE_COMPONENTS + 2)) != cudaSuccess) return E->fail(ABD_ERR_CUDA, "cudaMalloc info");
-    if (cudaMalloc(&D->comp_d, sizeof(long long) * 3 * MAX_LARGE_COMPONENTS) != cudaSuccess) return E->fail(ABD_ERR_CUDA, "cudaMalloc comps");
+    if (cudaMalloc(&D->imap_d, sizeof(int) * ni) != cudaSuccess) return fails("cudaMalloc maps");
+    if (cudaMallocHost(&D->imap_h, sizeof(int) * ni) != cudaSuccess) return fails("cudaMallocHost maps");
+    if (cudaMalloc(&D->info, sizeof(int) * (2 * MAX_LARGE_COMPONENTS + 2)) != cudaSuccess) return fails("cudaMalloc info");
+    if (cudaMalloc(&D->comp_d, sizeof(long long) * 3 * MAX_LARGE_COMPONENTS) != cudaSuccess) return fails("cudaMalloc comps");
     return ABD_OK;
 }
 
@@ -981,8 +982,10 @@ static int dense_reserve(Engine* E, DenseState* D, size_t a_elems, size_t rhs_el
         }
         D->work_bytes = ((size_t)std::max(lw1, lw2) + 32) * es;
         D->work_n = nmax;
-        if (cudaMalloc(&D->work, D->work_bytes) != cudaSuccess || cudaMalloc(&D->ipiv, sizeof(int) * nmax) != cudaSuccess)
+        if (cudaMalloc(&D->work, D->work_bytes) != cudaSuccess || cudaMalloc(&D->ipiv, sizeof(int) * nmax) != cudaSuccess) {
+            D->work_n = 0;
             return E->fail(ABD_ERR_CUDA, "cudaMalloc cusolver work");
+        }
     }
     return ABD_OK;
 }

@@ -12,6 +12,8 @@
 //   contacts[cap]     i32x4 {kind, a, b, 0} sorted by (kind, a, b)
 #pragma once
 #include "common.cuh"
+#include <algorithm>
+#include <climits>
 #include <string>
 #include <vector>
 
@@ -167,7 +169,7 @@ struct Engine {
     bool sw_inject_done = false;   // ABD_INJECT_SWEPT_FULL fired in this step
     // block keys and done flags of the last assembly, copied to pinned host
     // memory in the assembly's own sync for the direct solver's analysis
-    int* h_pattern = nullptr; int h_pattern_cap = 0; int* h_done = nullptr; bool keys_host = false;
+    int* h_pattern = nullptr; long long h_pattern_cap = 0; int* h_done = nullptr; bool keys_host = false;
     int* sw_flag = nullptr; int* sw_off = nullptr;
     int4* vchunk = nullptr; int nvchunk = 0;       // runs of <= VCHUNK vertices of one body {body, first, count, first run}
     bool x_fresh = false;          // x and xf are the vertices of st's nxt state
@@ -283,6 +285,37 @@ inline int grid_for(long n, int block = 256) {
     if (g > NUM_SMS * 16) g = NUM_SMS * 16;
     return (int)g;
 }
+// Growing arrays.  Capacities are ints and counters may pass them by the
+// threads in flight, so no list holds more than LIST_MAX entries.
+constexpr int LIST_MAX = INT_MAX - (1 << 20);
+// capacity for `need` entries: a quarter more, at least twice `have`; 0: above the limit
+inline int grown_cap(long long need, long long have, long long limit = LIST_MAX) {
+    if (need > limit) return 0;
+    return (int)std::min(std::max(need + need / 4 + 1024, 2 * have), limit);
+}
+// Arrays that take the place of others.  All are allocated before any old one is
+// freed: when one does not fit, the old ones stay as they are, with their
+// capacities, and the handle can still be used and destroyed.
+struct Replacement {
+    struct Item { void** slot; void* fresh; };
+    std::vector<Item> items;
+    bool ok = true;
+    template <class T> void add(T*& p, size_t n) { add_bytes(reinterpret_cast<void**>(&p), sizeof(T) * (n ? n : 1)); }
+    void add_bytes(void** slot, size_t bytes) {
+        void* p = nullptr;
+        if (ok && cudaMalloc(&p, bytes) != cudaSuccess) { ok = false; p = nullptr; cudaGetLastError(); }
+        items.push_back({slot, p});
+    }
+    bool commit() {
+        for (auto& i : items) {
+            if (!ok) { if (i.fresh) cudaFree(i.fresh); continue; }
+            if (*i.slot) cudaFree(*i.slot);
+            *i.slot = i.fresh;
+        }
+        items.clear();
+        return ok;
+    }
+};
 // index of block (r, c) in the block CSR, -1 when absent
 DV int find_block(const int* row_ptr, const int* bcol, int r, int c) {
     int lo = row_ptr[r], hi = row_ptr[r+1] - 1;

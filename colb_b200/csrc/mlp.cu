@@ -760,8 +760,10 @@ extern "C" int abd_set_mlp(AbdHandle* h, const float* params, const float* norm)
             cudaMalloc(&M->norm, sizeof(float) * ABD_MLP_NNORM) != cudaSuccess ||
             cudaMalloc(&M->y, sizeof(float) * MO * (size_t)E->nb) != cudaSuccess ||
             cudaMalloc(&M->feat, sizeof(float) * MI * (size_t)E->nb) != cudaSuccess ||
-            cudaMalloc(&M->err, sizeof(int)) != cudaSuccess)
+            cudaMalloc(&M->err, sizeof(int)) != cudaSuccess) {
+            eng_mlp_free(E);
             return E->fail(ABD_ERR_CUDA, "cudaMalloc mlp");
+        }
     }
     MlpDev* M = reinterpret_cast<MlpDev*>(E->mlp);
     float* P = nullptr;

@@ -226,7 +226,7 @@ int abd_create(const AbdParams* params, const AbdSceneDesc* scenes, int32_t n_sc
     if (!(P.dt > 0) || !(P.dhat > 0) || !(P.cand_dist >= P.dhat) || P.newton_max_iter <= 0 || P.lin_max_iter <= 0 ||
         P.barrier < 0 || P.barrier > 2 || P.contact_capacity <= 0 || P.linear_solver < 0 || P.linear_solver > 3 || (P.ccd && !(P.ccd_scale > 0 && P.ccd_scale < 1)) ||
         P.ls_groups < 0 || P.ls_groups > 1 || P.ls_graph < 0 || P.ls_graph > 1 || P.ccd_max_iter < 0 ||
-        (P.test_inject & ~(ABD_INJECT_DU_NONFINITE | ABD_INJECT_SWEPT_FULL))) {
+        (P.test_inject & ~(ABD_INJECT_DU_NONFINITE | ABD_INJECT_SWEPT_FULL | ABD_INJECT_BAND_CHECK))) {
         g_err = "abd_create: invalid parameters (dt, dhat <= cand_dist, iteration caps, barrier, capacity, ccd_scale, ls_groups, ls_graph)";
         return ABD_ERR_INVALID_ARG;
     }
@@ -599,8 +599,12 @@ int abd_solve(AbdHandle* h, double* du, int32_t* iters) {
     int it = 0;
     E->solver_capped = 0;
     if ((rc = eng_solve(E, &it))) return rc;
-    CUDA_TRY(cudaMemcpyAsync(du, E->du, sizeof(double) * 12 * E->nb, cudaMemcpyDeviceToHost, E->stream));
-    CUDA_TRY(cudaStreamSynchronize(E->stream));
+    for (bool again = true;; again = false) {
+        CUDA_TRY(cudaMemcpyAsync(du, E->du, sizeof(double) * 12 * E->nb, cudaMemcpyDeviceToHost, E->stream));
+        CUDA_TRY(cudaStreamSynchronize(E->stream));
+        if (!again || !eng_solve_failed(E)) break;
+        if ((rc = eng_solve_again(E, &it))) return rc;
+    }
     if (iters) *iters = it;
     if (E->solver_capped) return E->fail(ABD_ERR_SOLVER_CAP, "abd_solve: Krylov iteration cap reached above tolerance");
     return ABD_OK;

@@ -17,7 +17,8 @@
 //     column-major matrix and factored with cuSOLVER (Cholesky, or LU when
 //     Cholesky reports a non-positive pivot).
 // Mixed precision factors its FP32 blocks in FP64 on the band path, in FP32 on
-// the others.
+// the others.  A band solution that could have met a small pivot is checked
+// (band_check); where it fails, its component takes one of the last two paths in FP64.
 #include "engine.cuh"
 #include "block_inverse.cuh"
 #include <cstring>
@@ -26,9 +27,9 @@
 
 // Scatter the blocks of every body that belongs to a large component into
 // that component's dense column-major matrix (16 lanes per body row).
-template <class T>
+template <class TV, class T>
 __global__ void k_blocks_to_dense(int nb, const int* __restrict__ row_ptr, const int* __restrict__ bcol,
-                                  const T* __restrict__ vals, const int* __restrict__ bcomp,
+                                  const TV* __restrict__ vals, const int* __restrict__ bcomp,
                                   const int* __restrict__ blocal, const long long* __restrict__ comp_off,
                                   const long long* __restrict__ comp_n, int only_c, T* dense) {
     for (long base = (long)blockIdx.x * blockDim.x; base < (long)nb * 16; base += (long)gridDim.x * blockDim.x) {
@@ -42,9 +43,9 @@ __global__ void k_blocks_to_dense(int nb, const int* __restrict__ row_ptr, const
         long row = 12L * blocal[b] + l;
         for (int k = row_ptr[b]; k < row_ptr[b + 1]; k++) {
             long colb = 12L * blocal[bcol[k]];
-            const T* V = vals + (long)k * 144 + l;
+            const TV* V = vals + (long)k * 144 + l;
 #pragma unroll
-            for (int j = 0; j < 12; j++) A[(colb + j) * n + row] = V[j * 12];
+            for (int j = 0; j < 12; j++) A[(colb + j) * n + row] = (T)V[j * 12];
         }
     }
 }
@@ -57,32 +58,77 @@ __global__ void k_rhs_gather(int nb, const double* __restrict__ g, const int* __
         if (c >= 0) x[comp_rhs[c] + 12L * blocal[b] + i % 12] = (T)g[i];
     }
 }
+// Neither the unpivoted factorization of a signed matrix nor one that replaced
+// a pivot is backward stable: a small pivot grows without bound.  Every row of
+// the band components that could meet one is therefore checked:
+//   |g - A du|  <=  BAND_BACKWARD (|A| |du| + |g|) + |A - A^T| |du|
+// A body with a row above that, or with a non-finite one, is marked in `bad`
+// (pinned host memory; bad[nb]: any), and the host solves its component again
+// with pivoting, in FP64 (eng_solve_again).  The bound is one FP32 rounding; a
+// stable FP64 factorization is several orders below it (pivoted LU of nets in contact
+// 1e-13 to 3e-10).  The last term is there because the factorization reads one
+// entry of each symmetric pair, and FP32 blocks are symmetric only up to the
+// order of their sums.  One warp per body (all lanes call it); its time is a few
+// dependent loads, so the lanes look the transposed blocks up side by side.
+constexpr double BAND_BACKWARD = 5.9604644775390625e-8;     // 2^-24
+template <class T>
+DV void band_check(int b, int nb, int lane, int* transposed, const int* __restrict__ row_ptr, const int* __restrict__ bcol,
+                   const T* __restrict__ vals, const double* __restrict__ g, const double* __restrict__ du, int* bad) {
+    const int l = lane % 12, h = lane / 12;                 // row, half of a block's columns
+    double r = 0, s = 0, asym = 0;
+    if (lane < 12) { r = g[12L * b + l]; s = fabs(r); }
+    for (int k0 = row_ptr[b], k1 = row_ptr[b + 1]; k0 < k1; k0 += 32) {
+        // (the pattern is symmetric: every transposed block is there)
+        if (k0 + lane < k1) transposed[lane] = find_block(row_ptr, bcol, bcol[k0 + lane], b);
+        __syncwarp();
+        for (int k = k0; h < 2 && k < min(k0 + 32, k1); k++) {
+            const T* V = vals + (long)k * 144 + 72 * h + l;
+            const T* Vt = vals + (long)transposed[k - k0] * 144 + 12 * l + 6 * h;
+            const double* x = du + 12L * bcol[k] + 6 * h;
+#pragma unroll
+            for (int j = 0; j < 6; j++) {
+                const double a = V[j * 12], p = a * x[j];
+                r -= p; s += fabs(p);
+                asym += fabs((a - (double)Vt[j]) * x[j]);
+            }
+        }
+        __syncwarp();
+    }
+    r += __shfl_sync(0xffffffffu, r, (lane + 12) & 31);
+    s += __shfl_sync(0xffffffffu, s, (lane + 12) & 31);
+    asym += __shfl_sync(0xffffffffu, asym, (lane + 12) & 31);
+    if (lane < 12 && !(fabs(r) <= BAND_BACKWARD * s + asym && s <= DBL_MAX)) { bad[b] = 1; bad[nb] = 1; }
+}
+
 // du of every body, one warp each: large components from their dense solution, single
 // bodies through the inverse of their 12x12 block; bodies of small
-// components (bcomp -2) and band components (-3) were written by
-// k_small_solve / k_band_solve.  (The inverses of all bodies, single or not, in
+// components (bcomp -2) and band components (-3, -4) were written by
+// k_small_solve / k_band_solve, and the former band components are checked
+// (bad not null).  (The inverses of all bodies, single or not, in
 // a launch of their own took 12 us for 256 bodies and 39 for 4,096.)
 constexpr int DU_WARPS = 4;
-template <class T>
+template <class TV, class T>
 __global__ void __launch_bounds__(32 * DU_WARPS) k_du_scatter(int nb, const double* __restrict__ g, const int* __restrict__ bcomp,
                              const int* __restrict__ blocal, const long long* __restrict__ comp_rhs,
                              const T* __restrict__ x, const int* __restrict__ row_ptr, const int* __restrict__ bcol,
-                             const T* __restrict__ vals, const int* __restrict__ bscene,
-                             const int* __restrict__ ndone, double* du) {
+                             const TV* __restrict__ vals, const int* __restrict__ bscene,
+                             const int* __restrict__ ndone, double* du, int* bad) {
     __shared__ double sM[DU_WARPS][12][25];
+    __shared__ int transposed[DU_WARPS][32];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     double (*M)[25] = sM[w];
     for (int b = blockIdx.x * DU_WARPS + w; b < nb; b += gridDim.x * DU_WARPS) {
         const int c = bcomp[b];
+        if (c == -3 && bad) { band_check<TV>(b, nb, lane, transposed[w], row_ptr, bcol, vals, g, du, bad); continue; }
         if (c <= -2 || ndone[bscene[b]]) continue;
         if (c >= 0) { if (lane < 12) du[12L * b + lane] = (double)x[comp_rhs[c] + 12L * blocal[b] + lane]; continue; }
         const int bi = find_block(row_ptr, bcol, b, b);
-        const bool ok = block_inverse_warp<T>(vals + (long)bi * 144, M, lane);
+        const bool ok = block_inverse_warp<TV>(vals + (long)bi * 144, M, lane);
         if (lane < 12) {
             double acc = 0;
 #pragma unroll
             for (int k = 0; k < 12; k++)
-                acc += (double)(T)(ok ? M[lane][12 + k] : (lane == k ? 1.0 : 0.0)) * g[12L * b + k];
+                acc += (double)(TV)(ok ? M[lane][12 + k] : (lane == k ? 1.0 : 0.0)) * g[12L * b + k];
             du[12L * b + lane] = acc;
         }
         __syncwarp();
@@ -94,9 +140,9 @@ constexpr int SMALL_THREADS = 256;
 
 // Load the blocks of the component's bodies (local order sb[0..nbod)) into
 // the row-major n x n matrix A (leading dimension ld) and g into x.
-template <class T>
+template <class TV, class T>
 __device__ void small_fill(int nbod, int n, int ld, const int* sb, const int* __restrict__ blocal,
-                           const int* __restrict__ row_ptr, const int* __restrict__ bcol, const T* __restrict__ vals,
+                           const int* __restrict__ row_ptr, const int* __restrict__ bcol, const TV* __restrict__ vals,
                            const double* __restrict__ g, T* A, T* x) {
     for (int e = threadIdx.x; e < n * ld; e += blockDim.x) A[e] = 0;
     __syncthreads();
@@ -105,10 +151,10 @@ __device__ void small_fill(int nbod, int n, int ld, const int* sb, const int* __
         int b = sb[i];
         for (int k = row_ptr[b]; k < row_ptr[b + 1]; k++) {
             int j = blocal[bcol[k]];
-            const T* V = vals + (long)k * 144;
+            const TV* V = vals + (long)k * 144;
             for (int e = lane; e < 144; e += 32) {
                 int cc = e / 12, r = e % 12;        // blocks are column-major
-                A[(12 * i + r) * ld + 12 * j + cc] = V[e];
+                A[(12 * i + r) * ld + 12 * j + cc] = (T)V[e];
             }
         }
         if (lane < 12) x[12 * i + lane] = (T)g[12L * b + lane];
@@ -118,10 +164,10 @@ __device__ void small_fill(int nbod, int n, int ld, const int* sb, const int* __
 
 // One CTA per small component: A du = g in shared memory.  status bit 0 is
 // set when a component is singular (its du is zero).
-template <class T>
+template <class TV, class T>
 __global__ void __launch_bounds__(SMALL_THREADS) k_small_solve(int nsmall, const int* __restrict__ sptr,
         const int* __restrict__ sbody, const int* __restrict__ blocal, const int* __restrict__ row_ptr,
-        const int* __restrict__ bcol, const T* __restrict__ vals, const double* __restrict__ g, int try_chol,
+        const int* __restrict__ bcol, const TV* __restrict__ vals, const double* __restrict__ g, int try_chol,
         double* du, int* status) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ int flag, piv;
@@ -131,7 +177,7 @@ __global__ void __launch_bounds__(SMALL_THREADS) k_small_solve(int nsmall, const
         const int nbod = sptr[c + 1] - sptr[c], n = 12 * nbod, ld = n + 1;
         T* A = (T*)smem_raw;
         T* x = A + n * ld;
-        small_fill<T>(nbod, n, ld, sb, blocal, row_ptr, bcol, vals, g, A, x);
+        small_fill<TV, T>(nbod, n, ld, sb, blocal, row_ptr, bcol, vals, g, A, x);
         if (tid == 0) flag = try_chol ? 0 : 1;
         __syncthreads();
         // blocked right-looking Cholesky, lower triangle, 12-wide body columns;
@@ -219,7 +265,7 @@ __global__ void __launch_bounds__(SMALL_THREADS) k_small_solve(int nsmall, const
             }
         } else {
             // LU with partial pivoting on a fresh copy
-            small_fill<T>(nbod, n, ld, sb, blocal, row_ptr, bcol, vals, g, A, x);
+            small_fill<TV, T>(nbod, n, ld, sb, blocal, row_ptr, bcol, vals, g, A, x);
             bool singular = false;
             for (int k = 0; k < n; k++) {
                 if (warp == 0) {
@@ -898,17 +944,18 @@ struct DenseState {
     cusolverDnHandle_t h = nullptr;
     void* A = nullptr; size_t A_bytes = 0;
     void* rhs = nullptr; size_t rhs_bytes = 0;
-    void* work = nullptr; size_t work_bytes = 0; int work_n = 0;
+    void* work = nullptr; size_t work_bytes = 0, work_es = 0; int work_n = 0;   // work_es: widest type it fits
     int* ipiv = nullptr;
     int* info = nullptr;                             // 2 per large component, from [2] on
     long long* comp_d = nullptr;                     // per large component: offset | rhs offset | n
     int* imap_d = nullptr; int* imap_h = nullptr;    // bmap | blocal | sptr | sbody | band maps | band factor offsets (blocks) | status
     void* Lg = nullptr; size_t Lg_bytes = 0;         // band factors
     void* Ab = nullptr;                              // band blocks gathered in component order (Lg_bytes)
+    int* bad = nullptr;                              // pinned: bodies whose rows failed band_check, [nb]: any
     std::vector<unsigned long long> keys;
     std::vector<int> done, rp, col, act, parent, size, root, fill;
     std::vector<int> pos, members, mptr;
-    bool smem_set[2] = {false, false};
+    bool smem_set[3] = {false, false, false};
     bool band_smem_set[2][2] = {};
 };
 static DenseState* ds_of(Engine* E) { return reinterpret_cast<DenseState*>(E->dense_state); }
@@ -922,6 +969,7 @@ void eng_dense_free(Engine* E) {
     void* ps[] = {D->A, D->rhs, D->work, D->ipiv, D->info, D->comp_d, D->imap_d, D->Lg, D->Ab};
     for (void* p : ps) if (p) cudaFree(p);
     if (D->imap_h) cudaFreeHost(D->imap_h);
+    if (D->bad) cudaFreeHost(D->bad);
     delete D;
     E->dense_state = nullptr;
 }
@@ -948,6 +996,8 @@ static int dense_init(Engine* E) {
     size_t ni = 14 * (size_t)E->nb + 40;
     if (cudaMalloc(&D->imap_d, sizeof(int) * ni) != cudaSuccess) return fails("cudaMalloc maps");
     if (cudaMallocHost(&D->imap_h, sizeof(int) * ni) != cudaSuccess) return fails("cudaMallocHost maps");
+    if (cudaMallocHost(&D->bad, sizeof(int) * (E->nb + 1)) != cudaSuccess) return fails("cudaMallocHost check flags");
+    memset(D->bad, 0, sizeof(int) * (E->nb + 1));
     if (cudaMalloc(&D->info, sizeof(int) * (2 * MAX_LARGE_COMPONENTS + 2)) != cudaSuccess) return fails("cudaMalloc info");
     if (cudaMalloc(&D->comp_d, sizeof(long long) * 3 * MAX_LARGE_COMPONENTS) != cudaSuccess) return fails("cudaMalloc comps");
     return ABD_OK;
@@ -966,21 +1016,26 @@ static int dense_reserve(Engine* E, DenseState* D, size_t a_elems, size_t rhs_el
         D->rhs_bytes = rhs_elems * es + 4096;
         if (cudaMalloc(&D->rhs, D->rhs_bytes) != cudaSuccess) { D->rhs = nullptr; D->rhs_bytes = 0; return E->fail(ABD_ERR_CUDA, "cudaMalloc dense rhs"); }
     }
-    if (nmax > D->work_n || D->work_bytes % es) {
+    if (nmax > D->work_n || es > D->work_es) {
         // room for components up to twice this size (at most the whole handle)
         nmax = std::min(std::max(2 * nmax, 384), std::max(12 * E->nb, nmax));
         if (D->work) cudaFree(D->work);
         if (D->ipiv) cudaFree(D->ipiv);
         D->work = nullptr; D->ipiv = nullptr;
+        D->work_es = std::max(es, D->work_es);
+        size_t bytes = 0;
         int lw1 = 0, lw2 = 0;
-        if constexpr (sizeof(T) == 4) {
+        if (E->mixed) {
             cusolverDnSpotrf_bufferSize(D->h, CUBLAS_FILL_MODE_LOWER, nmax, (float*)D->A, nmax, &lw1);
             cusolverDnSgetrf_bufferSize(D->h, nmax, nmax, (float*)D->A, nmax, &lw2);
-        } else {
+            bytes = ((size_t)std::max(lw1, lw2) + 32) * sizeof(float);
+        }
+        if (D->work_es == sizeof(double)) {
             cusolverDnDpotrf_bufferSize(D->h, CUBLAS_FILL_MODE_LOWER, nmax, (double*)D->A, nmax, &lw1);
             cusolverDnDgetrf_bufferSize(D->h, nmax, nmax, (double*)D->A, nmax, &lw2);
+            bytes = std::max(bytes, ((size_t)std::max(lw1, lw2) + 32) * sizeof(double));
         }
-        D->work_bytes = ((size_t)std::max(lw1, lw2) + 32) * es;
+        D->work_bytes = bytes;
         D->work_n = nmax;
         if (cudaMalloc(&D->work, D->work_bytes) != cudaSuccess || cudaMalloc(&D->ipiv, sizeof(int) * nmax) != cudaSuccess) {
             D->work_n = 0;
@@ -1015,14 +1070,19 @@ static cusolverStatus_t lu_solve(DenseState* D, int n, T* A, T* x, T* work, int*
 
 // Returns 1 in *fallback when there are more large components than
 // MAX_LARGE_COMPONENTS or their matrices would exceed 4 GiB (the caller then
-// runs the Krylov solver).
-template <class T>
-static int dense_solve_t(Engine* E, int* iters, int* fallback) {
+// runs the Krylov solver).  TV: the stored blocks, T: the arithmetic outside the
+// band path.  again: the second solve of a system, in which the components that
+// failed band_check take the pivoted paths.
+template <class TV, class T>
+static int dense_solve_t(Engine* E, int* iters, int* fallback, bool again) {
     *fallback = 0;
     int rc = eng_asm_wait(E);
     if (rc) return rc;
     if ((rc = dense_init(E))) return rc;
     DenseState* D = ds_of(E);
+    std::vector<int> failed;
+    if (again) failed.assign(D->bad, D->bad + E->nb);
+    if (D->bad[E->nb]) memset(D->bad, 0, sizeof(int) * (E->nb + 1));
     cudaStream_t st = E->stream;
     const int* ndone = E->sci + SI_DONE * E->ns;
     const int nb = E->nb;
@@ -1141,15 +1201,24 @@ static int dense_solve_t(Engine* E, int* iters, int* fallback) {
         nsub++;
         return (int)B.bw.size() - 1;
     };
+    std::vector<char> checked;                   // per band component
+    auto has_failed = [&](int r) {
+        const int* m = D->members.data() + D->mptr[r];
+        for (int i = 0; i < D->size[r]; i++) if (failed[m[i]]) return true;
+        return false;
+    };
     for (int b : act) {
         int r = find(b), sz = D->size[r];
         // the band path takes every component of body bandwidth <= BAND_WIDE
         // of a projected Hessian, large ones split between the two CTAs of a
-        // cluster, and cuSOLVER only wider ones
-        if (D->root[r] == -1 && projected) {
+        // cluster; cuSOLVER takes wider ones, and the pivoted paths those that
+        // failed the check of the band solution
+        if (D->root[r] == -1 && projected && !(again && has_failed(r))) {
             int bw = rcm(r, ord);
             if (bw >= 1 && bw <= BAND_WIDE && sz <= BAND_ORD_MAX) {
                 D->root[r] = -10 - ncomp_band++;          // marks a band component
+                // FP64 of a narrow band replaces a pivot that is not positive and is not checked
+                checked.push_back(sizeof(TV) == 4 || bw > BAND_MAX);
                 BandSet& B = sets[bw > BAND_MAX];
                 const int m = band_split_point(sz, bw);
                 if (m > 0) {
@@ -1164,7 +1233,7 @@ static int dense_solve_t(Engine* E, int* iters, int* fallback) {
                 }
             }
         }
-        if (D->root[r] <= -10) { h_bmap[b] = -3; continue; }
+        if (D->root[r] <= -10) { h_bmap[b] = checked[-10 - D->root[r]] ? -3 : -4; continue; }
         if (D->root[r] < 0) {
             if (sz <= SMALL_MAX_BODIES) {
                 D->root[r] = (int)small_root.size();
@@ -1254,14 +1323,15 @@ static int dense_solve_t(Engine* E, int* iters, int* fallback) {
             const long long* d_loff = reinterpret_cast<const long long*>(D->imap_d + loff_first) + (q ? sets[0].bw.size() : 0);
             double* Ab = (double*)D->Ab + (q ? doubles[0] : 0);
             double* Lg = (double*)D->Lg + (q ? doubles[0] : 0);
-            auto kernel = q ? k_band_solve<BAND_WIDE + 1, sizeof(T) == 4> : k_band_solve<BAND_W, sizeof(T) == 4>;
+            constexpr bool mixed = sizeof(TV) == 4;
+            auto kernel = q ? k_band_solve<BAND_WIDE + 1, mixed> : k_band_solve<BAND_W, mixed>;
             const size_t smem = (size_t)band_smem_doubles(B.stride) * sizeof(double);
-            if (!D->band_smem_set[q][sizeof(T) == 8]) {
+            if (!D->band_smem_set[q][mixed]) {
                 CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-                D->band_smem_set[q][sizeof(T) == 8] = true;
+                D->band_smem_set[q][mixed] = true;
             }
-            k_band_gather<T><<<grid_for(32L * npos * B.stride), 256, 0, st>>>(B.stride, npos, d_pcomp, d_cptr, d_ord, d_bw, d_loff,
-                                                                             E->row_ptr, E->bcol, (const T*)E->vals, Ab);
+            k_band_gather<TV><<<grid_for(32L * npos * B.stride), 256, 0, st>>>(B.stride, npos, d_pcomp, d_cptr, d_ord, d_bw, d_loff,
+                                                                             E->row_ptr, E->bcol, (const TV*)E->vals, Ab);
             // one cluster of two CTAs per job
             kernel<<<2 * njobs, BAND_THREADS, smem, st>>>(njobs, d_jobs, d_cptr, d_ord, d_bw, d_loff, Ab, B.blocks, E->g, Lg,
                                                           E->du, d_status);
@@ -1272,17 +1342,22 @@ static int dense_solve_t(Engine* E, int* iters, int* fallback) {
                 bytes += (B.cptr[c + 1] - B.cptr[c]) * ((B.bw[c] + 1) * 144.0 * sizeof(double) * 3 + 96.0 * 4);
         }
         phase_end(E, ph, bytes);
+        if (!again && (E->P.test_inject & ABD_INJECT_BAND_CHECK)) {      // test hook: every band component fails
+            for (int b : act) if (h_bmap[b] <= -3) D->bad[b] = 1;
+            D->bad[nb] = 1;
+        }
     }
     if (nsmall > 0) {
         size_t smem = ((size_t)nmax_small * (nmax_small + 1) + nmax_small) * sizeof(T);
-        if (!D->smem_set[sizeof(T) == 8]) {
+        constexpr int attr = (sizeof(TV) == 8) + (sizeof(T) == 8);
+        if (!D->smem_set[attr]) {
             const size_t nm = 12 * SMALL_MAX_BODIES;
-            CUDA_TRY(cudaFuncSetAttribute(k_small_solve<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+            CUDA_TRY(cudaFuncSetAttribute(k_small_solve<TV, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           (int)((nm * (nm + 1) + nm) * sizeof(T))));
-            D->smem_set[sizeof(T) == 8] = true;
+            D->smem_set[attr] = true;
         }
-        k_small_solve<T><<<nsmall, SMALL_THREADS, smem, st>>>(nsmall, d_sptr, d_sbody, d_blocal, E->row_ptr, E->bcol,
-                                                              (const T*)E->vals, E->g, projected ? 1 : 0, E->du, d_status);
+        k_small_solve<TV, T><<<nsmall, SMALL_THREADS, smem, st>>>(nsmall, d_sptr, d_sbody, d_blocal, E->row_ptr, E->bcol,
+                                                              (const TV*)E->vals, E->g, projected ? 1 : 0, E->du, d_status);
         E->launches++;
     }
     T* x = nullptr;
@@ -1295,7 +1370,7 @@ static int dense_solve_t(Engine* E, int* iters, int* fallback) {
         T* A = (T*)D->A;
         x = (T*)D->rhs;
         CUDA_TRY(cudaMemsetAsync(A, 0, sizeof(T) * (size_t)aoff, st));
-        k_blocks_to_dense<T><<<grid_for(16L * nb), 256, 0, st>>>(nb, E->row_ptr, E->bcol, (const T*)E->vals, d_bmap,
+        k_blocks_to_dense<TV, T><<<grid_for(16L * nb), 256, 0, st>>>(nb, E->row_ptr, E->bcol, (const TV*)E->vals, d_bmap,
                                                                 d_blocal, d_off, d_n, -1, A);
         k_rhs_gather<T><<<grid_for(12L * nb), 256, 0, st>>>(nb, E->g, d_bmap, d_blocal, d_rhs, x);
         E->launches += 2;
@@ -1314,7 +1389,7 @@ static int dense_solve_t(Engine* E, int* iters, int* fallback) {
                     // not positive definite after all: rebuild this component for LU
                     use_lu[c] = 1;
                     CUDA_TRY(cudaMemsetAsync(A + large_off[c], 0, sizeof(T) * (size_t)large_n[c] * large_n[c], st));
-                    k_blocks_to_dense<T><<<grid_for(16L * nb), 256, 0, st>>>(nb, E->row_ptr, E->bcol, (const T*)E->vals, d_bmap,
+                    k_blocks_to_dense<TV, T><<<grid_for(16L * nb), 256, 0, st>>>(nb, E->row_ptr, E->bcol, (const TV*)E->vals, d_bmap,
                                                                             d_blocal, d_off, d_n, c, A);
                     E->launches++;
                 } else if (potrs<T>(D, large_n[c], A + large_off[c], x + large_rhs[c], D->info + 3 + 2 * c) != CUSOLVER_STATUS_SUCCESS) {
@@ -1326,14 +1401,20 @@ static int dense_solve_t(Engine* E, int* iters, int* fallback) {
             if (use_lu[c] && lu_solve<T>(D, large_n[c], A + large_off[c], x + large_rhs[c], work, D->info + 2 + 2 * c) != CUSOLVER_STATUS_SUCCESS)
                 return E->fail(ABD_ERR_CUDA, "cusolver getrf/getrs");
     }
-    k_du_scatter<T><<<grid_for(32L * nb, 32 * DU_WARPS), 32 * DU_WARPS, 0, st>>>(nb, E->g, d_bmap, d_blocal,
-        nlarge ? D->comp_d + nlarge : nullptr, x, E->row_ptr, E->bcol, (const T*)E->vals, E->bscene, ndone, E->du);
+    k_du_scatter<TV, T><<<grid_for(32L * nb, 32 * DU_WARPS), 32 * DU_WARPS, 0, st>>>(nb, E->g, d_bmap, d_blocal,
+        nlarge ? D->comp_d + nlarge : nullptr, x, E->row_ptr, E->bcol, (const TV*)E->vals, E->bscene, ndone, E->du, again ? nullptr : D->bad);
     E->launches++;
     *iters = 1;
     return ABD_OK;
 }
 
-int eng_solve_direct(Engine* E, int* iters, int* fallback) {
-    if (E->mixed) return dense_solve_t<float>(E, iters, fallback);
-    return dense_solve_t<double>(E, iters, fallback);
+int eng_solve_direct(Engine* E, int* iters, int* fallback, bool again) {
+    if (E->mixed && !again) return dense_solve_t<float, float>(E, iters, fallback, false);
+    if (E->mixed) return dense_solve_t<float, double>(E, iters, fallback, true);
+    return dense_solve_t<double, double>(E, iters, fallback, again);
+}
+// after the host has waited for the last solve: a band solution failed its check
+bool eng_solve_failed(const Engine* E) {
+    const auto* D = reinterpret_cast<const DenseState*>(E->dense_state);
+    return D && D->bad && *(volatile int*)(D->bad + E->nb);
 }

@@ -126,6 +126,7 @@ struct Engine {
     std::string err;
     int launches = 0;
     int comp_band = 0, comp_small = 0, comp_large = 0, krylov_fallbacks = 0;   // direct-solver counters
+    int solve_before[4] = {0, 0, 0, 0};            // those before the last eng_solve
     int solver_capped = 0;         // Krylov solves that ended at lin_max_iter above tolerance
     int du_guard_hits = 0;         // mixed-precision increments replaced by the block-Jacobi direction
     int host_syncs = 0;            // stream synchronisations of the current call
@@ -348,7 +349,9 @@ int eng_detect(Engine* E, double filt);               // sorted candidate list a
 int eng_energy(Engine* E, int slot);                   // per-scene energy into scd[slot]
 int eng_assemble(Engine* E);                           // g and blocks at the nxt state (uses the candidate list)
 int eng_solve(Engine* E, int* iters, bool first_iter = false);   // du = A^-1 g for scenes not done
-int eng_solve_direct(Engine* E, int* iters, int* fallback);   // dense factorization per connected component
+bool eng_solve_failed(const Engine* E);                          // after a host sync: solve once more with eng_solve_again
+int eng_solve_again(Engine* E, int* iters, bool first_iter = false);
+int eng_solve_direct(Engine* E, int* iters, int* fallback, bool again);   // factorization per connected component
 void eng_dense_free(Engine* E);
 void eng_features_free(Engine* E);
 void eng_mlp_free(Engine* E);

@@ -618,12 +618,12 @@ __global__ void k_du_jacobi(int nb, const float* __restrict__ dinv, const double
     }
 }
 // counts the scenes whose increment the guard replaced (read with the
-// step's statistics, no sync of its own)
-__global__ void k_du_guard_count(int ns, const int* __restrict__ bad, Counters* cnt) {
+// step's statistics, no sync of its own); sign -1 takes the count back
+__global__ void k_du_guard_count(int ns, const int* __restrict__ bad, Counters* cnt, int sign) {
     int n = 0;
     for (int s = threadIdx.x; s < ns; s += blockDim.x) n += bad[s];
     for (int o = 16; o > 0; o >>= 1) n += __shfl_xor_sync(0xffffffffu, n, o);
-    if ((threadIdx.x & 31) == 0 && n) atomicAdd(&cnt->du_guard, n);
+    if ((threadIdx.x & 31) == 0 && n) atomicAdd(&cnt->du_guard, sign * n);
 }
 // test hook (AbdParams.test_inject): a non-finite increment in scene 0,
 // written over the solver's output on the host's request; no kernel reads
@@ -641,25 +641,17 @@ static int du_guard(Engine* E, bool inject) {
     CUDA_TRY(cudaMemsetAsync(bad, 0, sizeof(int) * E->ns, s));
     k_du_nonfinite<<<grid_for(12L * E->nb), 256, 0, s>>>(E->nb, E->du, E->bscene, E->sci + SI_DONE * E->ns, bad);
     k_du_jacobi<<<grid_for(12L * E->nb), 256, 0, s>>>(E->nb, (const float*)E->dinv, E->g, E->bscene, bad, E->du);
-    k_du_guard_count<<<1, 256, 0, s>>>(E->ns, bad, E->dcnt);
+    k_du_guard_count<<<1, 256, 0, s>>>(E->ns, bad, E->dcnt, 1);
     E->launches += 3;
     return ABD_OK;
 }
-static int solve_any(Engine* E, int* iters);
 int eng_block_inverse(Engine* E);
-int eng_solve(Engine* E, int* iters, bool first_iter) {
-    // the guard's increment, and the Krylov solves' preconditioner
-    if (E->mixed) { int rc = eng_block_inverse(E); if (rc) return rc; }
-    int rc = solve_any(E, iters);
-    if (rc || !E->mixed) return rc;
-    return du_guard(E, first_iter && (E->P.test_inject & ABD_INJECT_DU_NONFINITE));
-}
-static int solve_any(Engine* E, int* iters) {
+static int solve_any(Engine* E, int* iters, bool again) {
     int kind = resolved_solver(E);
     if (kind == ABD_SOLVER_DIRECT) {
         int ph = phase_begin(E, PH_DENSE);
         int fallback = 0;
-        int rc = eng_solve_direct(E, iters, &fallback);
+        int rc = eng_solve_direct(E, iters, &fallback, again);
         phase_end(E, ph, 0);
         if (rc || !fallback) return rc;
         // too many large components for one factorization each
@@ -669,4 +661,28 @@ static int solve_any(Engine* E, int* iters) {
     KrylovKind kk(E, kind);
     if (E->mixed) return solve_t<float>(E, iters);
     return solve_t<double>(E, iters);
+}
+static int solve_guarded(Engine* E, int* iters, bool first_iter, bool again) {
+    int rc = solve_any(E, iters, again);
+    if (rc || !E->mixed) return rc;
+    return du_guard(E, first_iter && (E->P.test_inject & ABD_INJECT_DU_NONFINITE));
+}
+int eng_solve(Engine* E, int* iters, bool first_iter) {
+    const int before[4] = {E->comp_band, E->comp_small, E->comp_large, E->krylov_fallbacks};
+    std::copy(before, before + 4, E->solve_before);
+    // the guard's increment, and the Krylov solves' preconditioner
+    if (E->mixed) { int rc = eng_block_inverse(E); if (rc) return rc; }
+    return solve_guarded(E, iters, first_iter, false);
+}
+// The system of the last eng_solve once more, for eng_solve_failed: components
+// whose band solution failed its check take the pivoted paths.  What the first
+// solve counted is taken back.
+int eng_solve_again(Engine* E, int* iters, bool first_iter) {
+    E->comp_band = E->solve_before[0]; E->comp_small = E->solve_before[1];
+    E->comp_large = E->solve_before[2]; E->krylov_fallbacks = E->solve_before[3];
+    if (E->mixed) {
+        k_du_guard_count<<<1, 256, 0, E->stream>>>(E->ns, E->sci + SI_DUBAD * E->ns, E->dcnt, -1);
+        E->launches++;
+    }
+    return solve_guarded(E, iters, first_iter, true);
 }

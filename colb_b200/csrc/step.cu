@@ -262,7 +262,6 @@ int eng_step(Engine* E, int n_steps, AbdStepStats* stats) {
             // abd.py:690 / :631-658 solve
             int li = 0;
             { int ph = phase_begin(E, PH_SOLVE); rc = eng_solve(E, &li, it == 0); phase_end(E, ph, 0); if (rc) return rc; }
-            st.lin_iters += li;
             st.n_active = E->hcnt->n_active;
             // candidates along x -> x - J du, shared by CCD, every energy
             // of the line search and the next detection
@@ -271,8 +270,17 @@ int eng_step(Engine* E, int n_steps, AbdStepStats* stats) {
                 rc = eng_swept(E, E->du, -1.0, done);
                 // positions, rest positions, increments per vertex; topology; the listed pairs
                 phase_end(E, ph, E->nv * (24.0 + 24.0 + 4.0) + E->nb * 96.0 + E->ne * 8.0 + E->nt * 12.0 + E->n_sw * 24.0);
+                // the list's host sync has also brought the check of the solve
+                if ((!rc || rc == ABD_ERR_CONTACT_OVERFLOW) && eng_solve_failed(E)) {
+                    E->err.clear();
+                    ph = phase_begin(E, PH_SOLVE);
+                    rc = eng_solve_again(E, &li, it == 0);
+                    phase_end(E, ph, 0);
+                    if (!rc) rc = eng_swept(E, E->du, -1.0, done);
+                }
                 if (rc) return rc;
             }
+            st.lin_iters += li;
             // the line search runs per scene, or per contact group of the
             // listed step (ls_groups): each unit has its own CCD bound,
             // energies, step length and back-off

@@ -131,13 +131,17 @@ typedef struct AbdParams {
                                runs (the guard must replace it by the block-Jacobi direction);
                                ABD_INJECT_SWEPT_FULL makes the first swept candidate list of every
                                step report that it does not fit (the list must then be built for a
-                               shorter step, and the step length capped to it) */
+                               shorter step, and the step length capped to it);
+                               ABD_INJECT_BAND_CHECK makes every band component of a direct solve
+                               fail the check of its solution (it must then be solved again on the
+                               pivoted paths) */
     int32_t reserved[1];
 } AbdParams;
 
 #define ABD_CCD_MAX_ITER 100000
 #define ABD_INJECT_DU_NONFINITE 1
 #define ABD_INJECT_SWEPT_FULL 2
+#define ABD_INJECT_BAND_CHECK 4
 
 /* ---- one scene: concatenated affine bodies (geometry.py:22-73) ------- */
 typedef struct AbdSceneDesc {

@@ -249,9 +249,10 @@ __global__ void __launch_bounds__(256) k_st_find(int ne, StaticGrid G, StaticFla
     }
 }
 // Writes vertex quadruples, by edge and partner, the rows that fit below cap.
-// An edge without a list (see k_st_find) visits its partners again and
-// orders them where they are written; one whose rows cross cap then keeps the
-// ones it visited first.
+// An edge without a list (see k_st_find) visits its partners again and orders
+// them where they are written.  The order of a visit is not fixed (k_st_keys),
+// so the one edge whose rows may cross cap keeps its smallest partners, each
+// put in its place as it is found: the rows are the first ones of the complete list.
 __global__ void __launch_bounds__(256) k_st_write(int ne, StaticGrid G, const StaticFlags* F, const int* __restrict__ count,
                                                   const int* __restrict__ off, const int* __restrict__ at,
                                                   const int* __restrict__ pool, int* out4, int cap, int* n_out) {
@@ -264,7 +265,19 @@ __global__ void __launch_bounds__(256) k_st_write(int ne, StaticGrid G, const St
         const int c = count[i], base = off[i], from = at[i];
         if (c == 0 || base >= cap) continue;
         const int rows = min(c, cap - base);
-        if (from < 0) {
+        if (from < 0 && rows < c) {
+            int have = 0;                                    // lane 0's: rows so far, in order
+            st_visit(G, h, i, s_queue[w], [&](bool found, int j) {
+                for (unsigned m = __ballot_sync(0xffffffffu, found); m; m &= m - 1) {
+                    const int v = __shfl_sync(0xffffffffu, j, __ffs(m) - 1);
+                    if (lane > 0 || (have == rows && out4[4L*(base+rows-1)+2] < v)) continue;
+                    int k = base + (have < rows ? have++ : rows - 1);
+                    for (; k > base && out4[4L*(k-1)+2] > v; k--) out4[4L*k+2] = out4[4L*(k-1)+2];
+                    out4[4L*k+2] = v;
+                }
+            });
+            __syncwarp();
+        } else if (from < 0) {
             int k0 = base;
             st_visit(G, h, i, s_queue[w], [&](bool found, int j) {
                 const unsigned m = __ballot_sync(0xffffffffu, found);

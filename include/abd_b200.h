@@ -357,7 +357,7 @@ int abd_get_timing(AbdHandle* h, double* ms, int64_t* launches, double* bytes);
  * legacy default stream) and the call waits for that stream before it
  * returns.  ABD_ERR_CONTACT_OVERFLOW if more than cap pairs exist:
  * *n_pairs_dev holds the full count, nothing is written at or beyond row
- * cap, and which pairs the first cap rows hold is unspecified.
+ * cap, and the rows below it are the first ones of the complete list.
  * Errors: abd_last_error(NULL). */
 #define ABD_STATIC_MAX_EDGES (1 << 16)
 int abd_ee_pairs_static(const double* x_dev, const int32_t* edges_dev, int32_t n_verts, int32_t n_edges,

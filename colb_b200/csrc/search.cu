@@ -24,11 +24,15 @@
 // Body boxes of the listed step (bpair.cu), for skipping vertices that stay
 // away from every half-space; null when the step was listed by the grid.
 struct StepBoxes { const float4* lo; const float4* hi; };
-// smallest and largest signed distance of a box to a half-space
-DV void box_plane(float4 lo, float4 hi, const double* n, double& dmin, double& dmax) {
+// A body's swept box may reach a half-space: it comes within the barrier's
+// distance or (ccd) holds a vertex whose distance may fall below ccd_scale times
+// its present one.  A box that overflowed FP32 (a diverged increment) gives no
+// distances and counts as near.
+DV bool box_near_plane(float4 lo, float4 hi, const double* n, double dhat, bool ccd, double ccd_scale) {
     const double a0 = n[0] * lo.x, a1 = n[0] * hi.x, b0 = n[1] * lo.y, b1 = n[1] * hi.y, c0 = n[2] * lo.z, c1 = n[2] * hi.z;
-    dmin = fmin(a0, a1) + fmin(b0, b1) + fmin(c0, c1) - n[3];
-    dmax = fmax(a0, a1) + fmax(b0, b1) + fmax(c0, c1) - n[3];
+    const double dmin = fmin(a0, a1) + fmin(b0, b1) + fmin(c0, c1) - n[3];
+    const double dmax = fmax(a0, a1) + fmax(b0, b1) + fmax(c0, c1) - n[3];
+    return !(dmin >= dhat) || (ccd && !(dmin >= ccd_scale * dmax));
 }
 // grid split over the three kinds of work; a warp looks at `group` chunks at
 // once and then works on the live ones
@@ -49,7 +53,7 @@ struct LsArgs {
     const double* st; const double* J; double* backup;
     const double* g; const int* bscene; double* gg;   // gradient, and its squared norm per scene
     const int* unit; const int* skip;            // unit of a body; units left alone
-    BodyTerms B; PairTerms T; StepBoxes box; int npl;
+    BodyTerms B; PairTerms T; StepBoxes box;
     int ccd; double ccd_scale; int ccd_it;
     double* E; double* En; double* toi;
 };
@@ -120,9 +124,7 @@ DV void ls_terms(const LsArgs& A, const LsGrid& g, int* capped) {
         const int w0 = ((blockIdx.x - g.bodies - g.pairs) * blockDim.x + threadIdx.x) >> 5;
         for (int w = w0 * g.group; w < A.nchunks; w += ((g.chunks * blockDim.x) >> 5) * g.group) {
             // the lanes look at one chunk each: its unit still searches, and
-            // the body's swept box can reach a half-space, that is, comes
-            // within the barrier's distance or (CCD) holds a vertex whose
-            // distance may fall below ccd_scale times its present one
+            // the body's swept box can reach a half-space
             int4 mine = make_int4(0, 0, 0, 0);
             bool live = false;
             if (lane < g.group && w + lane < A.nchunks) {
@@ -130,12 +132,8 @@ DV void ls_terms(const LsArgs& A, const LsGrid& g, int* capped) {
                 if (!A.skip[A.unit[mine.x]]) {
                     const int s = G.bscene[mine.x];
                     for (int pl = G.sc_plane_begin[s]; pl < G.sc_plane_begin[s + 1] && !live; pl++) {
-                        live = true;
-                        if (A.box.lo) {
-                            double dmin, dmax;
-                            box_plane(A.box.lo[mine.x], A.box.hi[mine.x], G.planes + 4 * pl, dmin, dmax);
-                            live = dmin < A.T.dhat || (BEGIN && A.ccd && dmin < A.ccd_scale * dmax);
-                        }
+                        live = !A.box.lo || box_near_plane(A.box.lo[mine.x], A.box.hi[mine.x], G.planes + 4 * pl, A.T.dhat,
+                                                           BEGIN && A.ccd, A.ccd_scale);
                     }
                 }
             }
@@ -275,7 +273,7 @@ static LsArgs ls_args(Engine* E, const LsUnits& U, const int* skip, int slot) {
     A.unit = U.bunit; A.skip = skip; A.B = body_terms(P); A.T = pair_terms(P);
     A.box = StepBoxes{nullptr, nullptr};
     eng_step_boxes(E, &A.box.lo, &A.box.hi);
-    A.npl = E->npl; A.ccd = P.ccd; A.ccd_scale = P.ccd_scale; A.ccd_it = ccd_iters(P);
+    A.ccd = P.ccd; A.ccd_scale = P.ccd_scale; A.ccd_it = ccd_iters(P);
     A.E = U.d + slot * U.n; A.En = U.d + (slot == SD_E0 ? SD_E0N : SD_E1N) * U.n; A.toi = U.d + SD_TOI * U.n;
     return A;
 }

@@ -61,7 +61,7 @@ DV void stencil_hessian(int type, const d3* x, const double* pl, Stencil5& S) {
         n = mk3(pl[0], pl[1], pl[2]);
         S.d = dot(n, x[0]) - pl[3];
         S.c[0] = 1.0; S.cn = 1.0;
-        perp_frame(n, e1, e2);
+        e1 = e2 = mk3(0, 0, 0);                     // nothing but n; a frame would divide by its length, which may be 0
         S.a[s5(0, 0)] = 2.0;
     } else if (type == T_PP) {
         const d3 r = x[0] - x[1];

@@ -1,7 +1,8 @@
 // warp_eig.cuh — one warp projects a small symmetric matrix (n <= 12) held
-// in shared memory onto the PSD cone: V max(L, 0) V^T.  The contact assembly
-// takes the 5 x 5 form of contact_hess.cuh; this general one is what the CPU
-// test checks projections against.
+// in shared memory onto the PSD cone: V max(L, 0) V^T.  No kernel includes this
+// general form any more: the contact assembly projects 5 x 5 matrices in
+// registers (contact_hess.cuh, checked in tests/test_contact_hess_cpu.py).  It is
+// kept for its CPU test, which compares its two variants with each other.
 //
 // Parallel cyclic Jacobi with round-robin ("tournament") pair ordering:
 // each round rotates n/2 disjoint index pairs at once, so for a product R of

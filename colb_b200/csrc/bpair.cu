@@ -264,12 +264,13 @@ __global__ void __launch_bounds__(BOX_THREADS) k_bp_clboxes(int nb, const int* _
 // ---- step 3: overlapping cluster pairs of each body pair, as primitive
 // ranges {first of a, first of b, counts | kind | same body}.  The counter
 // is 64-bit and exact: the host grows the list once and runs the kernel
-// again.  `q0`, `q1`: the slice of body pairs to expand.
+// again.  `q0`, `q1`: the slice of body pairs to expand; `c0`, `c1`: of the
+// clusters of their first sides (whole groups of 32).
 DV int4 cl_item(int a0, int na, int b0, int nb, int kind, int same) {
     return make_int4(a0, b0, min(na, BP_CL) | (min(nb, BP_CL) << 8) | (kind << 16) | (same << 17), 0);
 }
 __global__ void k_bp_clusters(const int2* __restrict__ bpairs, const int* __restrict__ npairs, int bp_cap, int q0, int q1,
-                              const int* __restrict__ vbeg, const int* __restrict__ ebeg, const int* __restrict__ tbeg,
+                              int c0, int c1, const int* __restrict__ vbeg, const int* __restrict__ ebeg, const int* __restrict__ tbeg,
                               BpBoxes B, int do_ee, int do_pt, int4* out, long long cap, unsigned long long* count) {
     const int lane = threadIdx.x & 31;
     const int n = min(min(*npairs, bp_cap), q1);     // an overflowing pair list is rebuilt larger by the host
@@ -295,7 +296,7 @@ __global__ void k_bp_clusters(const int2* __restrict__ bpairs, const int* __rest
             const float4* BH = pass == 0 ? B.ch[1] : B.ch[2];
             const int na = cl_count(abeg, ba), nb = cl_count(bbeg, bb);
             const int ca = cl_first(abeg, ba), cb = cl_first(bbeg, bb);
-            for (int a0 = 0; a0 < na; a0 += 32) {
+            for (int a0 = c0; a0 < min(na, c1); a0 += 32) {
                 float4 al, ah;
                 empty_box(al, ah);
                 if (a0 + lane < na) { al = AL[ca + a0 + lane]; ah = AH[ca + a0 + lane]; }
@@ -563,13 +564,13 @@ static int bp_build(Engine* E, const BpDisp& disp, double lim, double filt, int 
         A.lim = lim; A.filt = filt; A.mode = mode; A.f32 = P.ee_f32;
         A.out = S->keys; A.cap = S->key_cap; A.count = S->cnt + 1;
         unsigned long long* nitems = reinterpret_cast<unsigned long long*>(S->cnt + 4);
-        auto expand = [&](int q0, int q1) {
-            k_bp_clusters<<<NUM_SMS * 4, 256, 0, s>>>(S->bpairs, S->cnt, S->bp_cap, q0, q1, E->bd_vbeg, E->bd_ebeg, E->bd_tbeg,
+        auto expand = [&](int q0, int q1, int c0, int c1) {
+            k_bp_clusters<<<NUM_SMS * 4, 256, 0, s>>>(S->bpairs, S->cnt, S->bp_cap, q0, q1, c0, c1, E->bd_vbeg, E->bd_ebeg, E->bd_tbeg,
                                                        S->B, do_ee, do_pt, S->items, S->item_cap, nitems);
             k_bp_prims<<<NUM_SMS * 8, PRIM_THREADS, 0, s>>>(S->items, nitems, S->item_cap, A);
             E->launches += 2;
         };
-        expand(0, INT_MAX);
+        expand(0, INT_MAX, 0, INT_MAX);
         k_bp_send<<<1, 32, 0, s>>>(S->cnt, E->hcnt->bp);
         E->launches += 3;
         CUDA_TRY(eng_stream_sync(E));
@@ -582,20 +583,24 @@ static int bp_build(Engine* E, const BpDisp& disp, double lim, double filt, int 
         }
         if (items > S->item_cap) {
             // more cluster pairs than the list may hold: slices of body pairs
-            // small enough to fit whatever they overlap
+            // small enough to fit whatever they overlap, and of a pair's
+            // clusters where a single one would not (one cluster meets at most
+            // `row` others, so a group of 32 fits up to 130 million primitives)
             auto most = [&](int n) { return (long long)n / 32 + 1; };
-            const long long per = most(E->ne) * most(E->ne) + 2 * most(E->nv) * most(E->nt);
-            const int step = (int)std::max<long long>(1, S->item_cap / std::max<long long>(per, 1));
+            const long long row = most(E->ne) + 2 * most(E->nt), rows = std::max(most(E->ne), most(E->nv)), per = row * rows;
+            const int step = (int)std::max<long long>(1, S->item_cap / per);
+            const long long cstep = per <= S->item_cap ? rows + 32 : std::max<long long>(32, S->item_cap / row / 32 * 32);
             CUDA_TRY(cudaMemsetAsync(S->cnt + 1, 0, sizeof(int), s));
-            for (int q0 = 0; q0 < npairs; q0 += step) {
-                CUDA_TRY(cudaMemsetAsync(nitems, 0, sizeof(long long), s));
-                expand(q0, std::min(npairs, q0 + step));
-                k_bp_send<<<1, 32, 0, s>>>(S->cnt, E->hcnt->bp);
-                E->launches++;
-                CUDA_TRY(eng_stream_sync(E));
-                memcpy(&items, E->hcnt->bp + 4, sizeof items);
-                if (items > S->item_cap) return E->fail(ABD_ERR_CONTACT_OVERFLOW, "body-pair broad phase: one body pair's cluster pairs do not fit");
-            }
+            for (int q0 = 0; q0 < npairs; q0 += step)
+                for (long long c0 = 0; c0 < rows; c0 += cstep) {
+                    CUDA_TRY(cudaMemsetAsync(nitems, 0, sizeof(long long), s));
+                    expand(q0, std::min(npairs, q0 + step), (int)c0, (int)std::min<long long>(c0 + cstep, INT_MAX));
+                    k_bp_send<<<1, 32, 0, s>>>(S->cnt, E->hcnt->bp);
+                    E->launches++;
+                    CUDA_TRY(eng_stream_sync(E));
+                    memcpy(&items, E->hcnt->bp + 4, sizeof items);
+                    if (items > S->item_cap) return E->fail(ABD_ERR_CONTACT_OVERFLOW, "body-pair broad phase: one body pair's cluster pairs do not fit");
+                }
             if (E->hcnt->bp[1] > S->key_cap) {
                 if ((rc = bp_reserve(E, npairs, 0, E->hcnt->bp[1]))) return rc;
                 continue;

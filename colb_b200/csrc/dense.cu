@@ -10,9 +10,10 @@
 //     bandwidth of at most BAND_WIDE: a banded L D L^T with the active window in
 //     registers, all such components of bandwidth up to BAND_MAX in one launch
 //     and the wider ones in another;
-//   - otherwise up to SMALL_MAX_BODIES bodies: one CTA per component factors
-//     it in shared memory (blocked Cholesky by 12-wide body columns; LU with
-//     partial pivoting when a pivot is not positive), all in one launch;
+//   - otherwise (not projected, or a band solution that failed its check) up to
+//     SMALL_MAX_BODIES bodies: one CTA per component factors it in shared
+//     memory (blocked Cholesky by 12-wide body columns if projected; LU with
+//     partial pivoting if not or when a pivot is not positive), all in one launch;
 //   - larger components: the 12x12 blocks are scattered into a dense
 //     column-major matrix and factored with cuSOLVER (Cholesky, or LU when
 //     Cholesky reports a non-positive pivot).
@@ -363,9 +364,11 @@ DV void band_cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "
 //     factor, the two vectors of the rank-6 update and its right-hand side's;
 //   - the window threads publish the next pivot rows with that update applied,
 //     and then apply it to their registers while the row threads go on.
-// The chain (per pivot a reciprocal of 74 cycles and two operations of 8, per
-// six pivots two barriers and one publishing) bounds the kernel; everything
-// else is kept off it.  The right-hand side is one more column of the pivot
+// What bounds the kernel is this exchange, twice per body: each role waits for the
+// other (barrier stall 4.6 per issue, FP64 pipe 14 % busy).  The pivots' own
+// chain, a reciprocal of 74 cycles and two operations of 8 each, is about a
+// seventh of it: 25 bodies one way, 300 pivots, 14 of 97 us for the first example
+// below.  The right-hand side is one more column of the pivot
 // rows.  After a body's pivots the row threads form
 //   M_{k,d} = L_kk^-T L_{k+d,k}^T  and  a_k = L_kk^-T D^-1 y_k
 // row by row (independent solves) and store them instead of the factor, so the
@@ -379,7 +382,8 @@ DV void band_cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "
 // of *status and is replaced by its magnitude).  SIGNED: mixed precision, whose
 // FP32-rounded blocks can be indefinite (the 12-body blocks of a chain mail
 // in contact have eigenvalues down to -2.9e3 of 1e9), factors them in FP64 with
-// pivots of either sign.
+// pivots of either sign, without exchanges; what a small pivot may have spoilt is
+// found afterwards (band_check).
 constexpr int BAND_MAX = 8;            // body bandwidths up to here: narrow kernel
 constexpr int BAND_W = BAND_MAX + 1;   // its blocks per body
 constexpr int BAND_WIDE = 11;          // up to here: wide kernel (78 window entries per thread)

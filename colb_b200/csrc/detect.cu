@@ -1,5 +1,5 @@
 // detect.cu — vertex transform, uniform-grid broad phase, candidate pairs,
-// contact energy, CCD and the intersection check.
+// contact energy, the ordered filter of listed candidates and the intersection check.
 //
 //  transform ............ abd_simple.py:26-35
 //  EE candidates ........ contact.py:25-32, :143-169 (float32 predicate, i<j,

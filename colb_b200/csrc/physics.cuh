@@ -5,8 +5,7 @@
 //  segment closest pts . Ericson, Real-Time Collision Detection §5.1.9, as
 //                        called by contact.py:166 and abd.py:190 (float32)
 //  squared distances ... IPC (Li et al. 2020) point-point, point-line,
-//                        line-line and point-plane, with gradient and Hessian
-//  PSD projection ...... cyclic Jacobi eigen-decomposition (abd.py:247)
+//                        line-line and point-plane (derivatives: contact_hess.cuh)
 //  triangle region ..... Ericson §5.1.5
 //  additive CCD ........ Li, Kaufman, Jiang 2021 (C-IPC) Alg. 1
 #pragma once

@@ -591,10 +591,10 @@ static int resolved_solver(const Engine* E) {
 }
 
 // an increment entry above this (scene units for positions, dimensionless for
-// the affine rows) is no Newton step of a physical scene: it is taken as an
-// FP32 breakdown like a non-finite one
+// the affine rows) is no Newton step of a physical scene: it is taken as a
+// breakdown of the mixed solve like a non-finite one
 constexpr double DU_GUARD_MAX = 1e6;
-// Mixed precision: a scene whose FP32 solve left a non-finite entry in du
+// Mixed precision: a scene whose solve left a non-finite entry in du
 // takes the block-Jacobi direction du_b = D_b^-1 g_b instead (every body's
 // inverse diagonal block is finite: a singular block inverts to the
 // identity), so the line search gets a descent direction rather than NaN.

@@ -193,7 +193,7 @@ int eng_swept(Engine* E, const double* dq, double sign, const int* done) {
         // a candidate list that does not fit even after growing (an increment
         // that sweeps most primitives into reach) is built for a quarter of
         // the step, then a sixteenth, ...; the line search then caps its step
-        // length at that fraction (k_ls_init), so the list still covers every
+        // length at that fraction (k_ls_begin), so the list still covers every
         // position it visits
         for (double scale = 1.0;; scale *= 0.25) {
             if ((E->P.test_inject & ABD_INJECT_SWEPT_FULL) && !E->sw_inject_done && scale == 1.0) {

@@ -66,3 +66,19 @@ def test_failed_band_solutions_take_the_pivoted_paths(n, precision):
         x, xr = e.vertices(), ref.vertices()
         assert np.abs(x - xr).max() <= (1e-4 if precision else 1e-7) * np.abs(xr).max()
     assert e.count_intersections() == 0
+
+
+@pytest.mark.parametrize("extra", [30, 1500])
+def test_second_solves_by_block_pattern(extra):
+    """The second solve reads the block pattern back from the device, as rows (30 more bodies) or as sorted keys
+    (1,500 more): the increment of the first solve up to the rounding of two stable factorizations."""
+    net = _net(5)
+    p = dict(linear_solver=2, hess_mode=1)
+    _, H = Engine(P.config_params(**p), net).assemble()
+    d = [Engine(P.config_params(test_inject=inject, **p), [S.config5_pile(n=extra, seed=1), net]).solve()[0]
+         for inject in (0, ABD_INJECT_BAND_CHECK)]
+    assert np.all(np.isfinite(d[1]))
+    d0, d1 = (v[-12 * 25:] for v in d)
+    s = 1.0 / np.sqrt(np.diag(H))
+    kappa = np.linalg.cond(H * s[:, None] * s)
+    assert np.linalg.norm((d0 - d1) / s) <= 50 * 2.2e-16 * kappa * np.linalg.norm(d0 / s)

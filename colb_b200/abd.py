@@ -13,7 +13,7 @@ Differences from the reference, all deliberate:
   * the contact list is sorted and grows on demand instead of wrapping at
     10000 entries (contact.py:8, :137);
   * the linear solve (ABD_SOLVER_AUTO) is a direct solve per connected
-    component of the contact graph (banded block Cholesky, shared-memory
+    component of the contact graph (banded block L D L^T, shared-memory
     dense factorization, or block-Jacobi preconditioned BiCGSTAB / PCG when
     the components are too large), not Warp's unpreconditioned bicgstab;
     the reference's own solver_config="cg" choice maps to

@@ -329,7 +329,7 @@ int abd_count_intersections(AbdHandle* h, int32_t* count);
  *   9 assembly: bodies          10 assembly: contacts     11 assembly: block inverse
  *   12 dense factor + solve     13 swept candidate list   14 contact-energy list kernel
  *   15 line-search trials (apply + energy + decision)
- *   16 banded block-Cholesky kernel of the direct solver
+ *   16 banded block L D L^T kernel of the direct solver
  * abd_get_timing writes ms[17], launches[17] and the algorithmic bytes[17]
  * those phases moved (documented at each kernel); reset clears them. */
 #define ABD_NUM_PHASES 17
